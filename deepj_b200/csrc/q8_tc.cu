@@ -1,69 +1,80 @@
-// Q8 linear for many activation rows (prefill): tcgen05 tensor-core tiles with the
-// accumulator in tensor memory.
+// Q8 linear for many activation rows (prompts, several sequences at once): tcgen05 tensor-core tiles, one accumulation
+// per scale block.
 //
-// With M in the hundreds the work is a dense contraction, 2·M·K·N flops against K·N weight
-// bytes, and belongs on the 5th-generation tensor cores.  The Q8 format keeps one fp32 scale per
-// 32 weights, so the weights cannot stay int8 inside one long accumulation; instead each
-// 256 × 32 weight tile is dequantised on the fly, exactly once per CTA, into two fp16 tiles with
-//     w_hi + w_lo = code · scale   to ≈ 22 bits  (packed fp16 arithmetic, see the conversion loop)
-// and the activations are split the same way by a pre-pass (x_hi, x_lo, after a power-of-two row
-// scaling that keeps fp16 in range; RMSNorm is applied there too).  Three MMAs per k-step,
-//     D += X_hi·W_hi + X_lo·W_hi + X_hi·W_lo,
-// carry ≈ 22 bits of each operand into the fp32 accumulator — the dropped lo·lo term is 2^-22
-// relative — so the prefill path stays inside the decode path's tolerance at one third of the
-// fp16 tensor peak.
+// A Q8 weight is code · scale with one fp32 scale per 32 k, so a product over one block is scale · Σ x·code, and a code is
+// exact in fp16.  The kernel multiplies the raw codes, block by block, and applies the scale afterwards in fp32:
+//     D_b  = C_b · X_hi + C_b · X_lo          tensor cores, K = 32, fp32 accumulator in tensor memory
+//     acc += scale_b · D_b                    fp32 fused multiply-adds in registers
+// X_hi + X_lo is the activation as two fp16 values (≈ 22 bits, after a power-of-two row scaling by the pre-pass, which also
+// applies the norm).  Weights enter without any rounding, and two MMAs per k-step are enough.  Folding the scale into the
+// operand instead (weights as hi + lo fp16 pairs, accumulated over all of K) takes three, and the conversion costs 2.75
+// instructions per weight instead of 1.25.
 //
-// One CTA per 128 (activation rows) × 256 (weight rows) output tile, or — when the launch has enough tiles to
-// keep every SM busy that way — per pair of them: two 128 × 256 accumulators fill the SM's tensor memory and
-// share every dequantised weight tile, which halves the conversion work per flop.  k-tiles of 32, ten warps:
-//   warps 0-7  dequantise, as two groups of four that take the k-tiles in turn (a thread owns two weight rows of
-//              the tile: 32 code bytes + a scale each per k-tile from global memory, its next three k-tiles
-//              already in registers) and write the W_hi / W_lo tiles in the 64-byte-swizzled K-major layout the
-//              MMA reads; afterwards they are the epilogue: tcgen05.ld of a 32 × 128 piece of the accumulator
-//              each, row scale, bias, residual or SiLU-gate, 128-byte row stores through a shared-memory transpose;
-//   warp 8     one thread streams the activation tiles: the pre-pass leaves every 128 × 32 tile as a ready
-//              shared-memory image (hi and lo adjacent, 16 KB), so a stage is ONE plain bulk copy completing
-//              on an mbarrier — no tensor map;
-//   warp 9     one thread issues the MMAs (128 × 256 × 16, three per accumulator and 16-k step, each accumulator
-//              256 columns of tensor memory) and commits each stage back to its "empty" barriers.
-// 64 KB of activation stages (four of one 128-row tile, or two of a pair) and three weight stages of 32 KB.  Every wait is bounded: when a bound
-// expires the CTA records an error code, stops waiting for anything, frees its tensor memory and returns.
+// The tile is 128 weight rows × NT activation rows with the weights as the M side: a thread of the promoting warps owns a
+// tensor-memory lane = one weight row, so its block scale is one register and its result rows are stored 128 contiguous
+// bytes at a time.  The fp16 codes go to tensor memory too and enter the MMAs from there: with them in shared memory the
+// converters' stores and the MMAs' operand reads together asked for its whole 128 bytes a cycle (measured: 8 MMAs of
+// 128 × 64 × 16 took 780 cycles beside the converters and 392 alone).  20 warps:
+//   warps 0-7    read the block's accumulator (tcgen05.ld, 32 lanes × NT/2 columns each) and add it to registers;
+//                afterwards the epilogue
+//   warps 8-15   convert, as two groups of four that take the stages in turn: one weight row per thread, 32 codes → 64 bytes
+//                of fp16 per block, stored to its lane
+//   warp 16      copies the activation images (one plain bulk copy per stage)
+//   warp 17      streams the raw codes: 128-byte × 128-row boxes through the tensor-memory accelerator
+//   warps 18-19  issue the MMAs (128 × NT × 16, four per block) into a ring of accumulators and commit, taking the stages in
+//                turn: the waits and commits of one stage cost an issuing thread ≈ 400 cycles, in which the other one issues
+// SwiGLU takes 64 gate and 64 up rows per tile, so the pair meets in one epilogue.  When the grid leaves SMs idle the
+// reduction is split over the CTAs of a cluster, which add their parts through distributed shared memory in split order.
+// Every wait is bounded: when a bound expires the CTA records an error code, stops waiting, lets its copies in flight
+// land, frees its tensor memory and returns.
 #include "kernels.h"
+#include "q8_tma.cuh"
 #include "tc_common.cuh"
 #include <cuda_fp16.h>
 
 namespace dj {
 namespace {
 
-constexpr int kTileM = 128, kTileN = 256, kTileK = 32;
-constexpr int kStagesA = 4, kStagesB = 3;                // activation stages: four of one 128-row tile, or two of a pair of tiles
-constexpr int kATileBytes = kTileM * kTileK * 2;         // one fp16 activation tile: 8 KB
-constexpr int kBTileBytes = kTileN * kTileK * 2;         // one fp16 weight tile: 16 KB
-constexpr int kAImageBytes = 2 * kATileBytes;            // X_hi, X_lo of one 128-row tile, as the pre-pass lays them down
-constexpr int kARegionBytes = kStagesA * kAImageBytes;   // 64 KB of activation stages either way
-constexpr int kStageBBytes = 2 * kBTileBytes;            // W_hi, W_lo
-constexpr int kDqWarps = 8;                              // dequantising (later: epilogue) warps, one weight row per thread; then one copy warp, one MMA warp
-constexpr int kTcThreads = (kDqWarps + 2) * 32;
-constexpr int kTmemCols = 512;                            // two 128 × 256 fp32 accumulators: all of tensor memory
-constexpr int kRawRow = 144;                             // bytes per weight row in the raw-code buffer: 4 k-tiles of codes + their scales
+constexpr int kRows = 128;                               // weight rows of a tile
+constexpr int kBlockK = 32;                              // one scale block
+constexpr int kGroup = 4;                                // blocks per raw-code box: 128 bytes of a weight row
+constexpr int kRawBytes = kRows * kBlockK * kGroup;      // raw codes of one group: 16 KB
+constexpr int kPromoteWarps = 8, kConvertWarps = 8;      // converters: two groups of four
+constexpr int kCopyWarp = kPromoteWarps + kConvertWarps, kRawWarp = kCopyWarp + 1, kMmaWarp = kCopyWarp + 2;   // two MMA warps
+constexpr int kTcThreads = 640;
+constexpr int kMaxSplits = 8;                            // portable cluster size
+// Registers: 640 threads × 96 at launch; 256 × 168 + 384 × 48 = 61440 afterwards.
+constexpr int kPromoteRegs = 168, kOtherRegs = 48;
 
-// byte offset of 16-byte chunk c (0-3) of row r inside a 64-byte-swizzled K-major tile of 32 halves per row:
-// 8-row groups of 512 bytes, the chunk index XORed with bits 1-2 of the row
-__host__ __device__ __forceinline__ int swz_off(int r, int c) { return (r >> 3) * 512 + (r & 7) * 64 + ((c ^ ((r >> 1) & 3)) << 4); }
+// Below 128 activation rows a block's products take less time than the barriers around them: a pipeline stage then holds two
+// blocks (rows of 128 bytes, 128-byte swizzle) and accumulators are handed over in pairs.
+constexpr int blocks_per_stage(int nt) { return nt < 128 ? 2 : 1; }
+template <int NT> struct TileShape {
+    static constexpr int kPer = blocks_per_stage(NT);
+    static constexpr int kStages = kPer == 2 ? 4 : 6;
+    static constexpr int kRawStages = 4;
+    static constexpr int kRowBytes = 64 * kPer;
+    static constexpr int kXBytes = NT * kRowBytes;                   // one half (hi or lo) of a stage's activations
+    static constexpr int kStageBytes = 2 * kXBytes;
+    // tensor memory: accumulators, handed over kPer at a time, then per stage the fp16 codes (16 columns of two per block)
+    static constexpr int kAccStride = NT < 32 ? 32 : NT;
+    static constexpr int kSlots = kPer == 2 && NT <= 32 ? 4 : 2;
+    static constexpr int kWCols = 16 * kPer, kWBase = kSlots * kPer * kAccStride;
+    static constexpr int kCols = NT / 2;                             // accumulator columns per promoting warp
+    static constexpr size_t kPipe = (size_t)kStages * kStageBytes + (size_t)kRawStages * kRawBytes;
+    static constexpr size_t kSmem = kPipe + 1024;
+    static constexpr uint32_t kIdesc = (1u << 4) | ((uint32_t)(NT >> 3) << 17) | ((uint32_t)(kRows >> 4) << 24);   // fp16 × fp16 → fp32, K-major
+    // K-major: 8-row groups 8 · kRowBytes apart, descriptor version 1, layout type 4 (64-byte swizzle) or 2 (128-byte)
+    static constexpr uint64_t kDesc = ((uint64_t)1 << 16) | ((uint64_t)(8 * kRowBytes >> 4) << 32) | ((uint64_t)1 << 46) | ((uint64_t)(kPer == 1 ? 4 : 2) << 61);
+    static_assert(kWBase + kStages * kWCols <= 512, "tensor memory");
+    static_assert((size_t)NT * kRows * 4 <= kPipe, "the partial tile fits the pipeline's memory");
+    static_assert(kSmem <= 227 * 1024, "shared memory of one CTA");
+};
 
-// K-major, 64-byte swizzle: 8-row groups 512 bytes apart (stride byte offset), leading offset unused (1),
-// descriptor version 1, layout type 4.
-__device__ __forceinline__ uint64_t umma_desc(uint32_t smem_addr) {
-    uint64_t d = 0;
-    d |= (uint64_t)((smem_addr >> 4) & 0x3fff);
-    d |= (uint64_t)1 << 16;
-    d |= (uint64_t)(512 >> 4) << 32;
-    d |= (uint64_t)1 << 46;
-    d |= (uint64_t)4 << 61;
-    return d;
+// byte offset of 16-byte chunk c of row r inside a swizzled K-major tile of 32 or 64 halves per row
+__host__ __device__ __forceinline__ int swz_off(int r, int c, int per) {
+    return per == 1 ? r * 64 + ((c ^ ((r >> 1) & 3)) << 4) : r * 128 + ((c ^ (r & 7)) << 4);
 }
-// fp16 × fp16 → fp32, both operands K-major, M = 128, N = 256
-constexpr uint32_t kIdesc = (1u << 4) | ((uint32_t)(kTileN >> 3) << 17) | ((uint32_t)(kTileM >> 4) << 24);
 
 __device__ __forceinline__ uint32_t pack_h2(float lo, float hi) {
     uint32_t r;
@@ -71,464 +82,558 @@ __device__ __forceinline__ uint32_t pack_h2(float lo, float hi) {
     return r;
 }
 
-// ───────────── pre-pass: fp32 activations → hi/lo fp16 tile images ─────────────
-// One warp per activation row.  Output tiles [m-tile][k-tile]{hi 16 KB, lo 16 KB}; rowscale[m] undoes the
-// power-of-two scaling in the GEMM epilogue.  Rows ≥ M of the last m-tile are written as zeros.
-__global__ void __launch_bounds__(256) k_x_to_f16_tiles(const float* __restrict__ x, int ldx, const float* __restrict__ gamma, float eps,
-                                                         int M, int K, unsigned char* __restrict__ tiles, float* __restrict__ rowscale) {
-    pdl_wait();
+__device__ __forceinline__ void tmem_ld16_nowait(uint32_t taddr, uint32_t* v) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+                 : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]), "=r"(v[9]),
+                   "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
+                 : "r"(taddr));
+}
+__device__ __forceinline__ void tmem_ld8_nowait(uint32_t taddr, uint32_t* v) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                 : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]) : "r"(taddr));
+}
+__device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
+__device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint32_t (&v)[8]) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};"
+                 ::"r"(taddr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]) : "memory");
+}
+__device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+// D (tensor memory) = or += A (tensor memory) · B (shared memory)
+__device__ __forceinline__ void umma_f16_ts(uint32_t d, uint32_t a, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+    asm volatile("{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}"
+                 ::"r"(d), "r"(a), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
+}
+
+// acc (two floats) += v (two floats) · s (the same float twice).  Volatile: v comes from an asynchronous load, and no use of it
+// may be scheduled before the wait.
+__device__ __forceinline__ void fma2(unsigned long long& acc, uint32_t v0, uint32_t v1, unsigned long long s) {
+    asm volatile("{\n .reg .b64 v;\n mov.b64 v, {%1, %2};\n fma.rn.f32x2 %0, v, %3, %0;\n}" : "+l"(acc) : "r"(v0), "r"(v1), "l"(s));
+}
+
+// A whole warp waits.  The first try decides nearly always (the instruction itself waits for a while); entering the bounded
+// loop costs more than 100 cycles even when the barrier is ready (measured: 170 against 48).  The vote makes the result
+// uniform for the compiler, so that what follows (descriptors, stage addresses) can stay in uniform registers.
+__device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag, int* error, int code) {
+    if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
+    return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag, error, code));
+}
+__device__ __forceinline__ bool elect_one() {
+    uint32_t p;
+    asm volatile("{\n .reg .pred P;\n elect.sync _|P, 0xffffffff;\n selp.u32 %0, 1, 0, P;\n}" : "=r"(p));
+    return p != 0;
+}
+
+__device__ __forceinline__ void cluster_sync_all() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ float ld_peer(uint32_t addr, uint32_t rank) {
+    uint32_t a; float v;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(addr), "r"(rank));
+    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(a) : "memory");
+    return v;
+}
+
+// ───────────── pre-pass: fp32 activations → hi/lo fp16 images ─────────────
+// Image: per tile of nt rows and stage of per blocks, X_hi then X_lo in the swizzled layout that the MMA reads, so that a stage
+// is one contiguous copy.  Blocks that fill up the last stage are zeros.  rowscale[m] undoes the power-of-two row scaling in
+// the epilogue.  Rows from M on are left alone: they only reach result rows that are never stored.  One block per row; norm:
+// RMSNorm (γ) or LayerNorm (γ, β).
+constexpr int kXThreads = 256;
+__global__ void __launch_bounds__(kXThreads) k_x_images(const float* __restrict__ x, int ldx, const float* __restrict__ gamma, const float* __restrict__ beta,
+                                                        float eps, int K, int nS, int nt, int per, unsigned char* __restrict__ images, float* __restrict__ rowscale) {
+    __shared__ float red[3][kXThreads / 32];
     pdl_launch_dependents();
-    const int lane = threadIdx.x & 31;
-    const int m = blockIdx.x * 8 + (threadIdx.x >> 5);
-    const int mPad = (M + kTileM - 1) / kTileM * kTileM;
-    if (m >= mPad) return;
-    const int nK = K / kTileK;
-    unsigned char* mt = tiles + (size_t)(m / kTileM) * nK * (2 * kATileBytes);
-    const int r = m % kTileM;
-    if (m >= M) {
-        for (int c = lane; c < nK * 4; c += 32) {
-            unsigned char* t = mt + (size_t)(c >> 2) * (2 * kATileBytes) + swz_off(r, c & 3);
-            *reinterpret_cast<uint4*>(t) = make_uint4(0, 0, 0, 0);
-            *reinterpret_cast<uint4*>(t + kATileBytes) = make_uint4(0, 0, 0, 0);
-        }
-        if (lane == 0) rowscale[m] = 0.0f;
-        return;
-    }
+    pdl_wait();
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, m = blockIdx.x;
     const float* xr = x + (size_t)m * ldx;
-    float ss = 0.0f, amax = 0.0f;
-    for (int k = lane * 4; k < K; k += 128) {
-        const float4 v = *reinterpret_cast<const float4*>(xr + k);
-        ss = fmaf(v.x, v.x, ss); ss = fmaf(v.y, v.y, ss); ss = fmaf(v.z, v.z, ss); ss = fmaf(v.w, v.w, ss);
-        float4 g = make_float4(1.f, 1.f, 1.f, 1.f);
-        if (gamma) g = *reinterpret_cast<const float4*>(gamma + k);
-        amax = fmaxf(amax, fmaxf(fmaxf(fabsf(v.x * g.x), fabsf(v.y * g.y)), fmaxf(fabsf(v.z * g.z), fabsf(v.w * g.w))));
+    auto block_sum = [&](float v, float* r) {
+        for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+        if (lane == 0) r[warp] = v;
+        __syncthreads();
+        float t = 0.0f;
+#pragma unroll
+        for (int q = 0; q < kXThreads / 32; q++) t += r[q];
+        return t;
+    };
+    float mean = 0.0f, inv = 1.0f;
+    if (beta != nullptr) {
+        float sm = 0.0f;
+        for (int k = tid * 4; k < K; k += 4 * kXThreads) {
+            const float4 v = *reinterpret_cast<const float4*>(xr + k);
+            sm += (v.x + v.y) + (v.z + v.w);
+        }
+        mean = block_sum(sm, red[0]) * (1.0f / (float)K);
     }
-    for (int o = 16; o > 0; o >>= 1) { ss += __shfl_xor_sync(0xffffffffu, ss, o); amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o)); }
-    float inv = 1.0f;
-    if (gamma) inv = __frcp_rn(sqrtf(ss * (1.0f / (float)K) + eps));      // RMSNorm1D.forward: x / rms · γ
-    amax *= inv;
+    if (gamma != nullptr) {
+        float ss = 0.0f;
+        for (int k = tid * 4; k < K; k += 4 * kXThreads) {
+            float4 v = *reinterpret_cast<const float4*>(xr + k);
+            v.x -= mean; v.y -= mean; v.z -= mean; v.w -= mean;
+            ss = fmaf(v.x, v.x, ss); ss = fmaf(v.y, v.y, ss); ss = fmaf(v.z, v.z, ss); ss = fmaf(v.w, v.w, ss);
+        }
+        const float var = block_sum(ss, red[1]) * (1.0f / (float)K);
+        inv = beta != nullptr ? sqrtf(var + eps) : __frcp_rn(sqrtf(var + eps));      // LayerNorm divides by it, RMSNorm multiplies
+    }
+    auto value = [&](float v, float g, float b) {
+        if (beta != nullptr) return __fdiv_rn(v - mean, inv) * g + b;
+        return gamma != nullptr ? (v * inv) * g : v;
+    };
+    auto load4 = [&](int k, float (&v)[4]) {
+        const float4 a = *reinterpret_cast<const float4*>(xr + k);
+        float4 g = make_float4(1.f, 1.f, 1.f, 1.f), b = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (gamma) g = *reinterpret_cast<const float4*>(gamma + k);
+        if (beta) b = *reinterpret_cast<const float4*>(beta + k);
+        v[0] = value(a.x, g.x, b.x); v[1] = value(a.y, g.y, b.y); v[2] = value(a.z, g.z, b.z); v[3] = value(a.w, g.w, b.w);
+    };
+    float amax = 0.0f;
+    for (int k = tid * 4; k < K; k += 4 * kXThreads) {
+        float v[4];
+        load4(k, v);
+        amax = fmaxf(amax, fmaxf(fmaxf(fabsf(v[0]), fabsf(v[1])), fmaxf(fabsf(v[2]), fabsf(v[3]))));
+    }
+    for (int o = 16; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
+    if (lane == 0) red[2][warp] = amax;
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < kXThreads / 32; q++) amax = fmaxf(amax, red[2][q]);
     // 2^-e brings the row's largest value into [512, 1024)
     int ebits = 0x3f800000;
     if (amax > 0.0f && amax < 1e30f) ebits = __float_as_int(amax) & 0x7f800000;
     const float down = __int_as_float(0x7f000000 - ebits) * 512.0f;
-    if (lane == 0) rowscale[m] = __int_as_float(ebits) * (1.0f / 512.0f);
-    for (int c = lane; c < nK * 4; c += 32) {          // chunk c: values 8c … 8c+7
-        const float4 a = *reinterpret_cast<const float4*>(xr + c * 8), b = *reinterpret_cast<const float4*>(xr + c * 8 + 4);
-        float v[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
-        if (gamma) {
-            const float4 ga = *reinterpret_cast<const float4*>(gamma + c * 8), gb = *reinterpret_cast<const float4*>(gamma + c * 8 + 4);
-            const float g[8] = {ga.x, ga.y, ga.z, ga.w, gb.x, gb.y, gb.z, gb.w};
-#pragma unroll
-            for (int j = 0; j < 8; j++) v[j] = (v[j] * inv) * g[j];
-        }
+    if (tid == 0) rowscale[m] = __int_as_float(ebits) * (1.0f / 512.0f);
+    const int rowBytes = 64 * per, mt = m / nt, r = m - mt * nt;
+    unsigned char* const tile = images + (size_t)mt * nS * 2 * nt * rowBytes;
+    for (int c = tid; c < nS * per * 4; c += kXThreads) {    // chunk c: values 8c … 8c + 7; past K zeros
         uint32_t hi[4], lo[4];
 #pragma unroll
-        for (int j = 0; j < 4; j++) {
-            const float p = v[2 * j] * down, q = v[2 * j + 1] * down;
-            hi[j] = pack_h2(p, q);
-            const float2 back = __half22float2(*reinterpret_cast<const __half2*>(&hi[j]));
-            lo[j] = pack_h2(p - back.x, q - back.y);
+        for (int h = 0; h < 2; h++) {
+            float v[4] = {0.f, 0.f, 0.f, 0.f};
+            if (c * 8 + 4 * h < K) load4(c * 8 + 4 * h, v);
+#pragma unroll
+            for (int j = 0; j < 2; j++) {
+                const float p = v[2 * j] * down, q = v[2 * j + 1] * down;
+                hi[2 * h + j] = pack_h2(p, q);
+                const float2 back = __half22float2(*reinterpret_cast<const __half2*>(&hi[2 * h + j]));
+                lo[2 * h + j] = pack_h2(p - back.x, q - back.y);
+            }
         }
-        unsigned char* t = mt + (size_t)(c >> 2) * (2 * kATileBytes) + swz_off(r, c & 3);
+        const int st = c / (4 * per), cc = c - st * 4 * per;
+        unsigned char* t = tile + (size_t)st * 2 * nt * rowBytes + swz_off(r, cc, per);
         *reinterpret_cast<uint4*>(t) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
-        *reinterpret_cast<uint4*>(t + kATileBytes) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+        *reinterpret_cast<uint4*>(t + nt * rowBytes) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
     }
 }
 
 struct TcParams {
-    const unsigned char* xtiles; const float* rowscale;
-    const int8_t* codes; const float* scales; const float* bias;
+    CUtensorMap codes, codes2;          // boxes of 128 bytes × 128 rows (64 rows of each for SwiGLU)
+    const unsigned char* images; const float* rowscale;
+    const float* scales; const float* scales2;
+    const float* bias; const float* bias2;
     const float* residual; int ldr;
     float* out; int ldo;
-    int M, N, K, Kp, nb;
-    int mTiles;             // 128-row activation tiles
-    int pair;               // 1: a CTA takes tiles 2·blockIdx.y and 2·blockIdx.y + 1 (the second may not exist), two accumulators; 0: tile blockIdx.y
-    int mode;               // 0: out = acc + bias (+ residual);  1: out = SiLU(out) · (acc + bias)   (SwiGLU's second GEMM)
-    int ktPer;              // k-tiles per K split (blockIdx.z); a multiple of 4.  One split = the whole reduction
-    size_t splitStride;     // floats between the partial outputs of consecutive splits (0 when there is one split)
-    int terms;              // correction products on top of x_hi · w_hi: bit 0 adds x_lo · w_hi, bit 1 adds x_hi · w_lo
+    int M, N, nb, nK, nS;               // nK blocks, nS stages of the whole reduction
+    int swiglu, gelu;
+    int splits, ktPer;                  // CTAs of a cluster share the reduction, ktPer blocks (a multiple of 4) each
+    int lo;                             // 1: the X_lo product is added
+    int coarse;                         // 1: block scales rounded to 11 bits
     int* error;
-    unsigned long long* trace;      // optional: thread 0 of CTA (0,0) sums the time it spends waiting / converting / fencing
 };
 
-__global__ void __launch_bounds__(kTcThreads, 1) k_q8_gemm_tc(const TcParams p) {
-    extern __shared__ __align__(1024) unsigned char smem[];
-    __shared__ __align__(8) unsigned long long s_bar[2 * kStagesA + 2 * kStagesB + 5];
+// Four block scales from block k on; past the row's end zeros, which only meet blocks that do not exist.
+__device__ __forceinline__ float4 load_scales(const float* row, int k, int nb, bool vec, bool coarse) {
+    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (vec) {
+        if (k < nb) v = *reinterpret_cast<const float4*>(row + k);
+    } else {
+        if (k < nb) v.x = row[k];
+        if (k + 1 < nb) v.y = row[k + 1];
+        if (k + 2 < nb) v.z = row[k + 2];
+        if (k + 3 < nb) v.w = row[k + 3];
+    }
+    if (coarse) {
+        auto cut = [](float f) { return __half2float(__float2half_rn(f * 4096.0f)) * (1.0f / 4096.0f); };
+        v = make_float4(cut(v.x), cut(v.y), cut(v.z), cut(v.w));
+    }
+    return v;
+}
+
+template <int NT>
+__global__ void __launch_bounds__(kTcThreads, 1) k_q8_gemm_tc(const __grid_constant__ TcParams p) {
+    using S = TileShape<NT>;
+    extern __shared__ __align__(1024) unsigned char smem_raw[];
+    __shared__ __align__(8) unsigned long long s_bar[2 * S::kStages + 2 * S::kRawStages + 2 * S::kSlots];
     __shared__ uint32_t s_tmem;
     __shared__ volatile int s_abort;
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int tile0 = p.pair ? 2 * (int)blockIdx.y : (int)blockIdx.y;
-    const int n0 = blockIdx.x * kTileN, m0 = tile0 * kTileM;
-    const bool has1 = p.pair && tile0 + 1 < p.mTiles;           // a second 128-row tile for the second accumulator
-    const int nStA = p.pair ? kStagesA / 2 : kStagesA;          // activation stages in use, and their size
-    const uint32_t stABytes = p.pair ? 2 * kAImageBytes : kAImageBytes;
-    // K split blockIdx.z covers k-tiles kt0 … kt0 + nK − 1 of the nKfull of the reduction; everything below counts
-    // k-tiles from 0 within the split and only the global addresses know kt0
-    const int nKfull = p.K / kTileK;
-    const int kt0 = (int)blockIdx.z * p.ktPer;
-    const int nK = min(p.ktPer, nKfull - kt0);
-    const int8_t* const codes = p.codes + (size_t)kt0 * kTileK;
-    const float* const scales = p.scales + kt0;
-    float* const outp = p.out + (size_t)blockIdx.z * p.splitStride;
-    // the swizzled tiles want 1024-byte alignment: the dynamic segment carries 1 KB of slack for it
-    const uint32_t smem_raw = smem_u32(smem);
-    const uint32_t smem_s = (smem_raw + 1023u) & ~1023u;
-    unsigned char* const smem_al = smem + (smem_s - smem_raw);
-    // layout: activation stages [kStagesA][tile 0: X_hi 8 KB | X_lo 8 KB][tile 1: the same], then weight stages [kStagesB][W_hi 16 KB | W_lo 16 KB]
-    const uint32_t smemB_s = smem_s + kARegionBytes;
-    unsigned char* const smemB = smem_al + kARegionBytes;
-    auto bar_fullA = [&](int s) { return smem_u32(&s_bar[s]); };
-    auto bar_emptyA = [&](int s) { return smem_u32(&s_bar[kStagesA + s]); };
-    auto bar_fullB = [&](int s) { return smem_u32(&s_bar[2 * kStagesA + s]); };
-    auto bar_emptyB = [&](int s) { return smem_u32(&s_bar[2 * kStagesA + kStagesB + s]); };
-    const uint32_t bar_acc = smem_u32(&s_bar[2 * kStagesA + 2 * kStagesB]);
-    const uint32_t bar_rawFull = smem_u32(&s_bar[2 * kStagesA + 2 * kStagesB + 1]);
-    const uint32_t bar_rawEmpty = smem_u32(&s_bar[2 * kStagesA + 2 * kStagesB + 2]);
-    unsigned char* const raw = smemB + kStagesB * kStageBBytes;          // [256 rows][128 code bytes + 4 scales]
+    const int split = (int)blockIdx.x, m0 = (int)blockIdx.y * NT;
+    const int rowsOut = p.swiglu ? kRows / 2 : kRows;             // output columns of a tile
+    const int n0 = (int)blockIdx.z * rowsOut;
+    const int kt0 = split * p.ktPer;
+    const int nK = min(p.ktPer, p.nK - kt0);                      // blocks of this CTA; at least one
+    const uint32_t raw_s = smem_u32(smem_raw), base = (raw_s + 1023u) & ~1023u;      // the swizzled tiles want 1024-byte alignment
+    unsigned char* const smem = smem_raw + (base - raw_s);
+    // layout: [stage: X_hi | X_lo] × kStages, then [raw codes 16 KB] × kRawStages
+    const uint32_t rawBase = base + S::kStages * S::kStageBytes;
+    auto full = [&](int s) { return smem_u32(&s_bar[s]); };
+    auto empty = [&](int s) { return smem_u32(&s_bar[S::kStages + s]); };
+    auto rawFull = [&](int s) { return smem_u32(&s_bar[2 * S::kStages + s]); };
+    auto rawEmpty = [&](int s) { return smem_u32(&s_bar[2 * S::kStages + S::kRawStages + s]); };
+    auto accFull = [&](int a) { return smem_u32(&s_bar[2 * S::kStages + 2 * S::kRawStages + a]); };
+    auto accEmpty = [&](int a) { return smem_u32(&s_bar[2 * S::kStages + 2 * S::kRawStages + S::kSlots + a]); };
 
     if (tid == 0) {
-        for (int s = 0; s < kStagesA; s++) { mbar_init(bar_fullA(s), 1); mbar_init(bar_emptyA(s), 1); }
-        for (int s = 0; s < kStagesB; s++) { mbar_init(bar_fullB(s), 128); mbar_init(bar_emptyB(s), 1); }
-        mbar_init(bar_acc, 1);
-        mbar_init(bar_rawFull, kDqWarps * 32);
-        mbar_init(bar_rawEmpty, kDqWarps * 32);
+        for (int s = 0; s < S::kStages; s++) { mbar_init(full(s), 1 + kConvertWarps / 2); mbar_init(empty(s), 1); }
+        for (int s = 0; s < S::kRawStages; s++) { mbar_init(rawFull(s), 1); mbar_init(rawEmpty(s), kConvertWarps); }
+        for (int a = 0; a < S::kSlots; a++) { mbar_init(accFull(a), 1); mbar_init(accEmpty(a), kPromoteWarps); }
         s_abort = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    if (warp == kDqWarps) tmem_alloc(smem_u32(&s_tmem), kTmemCols);
+    if (warp == kMmaWarp) tmem_alloc(smem_u32(&s_tmem), 512);
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem_base = s_tmem;
-    pdl_wait();
+    const uint32_t tmem = s_tmem;
     pdl_launch_dependents();
 
-    if (warp < kDqWarps) {
-        // ── dequantise: two groups of four warps take the k-tiles in turn (group g: k-tiles g, g+2, …); thread r of a
-        // group owns weight rows n0 + r and n0 + r + 128 of the 256-row tile.  The raw codes and scales of four
-        // k-tiles at a time (256 rows × 128 code bytes + 4 scales) come through a shared-memory buffer filled with
-        // cp.async in row-contiguous runs — a warp's copy instruction touches 4 lines, where a load per row owner
-        // touched 32 and kept L1TEX saturated; every thread lifts its own pieces into registers, the buffer is
-        // refilled for the next four k-tiles behind a barrier, and the conversion runs from registers. ──
-        const int r = tid & 127, grp = tid >> 7;
-        const int nG = nK / 4;
-        auto issue_group = [&](int G) {
-            // chunk q = tid + 256·i → row q / 8 (clamped: rows past N are never stored), 16-byte piece q % 8
+    if (warp < kPromoteWarps) {
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kPromoteRegs));
+        const int quarter = warp & 3, half = warp >> 2;
+        const int r = quarter * 32 + lane;                        // tile row = tensor-memory lane
+        const bool second = p.swiglu && r >= kRows / 2;
+        const int n = min(n0 + (second ? r - kRows / 2 : r), p.N - 1);
+        const float* const srow = (second ? p.scales2 : p.scales) + (size_t)n * p.nb;
+        const bool vec = (p.nb & 3) == 0;
+        const uint32_t lane_base = tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(half * S::kCols);
+        unsigned long long acc[S::kCols / 2];
 #pragma unroll
-            for (int i = 0; i < 8; i++) {
-                const int row = (tid >> 3) + 32 * i, c = tid & 7;
-                const int n = min(n0 + row, p.N - 1);
-                cp_async16(raw + row * kRawRow + c * 16, codes + (size_t)n * p.Kp + (size_t)G * 128 + c * 16);
-            }
-            const int n = min(n0 + tid, p.N - 1);
-            cp_async16(raw + tid * kRawRow + 128, scales + (size_t)n * p.nb + (size_t)G * 4);
-            asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(bar_rawFull) : "memory");
-        };
-        issue_group(0);
-        const bool tracing = p.trace != nullptr && blockIdx.x == 0 && blockIdx.y == 0 && tid == 0;
-        unsigned long long tWait = 0, tConv = 0, tFence = 0, tStart = tracing ? gtime() : 0;
-        const bool wantLo = (p.terms & 2) != 0;              // without the x_hi · w_lo product the low halves are never read
-        for (int G = 0; G < nG; G++) {
-            uint4 cur4[2][2][2]; float scl4[2][2];            // [own k-tile of the group][row][16-byte half]
-            mbar_wait(bar_rawFull, G & 1, &s_abort, p.error, 206);
+        for (int j = 0; j < S::kCols / 2; j++) acc[j] = 0ull;
+        float4 next = load_scales(srow, kt0, p.nb, vec, p.coarse);
+        bool ok = true;
+        int slot = 0;
+        uint32_t round = 0;
+        for (int b0 = 0; b0 < nK && ok; b0 += kGroup) {
+            const float4 cur = next;
+            if (b0 + kGroup < nK) next = load_scales(srow, kt0 + b0 + kGroup, p.nb, vec, p.coarse);
 #pragma unroll
-            for (int o = 0; o < 2; o++)
-#pragma unroll
-                for (int h = 0; h < 2; h++) {
-                    const unsigned char* src = raw + (r + 128 * h) * kRawRow;
-                    const int j = grp + 2 * o;                   // k-tile inside the group
-                    cur4[o][h][0] = *reinterpret_cast<const uint4*>(src + 32 * j);
-                    cur4[o][h][1] = *reinterpret_cast<const uint4*>(src + 32 * j + 16);
-                    scl4[o][h] = *reinterpret_cast<const float*>(src + 128 + 4 * j);
-                }
-            mbar_arrive(bar_rawEmpty);
-            if (G + 1 < nG) {
-                mbar_wait(bar_rawEmpty, G & 1, &s_abort, p.error, 207);      // every thread has lifted its pieces
-                issue_group(G + 1);
-            }
-#pragma unroll
-            for (int o = 0; o < 2; o++) {
-                const int kt = 4 * G + grp + 2 * o;
-                const int s = kt % kStagesB;
-                uint4 cur[2][2]; float scl[2];
-#pragma unroll
-                for (int h = 0; h < 2; h++) { cur[h][0] = cur4[o][h][0]; cur[h][1] = cur4[o][h][1]; scl[h] = scl4[o][h]; }
-                unsigned long long t0 = tracing ? gtime() : 0;
-                if (kt >= kStagesB) mbar_wait(bar_emptyB(s), ((kt / kStagesB) - 1) & 1, &s_abort, p.error, 201);
-                unsigned long long t1 = tracing ? gtime() : 0;
-                unsigned char* bhi = smemB + (size_t)s * kStageBBytes;
-                unsigned char* blo = bhi + kBTileBytes;
-                // The block's scale (times 2^12, undone in the epilogue, so that it sits in fp16's normal range) as
-                // s_hi + s_lo, both fp16.  Per pair of codes, all in packed fp16 arithmetic:
-                //   c    = the codes as fp16, exactly (sign flip, byte under exponent 0x64, subtract 1152)
-                //   w_hi = rn(c · s_hi)
-                //   w_lo = rn(c · s_lo + (c · s_hi − w_hi))      — the product's rounding error is exact in one fma
-                // so w_hi + w_lo carries ≈ 22 bits of c · scale at 2.75 instructions per weight.
-#pragma unroll
-                for (int h = 0; h < 2; h++) {
-                    const int row = r + 128 * h;
-                    const float sv = scl[h] * 4096.0f;
-                    const __half sh1 = __float2half_rn(sv);
-                    const __half sl1 = __float2half_rn(sv - __half2float(sh1));
-                    const __half2 sh = __half2half2(sh1), sl = __half2half2(sl1);
-#pragma unroll
-                    for (int j = 0; j < 2; j++) {                  // 16 codes → two 16-byte chunks of hi and of lo
-                        const uint32_t w4[4] = {cur[h][j].x, cur[h][j].y, cur[h][j].z, cur[h][j].w};
-                        uint32_t hi[8], lo[8];
-#pragma unroll
-                        for (int q = 0; q < 4; q++) {
-                            const uint32_t u = w4[q] ^ 0x80808080u;
-                            uint32_t c01 = __byte_perm(u, 0x64646464u, 0x4140), c23 = __byte_perm(u, 0x64646464u, 0x4342);
-                            const uint32_t k1152 = 0x64806480u;
-                            asm("sub.f16x2 %0, %1, %2;" : "=r"(c01) : "r"(c01), "r"(k1152));
-                            asm("sub.f16x2 %0, %1, %2;" : "=r"(c23) : "r"(c23), "r"(k1152));
-#pragma unroll
-                            for (int e = 0; e < 2; e++) {
-                                const __half2 c = *reinterpret_cast<const __half2*>(e == 0 ? &c01 : &c23);
-                                const __half2 wh = __hmul2(c, sh);
-                                hi[2 * q + e] = *reinterpret_cast<const uint32_t*>(&wh);
-                                if (wantLo) {
-                                    const __half2 er = __hfma2(c, sh, __hneg2(wh));
-                                    const __half2 wl = __hfma2(c, sl, er);
-                                    lo[2 * q + e] = *reinterpret_cast<const uint32_t*>(&wl);
-                                }
-                            }
-                        }
-                        const int o0 = swz_off(row, 2 * j), o1 = swz_off(row, 2 * j + 1);
-                        *reinterpret_cast<uint4*>(bhi + o0) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
-                        *reinterpret_cast<uint4*>(bhi + o1) = make_uint4(hi[4], hi[5], hi[6], hi[7]);
-                        if (wantLo) {
-                            *reinterpret_cast<uint4*>(blo + o0) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
-                            *reinterpret_cast<uint4*>(blo + o1) = make_uint4(lo[4], lo[5], lo[6], lo[7]);
-                        }
-                    }
-                }
-                unsigned long long t2 = tracing ? gtime() : 0;
-                fence_proxy_async_smem();                      // generic-proxy stores → visible to the tensor-core (async) proxy
-                mbar_arrive(bar_fullB(s));
-                if (tracing) { const unsigned long long t3 = gtime(); tWait += t1 - t0; tConv += t2 - t1; tFence += t3 - t2; }
-            }
-        }
-        if (tracing) { p.trace[0] = tStart; p.trace[1] = tStart + tWait; p.trace[2] = p.trace[1] + tConv; p.trace[3] = p.trace[2] + tFence; p.trace[4] = gtime(); }
-        // ── epilogue: warp w reads accumulator rows 32(w%4) … +31, columns 128(w/4) … +127; each 32 × 32 block goes
-        // through a padded shared-memory square so that a warp stores 128 contiguous bytes of one output row ──
-        const bool ok = __all_sync(0xffffffffu, mbar_wait(bar_acc, 0, &s_abort, p.error, 202));
-        tc_fence_after();
-        const int q4 = warp & 3, chalf = warp >> 2;
-        float* stg = reinterpret_cast<float*>(smem_al) + warp * (32 * 33);       // the pipeline stages are idle by now
-#pragma unroll 1
-        for (int acc = 0; acc < (has1 ? 2 : 1); acc++) {
-        const int mbase = m0 + acc * kTileM + q4 * 32;
-        const int mrow = mbase + lane;
-        const float rs = (ok && mrow < p.M) ? p.rowscale[mrow] * (1.0f / 4096.0f) : 0.0f;       // the weights carry 2^12
-#pragma unroll 1
-        for (int c0 = chalf * 128; c0 < chalf * 128 + 128; c0 += 32) {
-            uint32_t v[32];
-            if (ok) tmem_ld32(tmem_base + ((uint32_t)(q4 * 32) << 16) + (uint32_t)(acc * kTileN + c0), v);      // warp-uniform
-            else {
-#pragma unroll
-                for (int j = 0; j < 32; j++) v[j] = 0u;
-            }
-#pragma unroll
-            for (int j = 0; j < 32; j++) stg[lane * 33 + j] = __uint_as_float(v[j]) * rs;
-            __syncwarp();
-            const int nn = n0 + c0 + lane;
-            const float bv = (p.bias && nn < p.N) ? p.bias[nn] : 0.0f;
-            for (int i = 0; i < 32; i++) {
-                const int m = mbase + i;
-                if (!ok || m >= p.M || nn >= p.N) continue;
-                float val = stg[i * 33 + lane] + bv;
-                float* o = outp + (size_t)m * p.ldo + nn;
-                if (p.mode == 0) {
-                    if (p.residual) val += p.residual[(size_t)m * p.ldr + nn];
-                    *o = val;
-                } else {
-                    const float gte = *o;
-                    const float sig = 1.0f / (1.0f + expf(-gte));
-                    *o = (gte * sig) * val;
-                }
-            }
-            __syncwarp();
-        }
-        }
-        if (tracing) { p.trace[5] = gtime(); p.trace[6] = p.trace[5]; }
-        tc_fence_before();
-    } else if (warp == kDqWarps) {
-        // ── activation tiles: one bulk copy of 16 KB (hi + lo) per 128-row tile and stage ──
-        if (lane == 0) {
-            const unsigned char* src = p.xtiles + ((size_t)tile0 * nKfull + kt0) * kAImageBytes;
-            for (int kt = 0; kt < nK; kt++) {
-                const int s = kt % nStA;
-                if (kt >= nStA && !mbar_wait(bar_emptyA(s), ((kt / nStA) - 1) & 1, &s_abort, p.error, 203)) break;
-                mbar_arrive_expect_tx(bar_fullA(s), has1 ? 2 * kAImageBytes : kAImageBytes);
-                bulk_g2s(smem_s + (uint32_t)s * stABytes, src + (size_t)kt * kAImageBytes, kAImageBytes, bar_fullA(s));
-                if (has1)
-                    bulk_g2s(smem_s + (uint32_t)s * stABytes + kAImageBytes, src + (size_t)(nKfull + kt) * kAImageBytes, kAImageBytes, bar_fullA(s));
-            }
-        }
-        __syncwarp();
-    } else {
-        // ── MMA issue: one thread ──
-        if (lane == 0) {
-            bool ok = true;
-            const bool xLo = (p.terms & 1) != 0, wLo = (p.terms & 2) != 0;
-            for (int kt = 0; kt < nK && ok; kt++) {
-                const int sa = kt % nStA, sb = kt % kStagesB;
-                ok = mbar_wait(bar_fullA(sa), (kt / nStA) & 1, &s_abort, p.error, 204) &&
-                     mbar_wait(bar_fullB(sb), (kt / kStagesB) & 1, &s_abort, p.error, 205);
+            for (int i = 0; i < kGroup; i += S::kPer) {
+                if (b0 + i >= nK) break;
+                ok = warp_wait(accFull(slot), round & 1, &s_abort, p.error, 202);
                 if (!ok) break;
                 tc_fence_after();
-                const uint32_t a_hi = smem_s + (uint32_t)sa * stABytes, a_lo = a_hi + kATileBytes;
-                const uint32_t b_hi = smemB_s + (uint32_t)sb * kStageBBytes, b_lo = b_hi + kBTileBytes;
+                const uint32_t from = lane_base + (uint32_t)(slot * S::kPer * S::kAccStride);
+                // 32 columns at a time (16, 8 where registers or columns are short), the next piece on its way while this one is added
+                constexpr int kStep = S::kCols % 32 == 0 && S::kCols <= 64 ? 32 : S::kCols % 16 == 0 ? 16 : 8;
+                constexpr int kPieces = S::kPer * S::kCols / kStep;
+                const int pieces = S::kPer == 2 && b0 + i + 1 >= nK ? kPieces / 2 : kPieces;       // an odd last block
+                uint32_t v[2][kStep];
+                auto load = [&](int q) {
+                    const uint32_t at = from + (uint32_t)((q * kStep / S::kCols) * S::kAccStride + q * kStep % S::kCols);
+                    if constexpr (kStep == 8) tmem_ld8_nowait(at, v[q & 1]); else tmem_ld16_nowait(at, v[q & 1]);
+                    if constexpr (kStep == 32) tmem_ld16_nowait(at + 16, v[q & 1] + 16);
+                };
+                load(0);
 #pragma unroll
-                for (int ks = 0; ks < kTileK / 16; ks++) {
-                    const uint32_t off = ks * 32;          // 16 halves along K inside the swizzled row
-                    umma_f16(tmem_base, umma_desc(a_hi + off), umma_desc(b_hi + off), kIdesc, (kt | ks) != 0);
-                    if (xLo) umma_f16(tmem_base, umma_desc(a_lo + off), umma_desc(b_hi + off), kIdesc, 1);
-                    if (wLo) umma_f16(tmem_base, umma_desc(a_hi + off), umma_desc(b_lo + off), kIdesc, 1);
-                    if (has1) {                            // the same weight tile against the second 128 rows → accumulator 2
-                        umma_f16(tmem_base + kTileN, umma_desc(a_hi + kAImageBytes + off), umma_desc(b_hi + off), kIdesc, (kt | ks) != 0);
-                        if (xLo) umma_f16(tmem_base + kTileN, umma_desc(a_lo + kAImageBytes + off), umma_desc(b_hi + off), kIdesc, 1);
-                        if (wLo) umma_f16(tmem_base + kTileN, umma_desc(a_hi + kAImageBytes + off), umma_desc(b_lo + off), kIdesc, 1);
+                for (int q = 0; q < kPieces; q++) {
+                    if (q < pieces) {
+                        tmem_wait_ld();
+                        if (q + 1 < pieces) load(q + 1);
+                        else {                                    // everything is read: the MMAs may write here again
+                            tc_fence_before();
+                            __syncwarp();
+                            if (lane == 0) mbar_arrive(accEmpty(slot));
+                        }
+                        const int blk = i + q * kStep / S::kCols;
+                        const float sc = blk == 0 ? cur.x : blk == 1 ? cur.y : blk == 2 ? cur.z : cur.w;
+                        unsigned long long ss;
+                        asm("mov.b64 %0, {%1, %1};" : "=l"(ss) : "f"(sc));
+#pragma unroll
+                        for (int j = 0; j < kStep / 2; j++) fma2(acc[(q * kStep % S::kCols) / 2 + j], v[q & 1][2 * j], v[q & 1][2 * j + 1], ss);
                     }
                 }
-                umma_commit(bar_emptyA(sa));               // both arrive when the MMAs above have finished reading the stages
-                umma_commit(bar_emptyB(sb));
+                if (++slot == S::kSlots) { slot = 0; round++; }
             }
-            if (ok) umma_commit(bar_acc);
+        }
+        // Every MMA of this CTA has completed (its last commits have been waited for) and every copy has landed: the pipeline's
+        // memory takes the tile as [activation row][weight row].
+        float* const part = reinterpret_cast<float*>(smem) + (size_t)half * S::kCols * kRows + r;
+#pragma unroll
+        for (int j = 0; j < S::kCols / 2; j++) {
+            float lo, hi;
+            asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(acc[j]));
+            part[(2 * j) * kRows] = lo;
+            part[(2 * j + 1) * kRows] = hi;
+        }
+        pdl_wait();                                               // the row scales, the residual, readers of what the output was
+        tc_fence_before();
+        __syncwarp();
+        if (p.splits > 1) cluster_sync_all(); else asm volatile("bar.sync 1, %0;" ::"n"(kPromoteWarps * 32) : "memory");
+        // ── epilogue: CTA `split` of the cluster finishes every splits-th activation row; a warp stores 128 contiguous bytes ──
+        const int chunks = rowsOut / 32, phases = kPromoteWarps / chunks;      // 4 × 2, or 2 × 4 for SwiGLU
+        const int rc = (warp % chunks) * 32 + lane, no = n0 + rc;
+        const float bv = p.bias != nullptr && no < p.N ? p.bias[no] : 0.0f, bv2 = p.bias2 != nullptr && no < p.N ? p.bias2[no] : 0.0f;
+        const int mEnd = min(NT, p.M - m0);
+        const float* const tile = reinterpret_cast<const float*>(smem) + rc;
+#pragma unroll 4
+        for (int c = split + p.splits * (warp / chunks); c < mEnd; c += p.splits * phases) {
+            const uint32_t at = base + (uint32_t)(c * kRows + rc) * 4;
+            const float rv = p.residual != nullptr && no < p.N ? p.residual[(size_t)(m0 + c) * p.ldr + no] : 0.0f, rs = p.rowscale[m0 + c];
+            float v = 0.0f, u = 0.0f;
+            if (p.splits == 1) {
+                v = tile[c * kRows];
+                if (p.swiglu) u = tile[c * kRows + kRows / 2];
+            } else {
+                for (int z = 0; z < p.splits; z++) {
+                    v += ld_peer(at, (uint32_t)z);
+                    if (p.swiglu) u += ld_peer(at + kRows / 2 * 4, (uint32_t)z);
+                }
+            }
+            v = v * rs + bv;
+            if (p.swiglu) {
+                const float sig = 1.0f / (1.0f + expf(-v));
+                v = (v * sig) * (u * rs + bv2);
+            } else if (p.gelu) v = gelu_ref(v);
+            if (p.residual != nullptr) v += rv;
+            if (no < p.N) p.out[(size_t)(m0 + c) * p.ldo + no] = v;
+        }
+    } else {
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kOtherRegs));
+        if (warp < kPromoteWarps + kConvertWarps) {
+            // ── codes → fp16: thread r of a group owns tile row r; group g takes stages g, g + 2, … ──
+            const int r = tid & 127, grp = (warp - kPromoteWarps) >> 2;
+            const uint32_t wLane = tmem + ((uint32_t)((warp & 3) * 32) << 16) + S::kWBase;
+            int rawAt = -1;                                       // raw group whose arrival has been waited for
+            for (int i = grp; i * S::kPer < nK; i += 2) {
+                const int b = i * S::kPer, g = b / kGroup, j = b % kGroup, rs = g % S::kRawStages, s = i % S::kStages;
+                if (g != rawAt) { warp_wait(rawFull(rs), (g / S::kRawStages) & 1, &s_abort, p.error, 206); rawAt = g; }
+                const unsigned char* src = smem + (size_t)S::kStages * S::kStageBytes + (size_t)rs * kRawBytes + r * 128;
+                uint4 w[2 * S::kPer];
+#pragma unroll
+                for (int q = 0; q < 2 * S::kPer; q++) w[q] = *reinterpret_cast<const uint4*>(src + (((2 * j + q) ^ (r & 7)) << 4));
+                if (i >= S::kStages) warp_wait(empty(s), (i / S::kStages - 1) & 1, &s_abort, p.error, 201);
+                tc_fence_after();
+#pragma unroll
+                for (int q = 0; q < 2 * S::kPer; q++) {           // 16 codes → 8 columns
+                    const uint32_t u4[4] = {w[q].x, w[q].y, w[q].z, w[q].w};
+                    uint32_t h[8];
+#pragma unroll
+                    for (int e = 0; e < 4; e++) {                 // sign flip, byte under exponent 0x64 = 1024 + 128 + code, subtract 1152: exact
+                        const uint32_t u = u4[e] ^ 0x80808080u;
+                        const uint32_t a01 = __byte_perm(u, 0x64646464u, 0x4140), a23 = __byte_perm(u, 0x64646464u, 0x4342);
+                        asm("sub.f16x2 %0, %1, %2;" : "=r"(h[2 * e]) : "r"(a01), "r"(0x64806480u));
+                        asm("sub.f16x2 %0, %1, %2;" : "=r"(h[2 * e + 1]) : "r"(a23), "r"(0x64806480u));
+                    }
+                    tmem_st8(wLane + (uint32_t)(s * S::kWCols + 8 * q), h);
+                }
+                tmem_wait_st();
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) {
+                    mbar_arrive(full(s));
+                    // only now, after this group's last stage of the box: the stores above waited for the raw codes to reach
+                    // registers; released right behind the load instructions, the buffer was refilled under them
+                    if (S::kPer == 2 || j >= 2) mbar_arrive(rawEmpty(rs));
+                }
+            }
+        } else if (warp == kCopyWarp) {
+            pdl_wait();                                           // the images come from the pre-pass
+            const unsigned char* src = p.images + ((size_t)blockIdx.y * p.nS + kt0 / S::kPer) * S::kStageBytes;
+            const int n = (nK + S::kPer - 1) / S::kPer;
+            int i = 0, s = 0;
+            for (uint32_t round = 0; i < n; i++, src += S::kStageBytes) {
+                if (round > 0 && !warp_wait(empty(s), (round - 1) & 1, &s_abort, p.error, 203)) break;
+                if (elect_one()) {
+                    mbar_arrive_expect_tx(full(s), S::kStageBytes);
+                    bulk_g2s(base + s * S::kStageBytes, src, S::kStageBytes, full(s));
+                }
+                __syncwarp();
+                if (++s == S::kStages) { s = 0; round++; }
+            }
+            if (i < n && lane == 0)                               // gave up: let the copies in flight land before the block goes
+                for (int back = i - 1; back >= 0 && back >= i - S::kStages; back--)
+                    for (unsigned w = 0; w < (1u << 16) && !mbar_try_wait(full(back % S::kStages), (back / S::kStages) & 1); w++) {}
+        } else if (warp >= kMmaWarp) {
+            const bool lo = p.lo != 0;
+            // One thread's instructions are this loop's length, so stage and accumulator numbers are compile-time constants: the
+            // descriptors become immediates on top of two uniform registers.
+            const int which = warp - kMmaWarp;
+            const uint32_t d0 = __shfl_sync(0xffffffffu, tmem, 0);
+            const uint64_t x0 = S::kDesc | (base >> 4);
+            bool ok = true;
+            for (uint32_t it = 0; it * (S::kStages * S::kPer) < (uint32_t)nK && ok; it++) {
+#pragma unroll
+                for (int u2 = 0; u2 < S::kStages; u2 += 2) {
+                    const int u = u2 + which;
+                    const int b = (int)it * S::kStages * S::kPer + u * S::kPer;
+                    if (b >= nK) break;
+                    static_assert(S::kSlots == 2 || (S::kSlots == 4 && S::kStages == 4), "a slot belongs to one issuing warp");
+                    const int a = u % S::kSlots;
+                    const uint32_t aRound = it * (S::kStages / S::kSlots) + u2 / S::kSlots;         // earlier uses of this accumulator
+                    ok = (aRound == 0 || warp_wait(accEmpty(a), (aRound - 1) & 1, &s_abort, p.error, 204)) &&
+                         warp_wait(full(u), it & 1, &s_abort, p.error, 205);
+                    if (!ok) break;
+                    tc_fence_after();
+                    if (elect_one()) {
+#pragma unroll
+                        for (int j = 0; j < S::kPer; j++) {
+                            if (j > 0 && b + j >= nK) break;
+                            // a block is 16 columns of the codes and 64 bytes of an activation row, a k-step of 16 half of that
+                            const uint32_t w = d0 + (uint32_t)(S::kWBase + u * S::kWCols + 16 * j);
+                            const uint64_t xh = x0 + (uint32_t)(u * S::kStageBytes / 16 + 4 * j), xl = xh + S::kXBytes / 16;
+                            const uint32_t d = d0 + (uint32_t)((a * S::kPer + j) * S::kAccStride);
+                            umma_f16_ts(d, w, xh, S::kIdesc, 0);
+                            umma_f16_ts(d, w + 8, xh + 2, S::kIdesc, 1);
+                            if (lo) {
+                                umma_f16_ts(d, w, xl, S::kIdesc, 1);
+                                umma_f16_ts(d, w + 8, xl + 2, S::kIdesc, 1);
+                            }
+                        }
+                        umma_commit(accFull(a));
+                        umma_commit(empty(u));
+                    }
+                    __syncwarp();
+                }
+            }
+        } else if (warp == kRawWarp) {
+            const int nG = (nK + kGroup - 1) / kGroup;            // weights depend on no earlier kernel: no wait before them
+            int g = 0, s = 0;
+            for (uint32_t round = 0; g < nG; g++) {
+                if (round > 0 && !warp_wait(rawEmpty(s), (round - 1) & 1, &s_abort, p.error, 207)) break;
+                if (elect_one()) {
+                    const uint32_t dst = rawBase + s * kRawBytes;
+                    const int kx = (kt0 + g * kGroup) * kBlockK;
+                    mbar_arrive_expect_tx(rawFull(s), kRawBytes);
+                    tma_box(dst, &p.codes, kx, n0, rawFull(s));
+                    if (p.swiglu) tma_box(dst + kRawBytes / 2, &p.codes2, kx, n0, rawFull(s));
+                }
+                __syncwarp();
+                if (++s == S::kRawStages) { s = 0; round++; }
+            }
+            if (g < nG && lane == 0)
+                for (int back = g - 1; back >= 0 && back >= g - S::kRawStages; back--)
+                    for (unsigned w = 0; w < (1u << 16) && !mbar_try_wait(rawFull(back % S::kRawStages), (back / S::kRawStages) & 1); w++) {}
         }
         __syncwarp();
+        pdl_wait();
+        if (p.splits > 1) cluster_sync_all();
     }
-    __syncthreads();
-    if (warp == kDqWarps) { tc_fence_after(); tmem_dealloc(tmem_base, kTmemCols); }
+    __syncwarp();
+    if (p.splits > 1) cluster_sync_all(); else __syncthreads();   // peers have read this CTA's part
+    if (warp == kMmaWarp) { tc_fence_after(); tmem_dealloc(tmem, 512); }
 }
 
-constexpr size_t kTcSmem = (size_t)kARegionBytes + (size_t)kStagesB * kStageBBytes + (size_t)kTileN * kRawRow + 1024;
+// ───────────── layout of a launch ─────────────
+struct TcPlan { int nt, mTiles, nTiles, splits, ktPer; double us; };
 
-// Adds the partial outputs of a K-split launch in split order and runs the epilogue that the GEMM kernel runs itself
-// when the reduction is not split: out = Σ + bias (+ residual), or out = SiLU(out) · (Σ + bias) for SwiGLU's second GEMM.
-__global__ void __launch_bounds__(256) k_q8_tc_split_reduce(const float* __restrict__ part, size_t splitStride, int splits, int M, int N,
-                                                            const float* __restrict__ bias, const float* __restrict__ residual, int ldr,
-                                                            float* __restrict__ out, int ldo, int mode) {
-    pdl_wait();
-    pdl_launch_dependents();
-    const size_t total = (size_t)M * N;
-    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
-        const int m = (int)(i / N), n = (int)(i - (size_t)m * N);
-        float v = 0.0f;
-        for (int z = 0; z < splits; z++) v += __ldcg(part + (size_t)z * splitStride + i);
-        if (bias) v += bias[n];
-        float* o = out + (size_t)m * ldo + n;
-        if (mode == 0) {
-            if (residual) v += residual[(size_t)m * ldr + n];
-            *o = v;
-        } else {
-            const float gte = *o;
-            const float sig = 1.0f / (1.0f + expf(-gte));
-            *o = (gte * sig) * v;
+// Tile width and reduction split with the least estimated time.
+TcPlan tc_plan(int M, int K, int N, bool swiglu) {
+    const int nK = (K + kBlockK - 1) / kBlockK, rowsOut = swiglu ? kRows / 2 : kRows;
+    const int nTiles = (N + rowsOut - 1) / rowsOut;
+    TcPlan best = {}; best.us = 1e30;
+    for (int nt : {16, 32, 64, 96, 128, 160, 192}) {
+        const int mTiles = (M + nt - 1) / nt;
+        const double perBlock = nt >= 64 ? 0.045 + 0.00105 * nt : 0.11;          // µs per 32-k block
+        for (int sp = 1; sp <= kMaxSplits; sp *= 2) {
+            const int ktPer = ((nK + sp - 1) / sp + kGroup - 1) / kGroup * kGroup;
+            if (sp > 1 && (sp - 1) * ktPer >= nK) continue;                       // a CTA without blocks
+            const int slots = sp == 1 ? g_num_sms : g_num_sms * 15 / 16 / sp * sp;   // clusters leave some SMs of a GPC unused
+            const long ctas = (long)mTiles * nTiles * sp;
+            const long rounds = (ctas + slots - 1) / slots;
+            const double us = (double)rounds * (perBlock * ktPer + 2.0 + 0.012 * nt + (sp > 1 ? 1.0 + 0.004 * nt : 0.0)) + 4.0;
+            if (us < best.us) best = {nt, mTiles, nTiles, sp, ktPer, us};
         }
     }
+    return best;
 }
 
-// How a launch is laid out: CTAs take one 128-row tile or a pair, and when that leaves most SMs without a tile (a few
-// dozen to a few hundred rows) the reduction is split over up to four CTAs whose partial outputs a small kernel adds.
-struct TcPlan { bool pair; int splits, ktPer; long ctas; };
-TcPlan tc_plan(int M, int K, int N) {
-    const long mTiles = (M + kTileM - 1) / kTileM, nTiles = (N + kTileN - 1) / kTileN;
-    const int nK = K / kTileK;
-    // Two accumulators per CTA halve the conversion work per flop but also the number of CTAs, and a paired CTA
-    // takes 1.55–1.7 × as long as a single one: pair when the rounds of CTAs over the SMs it saves outweigh that.
-    const long single = nTiles * mTiles, paired = nTiles * ((mTiles + 1) / 2);
-    const long roundsSingle = (single + g_num_sms - 1) / g_num_sms, roundsPaired = (paired + g_num_sms - 1) / g_num_sms;
-    TcPlan pl;
-    pl.pair = mTiles >= 2 && 1.7 * (double)roundsPaired < (double)roundsSingle;
-    pl.ctas = pl.pair ? paired : single;
-    pl.splits = 1;
-    if (M <= 256 && 2 * pl.ctas <= g_num_sms) {
-        int sp = (int)(g_num_sms / pl.ctas);
-        if (sp > 4) sp = 4;
-        while (sp > 1 && nK / sp < 16) sp--;              // at least 16 k-tiles (512 k) per split
-        pl.splits = sp;
+bool encode_codes(const Q8View& w, int rows, CUtensorMap* map) {
+    EncodeTiledFn enc = encode_tiled_fn();
+    if (!enc || ((uintptr_t)w.codes & 15) != 0 || w.Kp % 16 != 0) return false;
+    const cuuint64_t dims[2] = {(cuuint64_t)w.Kp, (cuuint64_t)w.N};
+    const cuuint64_t strides[1] = {(cuuint64_t)w.Kp};
+    const cuuint32_t box[2] = {(cuuint32_t)(kBlockK * kGroup), (cuuint32_t)rows};
+    const cuuint32_t estr[2] = {1u, 1u};
+    return enc(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<int8_t*>(w.codes), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+               CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+template <int NT> void run(const TcParams& p, const TcPlan& pl, cudaStream_t s) {
+    using S = TileShape<NT>;
+    static bool attr = false;
+    if (!attr) {
+        DJ_CUDA_CHECK(cudaFuncSetAttribute(k_q8_gemm_tc<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::kSmem));
+        attr = true;
     }
-    pl.ktPer = ((nK + pl.splits - 1) / pl.splits + 3) / 4 * 4;      // whole groups of four k-tiles (the raw-code buffer's unit)
-    pl.splits = (nK + pl.ktPer - 1) / pl.ktPer;
-    return pl;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)pl.splits, (unsigned)pl.mTiles, (unsigned)pl.nTiles);
+    cfg.blockDim = dim3(kTcThreads);
+    cfg.dynamicSmemBytes = S::kSmem;
+    cfg.stream = s;
+    cudaLaunchAttribute at[2];
+    int n = 0;
+    if (pl.splits > 1) {
+        at[n].id = cudaLaunchAttributeClusterDimension;
+        at[n].val.clusterDim.x = (unsigned)pl.splits; at[n].val.clusterDim.y = 1; at[n].val.clusterDim.z = 1;
+        n++;
+    }
+    if (g_use_pdl) { at[n].id = cudaLaunchAttributeProgrammaticStreamSerialization; at[n].val.programmaticStreamSerializationAllowed = 1; n++; }
+    cfg.attrs = at;
+    cfg.numAttrs = (unsigned)n;
+    g_launches++;
+    DJ_CUDA_CHECK(cudaLaunchKernelEx(&cfg, k_q8_gemm_tc<NT>, p));
 }
 
 }  // namespace
 
 int g_tc_terms = 3;
 
-// Rough duration of launch_q8_linear_tc in µs, for the choice between this path and passes of the 16-row kernel
-// when M is small: a CTA needs ≈ 0.75 µs per 32-k tile (1.2 µs when it carries two accumulators), CTAs run in
-// rounds over the SMs, the activation pre-pass costs a few µs, and a split reduction adds its small second kernel.
-double q8_tc_estimate_us(int M, int K, int N) {
-    const TcPlan pl = tc_plan(M, K, N);
-    const long rounds = (pl.ctas * pl.splits + g_num_sms - 1) / g_num_sms;
-    // 0.75 µs per k-tile measured with one wave of a few dozen CTAs, 0.95 µs with the ≈ 144 CTAs of a split launch
-    const double perCta = (pl.pair ? 1.2 : pl.splits > 1 ? 0.95 : 0.75) * pl.ktPer;
-    double t = perCta * rounds + 5.0;
-    if (pl.splits > 1) t += 4.0 + (double)pl.splits * M * N * 8.0 / 3.0e6;      // partial outputs written and read back at ≈ 3 TB/s
-    return t;
+double q8_tc_estimate_us(int M, int K, int N, bool swiglu) { return tc_plan(M, K, N, swiglu).us; }
+
+size_t q8_tc_ws_floats(int M, int K, int N, bool swiglu) {
+    const TcPlan pl = tc_plan(M, K, N, swiglu);
+    const size_t mPad = (size_t)pl.nt * pl.mTiles, nK = ((size_t)(K + kBlockK - 1) / kBlockK + 1) / 2 * 2;
+    return nK * mPad * kBlockK + mPad;          // hi + lo halves = 4 bytes per value, then the row scales
 }
 
-size_t q8_tc_ws_floats(int M, int K, int N) {
-    const size_t mPad = (size_t)(M + kTileM - 1) / kTileM * kTileM;
-    const TcPlan pl = tc_plan(M, K, N);
-    return mPad * K + mPad + (pl.splits > 1 ? (size_t)pl.splits * M * N : 0);          // hi + lo halves = 4 bytes per value, the row scales, the splits' partial outputs
-}
-
-// out = x · W (+ fused norm / bias / residual / SiLU-gate) for M ≥ 1 rows on the tensor cores.
-// Returns false when the shape is outside the kernel's domain (K must be a multiple of 128).
+// out = x · W (+ fused norm / bias / residual / GELU / SiLU-gate) for M ≥ 1 rows on the tensor cores.
+// Returns false when the shape is outside the kernel's domain.
 bool launch_q8_linear_tc(const Q8LinearArgs& a, float* ws, cudaStream_t s) {
     const int K = a.w.K, N = a.w.N, M = a.M;
-    if (K % 128 != 0 || a.w.Kp != K || ws == nullptr || M < 1) return false;      // raw codes travel four k-tiles (and their 4 scales = 16 bytes) at a time
-    if (((uintptr_t)a.x & 15) != 0 || a.ldx % 4 != 0 || (a.gamma && ((uintptr_t)a.gamma & 15) != 0)) return false;
-    static bool attrSet = false;
-    if (!attrSet) {
-        DJ_CUDA_CHECK(cudaFuncSetAttribute(k_q8_gemm_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTcSmem));
-        attrSet = true;
+    const bool swiglu = a.w2.codes != nullptr;
+    if (ws == nullptr || ((uintptr_t)ws & 127) != 0 || M < 1 || K % 4 != 0 || g_dev_error == nullptr) return false;
+    if (((uintptr_t)a.x & 15) != 0 || a.ldx % 4 != 0 || ((uintptr_t)a.gamma & 15) != 0 || ((uintptr_t)a.beta & 15) != 0) return false;
+    if (a.w.nb % 4 == 0 && (((uintptr_t)a.w.scales & 15) != 0 || (swiglu && ((uintptr_t)a.w2.scales & 15) != 0))) return false;
+    if (swiglu && a.act != 0) return false;
+    TcParams p = {};
+    if (!encode_codes(a.w, swiglu ? kRows / 2 : kRows, &p.codes) || (swiglu && !encode_codes(a.w2, kRows / 2, &p.codes2))) return false;
+    const TcPlan pl = tc_plan(M, K, N, swiglu);
+    if (pl.nTiles > 65535 || pl.mTiles > 65535) return false;
+    const int per = blocks_per_stage(pl.nt);
+    p.nK = (K + kBlockK - 1) / kBlockK; p.nS = (p.nK + per - 1) / per; p.nb = a.w.nb;
+    unsigned char* const images = reinterpret_cast<unsigned char*>(ws);
+    float* const rowscale = ws + (size_t)p.nS * per * kBlockK * pl.nt * pl.mTiles;
+    launch_k(k_x_images, dim3((unsigned)M), dim3(kXThreads), 0, s, true, a.x, a.ldx, a.gamma, a.beta, a.eps, K, p.nS, pl.nt, per, images, rowscale);
+    p.images = images; p.rowscale = rowscale;
+    p.scales = a.w.scales; p.scales2 = a.w2.scales; p.bias = a.bias; p.bias2 = a.bias2;
+    p.residual = a.residual; p.ldr = a.ldr; p.out = a.out; p.ldo = a.ldo;
+    p.M = M; p.N = N; p.swiglu = swiglu; p.gelu = a.act == 1;
+    p.splits = pl.splits; p.ktPer = pl.ktPer; p.lo = g_tc_terms & 1; p.coarse = (g_tc_terms & 2) == 0; p.error = g_dev_error;
+    switch (pl.nt) {
+        case 16: run<16>(p, pl, s); break;
+        case 32: run<32>(p, pl, s); break;
+        case 64: run<64>(p, pl, s); break;
+        case 96: run<96>(p, pl, s); break;
+        case 128: run<128>(p, pl, s); break;
+        case 160: run<160>(p, pl, s); break;
+        default: run<192>(p, pl, s); break;
     }
-    const int mTiles = (M + kTileM - 1) / kTileM, nTiles = (N + kTileN - 1) / kTileN;
-    const size_t mPad = (size_t)mTiles * kTileM;
-    unsigned char* tiles = reinterpret_cast<unsigned char*>(ws);
-    float* rowscale = ws + mPad * K;
-    float* part = rowscale + mPad;
-    launch_k(k_x_to_f16_tiles, dim3((unsigned)(mPad / 8)), dim3(256), 0, s, true, a.x, a.ldx, a.gamma, a.eps, M, K, tiles, rowscale);
-    const TcPlan pl = tc_plan(M, K, N);
-    const bool split = pl.splits > 1;
-    const dim3 grid(nTiles, pl.pair ? (mTiles + 1) / 2 : mTiles, pl.splits);
-    const int redBlocks = (int)(((size_t)M * N + 255) / 256 < (size_t)(4 * g_num_sms) ? ((size_t)M * N + 255) / 256 : (size_t)(4 * g_num_sms));
-    TcParams p;
-    p.xtiles = tiles; p.rowscale = rowscale;
-    p.M = M; p.N = N; p.K = K; p.Kp = a.w.Kp; p.nb = a.w.nb; p.mTiles = mTiles; p.pair = pl.pair ? 1 : 0;
-    p.ktPer = pl.ktPer; p.splitStride = split ? (size_t)M * N : 0;
-    p.terms = g_tc_terms; p.error = g_dev_error; p.trace = trace_slot();
-    auto run = [&](const Q8View& w, const float* bias, const float* residual, int mode) {
-        p.codes = w.codes; p.scales = w.scales;
-        if (split) {
-            // raw partial sums per split, the epilogue in the reduce kernel
-            p.bias = nullptr; p.residual = nullptr; p.ldr = 0; p.out = part; p.ldo = N; p.mode = 0;
-            launch_k(k_q8_gemm_tc, grid, dim3(kTcThreads), kTcSmem, s, true, p);
-            launch_k(k_q8_tc_split_reduce, dim3(redBlocks), dim3(256), 0, s, true, (const float*)part, p.splitStride, pl.splits, M, N, bias,
-                     residual, a.ldr, a.out, a.ldo, mode);
-        } else {
-            p.bias = bias; p.residual = residual; p.ldr = a.ldr; p.out = a.out; p.ldo = a.ldo; p.mode = mode;
-            launch_k(k_q8_gemm_tc, grid, dim3(kTcThreads), kTcSmem, s, true, p);
-        }
-    };
-    run(a.w, a.bias, a.residual, 0);
-    // SwiGLU: the gate projection is in `out`; the up projection's epilogue multiplies SiLU(gate) into it
-    if (a.w2.codes != nullptr) run(a.w2, a.bias2, nullptr, 1);
     return true;
 }
 
 }  // namespace dj
 
-// Which of the two fp16 correction products the tensor-core GEMM issues on top of x_hi · w_hi: bit 0 = x_lo · w_hi,
-// bit 1 = x_hi · w_lo.  3 (the default) carries ≈ 22 bits of both operands; 1, 2 and 0 trade bits for tensor-pipe time
-// (and, without bit 1, for half of the dequantisation stores).  Drops the cached CUDA graphs, which hold the old value.
+// Precision of the many-row path: bit 0 adds the X_lo product (activations at ≈ 22 bits, else 11), bit 1 keeps the block
+// scales in fp32 (else they are rounded to 11 bits).  Drops the cached CUDA graphs, which hold the old value.
 extern "C" int deepj_cuda_tc_configure(int32_t correction_terms) {
     if (correction_terms < 0 || correction_terms > 3) { dj::set_last_error("tc_configure: correction_terms must be 0..3"); return 1; }
     if (dj::g_tc_terms != correction_terms) { dj::g_tc_terms = correction_terms; dj::invalidate_graphs(); }
