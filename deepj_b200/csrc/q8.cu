@@ -316,14 +316,35 @@ void launch_gelu_rows(float* buf, int ld, int N, int M, cudaStream_t s) {
 
 namespace {
 void dispatch_q8_linear(const Q8LinearArgs& a, cudaStream_t s);
+
+bool batch_qualifies(const Q8LinearArgs& a) { return g_gemv_mode >= 1 && a.M >= 5 && a.ws != nullptr && a.w.K % 32 == 0 && a.w.Kp == a.w.K; }
+
+// Whether the tensor-core kernel is tried first.  Passes of the 16-row kernel against it, by estimated time: a pass of the TMA
+// kernel costs ≈ 7 µs + 0.33 ps per weight (measured: 12.1 µs at 4096 × 4096, 22.6 at 4096 × 12288, 33.7 for a pair of 4096 × 11008,
+// where the tensor-core kernel takes 13.7, 32 and 52), one of the cp.async kernel (K no multiple of 128) 13 µs up to 16 M weights
+// and 0.8 ps per weight beyond (13.4 µs at 1600 × 1600, 14.9 at 1600 × 4800, 36 at 4096 × 11008; the tensor-core kernel takes
+// 6-9 µs where its grid is one short round).
+bool runs_tc(const Q8LinearArgs& a) {
+    static const bool noTc = getenv("DEEPJ_CUDA_NO_TC") != nullptr;
+    if (g_gemv_mode < 1 || noTc || a.M < kTcMinRows || a.ws == nullptr) return false;
+    if (!batch_qualifies(a) || a.M > 256) return true;
+    const bool swiglu = a.w2.codes != nullptr, tmaKernel = g_gemv_mode == 2 && a.w.K % 128 == 0;
+    const double weights = (double)a.w.K * (double)a.w.N * (swiglu ? 2.0 : 1.0);
+    const double perPassUs = tmaKernel ? 7.0 + 0.33e-6 * weights : weights < 16e6 ? 13.0 : 0.8e-6 * weights;
+    const int rem = a.M % 16;
+    const double passes = (double)(a.M / 16) + (rem == 0 ? 0.0 : rem <= 8 ? 0.75 : 1.0);      // a last pass of up to eight rows issues half the MMAs
+    return passes * perPassUs >= q8_tc_estimate_us(a.M, a.w.K, a.w.N, swiglu);
+}
 }
 
 void launch_q8_linear(const Q8LinearArgs& a0, cudaStream_t s) {
     if (a0.M <= 0 || a0.w.N <= 0) return;
     if (a0.beta == nullptr && a0.act == 0) { dispatch_q8_linear(a0, s); return; }
-    // GPT blocks: up to four rows go through the GEMV, which takes LayerNorm and GELU itself; the many-row
+    // GPT blocks: up to four rows go through the GEMV, which takes LayerNorm and GELU itself; the 16-row
     // kernels see already normalised rows and get the activation applied to their output afterwards
     if (g_gemv_mode >= 1 && a0.M < 5 && q8_gemv_i8_fuses_gpt(a0)) { dispatch_q8_linear(a0, s); return; }
+    // the tensor-core kernel normalises in its pre-pass and activates in its epilogue; the 16-row kernel cannot
+    if (runs_tc(a0) && launch_q8_linear_tc(a0, a0.ws, s)) return;
     Q8LinearArgs a = a0;
     if (a.beta != nullptr) {
         if (a.ln_ws == nullptr) throw std::runtime_error("Q8 linear: LayerNorm needs its workspace");
@@ -348,20 +369,8 @@ void dispatch_q8_linear(const Q8LinearArgs& a, cudaStream_t s) {
     p.out = a.out; p.ldo = a.ldo;
     p.K = a.w.K; p.N = a.w.N; p.Kp = a.w.Kp; p.nb = a.w.nb;
     const bool swiglu = a.w2.codes != nullptr;
-    static const bool noTc = getenv("DEEPJ_CUDA_NO_TC") != nullptr;
-    const bool batchOk = g_gemv_mode >= 1 && a.M >= 5 && a.ws != nullptr && a.w.K % 32 == 0 && a.w.Kp == a.w.K;
-    // A few dozen rows leave most SMs without a 128 × 256 tile: passes of the 16-row kernel (≈ 3 µs + 0.5 ps per weight
-    // and pass with the TMA kernel, 0.9 ps with the cp.async one; measured on 4096 × 12288, 11008 × 4096 and 4096 × 4096)
-    // win until the tensor-core grid fills up.
-    bool preferBatch = false;
-    if (batchOk && a.M >= kTcMinRows && a.M <= 256) {
-        const bool tmaKernel = g_gemv_mode == 2 && a.w.K % 128 == 0;
-        const double perPassUs = tmaKernel ? 3.0 + 0.5e-6 * (double)a.w.K * (double)a.w.N : 0.9e-6 * (double)a.w.K * (double)a.w.N;
-        const int rem = a.M % 16;
-        const double passes = (double)(a.M / 16) + (rem == 0 ? 0.0 : rem <= 8 ? 0.75 : 1.0);      // a last pass of up to eight rows issues half the MMAs
-        preferBatch = passes * perPassUs < q8_tc_estimate_us(a.M, a.w.K, a.w.N, swiglu);
-    }
-    if (g_gemv_mode >= 1 && !noTc && !preferBatch && a.M >= kTcMinRows && a.ws != nullptr && launch_q8_linear_tc(a, a.ws, s)) return;
+    const bool batchOk = batch_qualifies(a);
+    if (runs_tc(a) && launch_q8_linear_tc(a, a.ws, s)) return;
     if (batchOk) {
         // five or more rows share one pass over the weights, 16 at a time (up to four are two GEMV passes, which is as fast)
         bool ok = true;

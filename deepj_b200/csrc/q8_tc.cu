@@ -14,14 +14,15 @@
 // tensor-memory lane = one weight row, so its block scale is one register and its result rows are stored 128 contiguous
 // bytes at a time.  The fp16 codes go to tensor memory too and enter the MMAs from there: with them in shared memory the
 // converters' stores and the MMAs' operand reads together asked for its whole 128 bytes a cycle (measured: 8 MMAs of
-// 128 × 64 × 16 took 780 cycles beside the converters and 392 alone).  20 warps:
-//   warps 0-7    read the block's accumulator (tcgen05.ld, 32 lanes × NT/2 columns each) and add it to registers;
-//                afterwards the epilogue
-//   warps 8-15   convert, as two groups of four that take the stages in turn: one weight row per thread, 32 codes → 64 bytes
+// 128 × 64 × 16 took 780 cycles beside the converters and 392 alone).  28 warps:
+//   warps 0-15   read the block's accumulator (tcgen05.ld, 32 lanes × NT/4 columns each) and add it to registers; afterwards
+//                the epilogue.  Half the time of such a step is the latency of its barrier and loads, so four warps per
+//                scheduler share it (eight warps of NT/2 columns: 832 cycles per pair of blocks at NT = 96)
+//   warps 16-23  convert, as two groups of four that take the stages in turn: one weight row per thread, 32 codes → 64 bytes
 //                of fp16 per block, stored to its lane
-//   warp 16      copies the activation images (one plain bulk copy per stage)
-//   warp 17      streams the raw codes: 128-byte × 128-row boxes through the tensor-memory accelerator
-//   warps 18-19  issue the MMAs (128 × NT × 16, four per block) into a ring of accumulators and commit, taking the stages in
+//   warp 24      copies the activation images (one plain bulk copy per stage)
+//   warp 25      streams the raw codes: 128-byte × 128-row boxes through the tensor-memory accelerator
+//   warps 26-27  issue the MMAs (128 × NT × 16, four per block) into a ring of accumulators and commit, taking the stages in
 //                turn: the waits and commits of one stage cost an issuing thread ≈ 400 cycles, in which the other one issues
 // SwiGLU takes 64 gate and 64 up rows per tile, so the pair meets in one epilogue.  When the grid leaves SMs idle the
 // reduction is split over the CTAs of a cluster, which add their parts through distributed shared memory in split order.
@@ -39,12 +40,12 @@ constexpr int kRows = 128;                               // weight rows of a til
 constexpr int kBlockK = 32;                              // one scale block
 constexpr int kGroup = 4;                                // blocks per raw-code box: 128 bytes of a weight row
 constexpr int kRawBytes = kRows * kBlockK * kGroup;      // raw codes of one group: 16 KB
-constexpr int kPromoteWarps = 8, kConvertWarps = 8;      // converters: two groups of four
+constexpr int kPromoteWarps = 16, kConvertWarps = 8;      // converters: two groups of four
 constexpr int kCopyWarp = kPromoteWarps + kConvertWarps, kRawWarp = kCopyWarp + 1, kMmaWarp = kCopyWarp + 2;   // two MMA warps
-constexpr int kTcThreads = 640;
+constexpr int kTcThreads = 896;
 constexpr int kMaxSplits = 8;                            // portable cluster size
-// Registers: 640 threads × 96 at launch; 256 × 168 + 384 × 48 = 61440 afterwards.
-constexpr int kPromoteRegs = 168, kOtherRegs = 48;
+// Registers: 896 threads × 72 at launch; 512 × 88 + 384 × 48 = 63488 afterwards.
+constexpr int kPromoteRegs = 88, kOtherRegs = 48;
 
 // Below 128 activation rows a block's products take less time than the barriers around them: a pipeline stage then holds two
 // blocks (rows of 128 bytes, 128-byte swizzle) and accumulators are handed over in pairs.
@@ -60,7 +61,7 @@ template <int NT> struct TileShape {
     static constexpr int kAccStride = NT < 32 ? 32 : NT;
     static constexpr int kSlots = kPer == 2 && NT <= 32 ? 4 : 2;
     static constexpr int kWCols = 16 * kPer, kWBase = kSlots * kPer * kAccStride;
-    static constexpr int kCols = NT / 2;                             // accumulator columns per promoting warp
+    static constexpr int kCols = NT / 4;                             // accumulator columns per promoting warp
     static constexpr size_t kPipe = (size_t)kStages * kStageBytes + (size_t)kRawStages * kRawBytes;
     static constexpr size_t kSmem = kPipe + 1024;
     static constexpr uint32_t kIdesc = (1u << 4) | ((uint32_t)(NT >> 3) << 17) | ((uint32_t)(kRows >> 4) << 24);   // fp16 × fp16 → fp32, K-major
@@ -82,15 +83,21 @@ __device__ __forceinline__ uint32_t pack_h2(float lo, float hi) {
     return r;
 }
 
-__device__ __forceinline__ void tmem_ld16_nowait(uint32_t taddr, uint32_t* v) {
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-                 : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]), "=r"(v[9]),
-                   "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
-                 : "r"(taddr));
-}
-__device__ __forceinline__ void tmem_ld8_nowait(uint32_t taddr, uint32_t* v) {
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
-                 : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]) : "r"(taddr));
+// NC consecutive columns of the warp's 32 lanes → v, asynchronously
+template <int NC> __device__ __forceinline__ void tmem_ld_nowait(uint32_t taddr, uint32_t* v) {
+    if constexpr (NC >= 16) {
+        asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+                     : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]), "=r"(v[9]),
+                       "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
+                     : "r"(taddr));
+        if constexpr (NC > 16) tmem_ld_nowait<NC - 16>(taddr + 16, v + 16);
+    } else if constexpr (NC == 8) {
+        asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                     : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]) : "r"(taddr));
+    } else {
+        static_assert(NC == 4, "columns come in fours, eights and sixteens");
+        asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];" : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]) : "r"(taddr));
+    }
 }
 __device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 __device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint32_t (&v)[8]) {
@@ -116,6 +123,13 @@ __device__ __forceinline__ void fma2(unsigned long long& acc, uint32_t v0, uint3
 __device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag, int* error, int code) {
     if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
     return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag, error, code));
+}
+// Whether a phase is over, without waiting for it.
+__device__ __forceinline__ bool mbar_test(uint32_t bar, uint32_t parity) {
+    uint32_t ok;
+    asm volatile("{\n .reg .pred p;\n mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}"
+                 : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
+    return ok != 0;
 }
 __device__ __forceinline__ bool elect_one() {
     uint32_t p;
@@ -298,78 +312,72 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_q8_gemm_tc(const __grid_const
 
     if (warp < kPromoteWarps) {
         asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kPromoteRegs));
-        const int quarter = warp & 3, half = warp >> 2;
+        const int quarter = warp & 3, part = warp >> 2;
         const int r = quarter * 32 + lane;                        // tile row = tensor-memory lane
         const bool second = p.swiglu && r >= kRows / 2;
         const int n = min(n0 + (second ? r - kRows / 2 : r), p.N - 1);
         const float* const srow = (second ? p.scales2 : p.scales) + (size_t)n * p.nb;
         const bool vec = (p.nb & 3) == 0;
-        const uint32_t lane_base = tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(half * S::kCols);
+        const uint32_t lane_base = tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(part * S::kCols);
         unsigned long long acc[S::kCols / 2];
 #pragma unroll
         for (int j = 0; j < S::kCols / 2; j++) acc[j] = 0ull;
         float4 next = load_scales(srow, kt0, p.nb, vec, p.coarse);
-        bool ok = true;
-        int slot = 0;
-        uint32_t round = 0;
-        for (int b0 = 0; b0 < nK && ok; b0 += kGroup) {
+        // accumulator and phase parity of the i-th block of group g
+        auto slot_of = [](int g, int i) { return S::kSlots == 4 ? (g & 1) * 2 + i / 2 : i / S::kPer % 2; };
+        auto parity_of = [](int g, int i) { return (uint32_t)(S::kSlots == 4 ? g >> 1 : S::kPer == 2 ? g : i >> 1) & 1u; };
+        auto add = [&](const uint32_t* v, float sc) {
+            unsigned long long ss;
+            asm("mov.b64 %0, {%1, %1};" : "=l"(ss) : "f"(sc));
+#pragma unroll
+            for (int j = 0; j < S::kCols / 2; j++) fma2(acc[j], v[2 * j], v[2 * j + 1], ss);
+        };
+        bool ok = true, ready = false;                            // ready: the next accumulator was seen complete already
+        for (int g = 0, b0 = 0; b0 < nK && ok; g++, b0 += kGroup) {
             const float4 cur = next;
             if (b0 + kGroup < nK) next = load_scales(srow, kt0 + b0 + kGroup, p.nb, vec, p.coarse);
 #pragma unroll
             for (int i = 0; i < kGroup; i += S::kPer) {
                 if (b0 + i >= nK) break;
-                ok = warp_wait(accFull(slot), round & 1, &s_abort, p.error, 202);
+                const int slot = slot_of(g, i);
+                if (!__all_sync(0xffffffffu, ready)) ok = warp_wait(accFull(slot), parity_of(g, i), &s_abort, p.error, 202);
                 if (!ok) break;
                 tc_fence_after();
                 const uint32_t from = lane_base + (uint32_t)(slot * S::kPer * S::kAccStride);
-                // 32 columns at a time (16, 8 where registers or columns are short), the next piece on its way while this one is added
-                constexpr int kStep = S::kCols % 32 == 0 && S::kCols <= 64 ? 32 : S::kCols % 16 == 0 ? 16 : 8;
-                constexpr int kPieces = S::kPer * S::kCols / kStep;
-                const int pieces = S::kPer == 2 && b0 + i + 1 >= nK ? kPieces / 2 : kPieces;       // an odd last block
-                uint32_t v[2][kStep];
-                auto load = [&](int q) {
-                    const uint32_t at = from + (uint32_t)((q * kStep / S::kCols) * S::kAccStride + q * kStep % S::kCols);
-                    if constexpr (kStep == 8) tmem_ld8_nowait(at, v[q & 1]); else tmem_ld16_nowait(at, v[q & 1]);
-                    if constexpr (kStep == 32) tmem_ld16_nowait(at + 16, v[q & 1] + 16);
-                };
-                load(0);
-#pragma unroll
-                for (int q = 0; q < kPieces; q++) {
-                    if (q < pieces) {
-                        tmem_wait_ld();
-                        if (q + 1 < pieces) load(q + 1);
-                        else {                                    // everything is read: the MMAs may write here again
-                            tc_fence_before();
-                            __syncwarp();
-                            if (lane == 0) mbar_arrive(accEmpty(slot));
-                        }
-                        const int blk = i + q * kStep / S::kCols;
-                        const float sc = blk == 0 ? cur.x : blk == 1 ? cur.y : blk == 2 ? cur.z : cur.w;
-                        unsigned long long ss;
-                        asm("mov.b64 %0, {%1, %1};" : "=l"(ss) : "f"(sc));
-#pragma unroll
-                        for (int j = 0; j < kStep / 2; j++) fma2(acc[(q * kStep % S::kCols) / 2 + j], v[q & 1][2 * j], v[q & 1][2 * j + 1], ss);
-                    }
+                const bool both = S::kPer == 2 && b0 + i + 1 < nK;                    // not an odd last block
+                uint32_t v[S::kPer][S::kCols];
+                tmem_ld_nowait<S::kCols>(from, v[0]);
+                tmem_wait_ld();
+                if (both) {
+                    tmem_ld_nowait<S::kCols>(from + S::kAccStride, v[S::kPer - 1]);
+                    add(v[0], i == 0 ? cur.x : i == 1 ? cur.y : i == 2 ? cur.z : cur.w);
+                    tmem_wait_ld();
                 }
-                if (++slot == S::kSlots) { slot = 0; round++; }
+                tc_fence_before();                                // everything is read: the MMAs may write here again
+                __syncwarp();
+                if (lane == 0) mbar_arrive(accEmpty(slot));
+                const int gn = i + S::kPer == kGroup ? g + 1 : g, in = (i + S::kPer) % kGroup;
+                ready = mbar_test(accFull(slot_of(gn, in)), parity_of(gn, in));
+                if (both) add(v[S::kPer - 1], i == 0 ? cur.y : cur.w);
+                else add(v[0], i == 0 ? cur.x : i == 1 ? cur.y : i == 2 ? cur.z : cur.w);
             }
         }
         // Every MMA of this CTA has completed (its last commits have been waited for) and every copy has landed: the pipeline's
         // memory takes the tile as [activation row][weight row].
-        float* const part = reinterpret_cast<float*>(smem) + (size_t)half * S::kCols * kRows + r;
+        float* const mine = reinterpret_cast<float*>(smem) + (size_t)part * S::kCols * kRows + r;
 #pragma unroll
         for (int j = 0; j < S::kCols / 2; j++) {
             float lo, hi;
             asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(acc[j]));
-            part[(2 * j) * kRows] = lo;
-            part[(2 * j + 1) * kRows] = hi;
+            mine[(2 * j) * kRows] = lo;
+            mine[(2 * j + 1) * kRows] = hi;
         }
         pdl_wait();                                               // the row scales, the residual, readers of what the output was
         tc_fence_before();
         __syncwarp();
         if (p.splits > 1) cluster_sync_all(); else asm volatile("bar.sync 1, %0;" ::"n"(kPromoteWarps * 32) : "memory");
         // ── epilogue: CTA `split` of the cluster finishes every splits-th activation row; a warp stores 128 contiguous bytes ──
-        const int chunks = rowsOut / 32, phases = kPromoteWarps / chunks;      // 4 × 2, or 2 × 4 for SwiGLU
+        const int chunks = rowsOut / 32, phases = kPromoteWarps / chunks;      // 4 × 4, or 2 × 8 for SwiGLU
         const int rc = (warp % chunks) * 32 + lane, no = n0 + rc;
         const float bv = p.bias != nullptr && no < p.N ? p.bias[no] : 0.0f, bv2 = p.bias2 != nullptr && no < p.N ? p.bias2[no] : 0.0f;
         const int mEnd = min(NT, p.M - m0);
@@ -525,21 +533,25 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_q8_gemm_tc(const __grid_const
 // ───────────── layout of a launch ─────────────
 struct TcPlan { int nt, mTiles, nTiles, splits, ktPer; double us; };
 
-// Tile width and reduction split with the least estimated time.
+// Tile width and reduction split with the least estimated time.  A CTA's time is proportional to its blocks; what one costs is
+// barriers and instructions more than products, so narrow tiles cost more per column and wide ones leave fewer CTAs.
+// Measured (4096 × 4096, one round of CTAs over the SMs): 0.165, 0.172, 0.258, 0.30 and 0.415 µs per block for 16, 32, 64, 96
+// and 128 rows; ≈ 2-3 µs per CTA besides, as much again for the sum over a cluster, 4.5 µs for the pre-pass and the launches.
 TcPlan tc_plan(int M, int K, int N, bool swiglu) {
+    static const struct { int nt; double block; } widths[] = {{16, 0.165}, {32, 0.172}, {64, 0.258}, {96, 0.30}, {128, 0.415}};
     const int nK = (K + kBlockK - 1) / kBlockK, rowsOut = swiglu ? kRows / 2 : kRows;
     const int nTiles = (N + rowsOut - 1) / rowsOut;
     TcPlan best = {}; best.us = 1e30;
-    for (int nt : {16, 32, 64, 96, 128, 160, 192}) {
+    for (const auto& w : widths) {
+        const int nt = w.nt;
         const int mTiles = (M + nt - 1) / nt;
-        const double perBlock = nt >= 64 ? 0.045 + 0.00105 * nt : 0.11;          // µs per 32-k block
         for (int sp = 1; sp <= kMaxSplits; sp *= 2) {
             const int ktPer = ((nK + sp - 1) / sp + kGroup - 1) / kGroup * kGroup;
             if (sp > 1 && (sp - 1) * ktPer >= nK) continue;                       // a CTA without blocks
             const int slots = sp == 1 ? g_num_sms : g_num_sms * 15 / 16 / sp * sp;   // clusters leave some SMs of a GPC unused
             const long ctas = (long)mTiles * nTiles * sp;
             const long rounds = (ctas + slots - 1) / slots;
-            const double us = (double)rounds * (perBlock * ktPer + 2.0 + 0.012 * nt + (sp > 1 ? 1.0 + 0.004 * nt : 0.0)) + 4.0;
+            const double us = (double)rounds * (w.block * ktPer + 1.5 + 0.01 * nt) + (sp > 1 ? 1.5 + 0.01 * nt : 0.0) + 4.5;
             if (us < best.us) best = {nt, mTiles, nTiles, sp, ktPer, us};
         }
     }
@@ -623,9 +635,7 @@ bool launch_q8_linear_tc(const Q8LinearArgs& a, float* ws, cudaStream_t s) {
         case 32: run<32>(p, pl, s); break;
         case 64: run<64>(p, pl, s); break;
         case 96: run<96>(p, pl, s); break;
-        case 128: run<128>(p, pl, s); break;
-        case 160: run<160>(p, pl, s); break;
-        default: run<192>(p, pl, s); break;
+        default: run<128>(p, pl, s); break;
     }
     return true;
 }
