@@ -304,9 +304,13 @@ class ComputeGraph:
         if not isinstance(buf, GpuBuffer) or not buf.cpu_stale:
             return
         self.flush()
-        flat = np.empty(buf.float_count(), dtype=np.float32)
+        # straight into the tensor's array where it is one: a second host copy of every result cost as much as the transfer
+        direct = isinstance(t.data, np.ndarray) and t.data.dtype == np.float32 and t.data.flags.c_contiguous and t.data.flags.writeable \
+            and t.data.size == buf.float_count()
+        flat = t.data.reshape(-1) if direct else np.empty(buf.float_count(), dtype=np.float32)
         self.runtime.download_buffer(buf.id, flat)
-        t.data[...] = flat.reshape(t.rows, t.cols)
+        if not direct:
+            t.data[...] = flat.reshape(t.rows, t.cols)
         buf.cpu_stale = False
 
     def release_all(self) -> None:

@@ -9,6 +9,8 @@
 #include "kernels.h"
 #include "q8_tma.cuh"
 
+#include <deque>
+#include <iterator>
 #include <algorithm>
 #include <cmath>
 #include <cstring>
@@ -132,8 +134,53 @@ void drop_graphs() {
     R.graphs.clear();
 }
 
+// Device blocks of released float buffers, kept for the next buffer of the same size: a training step through the drop-in
+// tensors makes and drops some twenty, and in a process that holds a few gigabytes a cudaMalloc and cudaFree pair costs
+// milliseconds.  Everything runs on one stream, so a block handed on is used behind its last use.  Bounded (the oldest go
+// first), given back when an allocation fails and at shutdown.
+constexpr size_t kSpareBlock = (size_t)64 << 20, kSpareTotal = (size_t)256 << 20;
+std::deque<std::pair<size_t, void*>> g_spare;         // (bytes, block), oldest first
+size_t g_spare_bytes = 0;
+
+size_t block_bytes(size_t bytes) { return (bytes + 511) / 512 * 512; }
+void drop_spare(size_t keep) {
+    while (g_spare_bytes > keep) {
+        cudaFree(g_spare.front().second);
+        g_spare_bytes -= g_spare.front().first;
+        g_spare.pop_front();
+    }
+}
+// cudaMalloc that gives the spare blocks back before it fails
+cudaError_t device_malloc(void** p, size_t bytes) {
+    cudaError_t e = cudaMalloc(p, bytes);
+    if (e == cudaErrorMemoryAllocation && !g_spare.empty()) {
+        cudaGetLastError();
+        drop_spare(0);
+        e = cudaMalloc(p, bytes);
+    }
+    return e;
+}
+void* take_block(size_t bytes) {
+    const size_t n = block_bytes(bytes);
+    for (auto it = g_spare.rbegin(); it != g_spare.rend(); ++it)
+        if (it->first == n) {
+            void* p = it->second;
+            g_spare.erase(std::next(it).base());
+            g_spare_bytes -= n;
+            return p;
+        }
+    void* p = nullptr;
+    DJ_CUDA_CHECK(device_malloc(&p, n));
+    return p;
+}
+
 void free_buf(Buf& b) {
-    if (b.ptr) cudaFree(b.ptr);
+    const size_t n = block_bytes(b.bytes);
+    if (b.ptr && b.kind == kF32 && n <= kSpareBlock) {
+        drop_spare(kSpareTotal - n);
+        g_spare.emplace_back(n, b.ptr);
+        g_spare_bytes += n;
+    } else if (b.ptr) cudaFree(b.ptr);
     b.ptr = nullptr;
 }
 
@@ -798,7 +845,7 @@ void ensure_ws(size_t floats) {
     DJ_CUDA_CHECK(cudaStreamSynchronize(R.stream));
     if (R.ws) cudaFree(R.ws);
     R.ws = nullptr; R.ws_floats = 0;
-    DJ_CUDA_CHECK(cudaMalloc((void**)&R.ws, floats * sizeof(float)));
+    DJ_CUDA_CHECK(device_malloc((void**)&R.ws, floats * sizeof(float)));
     R.ws_floats = floats;
     R.epoch++;
     drop_graphs();
@@ -959,6 +1006,7 @@ int deepj_cuda_shutdown(void) {
     drop_graphs();
     for (auto& kv : R.pool) free_buf(kv.second);
     R.pool.clear();
+    drop_spare(0);
     if (R.ws) cudaFree(R.ws);
     R.ws = nullptr; R.ws_floats = 0;
     R.epoch++;
@@ -973,7 +1021,7 @@ int deepj_cuda_alloc_buffers(const int32_t* ids, const int32_t* sizes, int32_t c
         if (sizes[i] < 0) throw std::runtime_error("negative buffer size for id=" + std::to_string(ids[i]));
         if (R.pool.count(ids[i])) continue;                    // native/deepj_metal_jni.mm:1489
         Buf b; b.kind = kF32; b.floats = (size_t)sizes[i]; b.bytes = std::max<size_t>(b.floats * 4, 4);
-        DJ_CUDA_CHECK(cudaMalloc(&b.ptr, b.bytes));
+        b.ptr = take_block(b.bytes);
         DJ_CUDA_CHECK(cudaMemsetAsync(b.ptr, 0, b.bytes, R.stream));
         b.serial = R.next_serial++;
         R.pool[ids[i]] = b;
@@ -1098,7 +1146,7 @@ int deepj_cuda_q8_alloc(int32_t id, int32_t K, int32_t N) {
     Buf b; b.kind = kQ8; b.K = K; b.N = N; b.Kp = (K + 15) / 16 * 16; b.nb = (K + 31) / 32;
     size_t codeBytes = ((size_t)N * b.Kp + 255) / 256 * 256;
     b.bytes = codeBytes + (size_t)N * b.nb * 4;
-    DJ_CUDA_CHECK(cudaMalloc(&b.ptr, b.bytes));
+    DJ_CUDA_CHECK(device_malloc(&b.ptr, b.bytes));
     DJ_CUDA_CHECK(cudaMemsetAsync(b.ptr, 0, b.bytes, R.stream));
     b.serial = R.next_serial++;
     R.pool[id] = b;
@@ -1165,7 +1213,7 @@ static int kv_alloc_impl(int32_t id, int32_t layers, int32_t batch, int32_t head
     b.kvHalf = half;
     if (half && head_dim % 16 != 0) throw std::runtime_error("kv_alloc: an fp16 cache needs a head dim that is a multiple of 16");
     b.bytes = plane * 2 * (half ? 2 : 4);
-    DJ_CUDA_CHECK(cudaMalloc(&b.ptr, b.bytes));
+    DJ_CUDA_CHECK(device_malloc(&b.ptr, b.bytes));
     DJ_CUDA_CHECK(cudaMemsetAsync(b.ptr, 0, b.bytes, R.stream));
     b.serial = R.next_serial++;
     R.pool[id] = b;
@@ -1179,7 +1227,7 @@ int deepj_cuda_bf16_alloc(int32_t id, int32_t K, int32_t N) {
     if (R.pool.count(id)) throw std::runtime_error("bf16_alloc: id " + std::to_string(id) + " already exists");
     Buf b; b.kind = kBf16; b.K = K; b.N = N; b.Kp = (K + 7) / 8 * 8;
     b.bytes = (size_t)N * b.Kp * 2;
-    DJ_CUDA_CHECK(cudaMalloc(&b.ptr, b.bytes));
+    DJ_CUDA_CHECK(device_malloc(&b.ptr, b.bytes));
     DJ_CUDA_CHECK(cudaMemsetAsync(b.ptr, 0, b.bytes, R.stream));
     b.serial = R.next_serial++;
     R.pool[id] = b;
@@ -1207,7 +1255,7 @@ int deepj_cuda_latent_alloc(int32_t id, int32_t batch, int32_t max_seq, int32_t 
     if (R.pool.count(id)) throw std::runtime_error("latent_alloc: id " + std::to_string(id) + " already exists");
     Buf b; b.kind = kLatent; b.B = batch; b.maxSeq = max_seq; b.hd = width; b.kvHalf = bf16;
     b.bytes = (size_t)batch * max_seq * width * (bf16 ? 2 : 4);
-    DJ_CUDA_CHECK(cudaMalloc(&b.ptr, b.bytes));
+    DJ_CUDA_CHECK(device_malloc(&b.ptr, b.bytes));
     DJ_CUDA_CHECK(cudaMemsetAsync(b.ptr, 0, b.bytes, R.stream));
     b.serial = R.next_serial++;
     R.pool[id] = b;
