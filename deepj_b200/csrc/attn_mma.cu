@@ -7,7 +7,9 @@
 // product a·b is accumulated as a_hi·b_hi + a_lo·b_hi + a_hi·b_lo (the dropped lo·lo term is
 // ≈ 2^-22 of the product) — the same split the many-row Q8 projection uses.
 //
-// grid (ceil(T / 64), heads, sequences), 128 threads.  Warp w owns query rows 16w … 16w+15 of the
+// grid (heads, ceil(T / 64), sequences), the last query tiles first: they have the most keys, and started last they left the
+// chip to a few blocks at the end (32 heads of 128, 2048 tokens: 695 µs with the query tiles as the fast grid axis in rising
+// order, 545 µs this way).  128 threads.  Warp w owns query rows 16w … 16w+15 of the
 // tile; the CTA walks the keys in tiles of 32: K and V rows come from the fp32 cache, are split and
 // laid down in shared memory as fp16 [key][dim] (row stride dim + 8 halves, so the eight rows an
 // ldmatrix fetches fall into different banks) — into the stage that is not being multiplied, the
@@ -70,7 +72,7 @@ __global__ void __launch_bounds__(128, 2) k_attn_prefill_mma(
     pdl_launch_dependents();
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int g = lane >> 2, t4 = lane & 3;
-    const int qt = blockIdx.x, h = blockIdx.y, b = blockIdx.z;
+    const int qt = (int)(gridDim.y - 1 - blockIdx.y), h = blockIdx.x, b = blockIdx.z;      // the tiles with the most keys first
     const int t0 = qt * kMQ;
     int pos0 = (int)posbuf[b];
     pos0 = pos0 < 0 ? 0 : pos0;
@@ -258,7 +260,7 @@ void launch_mma(const AttnDecodeArgs& a, int T, cudaStream_t s) {
         DJ_CUDA_CHECK(cudaFuncSetAttribute(k_attn_prefill_mma<HD, KT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)prefill_mma_smem<HD>()));
         attr = true;
     }
-    dim3 grid((T + kMQ - 1) / kMQ, a.H, a.B);
+    dim3 grid(a.H, (T + kMQ - 1) / kMQ, a.B);
     launch_k(k_attn_prefill_mma<HD, KT>, grid, dim3(128), prefill_mma_smem<HD>(), s, true, (const float*)a.qkv, a.q_off, a.ld,
              (const KT*)a.kcache, (const KT*)a.vcache, a.maxSeq, a.pos, a.cosT, a.sinT, a.out, a.ldo, a.H, a.scale, T);
 }
