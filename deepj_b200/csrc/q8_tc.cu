@@ -535,10 +535,10 @@ struct TcPlan { int nt, mTiles, nTiles, splits, ktPer; double us; };
 
 // Tile width and reduction split with the least estimated time.  A CTA's time is proportional to its blocks; what one costs is
 // barriers and instructions more than products, so narrow tiles cost more per column and wide ones leave fewer CTAs.
-// Measured (4096 × 4096, one round of CTAs over the SMs): 0.165, 0.172, 0.258, 0.30 and 0.415 µs per block for 16, 32, 64, 96
+// Measured (4096 × 4096, one round of CTAs over the SMs): 0.165, 0.172, 0.258, 0.29 and 0.425 µs per block for 16, 32, 64, 96
 // and 128 rows; ≈ 2-3 µs per CTA besides, as much again for the sum over a cluster, 4.5 µs for the pre-pass and the launches.
 TcPlan tc_plan(int M, int K, int N, bool swiglu) {
-    static const struct { int nt; double block; } widths[] = {{16, 0.165}, {32, 0.172}, {64, 0.258}, {96, 0.30}, {128, 0.415}};
+    static const struct { int nt; double block; } widths[] = {{16, 0.165}, {32, 0.172}, {64, 0.258}, {96, 0.29}, {128, 0.425}};
     const int nK = (K + kBlockK - 1) / kBlockK, rowsOut = swiglu ? kRows / 2 : kRows;
     const int nTiles = (N + rowsOut - 1) / rowsOut;
     TcPlan best = {}; best.us = 1e30;
