@@ -306,7 +306,7 @@ class ComputeGraph:
         self.flush()
         # straight into the tensor's array where it is one: a second host copy of every result cost as much as the transfer
         direct = isinstance(t.data, np.ndarray) and t.data.dtype == np.float32 and t.data.flags.c_contiguous and t.data.flags.writeable \
-            and t.data.size == buf.float_count()
+            and t.data.shape == (t.rows, t.cols) and t.data.size == buf.float_count()
         flat = t.data.reshape(-1) if direct else np.empty(buf.float_count(), dtype=np.float32)
         self.runtime.download_buffer(buf.id, flat)
         if not direct:
