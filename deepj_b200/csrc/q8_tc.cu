@@ -27,7 +27,9 @@
 // SwiGLU takes 64 gate and 64 up rows per tile, so the pair meets in one epilogue.  When the grid leaves SMs idle the
 // reduction is split over the CTAs of a cluster, which add their parts through distributed shared memory in split order.
 // Every wait is bounded: when a bound expires the CTA records an error code, stops waiting, lets its copies in flight
-// land, frees its tensor memory and returns.
+// land, frees its tensor memory and returns without storing its results.  A bound times this kernel alone: a wait that ends
+// only with the activation images, which an earlier kernel writes, comes behind the dependency wait, so an earlier kernel that
+// takes its time (an exchange polling a late peer) costs none of it.  The first weights are loaded and converted before that.
 #include "kernels.h"
 #include "q8_tma.cuh"
 #include "tc_common.cuh"
@@ -332,6 +334,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_q8_gemm_tc(const __grid_const
 #pragma unroll
             for (int j = 0; j < S::kCols / 2; j++) fma2(acc[j], v[2 * j], v[2 * j + 1], ss);
         };
+        pdl_wait();                                               // ahead of the first bounded wait
         bool ok = true, ready = false;                            // ready: the next accumulator was seen complete already
         for (int g = 0, b0 = 0; b0 < nK && ok; g++, b0 += kGroup) {
             const float4 cur = next;
@@ -372,7 +375,6 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_q8_gemm_tc(const __grid_const
             mine[(2 * j) * kRows] = lo;
             mine[(2 * j + 1) * kRows] = hi;
         }
-        pdl_wait();                                               // the row scales, the residual, readers of what the output was
         tc_fence_before();
         __syncwarp();
         if (p.splits > 1) cluster_sync_all(); else asm volatile("bar.sync 1, %0;" ::"n"(kPromoteWarps * 32) : "memory");
@@ -380,7 +382,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_q8_gemm_tc(const __grid_const
         const int chunks = rowsOut / 32, phases = kPromoteWarps / chunks;      // 4 × 4, or 2 × 8 for SwiGLU
         const int rc = (warp % chunks) * 32 + lane, no = n0 + rc;
         const float bv = p.bias != nullptr && no < p.N ? p.bias[no] : 0.0f, bv2 = p.bias2 != nullptr && no < p.N ? p.bias2[no] : 0.0f;
-        const int mEnd = min(NT, p.M - m0);
+        const int mEnd = s_abort ? 0 : min(NT, p.M - m0);
         const float* const tile = reinterpret_cast<const float*>(smem) + rc;
 #pragma unroll 4
         for (int c = split + p.splits * (warp / chunks); c < mEnd; c += p.splits * phases) {
@@ -413,6 +415,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_q8_gemm_tc(const __grid_const
             int rawAt = -1;                                       // raw group whose arrival has been waited for
             for (int i = grp; i * S::kPer < nK; i += 2) {
                 const int b = i * S::kPer, g = b / kGroup, j = b % kGroup, rs = g % S::kRawStages, s = i % S::kStages;
+                if (i >= S::kStages && i < S::kStages + 2) pdl_wait();    // from here on stages come back from the MMAs
                 if (g != rawAt) { warp_wait(rawFull(rs), (g / S::kRawStages) & 1, &s_abort, p.error, 206); rawAt = g; }
                 const unsigned char* src = smem + (size_t)S::kStages * S::kStageBytes + (size_t)rs * kRawBytes + r * 128;
                 uint4 w[2 * S::kPer];
@@ -467,6 +470,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_q8_gemm_tc(const __grid_const
             const int which = warp - kMmaWarp;
             const uint32_t d0 = __shfl_sync(0xffffffffu, tmem, 0);
             const uint64_t x0 = S::kDesc | (base >> 4);
+            pdl_wait();
             bool ok = true;
             for (uint32_t it = 0; it * (S::kStages * S::kPer) < (uint32_t)nK && ok; it++) {
 #pragma unroll
@@ -506,6 +510,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_q8_gemm_tc(const __grid_const
             const int nG = (nK + kGroup - 1) / kGroup;            // weights depend on no earlier kernel: no wait before them
             int g = 0, s = 0;
             for (uint32_t round = 0; g < nG; g++) {
+                if (g == S::kRawStages) pdl_wait();               // the first refill: the converters may be waiting for stages
                 if (round > 0 && !warp_wait(rawEmpty(s), (round - 1) & 1, &s_abort, p.error, 207)) break;
                 if (elect_one()) {
                     const uint32_t dst = rawBase + s * kRawBytes;
