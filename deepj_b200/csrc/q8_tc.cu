@@ -33,6 +33,7 @@
 #include "kernels.h"
 #include "q8_tma.cuh"
 #include "tc_common.cuh"
+#include <cfloat>
 #include <cuda_fp16.h>
 
 namespace dj {
@@ -212,11 +213,14 @@ __global__ void __launch_bounds__(kXThreads) k_x_images(const float* __restrict_
     __syncthreads();
 #pragma unroll
     for (int q = 0; q < kXThreads / 32; q++) amax = fmaxf(amax, red[2][q]);
-    // 2^-e brings the row's largest value into [512, 1024)
-    int ebits = 0x3f800000;
-    if (amax > 0.0f && amax < 1e30f) ebits = __float_as_int(amax) & 0x7f800000;
-    const float down = __int_as_float(0x7f000000 - ebits) * 512.0f;
-    if (tid == 0) rowscale[m] = __int_as_float(ebits) * (1.0f / 512.0f);
+    // A power of two brings the row's largest value into [512, 1024).  Both that factor and its inverse stay normal numbers: a
+    // largest value below 2^-117 is scaled as if it were that (a subnormal one then still has all its bits in fp16), and a row
+    // with an infinity as the largest finite exponent.  Such a row has no low halves: they would turn the infinity, and every
+    // result of the row is infinite or NaN with it, into NaN.
+    const int ebits = min(max(__float_as_int(amax) & 0x7f800000, 10 << 23), 254 << 23);
+    const float down = __uint_as_float((263u << 23) - (unsigned)ebits);
+    const bool finite = amax <= FLT_MAX;
+    if (tid == 0) rowscale[m] = __int_as_float(ebits - (9 << 23));
     const int rowBytes = 64 * per, mt = m / nt, r = m - mt * nt;
     unsigned char* const tile = images + (size_t)mt * nS * 2 * nt * rowBytes;
     for (int c = tid; c < nS * per * 4; c += kXThreads) {    // chunk c: values 8c … 8c + 7; past K zeros
@@ -230,7 +234,7 @@ __global__ void __launch_bounds__(kXThreads) k_x_images(const float* __restrict_
                 const float p = v[2 * j] * down, q = v[2 * j + 1] * down;
                 hi[2 * h + j] = pack_h2(p, q);
                 const float2 back = __half22float2(*reinterpret_cast<const __half2*>(&hi[2 * h + j]));
-                lo[2 * h + j] = pack_h2(p - back.x, q - back.y);
+                lo[2 * h + j] = finite ? pack_h2(p - back.x, q - back.y) : 0u;
             }
         }
         const int st = c / (4 * per), cc = c - st * 4 * per;
