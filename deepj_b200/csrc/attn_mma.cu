@@ -5,7 +5,7 @@
 // runs S = Q·Kᵀ and O += P·V as mma.sync.m16n8k16 (fp16 inputs, fp32 accumulate) while keeping
 // fp32-grade accuracy: every fp32 operand x is split into hi = fp16(x) and lo = fp16(x − hi), and a
 // product a·b is accumulated as a_hi·b_hi + a_lo·b_hi + a_hi·b_lo (the dropped lo·lo term is
-// ≈ 2^-22 of the product) — the same split the many-row Q8 projection uses.
+// ≈ 2^-22 of the product).
 //
 // grid (heads, ceil(T / 64), sequences), the last query tiles first: they have the most keys, and started last they left the
 // chip to a few blocks at the end (32 heads of 128, 2048 tokens: 695 µs with the query tiles as the fast grid axis in rising
