@@ -643,14 +643,44 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_q8_gemm_tc(const __grid_const
 // ───────────── layout of a launch ─────────────
 struct TcPlan { int nt, mTiles, nTiles, splits, ktPer; double us; };
 
-// Tile width and reduction split with the least estimated time.  A CTA's time is proportional to its blocks; what one costs is
-// barriers and instructions more than products, so narrow tiles cost more per column and wide ones leave fewer CTAs.
-// Measured (4096 × 4096, one round of CTAs over the SMs): 0.165, 0.172, 0.258, 0.29 and 0.425 µs per block for 16, 32, 64, 96
-// and 128 rows; ≈ 2-3 µs per CTA besides, as much again for the sum over a cluster, 4.5 µs for the pre-pass and the launches.
+// CTAs of this kernel that run at once in clusters of `sp`: one per SM, but a cluster stays inside a GPC, whose SMs are no
+// multiple of it (148 SMs take 74 clusters of two, 33 of four and 15 of eight).
+int cluster_slots(int sp) {
+    if (sp == 1) return g_num_sms;
+    auto ask = [](int size) {
+        constexpr size_t smem = TileShape<128, false>::kSmem;
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3((unsigned)size); cfg.blockDim = dim3(kTcThreads); cfg.dynamicSmemBytes = smem;
+        cudaLaunchAttribute at[1];
+        at[0].id = cudaLaunchAttributeClusterDimension;
+        at[0].val.clusterDim.x = (unsigned)size; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
+        cfg.attrs = at; cfg.numAttrs = 1;
+        int n = 0;
+        if (cudaFuncSetAttribute(k_q8_gemm_tc<128, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess ||
+            cudaOccupancyMaxActiveClusters(&n, k_q8_gemm_tc<128, false>, &cfg) != cudaSuccess || n < 1) {
+            cudaGetLastError();
+            n = g_num_sms * 13 / 16 / size;
+        }
+        return n * size;
+    };
+    static const int slots[3] = {ask(2), ask(4), ask(8)};
+    return slots[sp == 2 ? 0 : sp == 4 ? 1 : 2];
+}
+
+bool folds(int K, int ktPer) { return K % 128 != 0 && ktPer > kFold; }
+
+// Tile width and reduction split with the least estimated time: rounds of CTAs over the SMs, each round a fixed part and one per
+// block, the exchange of a cluster, and the pre-pass.  The costs of a width are from grids of whole rounds (148 r CTAs, two and six
+// rounds at K = 1024 and 4096); with totals a block costs what one round of K = 8208 takes.  One round of 8 or 32 blocks per CTA
+// takes 0.5-1.5, 0-1.4 and 1.0-3.7 µs more in clusters of 2, 4 and 8 than alone.  The pre-pass is from 64 to 512 rows of 2048 and 8192.
+// Over 34 shapes of 20 to 2048 rows the estimates are within 8 % of the times measured, and the choice is the fastest but for
+// 2048 x 2048 x 8192 (128 rows 222 µs, 96 rows 211).
 TcPlan tc_plan(int M, int K, int N, bool swiglu) {
-    static const struct { int nt; double block; } widths[] = {{16, 0.165}, {32, 0.172}, {64, 0.258}, {96, 0.29}, {128, 0.425}};
+    static const struct { int nt; double cta, block, blockFold; } widths[] = {
+        {16, 3.4, 0.158, 0.167}, {32, 3.9, 0.161, 0.171}, {64, 5.1, 0.200, 0.235}, {96, 7.4, 0.210, 0.27}, {128, 7.7, 0.333, 0.52}};
     const int nK = (K + kBlockK - 1) / kBlockK, rowsOut = swiglu ? kRows / 2 : kRows;
     const int nTiles = (N + rowsOut - 1) / rowsOut;
+    const double pre = 0.8 + 0.3e-3 * K + 2e-6 * (double)M * K;
     TcPlan best = {}; best.us = 1e30;
     for (const auto& w : widths) {
         const int nt = w.nt;
@@ -658,10 +688,11 @@ TcPlan tc_plan(int M, int K, int N, bool swiglu) {
         for (int sp = 1; sp <= kMaxSplits; sp *= 2) {
             const int ktPer = ((nK + sp - 1) / sp + kGroup - 1) / kGroup * kGroup;
             if (sp > 1 && (sp - 1) * ktPer >= nK) continue;                       // a CTA without blocks
-            const int slots = sp == 1 ? g_num_sms : g_num_sms * 15 / 16 / sp * sp;   // clusters leave some SMs of a GPC unused
+            const int slots = cluster_slots(sp);
             const long ctas = (long)mTiles * nTiles * sp;
             const long rounds = (ctas + slots - 1) / slots;
-            const double us = (double)rounds * (w.block * ktPer + 1.5 + 0.01 * nt) + (sp > 1 ? 1.5 + 0.01 * nt : 0.0) + 4.5;
+            const double block = folds(K, ktPer) ? w.blockFold : w.block;
+            const double us = pre + (double)rounds * (block * (ktPer < nK ? ktPer : nK) + w.cta) + (sp > 1 ? 0.4 + 0.15 * sp : 0.0);
             if (us < best.us) best = {nt, mTiles, nTiles, sp, ktPer, us};
         }
     }
@@ -744,7 +775,7 @@ bool launch_q8_linear_tc(const Q8LinearArgs& a, float* ws, cudaStream_t s) {
     p.M = M; p.N = N; p.swiglu = swiglu; p.gelu = a.act == 1;
     // K a multiple of 128: what runs these shapes with fewer rows keeps 16 bits of the activations, and a plain running sum is
     // far below that.  The kernels of the other lengths are 32-bit sums in short chains, and their error is the line here.
-    const bool fold = K % 128 != 0 && pl.ktPer > kFold;
+    const bool fold = folds(K, pl.ktPer);
     p.splits = pl.splits; p.ktPer = pl.ktPer; p.lo = g_tc_terms & 1; p.coarse = (g_tc_terms & 2) == 0; p.error = g_dev_error;
     switch (pl.nt) {
         case 16: run<16>(p, pl, fold, s); break;
