@@ -101,6 +101,7 @@ DJ_PART bool launch_q8_linear_batch_tma(const Q8LinearArgs& a, int m0, int rows,
 DJ_PART size_t q8_batch_ws_floats(int K, int N, bool swiglu);
 DJ_PART bool launch_q8_linear_tc(const Q8LinearArgs& a, float* ws, cudaStream_t s);
 DJ_PART size_t q8_tc_ws_floats(int M, int K, int N, bool swiglu);     // activation images and row scales
+DJ_PART void q8_tc_plan(int M, int K, int N, bool swiglu, int* tileRows, int* splits);
 DJ_PART double q8_tc_estimate_us(int M, int K, int N, bool swiglu);
 constexpr int kTcMinRows = 5;             // from this many activation rows on, a Q8 linear may run on the tcgen05 path
 

@@ -319,21 +319,28 @@ void dispatch_q8_linear(const Q8LinearArgs& a, cudaStream_t s);
 
 bool batch_qualifies(const Q8LinearArgs& a) { return g_gemv_mode >= 1 && a.M >= 5 && a.ws != nullptr && a.w.K % 32 == 0 && a.w.Kp == a.w.K; }
 
-// Whether the tensor-core kernel is tried first.  Passes of the 16-row kernel against it, by estimated time: a pass of the TMA
-// kernel costs ≈ 7 µs + 0.33 ps per weight (measured: 12.1 µs at 4096 × 4096, 22.6 at 4096 × 12288, 33.7 for a pair of 4096 × 11008,
-// where the tensor-core kernel takes 13.7, 32 and 52), one of the cp.async kernel (K no multiple of 128) 13 µs up to 16 M weights
-// and 0.8 ps per weight beyond (13.4 µs at 1600 × 1600, 14.9 at 1600 × 4800, 36 at 4096 × 11008; the tensor-core kernel takes
-// 6-9 µs where its grid is one short round).
+// Whether the tensor-core kernel is tried first: where its estimated time is at least a tenth below that of the kernel that would
+// run instead (near a tie the rows stay where fewer of them run).  That kernel, as measured:
+//  * K % 128 == 0: passes of the 16-row TMA kernel, 7 µs + 0.30 ps per weight (12.1 µs at 4096 × 4096, 22.6 at 4096 × 12288, 33.7 for
+//    a pair of 4096 × 11008, 46.2 at 4096 × 32000, where the tensor-core kernel takes 12, 26, 49 and 50.5);
+//  * K % 32 == 0: passes of the 16-row cp.async kernel, 13 µs up to 16 M weights and 0.8 ps per weight beyond (13.4 µs at 1600 × 1600,
+//    14.9 at 1600 × 4800, 36 at 4096 × 11008; the tensor-core kernel takes 8 where its grid is one short round);
+//  * else the FMA kernel, 0.5 µs + 2.5 ns per k + 0.37 ps per weight and row (8 × 688 × 256 2.4 µs, 64 × 688 × 256 7.5, 32 × 1392 × 512 12.6,
+//    200 × 5648 × 2048 830; the tensor-core kernel 6.0, 6.9, 7 and 35).
 bool runs_tc(const Q8LinearArgs& a) {
     static const bool noTc = getenv("DEEPJ_CUDA_NO_TC") != nullptr;
     if (g_gemv_mode < 1 || noTc || a.M < kTcMinRows || a.ws == nullptr) return false;
-    if (!batch_qualifies(a) || a.M > 256) return true;
     const bool swiglu = a.w2.codes != nullptr, tmaKernel = g_gemv_mode == 2 && a.w.K % 128 == 0;
     const double weights = (double)a.w.K * (double)a.w.N * (swiglu ? 2.0 : 1.0);
-    const double perPassUs = tmaKernel ? 7.0 + 0.33e-6 * weights : weights < 16e6 ? 13.0 : 0.8e-6 * weights;
-    const int rem = a.M % 16;
-    const double passes = (double)(a.M / 16) + (rem == 0 ? 0.0 : rem <= 8 ? 0.75 : 1.0);      // a last pass of up to eight rows issues half the MMAs
-    return passes * perPassUs >= q8_tc_estimate_us(a.M, a.w.K, a.w.N, swiglu);
+    double other;
+    if (batch_qualifies(a)) {
+        if (a.M > 256) return true;
+        const double perPassUs = tmaKernel ? 7.0 + 0.30e-6 * weights : weights < 16e6 ? 13.0 : 0.8e-6 * weights;
+        const int rem = a.M % 16;
+        const double passes = (double)(a.M / 16) + (rem == 0 ? 0.0 : rem <= 8 ? 0.75 : 1.0);      // a last pass of up to eight rows issues half the MMAs
+        other = passes * perPassUs;
+    } else other = 0.5 + 2.5e-3 * a.w.K + 0.37e-6 * weights * a.M;
+    return other >= 1.1 * q8_tc_estimate_us(a.M, a.w.K, a.w.N, swiglu);
 }
 }
 
@@ -389,3 +396,18 @@ void dispatch_q8_linear(const Q8LinearArgs& a, cudaStream_t s) {
 }  // namespace
 
 }  // namespace dj
+
+// Which way `rows` rows of a Q8 projection go: out[0] = 1 on the tensor-core kernel and 0 on the others, out[1] and out[2] its tile
+// rows and reduction splits.
+extern "C" int deepj_cuda_q8_route(int32_t rows, int32_t K, int32_t N, int32_t swiglu, int32_t* out) {
+    if (rows < 1 || K < 1 || N < 1 || out == nullptr) { dj::set_last_error("q8_route: bad arguments"); return 1; }
+    dj::Q8LinearArgs a = {};
+    static int8_t some;
+    static float scratch;
+    a.M = rows; a.ws = &scratch;                       // only asked whether they are there
+    a.w.K = K; a.w.N = N; a.w.Kp = (K + 15) / 16 * 16;
+    if (swiglu) a.w2.codes = &some;
+    out[0] = dj::runs_tc(a) && K % 4 == 0;
+    dj::q8_tc_plan(rows, K, N, swiglu != 0, &out[1], &out[2]);
+    return 0;
+}

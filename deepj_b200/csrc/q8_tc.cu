@@ -743,6 +743,10 @@ template <int NT> void run(const TcParams& p, const TcPlan& pl, bool fold, cudaS
 
 int g_tc_terms = 3;
 
+void q8_tc_plan(int M, int K, int N, bool swiglu, int* tileRows, int* splits) {
+    const TcPlan pl = tc_plan(M, K, N, swiglu);
+    *tileRows = pl.nt; *splits = pl.splits;
+}
 double q8_tc_estimate_us(int M, int K, int N, bool swiglu) { return tc_plan(M, K, N, swiglu).us; }
 
 size_t q8_tc_ws_floats(int M, int K, int N, bool swiglu) {

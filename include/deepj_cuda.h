@@ -166,6 +166,11 @@ int deepj_cuda_clear_device_error(void);
  * is fp32 throughout (native/deepj_metal_jni.mm:828-889). */
 int deepj_cuda_tc_configure(int32_t correction_terms);
 
+/* Which kernel `rows` rows of a Q8 projection K x N (swiglu: of a gate / up pair) run on: out[0] = 1 for the many-row (tcgen05)
+ * kernel, 0 for the others; out[1], out[2] = the tile rows and reduction splits the many-row kernel would take.  For tests and
+ * tuning; call deepj_cuda_init first.  No counterpart in the reference. */
+int deepj_cuda_q8_route(int32_t rows, int32_t K, int32_t N, int32_t swiglu, int32_t* out);
+
 /* Decode attention for callers that must not allocate.  No counterpart in the reference.
  *
  * Some hosts of this library cannot let a call reach cudaMalloc: a JVM thread inside a

@@ -19,7 +19,7 @@ def product(dev, x, q, N):  # noqa: F811
     return dev.get(ob, M * N).reshape(M, N).astype(np.float64)
 
 
-@pytest.mark.parametrize("M,K,N", [(40, 256, 300), (129, 688, 130), (300, 128, 96), (96, 1600, 70)])
+@pytest.mark.parametrize("M,K,N", [(40, 256, 300), (300, 688, 130), (300, 128, 96), (96, 1600, 70)])
 def test_rows_of_every_magnitude(dev, M, K, N):  # noqa: F811
     rng = np.random.default_rng(M + K)
     q, W = weights(dev, rng, K, N)
@@ -35,7 +35,7 @@ def test_rows_of_every_magnitude(dev, M, K, N):  # noqa: F811
     assert np.all(np.linalg.norm(got - want, axis=1) <= room)
 
 
-@pytest.mark.parametrize("M,K,N", [(40, 256, 300), (40, 688, 130), (96, 1600, 70)])
+@pytest.mark.parametrize("M,K,N", [(40, 256, 300), (300, 688, 130), (96, 1600, 70)])
 def test_infinities_and_nan_stay_in_their_rows(dev, M, K, N):  # noqa: F811
     """One infinity times a code is an infinity of the code's sign, and NaN where the code is zero; a NaN spoils its row."""
     rng = np.random.default_rng(M * K)
