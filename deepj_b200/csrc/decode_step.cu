@@ -1238,7 +1238,7 @@ extern "C" int deepj_cuda_decode_plan(int32_t plan_id, const int32_t* desc, int3
             weightBytes += (packed_bytes(srcs[i].w.K, srcs[i].w.N, srcs[i].sw) + 255) & ~(size_t)255;
         }
         char* block = nullptr;
-        DJ_CUDA_CHECK(cudaMalloc((void**)&block, tableBytes + scratchBytes + weightBytes));
+        DJ_CUDA_CHECK(device_malloc((void**)&block, tableBytes + scratchBytes + weightBytes));
         DJ_CUDA_CHECK(cudaMemset(block, 0, tableBytes + scratchBytes));
         unsigned char* wbase = reinterpret_cast<unsigned char*>(block + tableBytes + scratchBytes);
         for (size_t i = 0; i < srcs.size(); i++) pack_phase(srcs[i].w, srcs[i].sw ? &srcs[i].w2 : nullptr, wbase + wOff[i], runtime_stream());

@@ -302,6 +302,7 @@ DJ_PART void decode_step_check(int plan_id, std::vector<std::pair<int, unsigned 
 DJ_PART void launch_decode_step(int plan_id, int feed_back, cudaStream_t s);
 // The library's stream and device; the stream is null until the library has been initialised.
 cudaStream_t runtime_stream();
+cudaError_t device_malloc(void** p, size_t bytes);      // cudaMalloc that gives the kept blocks of released buffers back before it fails
 int runtime_device();
 // Drops every captured graph: called when addresses baked into kernel parameters (peer mappings, exchange
 // buffers) stop being valid, so that the next flush of a cached stream is captured afresh.

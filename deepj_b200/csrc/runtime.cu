@@ -11,6 +11,7 @@
 
 #include <deque>
 #include <iterator>
+#include <list>
 #include <algorithm>
 #include <cmath>
 #include <cstring>
@@ -136,39 +137,44 @@ void drop_graphs() {
 
 // Device blocks of released float buffers, kept for the next buffer of the same size: a training step through the drop-in
 // tensors makes and drops some twenty, and in a process that holds a few gigabytes a cudaMalloc and cudaFree pair costs
-// milliseconds.  Everything runs on one stream, so a block handed on is used behind its last use.  Bounded (the oldest go
-// first), given back when an allocation fails and at shutdown.
-constexpr size_t kSpareBlock = (size_t)64 << 20, kSpareTotal = (size_t)256 << 20;
-std::deque<std::pair<size_t, void*>> g_spare;         // (bytes, block), oldest first
+// milliseconds.  Everything runs on one stream, so a block handed on is used behind its last use.  Bounded in bytes and in
+// number (the oldest go first), given back when an allocation of this library fails and at shutdown.
+constexpr size_t kSpareBlock = (size_t)64 << 20, kSpareTotal = (size_t)256 << 20, kSpareCount = 4096;
+struct Spare { size_t bytes; void* ptr; };
+std::list<Spare> g_spare;                                                            // oldest first
+std::unordered_map<size_t, std::deque<std::list<Spare>::iterator>> g_spare_of;       // the blocks of one size, oldest first
 size_t g_spare_bytes = 0;
 
 size_t block_bytes(size_t bytes) { return (bytes + 511) / 512 * 512; }
-void drop_spare(size_t keep) {
-    while (g_spare_bytes > keep) {
-        cudaFree(g_spare.front().second);
-        g_spare_bytes -= g_spare.front().first;
+void drop_spare(size_t keepBytes, size_t keepCount) {
+    while (!g_spare.empty() && (g_spare_bytes > keepBytes || g_spare.size() > keepCount)) {
+        const Spare old = g_spare.front();
+        auto of = g_spare_of.find(old.bytes);
+        of->second.pop_front();                       // the oldest of all is the oldest of its size
+        if (of->second.empty()) g_spare_of.erase(of);
         g_spare.pop_front();
+        g_spare_bytes -= old.bytes;
+        cudaFree(old.ptr);
     }
 }
-// cudaMalloc that gives the spare blocks back before it fails
-cudaError_t device_malloc(void** p, size_t bytes) {
-    cudaError_t e = cudaMalloc(p, bytes);
-    if (e == cudaErrorMemoryAllocation && !g_spare.empty()) {
-        cudaGetLastError();
-        drop_spare(0);
-        e = cudaMalloc(p, bytes);
-    }
-    return e;
+void keep_block(void* ptr, size_t bytes) {            // bytes: a whole block, at most kSpareBlock
+    drop_spare(kSpareTotal - bytes, kSpareCount - 1);
+    g_spare.push_back({bytes, ptr});
+    g_spare_of[bytes].push_back(std::prev(g_spare.end()));
+    g_spare_bytes += bytes;
 }
 void* take_block(size_t bytes) {
     const size_t n = block_bytes(bytes);
-    for (auto it = g_spare.rbegin(); it != g_spare.rend(); ++it)
-        if (it->first == n) {
-            void* p = it->second;
-            g_spare.erase(std::next(it).base());
-            g_spare_bytes -= n;
-            return p;
-        }
+    auto of = g_spare_of.find(n);
+    if (of != g_spare_of.end()) {
+        auto it = of->second.back();                  // the one used last
+        of->second.pop_back();
+        if (of->second.empty()) g_spare_of.erase(of);
+        void* p = it->ptr;
+        g_spare.erase(it);
+        g_spare_bytes -= n;
+        return p;
+    }
     void* p = nullptr;
     DJ_CUDA_CHECK(device_malloc(&p, n));
     return p;
@@ -176,11 +182,8 @@ void* take_block(size_t bytes) {
 
 void free_buf(Buf& b) {
     const size_t n = block_bytes(b.bytes);
-    if (b.ptr && b.kind == kF32 && n <= kSpareBlock) {
-        drop_spare(kSpareTotal - n);
-        g_spare.emplace_back(n, b.ptr);
-        g_spare_bytes += n;
-    } else if (b.ptr) cudaFree(b.ptr);
+    if (b.ptr && b.kind == kF32 && n <= kSpareBlock) keep_block(b.ptr, n);
+    else if (b.ptr) cudaFree(b.ptr);
     b.ptr = nullptr;
 }
 
@@ -950,6 +953,15 @@ void flush(const int32_t* cmd, int len, bool sync) {
 }  // namespace
 
 namespace dj {
+cudaError_t device_malloc(void** p, size_t bytes) {
+    cudaError_t e = cudaMalloc(p, bytes);
+    if (e == cudaErrorMemoryAllocation && !g_spare.empty()) {
+        cudaGetLastError();
+        drop_spare(0, 0);
+        e = cudaMalloc(p, bytes);
+    }
+    return e;
+}
 bool pool_f32(int id, PoolF32* out) {
     auto it = R.pool.find(id);
     if (it == R.pool.end() || it->second.kind != kF32 || it->second.ptr == nullptr) return false;
@@ -1006,7 +1018,7 @@ int deepj_cuda_shutdown(void) {
     drop_graphs();
     for (auto& kv : R.pool) free_buf(kv.second);
     R.pool.clear();
-    drop_spare(0);
+    drop_spare(0, 0);
     if (R.ws) cudaFree(R.ws);
     R.ws = nullptr; R.ws_floats = 0;
     R.epoch++;
@@ -1022,7 +1034,8 @@ int deepj_cuda_alloc_buffers(const int32_t* ids, const int32_t* sizes, int32_t c
         if (R.pool.count(ids[i])) continue;                    // native/deepj_metal_jni.mm:1489
         Buf b; b.kind = kF32; b.floats = (size_t)sizes[i]; b.bytes = std::max<size_t>(b.floats * 4, 4);
         b.ptr = take_block(b.bytes);
-        DJ_CUDA_CHECK(cudaMemsetAsync(b.ptr, 0, b.bytes, R.stream));
+        const cudaError_t e = cudaMemsetAsync(b.ptr, 0, b.bytes, R.stream);
+        if (e != cudaSuccess) { free_buf(b); DJ_CUDA_CHECK(e); }
         b.serial = R.next_serial++;
         R.pool[ids[i]] = b;
     }
@@ -1121,8 +1134,8 @@ int deepj_cuda_stats(int64_t* counters, int32_t n) {
         DJ_CUDA_CHECK(cudaStreamSynchronize(R.stream));
         DJ_CUDA_CHECK(cudaMemcpy(&dev_err, g_dev_error, sizeof(int), cudaMemcpyDeviceToHost));
     }
-    int64_t v[6] = {g_launches, R.replays, R.captured, R.last_nodes, (int64_t)(R.ws_floats * 4), dev_err};
-    for (int i = 0; i < n && i < 6; i++) counters[i] = v[i];
+    int64_t v[8] = {g_launches, R.replays, R.captured, R.last_nodes, (int64_t)(R.ws_floats * 4), dev_err, (int64_t)g_spare_bytes, (int64_t)g_spare.size()};
+    for (int i = 0; i < n && i < 8; i++) counters[i] = v[i];
     DJ_CATCH
 }
 

@@ -218,7 +218,7 @@ int deepj_cuda_tp_create(int32_t rank, int32_t world, int64_t slot_floats, void*
         T.small_floats = std::min((size_t)slot_floats, (size_t)(2 * g_large_pairs + 3) / 4 * 4);
         const size_t dataBytes = tp_data_bytes();       // {bits, epoch} per value, both regions
         T.bytes = dataBytes + (size_t)(kTpCtas + kTpCtasLarge + 4) * sizeof(unsigned);
-        DJ_CUDA_CHECK(cudaMalloc(&T.local, T.bytes));
+        DJ_CUDA_CHECK(device_malloc(&T.local, T.bytes));
         DJ_CUDA_CHECK(cudaMemset(T.local, 0, T.bytes));
         DJ_CUDA_CHECK(cudaDeviceSynchronize());
         cudaIpcMemHandle_t h;
@@ -238,7 +238,7 @@ int deepj_cuda_tp_connect(const void* handles, int32_t world) {
             void* base = T.local;
             if (r != T.rank && handles == nullptr) {
                 // nobody will ever write here: this rank's pushes land in it, and its own buffer never sees rank r
-                DJ_CUDA_CHECK(cudaMalloc(&base, T.bytes));
+                DJ_CUDA_CHECK(device_malloc(&base, T.bytes));
                 DJ_CUDA_CHECK(cudaMemset(base, 0, T.bytes));
                 T.absent[r] = base;
             } else if (r != T.rank) {
