@@ -299,7 +299,7 @@ __device__ __forceinline__ float4 load_scales(const float* row, int k, int nb, b
         if (k + 3 < nb) v.w = row[k + 3];
     }
     if (coarse) {
-        auto cut = [](float f) { return __half2float(__float2half_rn(f * 4096.0f)) * (1.0f / 4096.0f); };
+        auto cut = [](float f) { return __uint_as_float((__float_as_uint(f) + 0x1000u) & 0xffffe000u); };      // 11 bits, at any size
         v = make_float4(cut(v.x), cut(v.y), cut(v.z), cut(v.w));
     }
     return v;
@@ -793,8 +793,9 @@ bool launch_q8_linear_tc(const Q8LinearArgs& a, float* ws, cudaStream_t s) {
 
 }  // namespace dj
 
-// Precision of the many-row path: bit 0 adds the X_lo product (activations at ≈ 22 bits, else 11), bit 1 keeps the block
-// scales in fp32 (else they are rounded to 11 bits).  Drops the cached CUDA graphs, which hold the old value.
+// Precision of the many-row path: bit 0 adds the X_lo product (activations at ≈ 22 bits, else 11 and half the products), bit 1
+// keeps the block scales in fp32 (else they are rounded to 11 bits, which saves nothing: the weights' part of the setting is
+// kept for callers that compare precisions).  Drops the cached CUDA graphs, which hold the old value.
 extern "C" int deepj_cuda_tc_configure(int32_t correction_terms) {
     if (correction_terms < 0 || correction_terms > 3) { dj::set_last_error("tc_configure: correction_terms must be 0..3"); return 1; }
     if (dj::g_tc_terms != correction_terms) { dj::g_tc_terms = correction_terms; dj::invalidate_graphs(); }

@@ -164,8 +164,9 @@ int deepj_cuda_clear_device_error(void);
 /* Precision of the many-row (tcgen05) Q8 projection, which multiplies fp16 halves x = x_hi + x_lo with the exact codes and
  * applies the block scales in fp32: x_hi * code is always issued; bit 0 of correction_terms adds x_lo * code, bit 1 keeps
  * the scales at 24 bits.  3 is the default (activations at about 22 bits, weights exact); without a bit its operand has 11
- * bits.  Takes effect on the next flush; cached CUDA graphs are dropped.  No counterpart in the reference, whose Q8 matmul
- * is fp32 throughout (native/deepj_metal_jni.mm:828-889). */
+ * bits.  Leaving out bit 0 halves the tensor-core work, leaving out bit 1 saves nothing.  Takes effect on the next flush;
+ * cached CUDA graphs are dropped.  No counterpart in the reference, whose Q8 matmul is fp32 throughout
+ * (native/deepj_metal_jni.mm:828-889). */
 int deepj_cuda_tc_configure(int32_t correction_terms);
 
 /* Which kernel `rows` rows of a Q8 projection K x N (swiglu: of a gate / up pair) run on: out[0] = 1 for the many-row (tcgen05)

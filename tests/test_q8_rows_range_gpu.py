@@ -3,6 +3,8 @@ not whole scale blocks: results are those of 32-bit arithmetic, not a question o
 import numpy as np
 import pytest
 
+import oracle
+from deepj_b200 import _lib
 from deepj_b200.compute_graph import OP_Q8_LINEAR
 from test_q8_gpu import dev  # noqa: F401
 from test_q8_rows_gpu import bound, weights
@@ -50,3 +52,21 @@ def test_infinities_and_nan_stay_in_their_rows(dev, M, K, N):  # noqa: F811
     assert np.all(np.isnan(got[4]))
     rest = [m for m in range(M) if m not in (1, 2, 4)]
     assert np.linalg.norm(got[rest] - plain[rest]) <= bound(K) * np.linalg.norm(plain[rest])
+
+
+@pytest.mark.parametrize("size", [1e-6, 0.02, 1e5])
+def test_the_coarse_settings_take_weights_of_any_size(dev, size):  # noqa: F811
+    """deepj_cuda_tc_configure without bit 1 rounds the block scales to 11 bits, whatever their size: an error of at most 2^-11."""
+    M, K, N = 300, 512, 160
+    rng = np.random.default_rng(3)
+    W = (rng.standard_normal((K, N)) * size).astype(np.float32)
+    q, Wq = dev.q8(W), oracle.q8_dequantize(*oracle.q8_quantize(W)).astype(np.float64)
+    x = rng.standard_normal((M, K)).astype(np.float32)
+    try:
+        _lib.check(dev.lib.deepj_cuda_tc_configure(1))
+        got = product(dev, x, q, N)
+    finally:
+        _lib.check(dev.lib.deepj_cuda_tc_configure(3))
+    want = x.astype(np.float64) @ Wq
+    err = np.linalg.norm(got - want) / np.linalg.norm(want)
+    assert 2.0 ** -15 < err <= 2.0 ** -11
