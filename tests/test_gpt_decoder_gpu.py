@@ -23,8 +23,9 @@ def dev():
     d.close()
 
 
-# rows 1-4: the GEMV with the norm and the activation fused; 6, 16 and 40: the 16-row kernel behind a
-# normalising pass; 300: the tcgen05 path; K = 100: the FMA fallback (no 32-element blocks)
+# rows 1-4: the GEMV with the norm and the activation fused; 6 and 16: the 16-row kernel behind a normalising pass; 40 and 300:
+# the tcgen05 path, which fuses both (test_q8_routes_gpu.py runs all of these with it switched off: 40 and 300 are then several
+# passes of the 16-row kernel); K = 100: the FMA fallback (no 32-element blocks)
 @pytest.mark.parametrize("M,K,N", [(1, 256, 96), (2, 512, 40), (4, 4096, 64), (3, 768, 33), (6, 512, 72), (16, 256, 128),
                                    (40, 256, 300), (300, 256, 300), (1, 100, 24), (5, 100, 24)])
 @pytest.mark.parametrize("act", [0, 1])

@@ -1,6 +1,6 @@
-"""The many-row Q8 projection (tensor cores, one accumulation per scale block) at the edges of its tiles and of its dispatch:
-tile widths and reduction splits, rows and columns that fill no tile, K of odd block counts and of no whole block, and the
-fused LayerNorm and GELU."""
+"""The many-row Q8 projection (tensor cores, one accumulation per scale block) in small sizes: rows and columns that fill no
+tile, K of odd block counts and of no whole block, strided windows, and the fused LayerNorm and GELU, on tiles of 16 to 64 rows; a
+few shapes lie just outside its dispatch.  test_q8_routes_gpu.py takes every tile width and split by name."""
 import numpy as np
 import pytest
 
