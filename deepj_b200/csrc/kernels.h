@@ -154,6 +154,7 @@ struct Bf16LinearArgs {
     int pair = kPairClamp;
     int M = 0;
     int exact = 0;                             // 1: fp32 products throughout
+    int trigger = 0;                           // 1: the kernel behind it may start before this one's dependency wait
     float* ws = nullptr;                       // bf16_linear_ws_floats
 };
 DJ_PART void launch_bf16_store(const float* src, int rows, int cols, __nv_bfloat16* dst, long long dst_ld, cudaStream_t s);
@@ -178,10 +179,13 @@ struct Bf16ExpertArgs {
     Bf16View up, down; int ff, d; float limit;
     const float* residual; int ldr; float* out; int ldo;
     int M, exact;
+    bool early;                                // token ids and table may be read before the dependency wait
+    int trigger = 0;                           // as above
     float* ws;                                 // bf16_experts_ws_floats
 };
 DJ_PART size_t bf16_experts_ws_floats(const Bf16ExpertArgs& e);
 DJ_PART void launch_bf16_experts(const Bf16ExpertArgs& e, cudaStream_t s);
+DJ_PART void launch_bf16_gemv(const Bf16LinearArgs& a, cudaStream_t s);      // 1-16 rows
 DJ_PART void launch_bf16_expert_gemv(const Bf16ExpertArgs& e, float* y, cudaStream_t s);
 
 // ── generalized delta rule (delta_rule.cu) ──

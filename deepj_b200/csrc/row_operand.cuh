@@ -24,14 +24,19 @@ __device__ __forceinline__ float pair_f(float g, float u, float limit, int pair)
 __device__ __forceinline__ float softcap_f(float v, float cap) { return cap > 0.0f ? cap * tanhf(v / cap) : v; }
 
 constexpr int kMaxNormGroups = 512;
-struct RowScratch { float part[kMaxNormGroups + 32]; float scale[kMaxNormGroups]; };
+// Shared memory of a norm: the groups' scales and the warps' parts of their sums of squares.
+constexpr int kRowScratchMax = 2 * kMaxNormGroups + 32;
+struct RowScratch {
+    float* scale; float* part;
+    __device__ __forceinline__ RowScratch(float* s, int groups) : scale(s), part(s + groups) {}
+};
 
 // Stages one segment of row m with the whole block (blockDim.x a multiple of 32).  `at(k)` is the fp32 storage of column k;
 // four columns from a multiple of four on are contiguous in it.  Ends with every element written, NOT with a barrier.
 // The loads of a pass are issued in batches of four 16-byte pieces per thread: a block stages a row of thousands of
 // values, and what it waits for is the round trip to L2.  `keep`: this block writes the sum of a row with a base.
 template <typename Store>
-__device__ __forceinline__ void stage_segment(const RowOperand& seg, int m, RowScratch& sc, Store at, bool keep = false) {
+__device__ __forceinline__ void stage_segment(const RowOperand& seg, int m, const RowScratch& sc, Store at, bool keep = false) {
     const int tid = threadIdx.x, nt = blockDim.x, lane = tid & 31, warp = tid >> 5, nw = nt >> 5;
     const float* x = seg.x + (size_t)m * seg.ldx;
     const float* gate = seg.gate ? seg.gate + (size_t)m * seg.ldg : nullptr;

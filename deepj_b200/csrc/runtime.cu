@@ -194,6 +194,8 @@ struct Ctx {
     cudaStream_t s;
     size_t ws_need = 0;
     int prev_op = 0;                   // op code before this one in the stream
+    const int32_t* prev = nullptr;     // and its words
+    int next_op = 0;                   // op code behind this one, 0 = none
     bool bounded_waits = false;        // the stream holds an op whose kernel waits on a peer (tensor-parallel exchange)
     std::vector<std::pair<int, unsigned long long>>* refs = nullptr;
 };
@@ -319,7 +321,11 @@ void do_op(Ctx& ctx, const int32_t* c) {
     // An op that keeps a state or a cache may read what earlier steps left in it before the dependency wait only when the
     // kernel right before it is a projection: that kernel has passed its own wait, so everything older is complete.
     const bool early = ctx.prev_op == DEEPJ_OP_BF16_LINEAR || ctx.prev_op == DEEPJ_OP_BF16_LINEAR_SUM || ctx.prev_op == DEEPJ_OP_BF16_BLOCK_LINEAR;
-    ctx.prev_op = op;
+    // A projection lets the kernel behind it in before its own wait where that one reads nothing but weights ahead of its wait
+    // (every older kernel may still run then, so nothing that keeps a state or a cache).
+    const bool trigger = ctx.next_op == DEEPJ_OP_BF16_LINEAR || ctx.next_op == DEEPJ_OP_BF16_LINEAR_SUM || ctx.next_op == DEEPJ_OP_NORM_ADD;
+    const int32_t* const prev = ctx.prev;
+    ctx.prev_op = op; ctx.prev = c;
     auto scratch = [&](size_t floats) {          // room in the shared workspace for this op
         if (floats > ctx.ws_need) ctx.ws_need = floats;
         return R.ws;
@@ -605,7 +611,7 @@ void do_op(Ctx& ctx, const int32_t* c) {
             a.a = row_operand(ctx, M, k1, c[1], c[2], c[3], c[4], c[5], bits_to_float(c[6]), c[7], c[8], c[9], what);
             if (c[11] >= 0) a.b = row_operand(ctx, M, k2, c[11], c[12], c[13], -1, 0, 0.0f, -1, 0, 0, what);
             a.w = bf16view(wb);
-            a.gluRow = c[22]; a.limit = bits_to_float(c[23]); a.softcap = bits_to_float(c[27]); a.exact = c[28]; a.M = M;
+            a.gluRow = c[22]; a.limit = bits_to_float(c[23]); a.softcap = bits_to_float(c[27]); a.exact = c[28]; a.M = M; a.trigger = trigger;
             require(a.gluRow >= 0 && a.gluRow <= N && (a.gluRow == N || (a.gluRow % 8 == 0 && (N - a.gluRow) % 2 == 0)), what, "bad first gated row");
             require(a.exact == 0 || a.exact == 1, what, "exact must be 0 or 1");
             if (a.gluRow > 0) {
@@ -820,6 +826,10 @@ void do_op(Ctx& ctx, const int32_t* c) {
             probe.a = e.x; probe.w = e.up;
             if (const char* msg = bf16_linear_check(probe)) require(false, what, msg);
             require((size_t)e.top * (down.Kp + 255) / 256 * 1024 <= 200 * 1024, what, "expert feed-forward too wide");
+            // token ids and table come from further back than the op before: it does not even name them
+            e.trigger = trigger;
+            e.early = early && std::find(prev, prev + op_stride(prev[0]), c[7]) == prev + op_stride(prev[0]) &&
+                      std::find(prev, prev + op_stride(prev[0]), c[8]) == prev + op_stride(prev[0]);
             e.ws = scratch(bf16_experts_ws_floats(e));
             if (go) launch_bf16_experts(e, s);
             break;
@@ -836,6 +846,7 @@ int walk(Ctx& ctx, const int32_t* cmd, int len) {
         int stride = op_stride(cmd[pos]);
         if (stride < 0) throw std::runtime_error("Unknown op code in command stream: " + std::to_string(cmd[pos]));
         if (pos + stride > len) throw std::runtime_error("Truncated command stream at int " + std::to_string(pos));
+        ctx.next_op = pos + stride < len ? cmd[pos + stride] : 0;
         do_op(ctx, cmd + pos);
         pos += stride;
         nops++;
