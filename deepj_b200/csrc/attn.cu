@@ -5,18 +5,20 @@
 // RotaryEmbedding.java:81-122).  Masked positions contribute exactly +0 to the
 // reference's softmax, so attending over 0..pos only is the same function.
 //
-// grid (splits, heads, batch), flash-decoding: a CTA rotates its head's q in
-// registers (interleaved pairs, x0·c − x1·s, x0·s + x1·c), streams its slice of the
-// cache once — hd/16 lanes per position, 128-bit loads, online softmax in fp32 — and
-// leaves (acc[hd], m, l) in a workspace.  The lane group that meets the newest
-// position takes k and v from the projection buffer instead, rotates k and appends
-// both to the cache.  The last CTA of a head to finish (a ticket counter that it
-// resets) merges the split partials into the merged-heads row, so no second launch
-// is needed.  HBM-bound: the algorithmic traffic is the K and V rows of 0..pos.
+// grid (splits, heads, batch), flash-decoding: a block rotates its head's q in registers (interleaved pairs,
+// x0·c − x1·s, x0·s + x1·c) and streams its slice of the cache once.  Cached rows of a head are contiguous, so a warp asks for
+// the K and the V rows of 32 / (hd / 16) positions with one bulk copy each, into a ring of its own, the first of them before the
+// dependency wait; hd/16 lanes per position, online softmax in fp32.  The block that owns the newest position takes k and v from the
+// projection buffer instead, rotates k and appends both to the cache.  Up to eight splits of a head are a cluster: each
+// block leaves (acc[hd], m, l) in the first one's shared memory, one cluster barrier, done.  More splits leave them in a workspace, and the last
+// block of a head to finish (a ticket counter that it resets) merges them: a fence, the ticket and the loads are 2 µs.
+// HBM-bound with long contexts: the algorithmic traffic is the K and V rows of 0..pos.  Measured between the projections around
+// it, against rows through registers and tickets for any split: 16 heads × 128, 300 positions 6.9 µs (10.3; the hand-overs are 2 of it),
+// 25 × 64, 210 positions ≈ 5 (7.3), 32 × 128, 2060 positions 16.1 (16.5, with less of the L1 that register loads want beside it).
 #include "../../include/deepj_cuda.h"
 #include "kernels.h"
 #include "kv_cache.cuh"
-#include "q8_common.cuh"
+#include "tc_common.cuh"
 #include <algorithm>
 #include <cmath>
 #include <cstdlib>
@@ -27,6 +29,9 @@ namespace {
 
 constexpr int kAttnWarps = 4;
 constexpr int kMaxSplits = 256;             // split partials a head can have (the merge keeps their weights in shared memory)
+constexpr int kClusterSplits = 8;           // up to so many splits are a cluster
+constexpr int kAttnSpinLimit = 1 << 22;     // polls of a barrier before the kernel gives up on it
+constexpr int kErrAttnWait = 332;           // device error code: a copy of cached rows never arrived
 
 // Prompt chunk: row z = (sequence b, token t) of the projection buffer holds k and v of position pos[b] + t.
 // One thread per interleaved pair: rotate k (x0·c − x1·s, x0·s + x1·c — RotaryEmbedding.java:81-122), copy v.
@@ -49,529 +54,292 @@ __global__ void k_kv_append(const float* __restrict__ qkv, int k_off, int v_off,
     KvIo<KT>::st2(vcache + dst, v2.x, v2.y);
 }
 
-template <int LPP, typename KT>   // lanes per position = hd / 16; cache element type
-__global__ void __launch_bounds__(kAttnWarps * 32, 4) k_attn_decode(
-        const float* __restrict__ qkv, int q_off, int k_off, int v_off, int ld,
-        KT* __restrict__ kcache, KT* __restrict__ vcache, int maxSeq,
-        const float* __restrict__ posbuf, const float* __restrict__ cosT, const float* __restrict__ sinT,
-        float* __restrict__ ws, int* __restrict__ tickets, float* __restrict__ out, int ldo, int H, float scale,
-        int T, int append) {
-    constexpr int HD = LPP * 16;
+// Ring items per warp: four blocks and a projection's beside them have to fit into an SM.
+template <typename KT> constexpr int kRingStages = sizeof(KT) == 4 ? 2 : 3;
+struct AttnDecodeParams {
+    const float* qkv; int q_off, k_off, v_off, ld;
+    void* kcache; void* vcache; int maxSeq;
+    const float* pos; const float* cosT; const float* sinT;
+    float* ws; int* tickets; float* out; int ldo, H; float scale; int T, append;
+    int* error;
+};
+
+// A lane holds elements 4·(c·LPP + gl) … +3, c = 0 … 3, of its position's rows: the lanes of a position read consecutive pieces.
+// CLUSTER: the splits of a head are one cluster, whose blocks leave their partials in the first one's shared memory.
+template <int LPP, typename KT, bool CLUSTER>   // lanes per position = hd / 16; cache element type
+__global__ void __launch_bounds__(kAttnWarps * 32, 4) k_attn_decode(const AttnDecodeParams p) {
+    constexpr int HD = LPP * 16, half = HD / 2;
     constexpr int PPW = 32 / LPP;                 // positions per warp iteration
-    constexpr int G = kAttnWarps * PPW;           // position groups per CTA
-    constexpr int kStages = 3;                    // ring stages per warp: two groups of positions in flight, one being folded in
-    constexpr int kStageElems = 2 * PPW * HD;     // a stage: K rows of PPW consecutive positions, then their V rows (1024 elements)
-    // dynamic shared memory: warp-private K/V rings [warps][kStages][kStageElems] of the cache type while the slice
-    // streams; afterwards the same bytes hold the CTA's partial rows (s_acc [G][HD], s_m [G], s_l [G])
-    extern __shared__ __align__(16) unsigned char dynsm[];
-    float (*s_acc)[HD] = reinterpret_cast<float (*)[HD]>(dynsm);
-    float* s_m = reinterpret_cast<float*>(dynsm) + G * HD;
-    float* s_l = s_m + G;
+    constexpr int G = kAttnWarps * PPW;           // positions per block iteration
+    constexpr int kStages = kRingStages<KT>, kPlane = PPW * HD * (int)sizeof(KT);      // ring items per warp: K rows of PPW consecutive positions, then their V rows
+    extern __shared__ __align__(128) unsigned char ring[];               // [warps][kStages][2][kPlane]
+    __shared__ __align__(8) unsigned long long s_bar[kAttnWarps * kStages];
+    __shared__ __align__(16) float s_acc[kAttnWarps][HD];
+    __shared__ float s_m[kAttnWarps], s_l[kAttnWarps];
     __shared__ int s_last;
+    __shared__ float s_w[CLUSTER ? 1 : kMaxSplits];
+    __shared__ float s_part[CLUSTER ? kClusterSplits : 1][CLUSTER ? HD + 2 : 1];       // the cluster's partials, in its first block
 
     // row z of the projection / output buffers is token t of sequence b: T = 1 (and append) for a decode step;
-    // T > 1 for a prompt chunk, whose k/v rows the append kernel has already written
+    // T > 1 for a short prompt chunk, whose k/v rows the append kernel has already written
     const int split = blockIdx.x, splits = gridDim.x, h = blockIdx.y, z = blockIdx.z;
-    const int b = z / T, tok = z - b * T;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int b = p.T == 1 ? z : z / p.T, tok = z - b * p.T;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int group = lane / LPP, gl = lane % LPP;
+    if constexpr (CLUSTER) asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
+    const uint32_t bars = smem_u32(&s_bar[warp * kStages]), mine = smem_u32(ring) + warp * (kStages * 2 * kPlane);
+    if (lane < kStages) mbar_init(bars + 8 * lane, 1);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    __syncwarp();
+
     // The cache rows below the current position were written by earlier steps, not by the kernel this one depends
-    // on, so the first two groups of K/V rows are requested BEFORE the wait and stream in while the projection kernel
-    // drains.  The position read here is re-read after the wait; in the (never observed) case that it moved, the
-    // speculative rows are dropped and requested again.
-    const int half = HD >> 1;
-    auto read_pos = [&]() {
-        int v = (int)__ldcg(posbuf + b) + tok;
-        return v < 0 ? 0 : (v >= maxSeq ? maxSeq - 1 : v);
+    // on, so the first rows are requested BEFORE the wait and stream in while the projection kernel drains.  The
+    // position read here is re-read after the wait; in the (never observed) case that it moved, the early rows are
+    // dropped and requested again.
+    auto read_pos = [&]() { return min(max((int)__ldcg(p.pos + b) + tok, 0), p.maxSeq - 1); };
+    int pos = read_pos(), at = 0, endc = 0;       // the warp's next position to request, the end of the block's cached ones
+    bool ownsNew = false;                         // the new token's position is this block's: not in the cache yet, folded in apart
+    auto slice = [&]() {
+        const int seq = pos + 1, chunk = (seq + splits - 1) / splits, start = split * chunk, end = min(seq, start + chunk);
+        ownsNew = p.append && pos >= start && pos < end;
+        endc = ownsNew ? pos : end;
+        at = start + warp * PPW;
     };
-    int pos = read_pos();
-    int seq = pos + 1;
-    int chunk = (seq + splits - 1) / splits;
-    int start = split * chunk;
-    int end = min(seq, start + chunk);
-    KT* khead = kcache + ((size_t)b * H + h) * maxSeq * HD;      // this head's rows [maxSeq][HD]
-    KT* vhead = vcache + ((size_t)b * H + h) * maxSeq * HD;
-    KT* kbase = khead + gl * 16;
-    KT* vbase = vhead + gl * 16;
-    KT* ring = reinterpret_cast<KT*>(dynsm) + (size_t)warp * kStages * kStageElems;
-    // Stage `st` ← the K and V rows of positions pb … pb+PPW−1 (consecutive rows are contiguous): 16-byte pieces, lane by
-    // lane.  Rows past the end of the cache are clamped to its last row (their lanes are masked out below).
-    constexpr int kPieces = PPW * HD * (int)sizeof(KT) / 16;       // per plane: 128 (fp32) or 64 (fp16)
-    constexpr int kPerRow = HD * (int)sizeof(KT) / 16;
-    auto issue = [&](int st, int pb) {
-        KT* dst = ring + (size_t)st * kStageElems;
+    const size_t plane = ((size_t)b * p.H + h) * p.maxSeq * HD;
+    KT* const khead = static_cast<KT*>(p.kcache) + plane;
+    KT* const vhead = static_cast<KT*>(p.vcache) + plane;
+    int asked = 0, taken = 0, limit = kAttnSpinLimit;                    // items since the start; item i is in slot i % kStages
+    auto request = [&]() {
+        if (lane == 0) {
+            const int slot = asked % kStages;
+            const uint32_t bytes = min(PPW, endc - at) * HD * (int)sizeof(KT), bar = bars + 8 * slot, to = mine + slot * (2 * kPlane);
+            mbar_arrive_expect_tx(bar, 2 * bytes);
+            bulk_g2s(to, khead + (size_t)at * HD, bytes, bar);
+            bulk_g2s(to + kPlane, vhead + (size_t)at * HD, bytes, bar);
+        }
+        asked++;
+        at += G;
+    };
+    auto take = [&]() {                           // the next item has arrived
+        const uint32_t bar = bars + 8 * (taken % kStages), parity = (taken / kStages) & 1;
+        bool ready = mbar_try_wait(bar, parity);
+#pragma unroll 1
+        for (int spin = 0; !ready && spin < limit; spin++) ready = mbar_try_wait(bar, parity);
+        if (!ready) {                             // never on a healthy device: flag it, stop waiting long, keep the control flow
+            if (lane == 0) atomicCAS(p.error, 0, kErrAttnWait);
+            limit = 64;
+        }
+        taken++;
+    };
+    slice();
+    int base = at;
+#pragma unroll 1
+    for (int i = 0; i < kStages && at < endc && p.T == 1; i++) request();      // a chunk's own rows were written by the kernel before this one
+    // the rotation tables are constants: the row of the early position is fetched before the wait too
+    float2 cs[4], sn[4];
+    auto load_tables = [&]() {
 #pragma unroll
-        for (int c0 = 0; c0 < kPieces; c0 += 32) {
-            const int c = c0 + lane;
-            const int prow = min(pb + c / kPerRow, maxSeq - 1);
-            const size_t src = (size_t)prow * HD + (size_t)(c % kPerRow) * (16 / sizeof(KT));
-            cp_async16(reinterpret_cast<unsigned char*>(dst) + (size_t)c * 16, khead + src);
-            cp_async16(reinterpret_cast<unsigned char*>(dst + PPW * HD) + (size_t)c * 16, vhead + src);
+        for (int c = 0; c < 4; c++) {
+            cs[c] = *reinterpret_cast<const float2*>(p.cosT + (size_t)pos * half + 2 * (c * LPP + gl));
+            sn[c] = *reinterpret_cast<const float2*>(p.sinT + (size_t)pos * half + 2 * (c * LPP + gl));
         }
     };
-    // iteration `it` of this warp covers positions start + warp·PPW + it·G … + PPW − 1
-    int nIter = 0;
-    auto count_iters = [&]() { const int first = start + warp * PPW; nIter = first < end ? (end - first + G - 1) / G : 0; };
-    count_iters();
-    const bool spec = T == 1;                     // a chunk's own rows were written by the kernel before this one: no early requests
-    if (spec) {
-#pragma unroll
-        for (int i = 0; i < kStages - 1; i++) {
-            if (i < nIter) issue(i, start + warp * PPW + i * G);
-            cp_async_commit();
-        }
-    }
-    // the rotation tables are constants: the row of the speculative position is fetched before the wait too
-    float cs[8], sn[8];
-    auto load_tables = [&](float (&cs)[8], float (&sn)[8]) {
-        const float4* cp = reinterpret_cast<const float4*>(cosT + (size_t)pos * half + gl * 8);
-        const float4* sp = reinterpret_cast<const float4*>(sinT + (size_t)pos * half + gl * 8);
-#pragma unroll
-        for (int j = 0; j < 2; j++) {
-            const float4 c4 = cp[j], s4 = sp[j];
-            cs[4 * j] = c4.x; cs[4 * j + 1] = c4.y; cs[4 * j + 2] = c4.z; cs[4 * j + 3] = c4.w;
-            sn[4 * j] = s4.x; sn[4 * j + 1] = s4.y; sn[4 * j + 2] = s4.z; sn[4 * j + 3] = s4.w;
-        }
-    };
-    load_tables(cs, sn);
-    const int specPos = pos;
+    load_tables();
+    const int early = pos;
     pdl_wait();
     pdl_launch_dependents();
     // the query row does not depend on the position: its loads go out together with the position's
-    const float* rowp = qkv + (size_t)z * ld;
-    float q[16];
-    {
-        const float4* qp = reinterpret_cast<const float4*>(rowp + q_off + h * HD + gl * 16);
+    const float* rowp = p.qkv + (size_t)z * p.ld + h * HD + 4 * gl;
+    auto load_row = [&](int off, float4 (&v)[4]) {
 #pragma unroll
-        for (int j = 0; j < 4; j++) { float4 v = qp[j]; q[4 * j] = v.x; q[4 * j + 1] = v.y; q[4 * j + 2] = v.z; q[4 * j + 3] = v.w; }
-    }
+        for (int c = 0; c < 4; c++) v[c] = *reinterpret_cast<const float4*>(rowp + off + c * (4 * LPP));
+    };
+    float4 q[4], kx[4], vx[4];
+    load_row(p.q_off, q);
     pos = read_pos();
-    if (pos != specPos || !spec) {
-        if (pos != specPos) load_tables(cs, sn);
-        seq = pos + 1;
-        chunk = (seq + splits - 1) / splits;
-        start = split * chunk;
-        end = min(seq, start + chunk);
-        cp_async_wait<0>();                       // whatever was requested for the old position is dropped
+    if (pos != early || p.T > 1) {
+#pragma unroll 1
+        while (taken < asked) take();
         __syncwarp();
-        count_iters();
-#pragma unroll
-        for (int i = 0; i < kStages - 1; i++) {
-            if (i < nIter) issue(i, start + warp * PPW + i * G);
-            cp_async_commit();
-        }
+        if (pos != early) load_tables();
+        slice();
+        base = at;
+#pragma unroll 1
+        for (int i = 0; i < kStages && at < endc; i++) request();
     }
-
-    // rotate 8 interleaved pairs held in v[16] by the table row of the current position (cs, sn)
-    auto rotate = [&](float (&v)[16], const float (&cs)[8], const float (&sn)[8]) {
+    // interleaved pairs (x0, x1) → (x0·c − x1·s, x0·s + x1·c)
+    auto rotate = [&](float4 (&v)[4]) {
 #pragma unroll
-        for (int i = 0; i < 8; i++) {
-            const float x0 = v[2 * i], x1 = v[2 * i + 1];
-            v[2 * i] = x0 * cs[i] - x1 * sn[i];
-            v[2 * i + 1] = x0 * sn[i] + x1 * cs[i];
-        }
-    };
-    rotate(q, cs, sn);
-
-    float m = -INFINITY, l = 0.0f, acc[16];
-#pragma unroll
-    for (int j = 0; j < 16; j++) acc[j] = 0.0f;
-    for (int it = 0; it < nIter; it++) {
-        // keep two groups in flight: the stage freed by the previous iteration takes the group two ahead
-        if (it + kStages - 1 < nIter) issue((it + kStages - 1) % kStages, start + warp * PPW + (it + kStages - 1) * G);
-        cp_async_commit();
-        cp_async_wait<kStages - 1>();
-        __syncwarp();
-        const int p = start + warp * PPW + it * G + group;
-        const bool valid = p < end;
-        float kf[16], vf[16];
-        if (valid && p == pos && append) {
-            // the new token: k and v come from the projections; rotate k, append both to the cache
-            const float4* kp = reinterpret_cast<const float4*>(rowp + k_off + h * HD + gl * 16);
-            const float4* vp = reinterpret_cast<const float4*>(rowp + v_off + h * HD + gl * 16);
-#pragma unroll
-            for (int j = 0; j < 4; j++) {
-                float4 a = kp[j], c = vp[j];
-                kf[4 * j] = a.x; kf[4 * j + 1] = a.y; kf[4 * j + 2] = a.z; kf[4 * j + 3] = a.w;
-                vf[4 * j] = c.x; vf[4 * j + 1] = c.y; vf[4 * j + 2] = c.z; vf[4 * j + 3] = c.w;
-            }
-            float ck[8], sk[8];              // fetched again here (a cache hit) rather than kept live through the loop
-            load_tables(ck, sk);
-            rotate(kf, ck, sk);
-            KvIo<KT>::st16(kbase + (size_t)p * HD, kf);
-            KvIo<KT>::st16(vbase + (size_t)p * HD, vf);
-            // this step attends to what later steps will read back (the rounded values of an fp16 cache)
-#pragma unroll
-            for (int j = 0; j < 16; j++) { kf[j] = KvIo<KT>::stored(kf[j]); vf[j] = KvIo<KT>::stored(vf[j]); }
-        } else if (valid) {
-            const KT* st = ring + (size_t)(it % kStages) * kStageElems + group * HD + gl * 16;
-            KvIo<KT>::ld16_shared(st, kf);
-            KvIo<KT>::ld16_shared(st + PPW * HD, vf);
-        } else {
-#pragma unroll
-            for (int j = 0; j < 16; j++) { kf[j] = 0.0f; vf[j] = 0.0f; }
-        }
-        float dot = 0.0f;
-#pragma unroll
-        for (int j = 0; j < 16; j++) dot = fmaf(q[j], kf[j], dot);
-#pragma unroll
-        for (int o = LPP / 2; o > 0; o >>= 1) dot += __shfl_xor_sync(0xffffffffu, dot, o);
-        if (valid) {
-            const float s = dot * scale;
-            const float mn = fmaxf(m, s);
-            const float corr = expf(m - mn);
-            const float pe = expf(s - mn);
-            l = l * corr + pe;
-#pragma unroll
-            for (int j = 0; j < 16; j++) acc[j] = fmaf(pe, vf[j], acc[j] * corr);
-            m = mn;
-        }
-        __syncwarp();                             // the stage is read out before a later request may overwrite it
-    }
-    cp_async_wait<0>();
-    __syncthreads();                              // every warp is done with its ring: the bytes become the partial rows
-    const int g = warp * PPW + group;
-#pragma unroll
-    for (int j = 0; j < 16; j++) s_acc[g][gl * 16 + j] = acc[j];
-    if (gl == 0) { s_m[g] = m; s_l[g] = l; }
-    __syncthreads();
-    float* mine = ws + (((size_t)z * H + h) * splits + split) * (HD + 2);
-    for (int j = threadIdx.x; j < HD; j += blockDim.x) {
-        float M = -INFINITY;
-        for (int gg = 0; gg < G; gg++) M = fmaxf(M, s_m[gg]);
-        float a = 0.0f, L = 0.0f;
-        if (M > -INFINITY) {
-            for (int gg = 0; gg < G; gg++) {
-                const float e = expf(s_m[gg] - M);
-                a = fmaf(s_acc[gg][j], e, a);
-                L = fmaf(s_l[gg], e, L);
-            }
-        }
-        mine[j] = a;
-        if (j == 0) { mine[HD] = M; mine[HD + 1] = L; }
-    }
-    if (splits == 1) {
-        // nothing to merge
-        __syncthreads();
-        for (int j = threadIdx.x; j < HD; j += blockDim.x) out[(size_t)z * ldo + h * HD + j] = mine[j] / mine[HD + 1];
-        return;
-    }
-    // ── the last CTA of this head merges the split partials ──
-    __threadfence();
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        const int ticket = atomicAdd(&tickets[z * H + h], 1);
-        s_last = ticket == splits - 1;
-        if (s_last) tickets[z * H + h] = 0;          // ready for the next launch
-    }
-    __syncthreads();
-    if (!s_last) return;
-    __threadfence();
-    // Every thread requests its own column of up to 24 split partials together with the (m, l) pairs, so the
-    // merge costs one load round trip (more splits: further rounds of 24).
-    const float* pbase = ws + ((size_t)z * H + h) * splits * (HD + 2);
-    float* s_m2 = &s_acc[0][0];                 // reused: the CTA's own partial has been written out
-    float* s_l2 = s_m2 + kMaxSplits;
-    for (int sp = threadIdx.x; sp < splits; sp += blockDim.x) {
-        s_m2[sp] = __ldcg(pbase + (size_t)sp * (HD + 2) + HD);
-        s_l2[sp] = __ldcg(pbase + (size_t)sp * (HD + 2) + HD + 1);
-    }
-    constexpr int kBatch = 24;
-    const int j0 = threadIdx.x;                 // HD ≤ 512 = 4 columns per thread at most; the first one is prefetched here
-    float first[kBatch];
-#pragma unroll
-    for (int q = 0; q < kBatch; q++) first[q] = (j0 < HD && q < splits) ? __ldcg(pbase + (size_t)q * (HD + 2) + j0) : 0.0f;
-    __syncthreads();
-    float M = -INFINITY;
-    for (int sp = 0; sp < splits; sp++) M = fmaxf(M, s_m2[sp]);
-    float L = 0.0f;
-    for (int sp = 0; sp < splits; sp++) L = fmaf(s_l2[sp], expf(s_m2[sp] - M), L);
-    __syncthreads();
-    for (int sp = threadIdx.x; sp < splits; sp += blockDim.x) s_m2[sp] = expf(s_m2[sp] - M);
-    __syncthreads();
-    for (int j = threadIdx.x; j < HD; j += blockDim.x) {
-        float a = 0.0f;
-        for (int s0 = 0; s0 < splits; s0 += kBatch) {
-            float part[kBatch];
-            if (j == j0 && s0 == 0) {
-#pragma unroll
-                for (int q = 0; q < kBatch; q++) part[q] = first[q];
-            } else {
-#pragma unroll
-                for (int q = 0; q < kBatch; q++) part[q] = s0 + q < splits ? __ldcg(pbase + (size_t)(s0 + q) * (HD + 2) + j) : 0.0f;
-            }
-#pragma unroll
-            for (int q = 0; q < kBatch; q++) if (s0 + q < splits) a = fmaf(part[q], s_m2[s0 + q], a);
-        }
-        out[(size_t)z * ldo + h * HD + j] = a / L;
-    }
-}
-
-
-// The same step with the K/V rows travelling through registers, one group of positions ahead: the form the fp32 cache
-// keeps — its 48 KB of rings per CTA would leave no room for this kernel's CTAs to move in beside the projection kernel
-// they follow, and measured slower (0.55 against 0.51 ms per 7B token at context 2063).
-template <int LPP, typename KT>   // lanes per position = hd / 16; cache element type
-__global__ void __launch_bounds__(kAttnWarps * 32, 4) k_attn_decode_regs(
-        const float* __restrict__ qkv, int q_off, int k_off, int v_off, int ld,
-        KT* __restrict__ kcache, KT* __restrict__ vcache, int maxSeq,
-        const float* __restrict__ posbuf, const float* __restrict__ cosT, const float* __restrict__ sinT,
-        float* __restrict__ ws, int* __restrict__ tickets, float* __restrict__ out, int ldo, int H, float scale,
-        int T, int append) {
-    constexpr int HD = LPP * 16;
-    constexpr int PPW = 32 / LPP;                 // positions per warp iteration
-    constexpr int G = kAttnWarps * PPW;           // position groups per CTA
-    __shared__ float s_acc[G][HD];
-    __shared__ float s_m[G], s_l[G];
-    __shared__ int s_last;
-
-    // row z of the projection / output buffers is token t of sequence b: T = 1 (and append) for a decode step;
-    // T > 1 for a prompt chunk, whose k/v rows the append kernel has already written
-    const int split = blockIdx.x, splits = gridDim.x, h = blockIdx.y, z = blockIdx.z;
-    const int b = z / T, tok = z - b * T;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int group = lane / LPP, gl = lane % LPP;
-    // The cache rows below the current position were written by earlier steps, not by the kernel
-    // this one depends on, so the first group of K/V rows is fetched BEFORE the wait and streams in
-    // while the projection kernel drains.  The position read here is re-read after the wait; in the
-    // (never observed) case that it moved, the speculative rows are dropped and fetched again.
-    const int half = HD >> 1;
-    auto read_pos = [&]() {
-        int v = (int)__ldcg(posbuf + b) + tok;
-        return v < 0 ? 0 : (v >= maxSeq ? maxSeq - 1 : v);
-    };
-    int pos = read_pos();
-    int seq = pos + 1;
-    int chunk = (seq + splits - 1) / splits;
-    int start = split * chunk;
-    int end = min(seq, start + chunk);
-    KT* kbase = kcache + ((size_t)b * H + h) * maxSeq * HD + gl * 16;
-    KT* vbase = vcache + ((size_t)b * H + h) * maxSeq * HD + gl * 16;
-    float kf[16], vf[16], kn[16], vn[16];
-    auto fetch_cached = [&](int p, bool valid, float (&kx)[16], float (&vx)[16]) {
-        if (valid) {
-            KvIo<KT>::ld16_stream(kbase + (size_t)p * HD, kx);
-            KvIo<KT>::ld16_stream(vbase + (size_t)p * HD, vx);
-        } else {
-#pragma unroll
-            for (int j = 0; j < 16; j++) { kx[j] = 0.0f; vx[j] = 0.0f; }
-        }
-    };
-    {
-        const int p0 = start + warp * PPW + group;
-        fetch_cached(p0, T == 1 && p0 < end && p0 != pos, kf, vf);      // a chunk's own rows were written by the kernel before this one
-    }
-    // the rotation tables are constants: the row of the speculative position is fetched before the wait too
-    float cs[8], sn[8];
-    auto load_tables = [&](float (&cs)[8], float (&sn)[8]) {
-        const float4* cp = reinterpret_cast<const float4*>(cosT + (size_t)pos * half + gl * 8);
-        const float4* sp = reinterpret_cast<const float4*>(sinT + (size_t)pos * half + gl * 8);
-#pragma unroll
-        for (int j = 0; j < 2; j++) {
-            const float4 c4 = cp[j], s4 = sp[j];
-            cs[4 * j] = c4.x; cs[4 * j + 1] = c4.y; cs[4 * j + 2] = c4.z; cs[4 * j + 3] = c4.w;
-            sn[4 * j] = s4.x; sn[4 * j + 1] = s4.y; sn[4 * j + 2] = s4.z; sn[4 * j + 3] = s4.w;
-        }
-    };
-    load_tables(cs, sn);
-    const int specPos = pos;
-    pdl_wait();
-    pdl_launch_dependents();
-    // the query row does not depend on the position: its loads go out together with the position's
-    const float* rowp = qkv + (size_t)z * ld;
-    float q[16];
-    {
-        const float4* qp = reinterpret_cast<const float4*>(rowp + q_off + h * HD + gl * 16);
-#pragma unroll
-        for (int j = 0; j < 4; j++) { float4 v = qp[j]; q[4 * j] = v.x; q[4 * j + 1] = v.y; q[4 * j + 2] = v.z; q[4 * j + 3] = v.w; }
-    }
-    pos = read_pos();
-    if (pos != specPos) load_tables(cs, sn);
-    seq = pos + 1;
-    chunk = (seq + splits - 1) / splits;
-    start = split * chunk;
-    end = min(seq, start + chunk);
-
-    // rotate 8 interleaved pairs held in v[16] by the table row of the current position (cs, sn)
-    auto rotate = [&](float (&v)[16], const float (&cs)[8], const float (&sn)[8]) {
-#pragma unroll
-        for (int i = 0; i < 8; i++) {
-            const float x0 = v[2 * i], x1 = v[2 * i + 1];
-            v[2 * i] = x0 * cs[i] - x1 * sn[i];
-            v[2 * i + 1] = x0 * sn[i] + x1 * cs[i];
-        }
-    };
-    rotate(q, cs, sn);
-
-    // K or V slice of a cached position p for this lane (zeros when the lane has no position)
-    auto load_k = [&](int p, bool valid, float (&kx)[16]) {
-        if (valid) KvIo<KT>::ld16_stream(kbase + (size_t)p * HD, kx);
-        else {
-#pragma unroll
-            for (int j = 0; j < 16; j++) kx[j] = 0.0f;
-        }
-    };
-    auto load_v = [&](int p, bool valid, float (&vx)[16]) {
-        if (valid) KvIo<KT>::ld16_stream(vbase + (size_t)p * HD, vx);
-        else {
-#pragma unroll
-            for (int j = 0; j < 16; j++) vx[j] = 0.0f;
-        }
+        for (int c = 0; c < 4; c++)
+            v[c] = make_float4(v[c].x * cs[c].x - v[c].y * sn[c].x, v[c].x * sn[c].x + v[c].y * cs[c].x, v[c].z * cs[c].y - v[c].w * sn[c].y,
+                               v[c].z * sn[c].y + v[c].w * cs[c].y);
     };
 
     float m = -INFINITY, l = 0.0f, acc[16];
 #pragma unroll
-    for (int j = 0; j < 16; j++) acc[j] = 0.0f;
-    auto fold = [&](bool valid, float dot, const float (&vx)[16]) {
+    for (int e = 0; e < 16; e++) acc[e] = 0.0f;
+    const bool folds = ownsNew && warp == 0;      // warp-uniform
+    if (folds) { load_row(p.k_off, kx); load_row(p.v_off, vx); }
+    rotate(q);
+    // one group of positions a time: the new token's first (lane group 0), then what the ring holds
+#pragma unroll 1
+    for (bool fresh = folds; fresh || base < endc; fresh = false) {
+        bool valid = fresh ? group == 0 : base + group < endc;
+        if (fresh) {
+            // k and v come from the projections; k is rotated, both are appended to the cache, and this step attends to what
+            // later steps will read back (the rounded values of an fp16 cache)
+            rotate(kx);
+#pragma unroll
+            for (int c = 0; c < 4; c++) {
+                if (valid) {
+                    KvIo<KT>::st4(khead + (size_t)pos * HD + 4 * (c * LPP + gl), kx[c]);
+                    KvIo<KT>::st4(vhead + (size_t)pos * HD + 4 * (c * LPP + gl), vx[c]);
+                }
+                kx[c] = make_float4(KvIo<KT>::stored(kx[c].x), KvIo<KT>::stored(kx[c].y), KvIo<KT>::stored(kx[c].z), KvIo<KT>::stored(kx[c].w));
+                vx[c] = make_float4(KvIo<KT>::stored(vx[c].x), KvIo<KT>::stored(vx[c].y), KvIo<KT>::stored(vx[c].z), KvIo<KT>::stored(vx[c].w));
+            }
+        } else {
+            const KT* item = reinterpret_cast<const KT*>(ring + (size_t)warp * (kStages * 2 * kPlane) + (taken % kStages) * (2 * kPlane)) + group * HD + 4 * gl;
+            take();
+#pragma unroll
+            for (int c = 0; c < 4; c++) { kx[c] = KvIo<KT>::ld4_shared(item + c * (4 * LPP)); vx[c] = KvIo<KT>::ld4_shared(item + PPW * HD + c * (4 * LPP)); }
+        }
+        float d[4];
+#pragma unroll
+        for (int c = 0; c < 4; c++) d[c] = fmaf(q[c].w, kx[c].w, fmaf(q[c].z, kx[c].z, fmaf(q[c].y, kx[c].y, q[c].x * kx[c].x)));
+        float dot = (d[0] + d[1]) + (d[2] + d[3]);
 #pragma unroll
         for (int o = LPP / 2; o > 0; o >>= 1) dot += __shfl_xor_sync(0xffffffffu, dot, o);
         if (valid) {
-            const float s = dot * scale;
-            const float mn = fmaxf(m, s);
-            const float corr = expf(m - mn);
-            const float pe = expf(s - mn);
+            const float sc = dot * p.scale, mn = fmaxf(m, sc), corr = expf(m - mn), pe = expf(sc - mn);
             l = l * corr + pe;
 #pragma unroll
-            for (int j = 0; j < 16; j++) acc[j] = fmaf(pe, vx[j], acc[j] * corr);
+            for (int c = 0; c < 4; c++) {
+                acc[4 * c] = fmaf(pe, vx[c].x, acc[4 * c] * corr);
+                acc[4 * c + 1] = fmaf(pe, vx[c].y, acc[4 * c + 1] * corr);
+                acc[4 * c + 2] = fmaf(pe, vx[c].z, acc[4 * c + 2] * corr);
+                acc[4 * c + 3] = fmaf(pe, vx[c].w, acc[4 * c + 3] * corr);
+            }
             m = mn;
         }
-    };
+        if (!fresh) {
+            base += G;
+            __syncwarp();                         // the slot is read out before a later request may overwrite it
+            if (at < endc) request();
+        }
+    }
 
-    // The cached rows: two groups of positions travel in two register sets.  A set's K registers are reloaded (two
-    // groups ahead) as soon as the dot product has read them, its V registers as soon as the accumulation has: between
-    // one and two groups of rows are in flight per warp at any time, with no register copies.  The new token's own
-    // position (the last one of the last split) is not in the cache yet and is folded in after the loop.
-    const bool ownsNew = append && pos >= start && pos < end;
-    const int endc = ownsNew ? pos : end;
-    int base = start + warp * PPW;
-    if (base < endc) {
-        const int p0 = base + group;
-        if (T > 1 || pos != specPos) {                                   // a prompt chunk, or a dropped speculation
-            load_k(p0, p0 < endc, kf);
-            load_v(p0, p0 < endc, vf);
+    // the warp's groups → one row per warp → the block's
+    {
+        float M = m;
+#pragma unroll
+        for (int o = LPP; o < 32; o <<= 1) M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, o));
+        const float f = m > -INFINITY ? expf(m - M) : 0.0f;
+        l *= f;
+#pragma unroll
+        for (int e = 0; e < 16; e++) acc[e] *= f;
+#pragma unroll
+        for (int o = LPP; o < 32; o <<= 1) {
+            l += __shfl_xor_sync(0xffffffffu, l, o);
+#pragma unroll
+            for (int e = 0; e < 16; e++) acc[e] += __shfl_xor_sync(0xffffffffu, acc[e], o);
         }
-        if (base + G < endc) {
-            load_k(base + G + group, base + G + group < endc, kn);
-            load_v(base + G + group, base + G + group < endc, vn);
+        if (group == 0) {
+#pragma unroll
+            for (int c = 0; c < 4; c++)
+                *reinterpret_cast<float4*>(&s_acc[warp][4 * (c * LPP + gl)]) = make_float4(acc[4 * c], acc[4 * c + 1], acc[4 * c + 2], acc[4 * c + 3]);
         }
+        if (lane == 0) { s_m[warp] = M; s_l[warp] = l; }
     }
-    auto consume = [&](float (&kx)[16], float (&vx)[16], int at, int reload) {
-        float dot = 0.0f;
-#pragma unroll
-        for (int j = 0; j < 16; j++) dot = fmaf(q[j], kx[j], dot);
-        if (reload < endc) load_k(reload + group, reload + group < endc, kx);
-        fold(at + group < endc, dot, vx);
-        if (reload < endc) load_v(reload + group, reload + group < endc, vx);
-    };
-    for (; base < endc; base += 2 * G) {
-        consume(kf, vf, base, base + 2 * G);
-        if (base + G >= endc) break;
-        consume(kn, vn, base + G, base + 3 * G);
-    }
-    if (ownsNew && warp == 0) {                                          // warp-uniform
-        // the new token: k and v come from the projections; k is rotated, both are appended to the cache, and this step
-        // attends to what later steps will read back (the rounded values of an fp16 cache).  Lane group 0 does it.
-        const bool mine = group == 0;
-        if (mine) {
-            const float4* kp = reinterpret_cast<const float4*>(rowp + k_off + h * HD + gl * 16);
-            const float4* vp = reinterpret_cast<const float4*>(rowp + v_off + h * HD + gl * 16);
-#pragma unroll
-            for (int j = 0; j < 4; j++) {
-                float4 a = kp[j], c = vp[j];
-                kf[4 * j] = a.x; kf[4 * j + 1] = a.y; kf[4 * j + 2] = a.z; kf[4 * j + 3] = a.w;
-                vf[4 * j] = c.x; vf[4 * j + 1] = c.y; vf[4 * j + 2] = c.z; vf[4 * j + 3] = c.w;
-            }
-            float ck[8], sk[8];              // fetched again here (a cache hit) rather than kept live through the loop
-            load_tables(ck, sk);
-            rotate(kf, ck, sk);
-            KvIo<KT>::st16(kbase + (size_t)pos * HD, kf);
-            KvIo<KT>::st16(vbase + (size_t)pos * HD, vf);
-#pragma unroll
-            for (int j = 0; j < 16; j++) { kf[j] = KvIo<KT>::stored(kf[j]); vf[j] = KvIo<KT>::stored(vf[j]); }
-        }
-        float dot = 0.0f;
-#pragma unroll
-        for (int j = 0; j < 16; j++) dot = fmaf(q[j], kf[j], dot);
-        fold(mine, dot, vf);
-    }
-    const int g = warp * PPW + group;
-#pragma unroll
-    for (int j = 0; j < 16; j++) s_acc[g][gl * 16 + j] = acc[j];
-    if (gl == 0) { s_m[g] = m; s_l[g] = l; }
     __syncthreads();
-    float* mine = ws + (((size_t)z * H + h) * splits + split) * (HD + 2);
-    for (int j = threadIdx.x; j < HD; j += blockDim.x) {
-        float M = -INFINITY;
-        for (int gg = 0; gg < G; gg++) M = fmaxf(M, s_m[gg]);
-        float a = 0.0f, L = 0.0f;
-        if (M > -INFINITY) {
-            for (int gg = 0; gg < G; gg++) {
-                const float e = expf(s_m[gg] - M);
-                a = fmaf(s_acc[gg][j], e, a);
-                L = fmaf(s_l[gg], e, L);
-            }
-        }
-        mine[j] = a;
-        if (j == 0) { mine[HD] = M; mine[HD + 1] = L; }
-    }
+    float M = fmaxf(fmaxf(s_m[0], s_m[1]), fmaxf(s_m[2], s_m[3])), L = 0.0f, w[kAttnWarps];
+#pragma unroll
+    for (int i = 0; i < kAttnWarps; i++) { w[i] = s_m[i] > -INFINITY ? expf(s_m[i] - M) : 0.0f; L = fmaf(s_l[i], w[i], L); }
+    auto blocks = [&](int j) {                    // column j of the block's sum
+        float a = 0.0f;
+#pragma unroll
+        for (int i = 0; i < kAttnWarps; i++) a = fmaf(s_acc[i][j], w[i], a);
+        return a;
+    };
+    float* const orow = p.out + (size_t)z * p.ldo + h * HD;
     if (splits == 1) {
-        // nothing to merge
-        __syncthreads();
-        for (int j = threadIdx.x; j < HD; j += blockDim.x) out[(size_t)z * ldo + h * HD + j] = mine[j] / mine[HD + 1];
+#pragma unroll 1
+        for (int j = tid; j < HD; j += kAttnWarps * 32) orow[j] = blocks(j) / L;
         return;
     }
-    // ── the last CTA of this head merges the split partials ──
+    if constexpr (CLUSTER) {
+        asm volatile("barrier.cluster.wait.aligned;" ::: "memory");      // every block of the cluster is running
+        uint32_t to;
+        asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(to) : "r"(smem_u32(&s_part[split][0])));
+        auto put = [&](int j, float v) { asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(to + 4 * j), "f"(v) : "memory"); };
+#pragma unroll 1
+        for (int j = tid; j < HD; j += kAttnWarps * 32) put(j, blocks(j));
+        if (tid == 0) { put(HD, M); put(HD + 1, L); }
+        asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+        if (split != 0) return;
+        asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+        M = -INFINITY;
+#pragma unroll 1
+        for (int i = 0; i < splits; i++) M = fmaxf(M, s_part[i][HD]);
+#pragma unroll 1
+        for (int j = tid; j < HD; j += kAttnWarps * 32) {
+            float a = 0.0f;
+            L = 0.0f;
+#pragma unroll 1
+            for (int i = 0; i < splits; i++) {
+                const float e = expf(s_part[i][HD] - M);                 // an empty split: exp(−inf) = 0
+                a = fmaf(s_part[i][j], e, a);
+                L = fmaf(s_part[i][HD + 1], e, L);
+            }
+            orow[j] = a / L;
+        }
+        return;
+    }
+    // ── the last block of this head merges the split partials ──
+    const float* const records = p.ws + ((size_t)z * p.H + h) * splits * (HD + 2);
+    float* const record = p.ws + (((size_t)z * p.H + h) * splits + split) * (HD + 2);
+#pragma unroll 1
+    for (int j = tid; j < HD; j += kAttnWarps * 32) record[j] = blocks(j);
+    if (tid == 0) { record[HD] = M; record[HD + 1] = L; }
     __threadfence();
     __syncthreads();
-    if (threadIdx.x == 0) {
-        const int ticket = atomicAdd(&tickets[z * H + h], 1);
+    if (tid == 0) {
+        const int ticket = atomicAdd(&p.tickets[z * p.H + h], 1);
         s_last = ticket == splits - 1;
-        if (s_last) tickets[z * H + h] = 0;          // ready for the next launch
+        if (s_last) p.tickets[z * p.H + h] = 0;   // ready for the next launch
     }
     __syncthreads();
     if (!s_last) return;
     __threadfence();
-    // Every thread requests its own column of up to 24 split partials together with the (m, l) pairs, so the
-    // merge costs one load round trip (more splits: further rounds of 24).
-    const float* pbase = ws + ((size_t)z * H + h) * splits * (HD + 2);
-    float* s_m2 = &s_acc[0][0];                 // reused: the CTA's own partial has been written out
-    float* s_l2 = s_m2 + kMaxSplits;
-    for (int sp = threadIdx.x; sp < splits; sp += blockDim.x) {
-        s_m2[sp] = __ldcg(pbase + (size_t)sp * (HD + 2) + HD);
-        s_l2[sp] = __ldcg(pbase + (size_t)sp * (HD + 2) + HD + 1);
-    }
-    constexpr int kBatch = 24;
-    const int j0 = threadIdx.x;                 // HD ≤ 512 = 4 columns per thread at most; the first one is prefetched here
+    // every thread asks for its column of the first splits together with the (m, l) pairs: one load round trip for most
+    constexpr int kBatch = 20;
     float first[kBatch];
 #pragma unroll
-    for (int q = 0; q < kBatch; q++) first[q] = (j0 < HD && q < splits) ? __ldcg(pbase + (size_t)q * (HD + 2) + j0) : 0.0f;
+    for (int i = 0; i < kBatch; i++) first[i] = tid < HD && i < splits ? __ldcg(records + (size_t)i * (HD + 2) + tid) : 0.0f;
+    M = -INFINITY;
+#pragma unroll 1
+    for (int i = lane; i < splits; i += 32) M = fmaxf(M, __ldcg(records + (size_t)i * (HD + 2) + HD));
+    for (int o = 16; o > 0; o >>= 1) M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, o));
+    L = 0.0f;
+#pragma unroll 1
+    for (int i = lane; i < splits; i += 32) {     // every warp for itself; the first one leaves the weights
+        const float e = expf(__ldcg(records + (size_t)i * (HD + 2) + HD) - M);
+        L = fmaf(__ldcg(records + (size_t)i * (HD + 2) + HD + 1), e, L);
+        if (warp == 0) s_w[i] = e;
+    }
+    for (int o = 16; o > 0; o >>= 1) L += __shfl_xor_sync(0xffffffffu, L, o);
     __syncthreads();
-    float M = -INFINITY;
-    for (int sp = 0; sp < splits; sp++) M = fmaxf(M, s_m2[sp]);
-    float L = 0.0f;
-    for (int sp = 0; sp < splits; sp++) L = fmaf(s_l2[sp], expf(s_m2[sp] - M), L);
-    __syncthreads();
-    for (int sp = threadIdx.x; sp < splits; sp += blockDim.x) s_m2[sp] = expf(s_m2[sp] - M);
-    __syncthreads();
-    for (int j = threadIdx.x; j < HD; j += blockDim.x) {
+    for (int j = tid; j < HD; j += kAttnWarps * 32) {
         float a = 0.0f;
-        for (int s0 = 0; s0 < splits; s0 += kBatch) {
-            float part[kBatch];
-            if (j == j0 && s0 == 0) {
+        if (j == tid) {
 #pragma unroll
-                for (int q = 0; q < kBatch; q++) part[q] = first[q];
-            } else {
-#pragma unroll
-                for (int q = 0; q < kBatch; q++) part[q] = s0 + q < splits ? __ldcg(pbase + (size_t)(s0 + q) * (HD + 2) + j) : 0.0f;
-            }
-#pragma unroll
-            for (int q = 0; q < kBatch; q++) if (s0 + q < splits) a = fmaf(part[q], s_m2[s0 + q], a);
+            for (int i = 0; i < kBatch; i++) if (i < splits) a = fmaf(first[i], s_w[i], a);
         }
-        out[(size_t)z * ldo + h * HD + j] = a / L;
+#pragma unroll 8
+        for (int i = j == tid ? kBatch : 0; i < splits; i++) a = fmaf(__ldcg(records + (size_t)i * (HD + 2) + j), s_w[i], a);
+        orow[j] = a / L;
     }
 }
-
-
 
 // ───────────── prompt chunks: tiled causal attention ─────────────
 // Row-wise decode attention re-reads every key once per query row.  For a chunk of T ≥ 32 tokens this kernel
@@ -758,22 +526,16 @@ void launch_attn_decode_t(const AttnDecodeArgs& a, cudaStream_t s) {
         }
         return;
     }
-    const int append = T == 1 ? 1 : 0;
-    int* tickets = a.tickets;
-    // fp16 cache: K/V stream through warp-private rings in dynamic shared memory (3 stages × 1024 elements each, reused for
-    // the partial rows afterwards); fp32 cache: through registers (k_attn_decode_regs)
-    const size_t smem = std::max<size_t>((size_t)kAttnWarps * 3 * 1024 * sizeof(KT), (size_t)(4 * 512 + 2 * 4 * 32) * sizeof(float));
-#define DJ_ATTN_CASE(L)                                                                                              \
-    case L: {                                                                                                        \
-        static bool attr = false;                                                                                    \
-        if (!attr) { DJ_CUDA_CHECK(cudaFuncSetAttribute(k_attn_decode<L, KT>, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024)); attr = true; } \
-        if (sizeof(KT) == 2)                                                                                         \
-            launch_k(k_attn_decode<L, KT>, grid, block, smem, s, true, (const float*)a.qkv, a.q_off, a.k_off, a.v_off, a.ld, \
-                     kc, vc, a.maxSeq, a.pos, a.cosT, a.sinT, a.ws, tickets, a.out, a.ldo, a.H, a.scale, T, append); \
-        else                                                                                                         \
-            launch_k(k_attn_decode_regs<L, KT>, grid, block, 0, s, true, (const float*)a.qkv, a.q_off, a.k_off, a.v_off, a.ld, \
-                     kc, vc, a.maxSeq, a.pos, a.cosT, a.sinT, a.ws, tickets, a.out, a.ldo, a.H, a.scale, T, append); \
-    } break;
+    AttnDecodeParams p = {a.qkv, a.q_off, a.k_off, a.v_off, a.ld, kc, vc, a.maxSeq, a.pos, a.cosT, a.sinT, a.ws, a.tickets, a.out, a.ldo, a.H, a.scale, T,
+                          T == 1 ? 1 : 0, g_dev_error};
+    const size_t smem = (size_t)kAttnWarps * kRingStages<KT> * 1024 * sizeof(KT);
+    // a few splits merge through the first block's shared memory instead of a ticket, a fence and a round trip to the partials
+    const bool cluster = a.splits > 1 && a.splits <= kClusterSplits;
+    auto go = [&](auto kernel) {
+        DJ_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024));
+        launch_k_cluster(kernel, grid, block, smem, s, cluster ? (unsigned)a.splits : 1u, p);
+    };
+#define DJ_ATTN_CASE(L) case L: if (cluster) go(k_attn_decode<L, KT, true>); else go(k_attn_decode<L, KT, false>); break;
     switch (lpp) {
         DJ_ATTN_CASE(1) DJ_ATTN_CASE(2) DJ_ATTN_CASE(4) DJ_ATTN_CASE(8) DJ_ATTN_CASE(16) DJ_ATTN_CASE(32)
     }

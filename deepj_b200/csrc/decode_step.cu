@@ -25,10 +25,9 @@
 // small bulk copy per warp the issuing warp stalled ≈ 450 cycles per copy.  The tile-major copy
 // costs the plan as much memory again as the Q8 weights it covers.
 //
-// The arithmetic is the per-operator kernels' (q8_gemv_i8.cu, attn.cu), instruction for
-// instruction: int8 codes as the A operand of mma.sync m16n8k32, activations as three base-256
-// digit columns with a power-of-two scale per 32-k block, split-KV attention with a ticket merge —
-// at the same tile, warp and split assignments, so one GPU produces the same bits either way.
+// The arithmetic is the per-operator kernels' (q8_gemv_tma.cu, attn.cu): int8 codes as the A operand of mma.sync
+// m16n8k32, activations as three base-256 digit columns with a power-of-two scale per 32-k block, split-KV attention;
+// sums are formed in another order, so the results agree to fp32 rounding.
 //
 // A CTA's 16 warps work as two halves of 8 (each half owns a weight-row tile at a time, like one
 // CTA of the GEMV kernel; the halves share the staged activations) and, in the attention phase,
@@ -1020,8 +1019,8 @@ __global__ void __launch_bounds__(kThreads, 1) k_decode_step(const DsParams p) {
 // 1024 + (2r + b)·4).  Rows past N repeat the last row (their results are never written); the missing second block
 // of an odd last pair is zeros with scale 0.  With codes2 != null a tile is 8 gate rows then 8 up rows.
 __global__ void k_pack_phase(const int8_t* __restrict__ codes, const float* __restrict__ scales, const int8_t* __restrict__ codes2,
-                             const float* __restrict__ scales2, int K, int N, unsigned char* __restrict__ out) {
-    const int nBlocks = K >> 5, nPairs = (nBlocks + 1) >> 1, nb = nBlocks;
+                             const float* __restrict__ scales2, int K, int N, int nb, unsigned char* __restrict__ out) {
+    const int nBlocks = K >> 5, nPairs = (nBlocks + 1) >> 1;
     const int tile = blockIdx.y, pi = blockIdx.x, i = threadIdx.x;
     const bool sw = codes2 != nullptr;
     const int rpt = sw ? 8 : 16;
@@ -1055,7 +1054,7 @@ size_t packed_bytes(int K, int N, bool swiglu) {
 void pack_phase(const Q8View& w, const Q8View* w2, unsigned char* out, cudaStream_t s) {
     const int rpt = w2 ? 8 : 16;
     const dim3 grid((unsigned)(((w.K >> 5) + 1) >> 1), (unsigned)((w.N + rpt - 1) / rpt));
-    k_pack_phase<<<grid, 96, 0, s>>>(w.codes, w.scales, w2 ? w2->codes : nullptr, w2 ? w2->scales : nullptr, w.K, w.N, out);
+    k_pack_phase<<<grid, 96, 0, s>>>(w.codes, w.scales, w2 ? w2->codes : nullptr, w2 ? w2->scales : nullptr, w.K, w.N, w.nb, out);
     DJ_CUDA_CHECK(cudaGetLastError());
 }
 

@@ -30,7 +30,7 @@ extern int g_num_sms;
 // When true, launchers attach the programmatic-dependent-launch attribute so that
 // a kernel's weight prefetch overlaps the tail of its predecessor.
 extern bool g_use_pdl;
-// Q8 GEMV kernel choice (environment DEEPJ_CUDA_GEMV = cpasync | fma to step down); shapes outside a
+// Q8 GEMV kernel choice (environment DEEPJ_CUDA_GEMV = cpasync | fma to step down: without the TMA kernels, without any tensor-pipe kernel); shapes outside a
 // kernel's domain fall through to the next one.
 extern int g_gemv_mode;
 extern int g_tc_terms;      // deepj_cuda_tc_configure
@@ -43,7 +43,8 @@ extern long long g_trace_launches;
 unsigned long long* trace_slot();
 
 // A Q8 weight as laid out in HBM: codes[N][Kp] int8 (Kp = K rounded up to 16, zero
-// padded) followed by scales[N][nb] fp32, nb = ceil(K/32).
+// padded) followed by scales[N][nb] fp32, nb = ceil(K/32) rounded up to 4 (a row of scales starts on a 16-byte boundary, as
+// tensor copies want it; zero padded).
 struct Q8View {
     const int8_t* codes;
     const float* scales;
@@ -91,9 +92,7 @@ struct Q8LinearArgs {
     const float* beta = nullptr; int act = 0; float* ln_ws = nullptr;
 };
 DJ_PART void launch_q8_linear(const Q8LinearArgs& a, cudaStream_t s);
-DJ_PART bool launch_q8_gemv_i8(const Q8LinearArgs& a, cudaStream_t s);
-DJ_PART bool launch_q8_gemv_tma(const Q8LinearArgs& a, cudaStream_t s);     // K a multiple of 128; false = outside its domain
-DJ_PART bool q8_gemv_i8_fuses_gpt(const Q8LinearArgs& a);     // true when launch_q8_gemv_i8 can take beta / act itself
+DJ_PART bool launch_q8_gemv_tma(const Q8LinearArgs& a, cudaStream_t s);     // false = outside its domain
 DJ_PART void launch_layernorm_rows(const float* x, int ldx, const float* gamma, const float* beta, float eps, float* out, int K, int M, cudaStream_t s);
 DJ_PART void launch_gelu_rows(float* buf, int ld, int N, int M, cudaStream_t s);
 DJ_PART bool launch_q8_linear_batch(const Q8LinearArgs& a, int m0, int rows, float* ws, int* tickets, cudaStream_t s);
@@ -313,6 +312,24 @@ int runtime_device();
 void invalidate_graphs();
 void set_last_error(const std::string& msg);
 
+// The same with clusters of `cluster` blocks along x and the PDL attribute.
+template <typename... KArgs, typename... Args>
+inline void launch_k_cluster(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, unsigned cluster, Args... args) {
+    g_launches++;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid; cfg.blockDim = block; cfg.dynamicSmemBytes = smem; cfg.stream = s;
+    cudaLaunchAttribute attr[2];
+    if (g_use_pdl) {
+        attr[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[cfg.numAttrs++].val.programmaticStreamSerializationAllowed = 1;
+    }
+    if (cluster > 1) {
+        attr[cfg.numAttrs].id = cudaLaunchAttributeClusterDimension;
+        attr[cfg.numAttrs].val.clusterDim.x = cluster; attr[cfg.numAttrs].val.clusterDim.y = 1; attr[cfg.numAttrs++].val.clusterDim.z = 1;
+    }
+    cfg.attrs = attr;
+    DJ_CUDA_CHECK(cudaLaunchKernelEx(&cfg, kernel, KArgs(args)...));
+}
 // Launch helper: plain <<<>>> or cudaLaunchKernelEx with the PDL attribute.
 template <typename... KArgs, typename... Args>
 inline void launch_k(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, bool pdl, Args... args) {

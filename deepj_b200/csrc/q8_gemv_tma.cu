@@ -1,23 +1,25 @@
-// Q8 GEMV on the integer tensor pipe with warp-private TMA rings — the decode hot kernel for up to two
-// activation rows per pass, for reduction lengths that are multiples of 128.
+// Q8 GEMV on the integer tensor pipe with warp-private TMA rings — the decode kernel for up to four activation rows per pass, for
+// reduction lengths that are multiples of 32.
 //
-// Same arithmetic as the cp.async kernel (q8_gemv_i8.cu: one int8 MMA m16n8k32 per 32-k block of 16 weight
-// rows, activations as three base-256 digit columns with a power-of-two block scale, exact integer block sums,
-// fp32 accumulation of (weight scale × activation scale) × sum), but the weights reach shared memory through the
-// tensor-memory accelerator instead of the load/store unit: one lane of a warp issues four tiled bulk copies per
-// item (two 8-row × 128-byte boxes of codes, two 8-row × 4 boxes of scales, straight from the [N][K] / [N][K/32]
-// layout of the format, 128-byte swizzle) that complete on a warp-private mbarrier, and the warp reads its MMA
-// operands with one ldmatrix.x4 per block.  Measured on the cp.async kernel: its copies landed in shared memory
-// sector by sector (≈ 11 wavefronts per 512-byte instruction, 58 % of all shared-memory wavefronts of the kernel)
-// and held the load/store pipe near saturation in the streaming phase, so the kernel ran at the same speed from
-// L2 as from HBM; here the pipe carries the operand reads only, and the conversion of the block sums to fp32 is
-// an integer add and a subtraction on the main pipes instead of a conversion-unit instruction.
+// One int8 MMA m16n8k32 per 32-k block of 16 weight rows; the codes are the A operand as they are, the activations three
+// base-256 digit columns with a power-of-two block scale; the integer block sums are exact, converted to fp32 exactly (an
+// integer add and a subtraction on the main pipes) and (weight scale × activation scale) × sum is accumulated in fp32.  One
+// lane of a warp issues four tiled bulk copies per item (two 8-row × 128-byte boxes of codes, two 8-row × 4 boxes of scales,
+// straight from the [N][K] / [N][K/32] layout of the format, 128-byte swizzle; boxes of 16 rows took 25 % longer in long
+// streams) that complete on a warp-private mbarrier, and the warp reads its MMA operands with one ldmatrix.x4 per block.
 //
-// Two CTAs of 8 warps per SM as before (the next kernel's CTAs move in while this one drains); warp w owns the
-// 128-k groups w, w+8, … of every tile of its CTA and stages exactly those groups of the activations itself;
-// two items (2304 bytes each) per warp in flight.  Projections with a fused LayerNorm or GELU (GPT blocks) stay on
-// the cp.async kernel.
+// Two blocks of 8 warps per SM; warp w owns the 128-k groups w, w+8, … of every tile of its block and stages exactly those groups of the
+// activations itself; its sums of a tile, the digits recombined, go to shared memory, and one barrier per 16 tiles (or at the
+// end) stands between them and the outputs.  (One block per SM with rings twice as deep: 5.9 against 4.7 ms for eight 7B steps, 8 warps
+// do not keep up with the stream.)  A launch of a few microseconds runs most of its code once, and fetching 1 KB of code
+// that another kernel has displaced takes 0.15 µs: the conversion is a loop over four groups in registers, rows that do not come in 16-byte
+// pieces take the FMA kernel.  Measured from the dependency wait to the last block's end, against the kernel with everything
+// unrolled and a barrier per tile: 2048 → 2048 1.9-2.6 µs (1.9-2.9), gate and up of 5632 5.9 (7.6), 5632 → 2048 5.7 (6.0), head of
+// 32000 × 2048 13.2 (15.6), gate and up of 11008 × 4096 18.0 (19.2), 4096 → 4096 4.0 (5.2).  GPT blocks (LayerNorm, GELU, reduction lengths of 1600)
+// came from a cp.async kernel of 8.0 µs per launch: gpt2xl_request 9.5 → 8.5 ms.
 #include <cuda.h>
+
+#include <algorithm>
 
 #include "kernels.h"
 #include "q8_common.cuh"
@@ -34,107 +36,171 @@ constexpr int kItemK = kTmaItemK;
 constexpr int kCodeBytes = 16 * kItemK;             // 16 rows × 128 code bytes, two 1024-byte swizzle atoms
 constexpr int kScaleBytes = 16 * 16;                // 16 rows × 4 block scales
 constexpr int kItemBytes = kCodeBytes + kScaleBytes;
-// Three items per warp: a deeper ring measured no faster back to back (the kernel waits on the handoff and on the
-// activations, not on bytes in flight) and slower inside the decode step, where a CTA pair of 2 × 96 KB and more takes
-// the L1 capacity that the attention kernel beside it uses.
-constexpr int kDepth = 3;
+constexpr int kMaxDepth = 4;
+constexpr int kChunk = 16;                          // tiles × activation rows between two barriers
 constexpr int kSpinLimit = 1 << 22;                 // polls of one item's barrier before the kernel gives up on it
 constexpr int kErrTmaWait = 330;                    // device error code: an item never arrived
 
 struct GemvTmaParams {
     CUtensorMap codes, scales, codes2, scales2;     // boxes of 8 rows; the second pair is the SwiGLU up projection
     const float* x; int ldx;
-    const float* gamma; float eps;
+    const float* gamma; const float* beta; float eps;      // beta: LayerNorm instead of RMSNorm
     const float* bias; const float* bias2;
     const float* residual; int ldr;
     float* out; int ldo;
-    int K, N, M;
-    int pre;                        // ring items a warp fetches before it waits for the previous kernel
+    int K, N, M, act;               // act 1: GELU behind the bias
+    int share, extra, depth;        // granules of 8 rows per block; the first `extra` blocks have one more; ring items per warp
     int* error;
     unsigned long long* trace;
 };
 
+__device__ __noinline__ float gelu_call(float v) { return gelu_ref(v); }
+
 // NM = 2 takes three or four activation rows in one pass over the weights (a second MMA per block).
-template <bool SWIGLU, int DEPTH, int NM>
+template <bool SWIGLU, int NM, bool GPT>
 __global__ void __launch_bounds__(kThreads, 2) k_q8_gemv_tma(const __grid_constant__ GemvTmaParams p) {
     extern __shared__ unsigned char smem_raw[];
-    __shared__ __align__(8) unsigned long long s_bar[kWarps * DEPTH];
-    __shared__ float s_ss[4 * kWarps];               // the warps' parts of Σx² per activation row (RMSNorm in the epilogue)
-    // layout (from a 1024-byte boundary, which the swizzle pattern wants): code rings [warps][DEPTH][2048], scale rings
-    // [warps][DEPTH][256], digits int8 [3M][K+pad], block scales fp32 [M][K/32], partials [2][warps][NM][16][8]
+    __shared__ __align__(8) unsigned long long s_bar[kWarps * kMaxDepth];
+    __shared__ __align__(16) float s_mean[GPT ? 4 * kWarps : 4];
+    __shared__ __align__(16) float s_ss[4 * kWarps]; // the warps' parts of Σx² per activation row (RMSNorm at the output)
+    // layout (from a 1024-byte boundary, which the swizzle pattern wants): code rings [warps][depth][2048], scale rings
+    // [warps][depth][256], digits int8 [3M][K+pad], block scales fp32 [M][K/32], sums [tiles of a chunk][M][16 rows][warps]
     const uint32_t raw_s = smem_u32(smem_raw);
     unsigned char* const smem = smem_raw + (((raw_s + 1023u) & ~1023u) - raw_s);
-    const int ldxs = p.K + kGemvXsPad;
-    unsigned char* const ringC = smem;
-    unsigned char* const ringS = smem + (size_t)kWarps * DEPTH * kCodeBytes;
-    int8_t* xd = reinterpret_cast<int8_t*>(ringS + (size_t)kWarps * DEPTH * kScaleBytes);
-    float* xsc = reinterpret_cast<float*>(reinterpret_cast<unsigned char*>(xd) + (size_t)kGemvColsPerRow * p.M * ldxs);
-    float* s_part = xsc + (size_t)p.M * (p.K >> 5);
+    const int nGroups = (p.K + kItemK - 1) / kItemK, nBlocks = nGroups * 4, ldxs = nGroups * kItemK + kGemvXsPad;
+    unsigned char* const ringS = smem + (size_t)kWarps * p.depth * kCodeBytes;
+    int8_t* const xd = reinterpret_cast<int8_t*>(ringS + (size_t)kWarps * p.depth * kScaleBytes);
+    float* const xsc = reinterpret_cast<float*>(reinterpret_cast<unsigned char*>(xd) + (size_t)kGemvColsPerRow * p.M * ldxs);
+    float* const s_part = xsc + (size_t)p.M * nBlocks;
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int g = lane >> 2, t = lane & 3;
-    constexpr int rowsPerTile = SWIGLU ? 8 : 16;
-    const int nTiles = (p.N + rowsPerTile - 1) / rowsPerTile;
-    const int nGroups = p.K / kItemK;
     const bool tracing = p.trace != nullptr && blockIdx.x == 0 && tid == 0;
     if (tracing) { p.trace[0] = gtime(); p.trace[6] = 0ull; }
+    // this block's granules; a tile is two of them (SwiGLU: one of the gate and the same of the up projection)
+    const int bx = blockIdx.x, granules = p.share + (bx < p.extra), row0 = (bx * p.share + min(bx, p.extra)) * 8;
+    const int tiles = SWIGLU ? granules : (granules + 1) / 2;
 
-    const uint32_t myC = smem_u32(ringC) + (uint32_t)warp * DEPTH * kCodeBytes;
-    const uint32_t myS = smem_u32(ringS) + (uint32_t)warp * DEPTH * kScaleBytes;
-    const uint32_t myBar = smem_u32(&s_bar[warp * DEPTH]);
-    if (lane == 0) {
-#pragma unroll
-        for (int d = 0; d < DEPTH; d++) mbar_init(myBar + 8 * d, 1);
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    }
+    const uint32_t myC = smem_u32(smem) + (uint32_t)(warp * p.depth) * kCodeBytes;
+    const uint32_t myS = smem_u32(ringS) + (uint32_t)(warp * p.depth) * kScaleBytes;
+    const uint32_t myBar = smem_u32(&s_bar[warp * kMaxDepth]);
+    if (lane < p.depth) mbar_init(myBar + 8 * lane, 1);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     __syncwarp();
 
-    // flat (tile, group) sequence of this warp, with a cursor running DEPTH-1 items ahead; rows past N and the
-    // second half of a tile that does not exist are filled with zeros by the copy engine and never stored
-    int itile = blockIdx.x, igrp = warp, islot = 0;
+    // flat (tile, group) sequence of this warp; rows past N are filled with zeros by the copy engine and never stored, the second
+    // half of a tile that is not this block's holds anything and is not stored either
+    int itile = 0, igrp = warp, islot = 0;
     auto issue_next = [&]() {
-        if (itile < nTiles && igrp < nGroups) {
-            if (lane == 0) {
-                const uint32_t bar = myBar + 8 * islot;
-                const uint32_t dc = myC + (uint32_t)islot * kCodeBytes, ds = myS + (uint32_t)islot * kScaleBytes;
-                const int row0 = itile * rowsPerTile;
+        if (igrp >= nGroups || itile >= tiles) return;
+        if (lane == 0) {
+            const uint32_t bar = myBar + 8 * islot, dc = myC + (uint32_t)islot * kCodeBytes, ds = myS + (uint32_t)islot * kScaleBytes;
+            const int row = row0 + itile * (SWIGLU ? 8 : 16);
+            if (SWIGLU) {
                 mbar_arrive_expect_tx(bar, kItemBytes);
-                tma_box(dc, &p.codes, igrp * kItemK, row0, bar);
-                tma_box(dc + kCodeBytes / 2, SWIGLU ? &p.codes2 : &p.codes, igrp * kItemK, SWIGLU ? row0 : row0 + 8, bar);
-                tma_box(ds, &p.scales, igrp * 4, row0, bar);
-                tma_box(ds + kScaleBytes / 2, SWIGLU ? &p.scales2 : &p.scales, igrp * 4, SWIGLU ? row0 : row0 + 8, bar);
+                tma_box(dc, &p.codes, igrp * kItemK, row, bar);
+                tma_box(dc + kCodeBytes / 2, &p.codes2, igrp * kItemK, row, bar);
+                tma_box(ds, &p.scales, igrp * 4, row, bar);
+                tma_box(ds + kScaleBytes / 2, &p.scales2, igrp * 4, row, bar);
+            } else {
+                const bool half = 2 * itile + 1 == granules;
+                mbar_arrive_expect_tx(bar, half ? kItemBytes / 2 : kItemBytes);
+                tma_box(dc, &p.codes, igrp * kItemK, row, bar);
+                if (!half) tma_box(dc + kCodeBytes / 2, &p.codes, igrp * kItemK, row + 8, bar);
+                tma_box(ds, &p.scales, igrp * 4, row, bar);
+                if (!half) tma_box(ds + kScaleBytes / 2, &p.scales, igrp * 4, row + 8, bar);
             }
-            igrp += kWarps;
-            if (igrp >= nGroups) { igrp = warp; itile += gridDim.x; }
         }
-        islot = islot + 1 == DEPTH ? 0 : islot + 1;
+        igrp += kWarps;
+        if (igrp >= nGroups) { igrp = warp; itile++; }
+        islot = islot + 1 == p.depth ? 0 : islot + 1;
     };
     // Weights never depend on the previous kernel, so streaming starts before the wait.
-    const int kPre = p.pre < DEPTH - 1 ? p.pre : DEPTH - 1;
-    for (int d = 0; d < kPre; d++) issue_next();
+#pragma unroll 1
+    for (int d = 0; d < p.depth; d++) issue_next();
     pdl_launch_dependents();
     if (tracing) p.trace[1] = gtime();
-    // the norm's gain is a weight as well: fetch it before the wait when four groups per warp cover the row
-    const bool gammaEarly = p.gamma != nullptr && nGroups <= 4 * kWarps && (reinterpret_cast<uintptr_t>(p.gamma) & 15) == 0;
-    float4 gpre4[4];
+    // the norm's gain is a weight as well
+    constexpr int kAhead = 4;                        // groups of a warp in registers
+    float4 xv[kAhead], gv[kAhead];
+    auto ld4 = [&](const float* q, int grp) {        // zeros behind the row's end
+        const int k = grp * kItemK + lane * 4;
+        return k < p.K ? *reinterpret_cast<const float4*>(q + k) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    };
+    auto load_gain = [&]() {
 #pragma unroll
-    for (int j = 0; j < 4; j++) gpre4[j] = make_float4(1.0f, 1.0f, 1.0f, 1.0f);
-    if (gammaEarly) {
-#pragma unroll
-        for (int j = 0; j < 4; j++)
-            if (warp + kWarps * j < nGroups) gpre4[j] = gemv_load4(p.gamma + (warp + kWarps * j) * 128 + lane * 4, true);
-    }
+        for (int u = 0; u < kAhead; u++)
+            if (p.gamma && warp + kWarps * u < nGroups) gv[u] = ld4(p.gamma, warp + kWarps * u);
+    };
+    load_gain();
     pdl_wait();
     if (tracing) p.trace[2] = gtime();
 
-    // activations → digit columns in the MMA fragment's order; the rest of the ring is queued behind the first loads.
-    // Every warp converts the groups it consumes and goes on by itself; RMSNorm's 1/rms is applied in the epilogue.
-    gemv_stage_warp_groups(p.x, p.ldx, p.gamma, p.K, p.M, xd, ldxs, xsc, s_ss, gpre4, gammaEarly, [&]() {
-        for (int d = kPre; d < DEPTH - 1; d++) issue_next();
-    });
-    if (warp >= nGroups) {                               // a warp without groups still owes the ring its issue slots
-        for (int d = kPre; d < DEPTH - 1; d++) issue_next();
+    auto sum8 = [](const float* q) {                 // in warp order
+        const float4 a = *reinterpret_cast<const float4*>(q), b = *reinterpret_cast<const float4*>(q + 4);
+        return ((((((a.x + a.y) + a.z) + a.w) + b.x) + b.y) + b.z) + b.w;
+    };
+    // activations → digit columns in the MMA fragment's order; every warp converts the groups it consumes and goes on by itself
+    const int j8 = lane & 7, pos = j8 < 4 ? 8 * j8 : 8 * (j8 - 4) + 4;
+#pragma unroll 1
+    for (int m = 0; m < p.M; m++) {
+        const float* xrow = p.x + (size_t)m * p.ldx;
+        int8_t* const dcol = xd + (size_t)(kGemvColsPerRow * m) * ldxs;
+        float* const xscRow = xsc + (size_t)m * nBlocks;
+        float ss = 0.0f, mean = 0.0f, inv = 1.0f;
+#pragma unroll
+        for (int u = 0; u < kAhead; u++)
+            if (warp + kWarps * u < nGroups) xv[u] = ld4(xrow, warp + kWarps * u);
+        if (m > 0) load_gain();
+        if (GPT && p.beta) {                         // LayerNorm1D (norm/LayerNorm1D.java:34-71): the row's mean, then its biased variance, over the block
+#pragma unroll 1
+            for (int pass = 0; pass < 2; pass++) {
+                float part = 0.0f;
+                auto add = [&](const float4& v, int grp) {
+                    if (grp * kItemK + lane * 4 >= p.K) return;
+                    const float d[4] = {v.x - mean, v.y - mean, v.z - mean, v.w - mean};
+#pragma unroll
+                    for (int e = 0; e < 4; e++) part = pass ? fmaf(d[e], d[e], part) : part + d[e];
+                };
+#pragma unroll
+                for (int u = 0; u < kAhead; u++)
+                    if (warp + kWarps * u < nGroups) add(xv[u], warp + kWarps * u);
+#pragma unroll 1
+                for (int grp = warp + kWarps * kAhead; grp < nGroups; grp += kWarps) add(ld4(xrow, grp), grp);
+                for (int o = 16; o > 0; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
+                float* const to = (pass ? s_ss : s_mean) + m * kWarps;
+                if (lane == 0) to[warp] = part;
+                __syncthreads();
+                const float all = sum8(to) * (1.0f / (float)p.K);
+                if (pass) inv = __frcp_rn(sqrtf(all + p.eps)); else mean = all;
+            }
+        }
+#pragma unroll 1
+        for (int g0 = warp; g0 < nGroups; g0 += kWarps * kAhead) {
+#pragma unroll
+            for (int u = 0; u < kAhead; u++) {
+                const int grp = g0 + kWarps * u;
+                if (grp >= nGroups) break;                           // warp-uniform
+                float4 v = xv[u];
+                if (GPT && p.beta) {                 // (the gain is zero behind the row's end)
+                    const float4 b = ld4(p.beta, grp);
+                    v = make_float4(((v.x - mean) * inv) * gv[u].x + b.x, ((v.y - mean) * inv) * gv[u].y + b.y, ((v.z - mean) * inv) * gv[u].z + b.z,
+                                    ((v.w - mean) * inv) * gv[u].w + b.w);
+                }
+                gemv_digits4(v, gv[u], p.gamma != nullptr && !(GPT && p.beta), ss, dcol + grp * kItemK + (lane >> 3) * 32 + pos, ldxs, j8 == 0,
+                             xscRow + grp * 4 + (lane >> 3));
+                if (grp + kWarps * kAhead < nGroups) {
+                    xv[u] = ld4(xrow, grp + kWarps * kAhead);
+                    if (p.gamma) gv[u] = ld4(p.gamma, grp + kWarps * kAhead);
+                }
+            }
+        }
+        if (p.gamma && !(GPT && p.beta)) {
+            for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+            if (lane == 0) s_ss[m * kWarps + warp] = ss;
+        }
     }
+    __syncwarp();
     if (tracing) p.trace[3] = gtime();
 
     // lane (g,t) feeds column g of MMA q: activation row 2q + g/4, digit g%4 (digit 3 does not exist)
@@ -147,92 +213,144 @@ __global__ void __launch_bounds__(kThreads, 2) k_q8_gemv_tma(const __grid_consta
         xcol[q] = reinterpret_cast<const unsigned char*>(xd) + (size_t)(hasCol[q] ? kGemvColsPerRow * mrow + (g & 3) : 0) * ldxs + t * 8;
         // the lane's two result columns 2t, 2t+1 belong to activation row 2q + t/2
         const int rrow = 2 * q + (t >> 1);
-        myxsc[q] = xsc + (size_t)(rrow < p.M ? rrow : 0) * (p.K >> 5);
-        acc[q][0] = acc[q][1] = acc[q][2] = acc[q][3] = 0.0f;
+        myxsc[q] = xsc + (size_t)(rrow < p.M ? rrow : 0) * nBlocks;
     }
     // ldmatrix.x4 addresses: lanes 0-7 rows 0-7 of the block's first 16-byte chunk, 8-15 rows 8-15 of it, 16-23 and
     // 24-31 the same rows of the second chunk; chunk c of row r sits at r·128 + ((c ^ (r & 7)) · 16)
     const int lrow = (lane & 7) + ((lane >> 3) & 1) * 8;
     const uint32_t lmBase = (uint32_t)lrow * 128u;
     const uint32_t lmChunk = (uint32_t)((lane >> 4) ^ (lrow & 7));
-    int cslot = 0, buf = 0, limit = kSpinLimit;
+    int cslot = 0, limit = kSpinLimit;
     uint32_t phases = 0;
-    for (int tile = blockIdx.x; tile < nTiles; tile += gridDim.x) {
-        const GemvEpilogueOperands eo = gemv_epilogue_fetch<SWIGLU>(tile, p.M, p.N, p.bias, p.bias2, p.residual, p.ldr);
-        for (int grp = warp; grp < nGroups; grp += kWarps) {
-            issue_next();
-            const uint32_t bar = myBar + 8 * cslot;
-            const uint32_t parity = (phases >> cslot) & 1u;
-            bool ready = mbar_try_wait(bar, parity);
-            for (int spin = 0; !ready && spin < limit; spin++) ready = mbar_try_wait(bar, parity);
-            if (!ready) {                               // never on a healthy device: flag it, stop waiting long, keep the control flow
-                if (lane == 0) atomicCAS(p.error, 0, kErrTmaWait);
-                limit = 64;
-            }
-            phases ^= 1u << cslot;
-            const uint32_t sc = myC + (uint32_t)cslot * kCodeBytes;
-            const unsigned char* ss = ringS + ((size_t)warp * DEPTH + cslot) * kScaleBytes;
-            const float4 s0 = *reinterpret_cast<const float4*>(ss + g * 16);            // row g: its four block scales
-            const float4 s1 = *reinterpret_cast<const float4*>(ss + (g + 8) * 16);      // row g+8
-            const float s0v[4] = {s0.x, s0.y, s0.z, s0.w}, s1v[4] = {s1.x, s1.y, s1.z, s1.w};
-            float xsv[NM][4];
+    const int chunk = kChunk / p.M;                  // tiles between two barriers
+#pragma unroll 1
+    for (int tile0 = 0; tile0 < tiles; tile0 += chunk) {
+        const int many = min(chunk, tiles - tile0);
+        // output o of the chunk: tile o / (M·rows), activation row, row; its operands are fetched ahead of the tiles
+        constexpr int kRows = SWIGLU ? 8 : 16;
+        const int perTile = p.M * kRows, ot = tid / perTile, om = (tid - ot * perTile) / kRows, orow = tid % kRows;
+        const int n = row0 + (tile0 + ot) * kRows + orow;
+        const bool mine = ot < many && n < p.N && n < row0 + granules * 8;
+        float bias = 0.0f, other = 0.0f;
+        if (mine) {
+            if (p.bias) bias = p.bias[n];
+            if (SWIGLU) { if (p.bias2) other = p.bias2[n]; }
+            else if (p.residual) other = p.residual[(size_t)om * p.ldr + n];
+        }
+#pragma unroll 1
+        for (int i = 0; i < many; i++) {
 #pragma unroll
-            for (int q = 0; q < NM; q++) {
-                const float4 v = *reinterpret_cast<const float4*>(myxsc[q] + grp * 4);
-                xsv[q][0] = v.x; xsv[q][1] = v.y; xsv[q][2] = v.z; xsv[q][3] = v.w;
-            }
-#pragma unroll
-            for (int b = 0; b < 4; b++) {
-                uint32_t a[4];
-                ldmatrix_x4(a, sc + lmBase + ((lmChunk ^ (uint32_t)(2 * b)) << 4));
-                const int blk = grp * 4 + b;
+            for (int q = 0; q < NM; q++) acc[q][0] = acc[q][1] = acc[q][2] = acc[q][3] = 0.0f;
+#pragma unroll 1
+            for (int grp = warp; grp < nGroups; grp += kWarps) {
+                const uint32_t bar = myBar + 8 * cslot;
+                const uint32_t parity = (phases >> cslot) & 1u;
+                bool ready = mbar_try_wait(bar, parity);
+#pragma unroll 1
+                for (int spin = 0; !ready && spin < limit; spin++) ready = mbar_try_wait(bar, parity);
+                if (!ready) {                               // never on a healthy device: flag it, stop waiting long, keep the control flow
+                    if (lane == 0) atomicCAS(p.error, 0, kErrTmaWait);
+                    limit = 64;
+                }
+                phases ^= 1u << cslot;
+                const uint32_t sc = myC + (uint32_t)cslot * kCodeBytes;
+                const unsigned char* ss = ringS + ((size_t)warp * p.depth + cslot) * kScaleBytes;
+                const float4 s0 = *reinterpret_cast<const float4*>(ss + g * 16);            // row g: its four block scales
+                const float4 s1 = *reinterpret_cast<const float4*>(ss + (g + 8) * 16);      // row g+8
+                const float s0v[4] = {s0.x, s0.y, s0.z, s0.w}, s1v[4] = {s1.x, s1.y, s1.z, s1.w};
+                float xsv[NM][4];
 #pragma unroll
                 for (int q = 0; q < NM; q++) {
-                    uint2 xb = make_uint2(0u, 0u);
-                    if (hasCol[q]) xb = *reinterpret_cast<const uint2*>(xcol[q] + blk * 32);
-                    int cc[4] = {0, 0, 0, 0};
-                    mma_s8_16832(cc, a[0], a[1], a[2], a[3], xb.x, xb.y);
-                    const float f0 = s0v[b] * xsv[q][b], f1 = s1v[b] * xsv[q][b];
-                    acc[q][0] = fmaf(f0, int_to_float_exact(cc[0]), acc[q][0]);
-                    acc[q][1] = fmaf(f0, int_to_float_exact(cc[1]), acc[q][1]);
-                    acc[q][2] = fmaf(f1, int_to_float_exact(cc[2]), acc[q][2]);
-                    acc[q][3] = fmaf(f1, int_to_float_exact(cc[3]), acc[q][3]);
+                    const float4 v = *reinterpret_cast<const float4*>(myxsc[q] + grp * 4);
+                    xsv[q][0] = v.x; xsv[q][1] = v.y; xsv[q][2] = v.z; xsv[q][3] = v.w;
+                }
+#pragma unroll
+                for (int b = 0; b < 4; b++) {
+                    uint32_t a[4];
+                    ldmatrix_x4(a, sc + lmBase + ((lmChunk ^ (uint32_t)(2 * b)) << 4));
+                    const int blk = grp * 4 + b;
+#pragma unroll
+                    for (int q = 0; q < NM; q++) {
+                        uint2 xb = make_uint2(0u, 0u);
+                        if (hasCol[q]) xb = *reinterpret_cast<const uint2*>(xcol[q] + blk * 32);
+                        int cc[4] = {0, 0, 0, 0};
+                        mma_s8_16832(cc, a[0], a[1], a[2], a[3], xb.x, xb.y);
+                        const float f0 = s0v[b] * xsv[q][b], f1 = s1v[b] * xsv[q][b];
+                        acc[q][0] = fmaf(f0, int_to_float_exact(cc[0]), acc[q][0]);
+                        acc[q][1] = fmaf(f0, int_to_float_exact(cc[1]), acc[q][1]);
+                        acc[q][2] = fmaf(f1, int_to_float_exact(cc[2]), acc[q][2]);
+                        acc[q][3] = fmaf(f1, int_to_float_exact(cc[3]), acc[q][3]);
+                    }
+                }
+                __syncwarp();           // every lane has read the slot before lane 0 hands it to the copy engine again
+                issue_next();
+                cslot = cslot + 1 == p.depth ? 0 : cslot + 1;
+            }
+            // the warp's sums, digits recombined: lanes of even t hold the upper two digits of activation row 2q + t/2, their neighbours the last
+#pragma unroll
+            for (int q = 0; q < NM; q++) {
+                const float d0 = __shfl_down_sync(0xffffffffu, acc[q][0], 1), d1 = __shfl_down_sync(0xffffffffu, acc[q][2], 1);
+                const int m = 2 * q + (t >> 1);
+                if ((t & 1) == 0 && m < p.M) {
+                    float* to = s_part + ((i * p.M + m) * 16 + g) * kWarps + warp;
+                    to[0] = fmaf(acc[q][0], 65536.0f, fmaf(acc[q][1], 256.0f, d0));
+                    to[8 * kWarps] = fmaf(acc[q][2], 65536.0f, fmaf(acc[q][3], 256.0f, d1));
                 }
             }
-            __syncwarp();           // every lane has read the slot before lane 0 hands it to the copy engine again
-            cslot = cslot + 1 == DEPTH ? 0 : cslot + 1;
         }
-        if (tracing && tile == blockIdx.x) p.trace[4] = gtime();
-        gemv_tile_epilogue<SWIGLU, false, NM>(acc, s_part + (size_t)buf * kWarps * NM * 128, tile, p.M, p.N, eo, p.bias != nullptr,
-                                            p.bias2 != nullptr, p.residual != nullptr, 0, p.out, p.ldo,
-                                            p.gamma ? s_ss : nullptr, p.eps, p.K);
-        buf ^= 1;
+        if (tracing && tile0 == 0) p.trace[4] = gtime();
+        __syncthreads();
+        if (mine) {
+            const float* from = s_part + ((ot * p.M + om) * 16 + orow) * kWarps;
+            float v = sum8(from), inv = 1.0f;
+            if (p.gamma && !(GPT && p.beta)) {
+                inv = __frcp_rn(sqrtf(sum8(s_ss + om * kWarps) * (1.0f / (float)p.K) + p.eps));
+                v *= inv;
+            }
+            if (p.bias) v += bias;
+            if (GPT && p.act == 1) v = gelu_call(v);
+            if (SWIGLU) {
+                float u = sum8(from + 8 * kWarps) * inv;
+                if (p.bias2) u += other;
+                const float sig = 1.0f / (1.0f + expf(-v));
+                v = (v * sig) * u;                   // SiLU(gate) ⊙ up
+            } else if (p.residual) v += other;
+            p.out[(size_t)om * p.ldo + n] = v;
+        }
+        if (tile0 + chunk < tiles) __syncthreads();
     }
     if (tracing) p.trace[5] = gtime();
     if (p.trace != nullptr && tid == 0) atomicMax(p.trace + 6, gtime());
 }
 
 size_t tma_smem_bytes(int K, int M, int depth) {
-    return 1024 + (size_t)kWarps * depth * kItemBytes + (size_t)kGemvColsPerRow * M * (K + kGemvXsPad) + (size_t)M * (K / 32) * 4 +
-           (size_t)2 * kWarps * (M > 2 ? 2 : 1) * 128 * 4;
+    const size_t groups = (K + kItemK - 1) / kItemK;
+    return 1024 + (size_t)kWarps * depth * kItemBytes + (size_t)kGemvColsPerRow * M * (groups * kItemK + kGemvXsPad) + M * groups * 16 +
+           (size_t)(kChunk / M) * M * 16 * kWarps * 4;
 }
-constexpr size_t kSmemBudget = 112 * 1024;       // two CTAs per SM
+constexpr size_t kSmemHalf = 111 * 1024;         // two blocks per SM
+constexpr size_t kSmemWhole = 224 * 1024;        // a block with its SM to itself
+constexpr int kMinDepth = 3;
 
-template <bool SWIGLU, int DEPTH, int NM>
-void launch_tma(const GemvTmaParams& p, cudaStream_t s) {
+// Ring items per warp, so that two blocks share an SM where that can be;
+// 0: no ring fits.
+int ring_depth(int K, int M) {
+    for (int d = kMaxDepth; d >= kMinDepth; d--)
+        if (tma_smem_bytes(K, M, d) <= kSmemHalf) return d;
+    return tma_smem_bytes(K, M, kMinDepth) <= kSmemWhole ? kMinDepth : 0;
+}
+
+template <bool SWIGLU, int NM, bool GPT>
+void launch_tma(GemvTmaParams& p, cudaStream_t s) {
     static bool attrSet = false;
     if (!attrSet) {
-        DJ_CUDA_CHECK(cudaFuncSetAttribute(k_q8_gemv_tma<SWIGLU, DEPTH, NM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBudget));
+        DJ_CUDA_CHECK(cudaFuncSetAttribute(k_q8_gemv_tma<SWIGLU, NM, GPT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemWhole));
         attrSet = true;
     }
-    const int rowsPerTile = SWIGLU ? 8 : 16;
-    const int nTiles = (p.N + rowsPerTile - 1) / rowsPerTile;
-    // every CTA gets the same number of tiles (±1 only in the last round): the grid is the smallest one that
-    // keeps the rounds of the full grid
-    const int cap = 2 * g_num_sms;
-    const int rounds = (nTiles + cap - 1) / cap;
-    const int gx = (nTiles + rounds - 1) / rounds;
-    launch_k(k_q8_gemv_tma<SWIGLU, DEPTH, NM>, dim3(gx), dim3(kThreads), tma_smem_bytes(p.K, p.M, DEPTH), s, true, p);
+    const int granules = (p.N + 7) / 8, gx = std::min(SWIGLU ? granules : (granules + 1) / 2, 2 * g_num_sms);
+    p.share = granules / gx; p.extra = granules % gx;
+    p.depth = ring_depth(p.K, p.M);
+    launch_k(k_q8_gemv_tma<SWIGLU, NM, GPT>, dim3(gx), dim3(kThreads), tma_smem_bytes(p.K, p.M, p.depth), s, true, p);
 }
 
 }  // namespace
@@ -265,43 +383,32 @@ bool q8_encode_weight_maps(const Q8View& w, CUtensorMap* codes, CUtensorMap* sca
     return true;
 }
 
-// Returns false when the shape is outside this kernel's domain (K a multiple of 128, no LayerNorm / GELU, the
-// digits of all rows of the call — up to four — beside the ring in shared memory); the caller then takes the cp.async
-// kernel.
+// Returns false when the shape is outside this kernel's domain: rows in 16-byte pieces, a ring beside the digits of one row, whole
+// blocks (the FMA kernel rounds less than the digits do: 1.0e-7 against 2e-7 of the result, and other lengths stay with it).
 bool launch_q8_gemv_tma(const Q8LinearArgs& a, cudaStream_t s) {
     const int K = a.w.K;
-    if (K % kItemK != 0 || a.w.Kp != K || g_dev_error == nullptr) return false;
-    const bool swiglu = a.w2.codes != nullptr;
-    // LayerNorm needs the row's mean before any digit, i.e. CTA-wide staging: the cp.async kernel has it (and measured
-    // 1.5 % faster per GPT-2 XL token than this kernel with the same staging)
-    if (a.beta != nullptr || a.act != 0) return false;
-    if (swiglu && (a.w2.K != K || a.w2.Kp != K || a.w2.N != a.w.N)) return false;
-    // all rows (up to four) in one pass, or not at all: where the digits of the rows do not fit beside the ring, the
-    // cp.async kernel with its smaller ring items takes them in fewer passes
-    if (tma_smem_bytes(K, a.M < 4 ? a.M : 4, kDepth) > kSmemBudget) return false;
+    const bool swiglu = a.w2.codes != nullptr, gpt = a.beta != nullptr || a.act != 0;
+    if (K % 32 != 0 || g_dev_error == nullptr || (swiglu && (gpt || a.w2.K != K || a.w2.Kp != a.w.Kp || a.w2.N != a.w.N))) return false;
+    if (((reinterpret_cast<uintptr_t>(a.x) | reinterpret_cast<uintptr_t>(a.gamma) | reinterpret_cast<uintptr_t>(a.beta)) & 15) != 0 || (a.M > 1 && a.ldx % 4 != 0)) return false;
+    if (ring_depth(K, 1) == 0) return false;
     GemvTmaParams p;
     if (!q8_encode_weight_maps(a.w, &p.codes, &p.scales)) return false;
     if (swiglu) {
         if (!q8_encode_weight_maps(a.w2, &p.codes2, &p.scales2)) return false;
-    } else {
-        p.codes2 = p.codes; p.scales2 = p.scales;
-    }
+    } else { p.codes2 = p.codes; p.scales2 = p.scales; }
     for (int m0 = 0; m0 < a.M;) {
-        int rows = a.M - m0 < 4 ? a.M - m0 : 4;      // 8 MMA columns = 2 activation rows × (3 digits + 1 unused); 3-4 rows take a second MMA
-        while (rows > 1 && tma_smem_bytes(K, rows, kDepth) > kSmemBudget) rows--;
-        p.x = a.x + (size_t)m0 * a.ldx; p.ldx = a.ldx; p.gamma = a.gamma; p.eps = a.eps;
-        p.bias = a.bias; p.bias2 = a.bias2;
+        int rows = std::min(a.M - m0, 4);            // 8 MMA columns = 2 activation rows × (3 digits + 1 unused); 3-4 rows take a second MMA
+        while (rows > 1 && ring_depth(K, rows) == 0) rows--;
+        p.x = a.x + (size_t)m0 * a.ldx; p.ldx = a.ldx; p.gamma = a.gamma; p.beta = a.gamma ? a.beta : nullptr; p.eps = a.eps;
+        p.bias = a.bias; p.bias2 = a.bias2; p.act = a.act;
         p.residual = a.residual ? a.residual + (size_t)m0 * a.ldr : nullptr; p.ldr = a.ldr;
         p.out = a.out + (size_t)m0 * a.ldo; p.ldo = a.ldo;
         p.K = K; p.N = a.w.N; p.M = rows;
-        p.pre = 2;
         p.error = g_dev_error;
         p.trace = trace_slot();
-        if (rows > 2) {
-            if (swiglu) launch_tma<true, kDepth, 2>(p, s); else launch_tma<false, kDepth, 2>(p, s);
-        } else {
-            if (swiglu) launch_tma<true, kDepth, 1>(p, s); else launch_tma<false, kDepth, 1>(p, s);
-        }
+        if (swiglu) { if (rows > 2) launch_tma<true, 2, false>(p, s); else launch_tma<true, 1, false>(p, s); }
+        else if (gpt) { if (rows > 2) launch_tma<false, 2, true>(p, s); else launch_tma<false, 1, true>(p, s); }
+        else { if (rows > 2) launch_tma<false, 2, false>(p, s); else launch_tma<false, 1, false>(p, s); }
         m0 += rows;
     }
     return true;

@@ -1167,7 +1167,7 @@ int deepj_cuda_q8_alloc(int32_t id, int32_t K, int32_t N) {
     ensure_init();
     if (K <= 0 || N <= 0) throw std::runtime_error("q8_alloc: K and N must be positive");
     if (R.pool.count(id)) throw std::runtime_error("q8_alloc: id " + std::to_string(id) + " already exists");
-    Buf b; b.kind = kQ8; b.K = K; b.N = N; b.Kp = (K + 15) / 16 * 16; b.nb = (K + 31) / 32;
+    Buf b; b.kind = kQ8; b.K = K; b.N = N; b.Kp = (K + 15) / 16 * 16; b.nb = (K + 127) / 128 * 4;
     size_t codeBytes = ((size_t)N * b.Kp + 255) / 256 * 256;
     b.bytes = codeBytes + (size_t)N * b.nb * 4;
     DJ_CUDA_CHECK(device_malloc(&b.ptr, b.bytes));
@@ -1200,7 +1200,8 @@ int deepj_cuda_q8_upload(int32_t q8_id, const int8_t* codes, const float* scales
     Buf& q = find_buf(c, q8_id, kQ8, "q8_upload");
     Q8View v = q8view(q);
     DJ_CUDA_CHECK(cudaMemcpy2DAsync((void*)v.codes, q.Kp, codes, q.K, q.K, q.N, cudaMemcpyHostToDevice, R.stream));
-    DJ_CUDA_CHECK(cudaMemcpyAsync((void*)v.scales, scales, (size_t)q.N * q.nb * 4, cudaMemcpyHostToDevice, R.stream));
+    const size_t nb = (size_t)(q.K + 31) / 32 * 4;
+    DJ_CUDA_CHECK(cudaMemcpy2DAsync((void*)v.scales, (size_t)q.nb * 4, scales, nb, nb, q.N, cudaMemcpyHostToDevice, R.stream));
     DJ_CUDA_CHECK(cudaStreamSynchronize(R.stream));
     DJ_CATCH
 }
@@ -1212,7 +1213,8 @@ int deepj_cuda_q8_download(int32_t q8_id, int8_t* codes, float* scales) {
     Buf& q = find_buf(c, q8_id, kQ8, "q8_download");
     Q8View v = q8view(q);
     DJ_CUDA_CHECK(cudaMemcpy2DAsync(codes, q.K, v.codes, q.Kp, q.K, q.N, cudaMemcpyDeviceToHost, R.stream));
-    DJ_CUDA_CHECK(cudaMemcpyAsync(scales, v.scales, (size_t)q.N * q.nb * 4, cudaMemcpyDeviceToHost, R.stream));
+    const size_t nb = (size_t)(q.K + 31) / 32 * 4;
+    DJ_CUDA_CHECK(cudaMemcpy2DAsync(scales, nb, v.scales, (size_t)q.nb * 4, nb, q.N, cudaMemcpyDeviceToHost, R.stream));
     DJ_CUDA_CHECK(cudaStreamSynchronize(R.stream));
     DJ_CATCH
 }

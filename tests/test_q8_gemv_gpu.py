@@ -1,0 +1,54 @@
+"""The few-row Q8 kernel at the edges of its groups (128), its warps (8 groups), its register rounds (4 groups a warp), its tiles (16 rows,
+half tiles) and its chunks (16 tiles × rows), with RMSNorm, LayerNorm, GELU and the gated pair, against float64."""
+import numpy as np
+import pytest
+
+from deepj_b200.compute_graph import OP_Q8_LINEAR, OP_Q8_LINEAR_LN, OP_Q8_SWIGLU, float_bits
+from test_q8_gpu import Dev
+
+pytestmark = pytest.mark.gpu
+
+SHAPES = [(32, 8), (96, 40), (128, 17), (160, 2400), (992, 24), (1024, 33), (1056, 1200), (1600, 4800), (4096, 72), (4128, 40), (8352, 16), (128, 40000)]
+
+
+def dequantized(dev, q, K, N):
+    codes, scales = dev.q8_download(q, K, N)
+    return codes.astype(np.float64) * np.repeat(scales.astype(np.float64), 32, axis=1)[:, :K]      # [N × K]
+
+
+@pytest.mark.parametrize("K,N", SHAPES)
+@pytest.mark.parametrize("M", [1, 2, 4])
+def test_few_rows(K, N, M):
+    dev = Dev(9 << 20)
+    try:
+        rng = np.random.default_rng(K + N + M)
+        x = rng.standard_normal((M, K)).astype(np.float32) + 0.3
+        gamma, beta = rng.uniform(0.5, 1.5, K).astype(np.float32), rng.standard_normal(K).astype(np.float32)
+        bias, res = rng.standard_normal(N).astype(np.float32), rng.standard_normal((M, N)).astype(np.float32)
+        q, q2 = (dev.q8((rng.standard_normal((K, N)) * 0.05).astype(np.float32)) for _ in range(2))
+        w, w2 = dequantized(dev, q, K, N), dequantized(dev, q2, K, N)
+        xb, gb, tb, bb, rb = (dev.buf(a.size, a) for a in (x, gamma, beta, bias, res))
+        ob = dev.buf(M * N)
+        x64 = x.astype(np.float64)
+        rms = x64 / np.sqrt((x64 ** 2).mean(1, keepdims=True) + 1e-5) * gamma
+        mean = x64.mean(1, keepdims=True)
+        ln = (x64 - mean) / np.sqrt(((x64 - mean) ** 2).mean(1, keepdims=True) + 1e-5) * gamma + beta
+
+        def check(row, want, weights, what):
+            # a digit is within 2^-22 of its block's largest value; 32-bit sums of K / 32 / 8 blocks per warp; activations are 1-Lipschitz or nearly so
+            got = dev.get(ob, M * N).reshape(M, N)
+            size = (np.abs(row).max(1, keepdims=True) * np.abs(weights).sum(1)[None]) * (2.0 ** -22 + K / 256 * 2.0 ** -24) + 1e-6 * (np.abs(want) + 4)
+            assert (np.abs(got - want) <= 2 * size).all(), (what, np.abs(got - want).max())
+
+        dev.flush([OP_Q8_LINEAR, xb, 0, K, -1, 0, q, -1, -1, 0, 0, ob, 0, N, M])
+        check(x64, x64 @ w.T, w, "plain")
+        dev.flush([OP_Q8_LINEAR, xb, 0, K, gb, float_bits(1e-5), q, bb, rb, 0, N, ob, 0, N, M])
+        check(rms, rms @ w.T + bias + res, w, "rms")
+        dev.flush([OP_Q8_LINEAR_LN, xb, 0, K, gb, tb, float_bits(1e-5), q, bb, -1, 0, 0, ob, 0, N, M, 1])
+        z = ln @ w.T + bias
+        check(ln, 0.5 * z * (1 + np.tanh(np.sqrt(2 / np.float64(np.float32(np.pi))) * (z + 0.044715 * z ** 3))), w, "layer norm and gelu")
+        dev.flush([OP_Q8_SWIGLU, xb, 0, K, gb, float_bits(1e-5), q, bb, q2, -1, ob, 0, N, M])
+        g, u = rms @ w.T + bias, rms @ w2.T
+        check(rms * np.abs(u).max(), g / (1 + np.exp(-g)) * u, np.maximum(np.abs(w), np.abs(w2)) + np.abs(g).max() * np.abs(w2) / np.abs(u).max(), "gated pair")
+    finally:
+        dev.close()
