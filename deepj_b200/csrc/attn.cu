@@ -34,24 +34,28 @@ constexpr int kAttnSpinLimit = 1 << 22;     // polls of a barrier before the ker
 constexpr int kErrAttnWait = 332;           // device error code: a copy of cached rows never arrived
 
 // Prompt chunk: row z = (sequence b, token t) of the projection buffer holds k and v of position pos[b] + t.
-// One thread per interleaved pair: rotate k (x0·c − x1·s, x0·s + x1·c — RotaryEmbedding.java:81-122), copy v.
+// A block per row, a thread per two interleaved pairs: rotate k (x0·c − x1·s, x0·s + x1·c — RotaryEmbedding.java:81-122), copy v.
+// 2048 rows of 32 heads × 128 took 71 µs as a block of 64 threads per head and row, 24 this way (21 µs at the copy bandwidth).
 template <typename KT>
-__global__ void k_kv_append(const float* __restrict__ qkv, int k_off, int v_off, int ld, KT* __restrict__ kcache,
+__global__ void __launch_bounds__(256) k_kv_append(const float* __restrict__ qkv, int k_off, int v_off, int ld, KT* __restrict__ kcache,
                             KT* __restrict__ vcache, int maxSeq, const float* __restrict__ posbuf,
                             const float* __restrict__ cosT, const float* __restrict__ sinT, int H, int hd, int T) {
     pdl_wait();
     pdl_launch_dependents();
-    const int h = blockIdx.x, z = blockIdx.y, i = threadIdx.x;
-    const int b = z / T, tok = z - b * T;
+    const int z = blockIdx.x, b = z / T, tok = z - b * T;
     const int p = (int)posbuf[b] + tok;
     if (p < 0 || p >= maxSeq) return;
     const float* row = qkv + (size_t)z * ld;
-    const float2 k2 = *reinterpret_cast<const float2*>(row + k_off + h * hd + 2 * i);
-    const float2 v2 = *reinterpret_cast<const float2*>(row + v_off + h * hd + 2 * i);
-    const float c = cosT[(size_t)p * (hd >> 1) + i], s = sinT[(size_t)p * (hd >> 1) + i];
-    const size_t dst = (((size_t)b * H + h) * maxSeq + p) * hd + 2 * i;
-    KvIo<KT>::st2(kcache + dst, k2.x * c - k2.y * s, k2.x * s + k2.y * c);
-    KvIo<KT>::st2(vcache + dst, v2.x, v2.y);
+    const int per = hd >> 2, n = H * per;         // hd is a multiple of 16
+#pragma unroll 2
+    for (int i = threadIdx.x; i < n; i += 256) {
+        const int h = i / per, e = i - h * per;
+        const float4 k = *reinterpret_cast<const float4*>(row + k_off + 4 * i), v = *reinterpret_cast<const float4*>(row + v_off + 4 * i);
+        const float2 c = *reinterpret_cast<const float2*>(cosT + (size_t)p * (hd >> 1) + 2 * e), s = *reinterpret_cast<const float2*>(sinT + (size_t)p * (hd >> 1) + 2 * e);
+        const size_t dst = (((size_t)b * H + h) * maxSeq + p) * hd + 4 * e;
+        KvIo<KT>::st4(kcache + dst, make_float4(k.x * c.x - k.y * s.x, k.x * s.x + k.y * c.x, k.z * c.y - k.w * s.y, k.z * s.y + k.w * c.y));
+        KvIo<KT>::st4(vcache + dst, v);
+    }
 }
 
 // Ring items per warp: four blocks and a projection's beside them have to fit into an SM.
@@ -504,8 +508,7 @@ void launch_attn_decode_t(const AttnDecodeArgs& a, cudaStream_t s) {
     KT* vc = static_cast<KT*>(a.vcache);
     if (T > 1) {
         // the chunk's keys (rotated) and values go into the cache first; the attention kernel then only reads
-        dim3 ag(a.H, (unsigned)rows);
-        launch_k(k_kv_append<KT>, ag, dim3(a.hd / 2), 0, s, true, (const float*)a.qkv, a.k_off, a.v_off, a.ld, kc, vc, a.maxSeq,
+        launch_k(k_kv_append<KT>, dim3((unsigned)rows), dim3(256), 0, s, true, (const float*)a.qkv, a.k_off, a.v_off, a.ld, kc, vc, a.maxSeq,
                  a.pos, a.cosT, a.sinT, a.H, a.hd, T);
     }
     static const bool noTiled = getenv("DEEPJ_CUDA_NO_TILED_PREFILL") != nullptr;
@@ -533,7 +536,7 @@ void launch_attn_decode_t(const AttnDecodeArgs& a, cudaStream_t s) {
     const bool cluster = a.splits > 1 && a.splits <= kClusterSplits;
     auto go = [&](auto kernel) {
         DJ_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024));
-        launch_k_cluster(kernel, grid, block, smem, s, cluster ? (unsigned)a.splits : 1u, p);
+        launch_k_cluster(kernel, grid, block, smem, s, dim3(cluster ? a.splits : 1), p);
     };
 #define DJ_ATTN_CASE(L) case L: if (cluster) go(k_attn_decode<L, KT, true>); else go(k_attn_decode<L, KT, false>); break;
     switch (lpp) {

@@ -7,7 +7,7 @@
 // product a·b is accumulated as a_hi·b_hi + a_lo·b_hi + a_hi·b_lo (the dropped lo·lo term is
 // ≈ 2^-22 of the product).
 //
-// grid (heads, ceil(T / 64), sequences), the last query tiles first: they have the most keys, and started last they left the
+// grid (heads, ceil(T / 64), sequences × splits of the keys), the last query tiles first: they have the most keys, and started last they left the
 // chip to a few blocks at the end (32 heads of 128, 2048 tokens: 695 µs with the query tiles as the fast grid axis in rising
 // order, 545 µs this way).  128 threads.  Warp w owns query rows 16w … 16w+15 of the
 // tile; the CTA walks the keys in tiles of 32: K and V rows come from the fp32 cache, are split and
@@ -58,7 +58,7 @@ template <int HD, typename KT>
 __global__ void __launch_bounds__(128, 2) k_attn_prefill_mma(
         const float* __restrict__ qkv, int q_off, int ld, const KT* __restrict__ kcache, const KT* __restrict__ vcache,
         int maxSeq, const float* __restrict__ posbuf, const float* __restrict__ cosT, const float* __restrict__ sinT,
-        float* __restrict__ out, int ldo, int H, float scale, int T) {
+        float* __restrict__ out, int ldo, int H, float scale, int T, int splits) {
     constexpr int LDS = HD + 8;                     // halves per shared-memory row
     constexpr int KS = HD / 16;                     // k-steps of Q·Kᵀ, and pairs of output n-tiles
     extern __shared__ __align__(16) __half smh[];
@@ -72,28 +72,12 @@ __global__ void __launch_bounds__(128, 2) k_attn_prefill_mma(
     pdl_launch_dependents();
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int g = lane >> 2, t4 = lane & 3;
-    const int qt = (int)(gridDim.y - 1 - blockIdx.y), h = blockIdx.x, b = blockIdx.z;      // the tiles with the most keys first
+    const int qt = (int)(gridDim.y - 1 - blockIdx.y), h = blockIdx.x, b = blockIdx.z / splits, split = blockIdx.z - b * splits;      // the tiles with the most keys first
     const int t0 = qt * kMQ;
     int pos0 = (int)posbuf[b];
     pos0 = pos0 < 0 ? 0 : pos0;
     constexpr int half_ = HD >> 1;
 
-    // Q tile: rotate the interleaved pairs at position pos0 + t, fold in 1/sqrt(hd), split
-    for (int i = tid; i < kMQ * half_; i += 128) {
-        const int r = i / half_, pr = i % half_;
-        const int t = t0 + r;
-        float x0 = 0.0f, x1 = 0.0f;
-        if (t < T && pos0 + t < maxSeq) {
-            const float2 v = *reinterpret_cast<const float2*>(qkv + (size_t)(b * T + t) * ld + q_off + h * HD + 2 * pr);
-            const float c = cosT[(size_t)(pos0 + t) * half_ + pr], s = sinT[(size_t)(pos0 + t) * half_ + pr];
-            x0 = (v.x * c - v.y * s) * scale;
-            x1 = (v.x * s + v.y * c) * scale;
-        }
-        uint32_t hi, lo;
-        split2(x0, x1, hi, lo);
-        *reinterpret_cast<uint32_t*>(Qh + r * LDS + 2 * pr) = hi;
-        *reinterpret_cast<uint32_t*>(Ql + r * LDS + 2 * pr) = lo;
-    }
     const KT* kb = kcache + ((size_t)b * H + h) * maxSeq * HD;
     const KT* vb = vcache + ((size_t)b * H + h) * maxSeq * HD;
     const int lastKey = min(maxSeq - 1, pos0 + min(T, t0 + kMQ) - 1);       // newest key any row of this tile may see
@@ -138,15 +122,37 @@ __global__ void __launch_bounds__(128, 2) k_attn_prefill_mma(
     constexpr int kStageHalves = 4 * kMK * LDS;     // K_hi, K_lo, V_hi, V_lo of one tile
     constexpr uint32_t kStageBytes = kStageHalves * 2;
 
-    // first tile into stage 0
-    fetch(kb, 0); put(Kh, Kl);
-    fetch(vb, 0); put(Vh, Vl);
+    // Q tile: rotate the interleaved pairs at position pos0 + t, fold in 1/sqrt(hd), split; the loads of eight pieces a time in flight
+    auto stage_q = [&] {
+#pragma unroll 8
+        for (int i = tid; i < kMQ * (HD / 4); i += 128) {
+            const int r = i / (HD / 4), c = i % (HD / 4), t = t0 + r;
+            float4 x = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            if (t < T && pos0 + t < maxSeq) {
+                const float4 v = *reinterpret_cast<const float4*>(qkv + (size_t)(b * T + t) * ld + q_off + h * HD + 4 * c);
+                const float2 cs = *reinterpret_cast<const float2*>(cosT + (size_t)(pos0 + t) * half_ + 2 * c), sn = *reinterpret_cast<const float2*>(sinT + (size_t)(pos0 + t) * half_ + 2 * c);
+                x = make_float4((v.x * cs.x - v.y * sn.x) * scale, (v.x * sn.x + v.y * cs.x) * scale, (v.z * cs.y - v.w * sn.y) * scale, (v.z * sn.y + v.w * cs.y) * scale);
+            }
+            uint2 hi, lo;
+            split2(x.x, x.y, hi.x, lo.x); split2(x.z, x.w, hi.y, lo.y);
+            *reinterpret_cast<uint2*>(Qh + r * LDS + 4 * c) = hi;
+            *reinterpret_cast<uint2*>(Ql + r * LDS + 4 * c) = lo;
+        }
+    };
+    // this block's tiles [from, nTiles) of the row tile's; the first into stage 0
+    const int allTiles = lastKey / kMK + 1, share = (allTiles + splits - 1) / splits;
+    const int from = split * share, nTiles = min(allTiles, from + share);
+    if (from < nTiles) {
+        fetch(kb, from * kMK);                      // on its way while the queries are staged
+        stage_q();
+        put(Kh, Kl);
+        fetch(vb, from * kMK); put(Vh, Vl);
+    }
     __syncthreads();
-    const int nTiles = lastKey / kMK + 1;
-    for (int it = 0; it < nTiles; it++) {
+    for (int it = from; it < nTiles; it++) {
         const int k0 = it * kMK;
-        const uint32_t cur = (uint32_t)(it & 1) * kStageBytes;
-        __half* const nKh = Kh + ((it + 1) & 1) * kStageHalves;
+        const uint32_t cur = (uint32_t)((it - from) & 1) * kStageBytes;
+        __half* const nKh = Kh + ((it - from + 1) & 1) * kStageHalves;
         const bool more = it + 1 < nTiles;
         if (more) fetch(kb, k0 + kMK);              // the next tile's keys travel while this tile's Q·Kᵀ runs
 
@@ -239,6 +245,53 @@ __global__ void __launch_bounds__(128, 2) k_attn_prefill_mma(
     }
     l0 += __shfl_xor_sync(0xffffffffu, l0, 1); l0 += __shfl_xor_sync(0xffffffffu, l0, 2);
     l1 += __shfl_xor_sync(0xffffffffu, l1, 1); l1 += __shfl_xor_sync(0xffffffffu, l1, 2);
+    if (splits > 1) {
+        // the splits of a row tile are a cluster: every block leaves its unnormalised rows in its own shared memory (the stages have been
+        // read out) and adds up a share of the rows over all blocks
+        constexpr int LP = HD + 4;
+        float* const po = reinterpret_cast<float*>(Kh);                  // [64][LP], then the rows' maxima and sums
+        float* const pm = po + kMQ * LP;
+        float* const pl = pm + kMQ;
+#pragma unroll
+        for (int j = 0; j < 2 * KS; j++) {
+            *reinterpret_cast<float2*>(po + row0 * LP + 2 * t4 + j * 8) = make_float2(o[j][0], o[j][1]);
+            *reinterpret_cast<float2*>(po + row1 * LP + 2 * t4 + j * 8) = make_float2(o[j][2], o[j][3]);
+        }
+        if (t4 == 0) { pm[row0] = m0; pm[row1] = m1; pl[row0] = l0; pl[row1] = l1; }
+        asm volatile("barrier.cluster.arrive.release.aligned;\n barrier.cluster.wait.acquire.aligned;" ::: "memory");
+        constexpr int LANES = HD / 4;                                    // threads of a row
+        auto peer = [&](const float* p, int rank) {
+            uint32_t a;
+            asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_u32(p)), "r"(rank));
+            return a;
+        };
+        for (int r = split + splits * (tid / LANES); r < kMQ && t0 + r < T; r += splits * (128 / LANES)) {
+            const int c = tid % LANES * 4;
+            float M = -INFINITY, L = 0.0f;
+            for (int q = 0; q < splits; q++) {
+                float m;
+                asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(m) : "r"(peer(pm + r, q)) : "memory");
+                M = fmaxf(M, m);
+            }
+            float4 sum = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            for (int q = 0; q < splits; q++) {
+                float m, l; float4 v;
+                asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(m) : "r"(peer(pm + r, q)) : "memory");
+                asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(l) : "r"(peer(pl + r, q)) : "memory");
+                asm volatile("ld.shared::cluster.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(peer(po + r * LP + c, q)) : "memory");
+                const float e = m > -INFINITY ? expf(m - M) : 0.0f;
+                L = fmaf(l, e, L);
+                sum.x = fmaf(v.x, e, sum.x); sum.y = fmaf(v.y, e, sum.y); sum.z = fmaf(v.z, e, sum.z); sum.w = fmaf(v.w, e, sum.w);
+            }
+            if (L > 0.0f) {
+                float* dst = out + (size_t)(b * T + t0 + r) * ldo + h * HD + c;
+                *reinterpret_cast<float2*>(dst) = make_float2(sum.x / L, sum.y / L);
+                *reinterpret_cast<float2*>(dst + 2) = make_float2(sum.z / L, sum.w / L);
+            }
+        }
+        asm volatile("barrier.cluster.arrive.release.aligned;\n barrier.cluster.wait.acquire.aligned;" ::: "memory");      // nobody reads this block any more
+        return;
+    }
     if (t0 + row0 < T && l0 > 0.0f) {
         float* dst = out + (size_t)(b * T + t0 + row0) * ldo + h * HD + 2 * t4;
 #pragma unroll
@@ -253,6 +306,14 @@ __global__ void __launch_bounds__(128, 2) k_attn_prefill_mma(
 
 template <int HD> constexpr size_t prefill_mma_smem() { return (size_t)(2 * kMQ + 2 * 4 * kMK) * (HD + 8) * sizeof(__half); }
 
+// Blocks that share a row tile's keys, a cluster of 2, 4 or 8: where the tiles alone leave half of the slots (two per SM) empty, and
+// the cache holds four key tiles for each.  32 heads × 64 behind 700 positions, 123 tokens: 64 blocks 79 µs, 256 blocks 32 (with the queries staged eight loads at a time behind the first keys).
+int prefill_splits(long long blocks, int maxSeq) {
+    int s = 1;
+    while (s < 8 && blocks * s * 2 <= 2 * g_num_sms && maxSeq >= s * 2 * 4 * kMK) s *= 2;
+    return s;
+}
+
 template <int HD, typename KT>
 void launch_mma(const AttnDecodeArgs& a, int T, cudaStream_t s) {
     static bool attr = false;
@@ -260,9 +321,10 @@ void launch_mma(const AttnDecodeArgs& a, int T, cudaStream_t s) {
         DJ_CUDA_CHECK(cudaFuncSetAttribute(k_attn_prefill_mma<HD, KT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)prefill_mma_smem<HD>()));
         attr = true;
     }
-    dim3 grid(a.H, (T + kMQ - 1) / kMQ, a.B);
-    launch_k(k_attn_prefill_mma<HD, KT>, grid, dim3(128), prefill_mma_smem<HD>(), s, true, (const float*)a.qkv, a.q_off, a.ld,
-             (const KT*)a.kcache, (const KT*)a.vcache, a.maxSeq, a.pos, a.cosT, a.sinT, a.out, a.ldo, a.H, a.scale, T);
+    const int qTiles = (T + kMQ - 1) / kMQ, splits = prefill_splits((long long)a.H * qTiles * a.B, a.maxSeq);
+    const dim3 grid(a.H, qTiles, a.B * splits);
+    launch_k_cluster(k_attn_prefill_mma<HD, KT>, grid, dim3(128), prefill_mma_smem<HD>(), s, dim3(1, 1, splits), (const float*)a.qkv, a.q_off, a.ld,
+                     (const KT*)a.kcache, (const KT*)a.vcache, a.maxSeq, a.pos, a.cosT, a.sinT, a.out, a.ldo, a.H, a.scale, T, splits);
 }
 
 }  // namespace

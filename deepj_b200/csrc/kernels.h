@@ -312,9 +312,9 @@ int runtime_device();
 void invalidate_graphs();
 void set_last_error(const std::string& msg);
 
-// The same with clusters of `cluster` blocks along x and the PDL attribute.
+// The same with clusters of blocks and the PDL attribute.
 template <typename... KArgs, typename... Args>
-inline void launch_k_cluster(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, unsigned cluster, Args... args) {
+inline void launch_k_cluster(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, dim3 cluster, Args... args) {
     g_launches++;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid; cfg.blockDim = block; cfg.dynamicSmemBytes = smem; cfg.stream = s;
@@ -323,9 +323,9 @@ inline void launch_k_cluster(void (*kernel)(KArgs...), dim3 grid, dim3 block, si
         attr[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
         attr[cfg.numAttrs++].val.programmaticStreamSerializationAllowed = 1;
     }
-    if (cluster > 1) {
+    if (cluster.x * cluster.y * cluster.z > 1) {
         attr[cfg.numAttrs].id = cudaLaunchAttributeClusterDimension;
-        attr[cfg.numAttrs].val.clusterDim.x = cluster; attr[cfg.numAttrs].val.clusterDim.y = 1; attr[cfg.numAttrs++].val.clusterDim.z = 1;
+        attr[cfg.numAttrs].val.clusterDim.x = cluster.x; attr[cfg.numAttrs].val.clusterDim.y = cluster.y; attr[cfg.numAttrs++].val.clusterDim.z = cluster.z;
     }
     cfg.attrs = attr;
     DJ_CUDA_CHECK(cudaLaunchKernelEx(&cfg, kernel, KArgs(args)...));

@@ -12,15 +12,22 @@ __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepc
 // Embedding.forward → Tensor.sliceRows (transformer/embeddings/Embedding.java:28-34):
 // out[r] = table[ids[r]].  The reference throws on an out-of-range id before any
 // work; the runtime cannot see device-resident ids, so such a row is filled with NaN.
-__global__ void k_embed_gather(const float* __restrict__ table, const float* __restrict__ ids, float* __restrict__ out,
+// grid (rows, column blocks): a row of a table that lies in HBM is one load round trip, not one per 256 columns.
+constexpr int kEmbedCols = 1024;
+__global__ void __launch_bounds__(256) k_embed_gather(const float* __restrict__ table, const float* __restrict__ ids, float* __restrict__ out,
                                int rows, int d, int vocab) {
     pdl_wait();
     pdl_launch_dependents();
-    int r = blockIdx.x;
-    int id = (int)ids[r];
-    bool ok = id >= 0 && id < vocab;
-    for (int c = threadIdx.x; c < d; c += blockDim.x)
-        out[(size_t)r * d + c] = ok ? table[(size_t)id * d + c] : NAN;
+    const int r = blockIdx.x, id = (int)ids[r], c0 = blockIdx.y * kEmbedCols;
+    const bool ok = id >= 0 && id < vocab;
+    const float* src = table + (size_t)id * d;
+    float* dst = out + (size_t)r * d;
+    if (((reinterpret_cast<uintptr_t>(table) | reinterpret_cast<uintptr_t>(out)) & 15) == 0 && (d & 3) == 0) {
+        const int c = c0 + threadIdx.x * 4;
+        if (c < d) *reinterpret_cast<float4*>(dst + c) = ok ? *reinterpret_cast<const float4*>(src + c) : make_float4(NAN, NAN, NAN, NAN);
+        return;
+    }
+    for (int c = c0 + threadIdx.x; c < min(d, c0 + kEmbedCols); c += 256) dst[c] = ok ? src[c] : NAN;
 }
 
 // Total order of Float.compare (models/TextGenerator.java:163-170): -0.0 < +0.0,
@@ -310,7 +317,7 @@ unsigned long long h_splitmix64(unsigned long long z) {
 
 void launch_embed_gather(const float* table, const float* ids, float* out, int rows, int d, int vocab, cudaStream_t s) {
     if (rows <= 0) return;
-    launch_k(k_embed_gather, dim3(rows), dim3(256), 0, s, true, table, ids, out, rows, d, vocab);
+    launch_k(k_embed_gather, dim3(rows, (d + kEmbedCols - 1) / kEmbedCols), dim3(256), 0, s, true, table, ids, out, rows, d, vocab);
 }
 void launch_argmax_rows(const float* in, float* out, int rows, int cols, int* scratch, int* tickets, cudaStream_t s) {
     if (rows <= 0) return;
