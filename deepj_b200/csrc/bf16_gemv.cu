@@ -29,7 +29,7 @@ constexpr int kRgSmemHalf = 111 * 1024;          // of two blocks that share one
 constexpr int kRgMaxDepth = 6, kRgMaxWarps = 16;
 constexpr int kRgSpinLimit = 1 << 22;            // polls of a barrier before the kernel gives up on it
 constexpr int kRgMaxGroups = 512;                // row groups of a block, at most
-constexpr int kErrRingWait = 331;                // device error code: a copy never arrived
+constexpr int kErrRingWait = 333;                // device error code: a copy never arrived
 constexpr int kPieces = 4;                       // 16-byte pieces of a row's gain, gate or base that a thread holds while the row is on its way
 
 __device__ __forceinline__ float bf_lo(uint32_t u) { return __uint_as_float(u << 16); }
