@@ -48,6 +48,56 @@ template <int BN> struct GemmShape {
     static constexpr uint32_t kIdesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(kGM >> 4) << 24);
 };
 
+// A warp's 32 rows of an accumulator (from column 0 of it) → the outputs of rows mBase … and columns n0 ….
+template <int BN>
+__device__ __forceinline__ void store_tile(const GemmTcParams& p, uint32_t acc, int mBase, int rows, int n0, float* stg, int warp, int lane) {
+    int myRow = mBase + lane < rows ? mBase + lane : -1;      // output row of tile row `lane`
+    if (myRow >= 0 && p.rowMap != nullptr) myRow = p.rowMap[myRow];
+#pragma unroll 1
+    for (int c0 = 0; c0 < BN && n0 + c0 < p.N; c0 += 32) {
+        uint32_t v[32];
+        tmem_ld32(acc + ((uint32_t)(warp * 32) << 16) + (uint32_t)c0, v);
+#pragma unroll
+        for (int j = 0; j < 32; j++) stg[lane * 33 + j] = __uint_as_float(v[j]);
+        __syncwarp();
+        const int nb = n0 + c0, nn = nb + lane;
+        if (p.outHalf != nullptr) {
+#pragma unroll 8
+            for (int i = 0; i < 32; i += 2) {
+                const int r = i + (lane >> 4), row = __shfl_sync(0xffffffffu, myRow, r), c = 2 * (lane & 15);
+                if (row >= 0 && nb + c < p.N)
+                    *reinterpret_cast<__nv_bfloat162*>(p.outHalf + (size_t)row * p.ldo + nb + c) = __floats2bfloat162_rn(stg[r * 33 + c], stg[r * 33 + c + 1]);
+            }
+            __syncwarp();
+            continue;
+        }
+        if (nb < p.gluRow) {
+            const float myBias = p.bias != nullptr && nn < p.gluRow ? p.bias[nn] : 0.0f;
+#pragma unroll 8
+            for (int i = 0; i < 32; i++) {
+                const int row = __shfl_sync(0xffffffffu, myRow, i);
+                if (row >= 0 && nn < p.gluRow) {
+                    float val = stg[i * 33 + lane] + myBias;
+                    if (p.residual) val += p.residual[(size_t)row * p.ldr + nn];
+                    p.out[(size_t)row * p.ldo + nn] = softcap_f(val, p.softcap);
+                }
+            }
+        }
+        if (nb + 32 > p.gluRow && p.gluRow < p.N) {
+            const int pair = nb + 2 * (lane & 15);
+#pragma unroll 4
+            for (int i = 0; i < 32; i += 2) {
+                const int r = i + (lane >> 4), row = __shfl_sync(0xffffffffu, myRow, r);
+                if (row >= 0 && pair >= p.gluRow && pair < p.N) {
+                    const float g = stg[r * 33 + 2 * (lane & 15)], u = stg[r * 33 + 2 * (lane & 15) + 1];
+                    p.glu[(size_t)row * p.ldglu + ((pair - p.gluRow) >> 1)] = pair_f(g, u, p.limit, p.pair);
+                }
+            }
+        }
+        __syncwarp();
+    }
+}
+
 template <int BN>
 __global__ void __launch_bounds__(kGThreads, 1) k_bf16_gemm_tc(const __grid_constant__ GemmTcParams p) {
     using S = GemmShape<BN>;
@@ -161,52 +211,7 @@ __global__ void __launch_bounds__(kGThreads, 1) k_bf16_gemm_tc(const __grid_cons
             const int a = n & 1;
             if (!__all_sync(0xffffffffu, mbar_wait(accFull(a), (n / 2) & 1, &s_abort, p.error, 214))) break;
             tc_fence_after();
-            const int mBase = mt * kGM + warp * 32;
-            int myRow = mBase + lane < rows ? mBase + lane : -1;      // output row of tile row `lane`
-            if (myRow >= 0 && p.rowMap != nullptr) myRow = p.rowMap[myRow];
-#pragma unroll 1
-            for (int c0 = 0; c0 < BN && n0 + c0 < p.N; c0 += 32) {
-                uint32_t v[32];
-                tmem_ld32(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)(a * BN + c0), v);
-#pragma unroll
-                for (int j = 0; j < 32; j++) stg[lane * 33 + j] = __uint_as_float(v[j]);
-                __syncwarp();
-                const int nb = n0 + c0, nn = nb + lane;
-                if (p.outHalf != nullptr) {
-#pragma unroll 8
-                    for (int i = 0; i < 32; i += 2) {
-                        const int r = i + (lane >> 4), row = __shfl_sync(0xffffffffu, myRow, r), c = 2 * (lane & 15);
-                        if (row >= 0 && nb + c < p.N)
-                            *reinterpret_cast<__nv_bfloat162*>(p.outHalf + (size_t)row * p.ldo + nb + c) = __floats2bfloat162_rn(stg[r * 33 + c], stg[r * 33 + c + 1]);
-                    }
-                    __syncwarp();
-                    continue;
-                }
-                if (nb < p.gluRow) {
-                    const float myBias = p.bias != nullptr && nn < p.gluRow ? p.bias[nn] : 0.0f;
-#pragma unroll 8
-                    for (int i = 0; i < 32; i++) {
-                        const int row = __shfl_sync(0xffffffffu, myRow, i);
-                        if (row >= 0 && nn < p.gluRow) {
-                            float val = stg[i * 33 + lane] + myBias;
-                            if (p.residual) val += p.residual[(size_t)row * p.ldr + nn];
-                            p.out[(size_t)row * p.ldo + nn] = softcap_f(val, p.softcap);
-                        }
-                    }
-                }
-                if (nb + 32 > p.gluRow && p.gluRow < p.N) {
-                    const int pair = nb + 2 * (lane & 15);
-#pragma unroll 4
-                    for (int i = 0; i < 32; i += 2) {
-                        const int r = i + (lane >> 4), row = __shfl_sync(0xffffffffu, myRow, r);
-                        if (row >= 0 && pair >= p.gluRow && pair < p.N) {
-                            const float g = stg[r * 33 + 2 * (lane & 15)], u = stg[r * 33 + 2 * (lane & 15) + 1];
-                            p.glu[(size_t)row * p.ldglu + ((pair - p.gluRow) >> 1)] = pair_f(g, u, p.limit, p.pair);
-                        }
-                    }
-                }
-                __syncwarp();
-            }
+            store_tile<BN>(p, tmem + (uint32_t)(a * BN), mt * kGM + warp * 32, rows, n0, stg, warp, lane);
             tc_fence_before();
             mbar_arrive(accEmpty(a));
             n++;
@@ -214,6 +219,147 @@ __global__ void __launch_bounds__(kGThreads, 1) k_bf16_gemm_tc(const __grid_cons
     }
     __syncthreads();
     if (warp == 4) { tc_fence_after(); tmem_dealloc(tmem, S::kTmem); }
+}
+
+// ───────────── two SMs on one tile ─────────────
+// A cluster of two CTAs multiplies 256 × 256 tiles with tcgen05.mma of cta_group::2: each CTA holds its own 128 rows of A and half of
+// the weight rows, and the tensor cores read the other half from the neighbour.  Per k-step of 16 an SM's shared memory is written
+// 8 KB and read 8 KB in 135 cycles instead of 12 and 12 KB, which at 128 bytes a cycle was what bound the single-CTA form.  2048 rows through
+// [40960 … 44032 × 4096] and [4096 × 15104], four layers: 3.78 ms in place of 4.03; [8192 … 22016 × 4096], [4096 × 4096 and 11008], four layers:
+// 2.84 in place of 3.09.  What bounds it now is the tiles' way out of L2, about 9.5 TB/s.
+// The barriers that the MMAs wait for are the first CTA's: both CTAs' copies complete on its `full`, both CTAs' epilogue warps arrive
+// on its accEmpty; a commit arrives on both CTAs' `empty` and accFull.  Everything else is the kernel above.
+constexpr int kPN = 256, kPStages = 6, kPBytes = kABytes + kPN / 2 * kGK * 2;
+constexpr size_t kPSmem = (size_t)kPStages * kPBytes + kEpiBytes + 1024;
+constexpr uint32_t kPIdesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(kPN >> 3) << 17) | ((uint32_t)(2 * kGM >> 4) << 24);
+
+__device__ __forceinline__ uint32_t in_first(uint32_t addr) {            // the same place in the cluster's first CTA
+    uint32_t a;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(a) : "r"(addr));
+    return a;
+}
+__device__ __forceinline__ void tma_box_pair(uint32_t dst, const CUtensorMap* map, int x, int y, uint32_t bar) {
+    asm volatile("cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
+                 ::"r"(dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(bar) : "memory");
+}
+__device__ __forceinline__ void umma_f16_pair(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+    asm volatile("{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n}"
+                 ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
+}
+__device__ __forceinline__ void umma_commit_pair(uint32_t bar) {
+    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(bar), "h"((uint16_t)3) : "memory");
+}
+__device__ __forceinline__ void cluster_barrier() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\n barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+__global__ void __launch_bounds__(kGThreads, 1) k_bf16_gemm_pair(const __grid_constant__ GemmTcParams p) {
+    extern __shared__ __align__(1024) unsigned char smem[];
+    __shared__ __align__(8) unsigned long long s_bar[2 * kPStages + 4];
+    __shared__ uint32_t s_tmem;
+    __shared__ volatile int s_abort;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, rank = (int)(blockIdx.x & 1);
+    const uint32_t raw = smem_u32(smem), base = (raw + 1023u) & ~1023u;
+    float* const stg = reinterpret_cast<float*>(smem + (base - raw) + (size_t)kPStages * kPBytes) + warp * (32 * 33);
+    auto full = [&](int s) { return smem_u32(&s_bar[s]); };
+    auto empty = [&](int s) { return smem_u32(&s_bar[kPStages + s]); };
+    auto accFull = [&](int a) { return smem_u32(&s_bar[2 * kPStages + a]); };
+    auto accEmpty = [&](int a) { return smem_u32(&s_bar[2 * kPStages + 2 + a]); };
+    if (tid == 0) {
+        for (int s = 0; s < kPStages; s++) { mbar_init(full(s), 1); mbar_init(empty(s), 1); }
+        for (int a = 0; a < 2; a++) { mbar_init(accFull(a), 1); mbar_init(accEmpty(a), 8); }
+        s_abort = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == 4) {
+        asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&s_tmem)), "r"(512u) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+    }
+    tc_fence_before();
+    __syncthreads();
+    cluster_barrier();                                       // both CTAs' barriers stand before anything arrives on them
+    tc_fence_after();
+    const uint32_t tmem = s_tmem;
+    const int tiles = p.mTiles * p.nTiles, first = (int)(blockIdx.x >> 1), stride = (int)(gridDim.x >> 1);
+
+    if (warp == 4) {
+        if (lane == 0) {
+            unsigned early = 0;                              // stages whose weights were requested before the wait
+            auto weights = [&](unsigned it, int kt, int n0) {
+                const int s = it % kPStages;
+                if (rank == 0) mbar_arrive_expect_tx(full(s), 2 * kPBytes);
+                tma_box_pair(base + s * kPBytes + kABytes, &p.w, kt * kGK, n0 + rank * (kPN / 2), in_first(full(s)));
+            };
+            if (first < tiles)
+                for (; early < (unsigned)kPStages && early < (unsigned)p.nK; early++) weights(early, (int)early, (first / p.mTiles) * kPN);
+            pdl_wait();
+            pdl_launch_dependents();
+            unsigned it = 0;
+            bool ok = true;
+            for (int t = first; t < tiles && ok; t += stride) {
+                const int row = (t % p.mTiles) * (2 * kGM) + rank * kGM, n0 = (t / p.mTiles) * kPN;
+                for (int kt = 0; kt < p.nK; kt++, it++) {
+                    const int s = it % kPStages;
+                    if (it >= early) {
+                        if (it >= (unsigned)kPStages && !mbar_wait(empty(s), (it / kPStages - 1) & 1, &s_abort, p.error, 215)) { ok = false; break; }
+                        weights(it, kt, n0);
+                    }
+                    tma_box_pair(base + s * kPBytes, &p.a, kt * kGK, row, in_first(full(s)));
+                }
+            }
+            if (!ok && rank == 0)                            // a wait ran out: let both CTAs' copies in flight land before the blocks go
+                for (unsigned back = 1; back <= (unsigned)kPStages && back <= it; back++) {
+                    const unsigned j = it - back;
+                    for (unsigned w = 0; w < (1u << 16) && !mbar_try_wait(full(j % kPStages), (j / kPStages) & 1); w++) {}
+                }
+        }
+        __syncwarp();
+    } else if (warp == 5) {
+        if (lane == 0 && rank == 0) {
+            pdl_wait();
+            pdl_launch_dependents();
+            unsigned it = 0, n = 0;
+            bool ok = true;
+            for (int t = first; t < tiles && ok; t += stride) {
+                const int a = n & 1;
+                if (n >= 2 && !mbar_wait(accEmpty(a), (n / 2 - 1) & 1, &s_abort, p.error, 216)) break;
+                tc_fence_after();
+                for (int kt = 0; kt < p.nK; kt++, it++) {
+                    const int s = it % kPStages;
+                    if (!mbar_wait(full(s), (it / kPStages) & 1, &s_abort, p.error, 217)) { ok = false; break; }
+                    tc_fence_after();
+                    const uint32_t sa = base + s * kPBytes, sw = sa + kABytes;
+#pragma unroll
+                    for (int k = 0; k < kGK / 16; k++)
+                        umma_f16_pair(tmem + (uint32_t)(a * kPN), desc_sw128(sa + k * 32), desc_sw128(sw + k * 32), kPIdesc, (kt | k) != 0);
+                    umma_commit_pair(empty(s));
+                }
+                if (ok) umma_commit_pair(accFull(a));
+                n++;
+            }
+        }
+        __syncwarp();
+    } else {
+        pdl_wait();
+        pdl_launch_dependents();
+        unsigned n = 0;
+        for (int t = first; t < tiles; t += stride) {
+            const int a = n & 1;
+            if (!__all_sync(0xffffffffu, mbar_wait(accFull(a), (n / 2) & 1, &s_abort, p.error, 218))) break;
+            tc_fence_after();
+            store_tile<kPN>(p, tmem + (uint32_t)(a * kPN), (t % p.mTiles) * (2 * kGM) + rank * kGM + warp * 32, p.M, (t / p.mTiles) * kPN, stg, warp, lane);
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(in_first(accEmpty(a))) : "memory");
+            n++;
+        }
+    }
+    __syncthreads();
+    cluster_barrier();                                       // neither CTA's memory is used from outside any more
+    if (warp == 4) {
+        tc_fence_after();
+        asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u) : "memory");
+    }
 }
 
 bool encode_rows(CUtensorMap* map, const void* base, size_t K, size_t pitch, size_t rows, int boxRows) {
@@ -242,14 +388,33 @@ bool run(GemmTcParams& p, const void* a, int aK, int aPitch, size_t aRows, const
     return true;
 }
 
+bool run_pair(GemmTcParams& p, const void* a, int aK, int aPitch, size_t aRows, const Bf16View& w, cudaStream_t s) {
+    if (!encode_rows(&p.a, a, aK, aPitch, aRows, kGM) || !encode_rows(&p.w, w.w, w.Kp, w.Kp, w.N, kPN / 2)) return false;
+    static bool attr = false;
+    if (!attr) {
+        DJ_CUDA_CHECK(cudaFuncSetAttribute(k_bf16_gemm_pair, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPSmem));
+        attr = true;
+    }
+    p.mTiles = (p.M + 2 * kGM - 1) / (2 * kGM); p.nTiles = (p.N + kPN - 1) / kPN;
+    const int pairs = std::min(p.mTiles * p.nTiles, g_num_sms / 2);
+    launch_k_cluster(k_bf16_gemm_pair, dim3((unsigned)(2 * pairs)), dim3(kGThreads), kPSmem, s, dim3(2), p);
+    return true;
+}
+// Rounds of pairs, each a little over four fifths of a round of single CTAs' 128 × 256 tiles; widths as below.
+double pair_cost(int M, int N) {
+    const long tiles = (long)((M + 2 * kGM - 1) / (2 * kGM)) * ((N + kPN - 1) / kPN);
+    return (double)((tiles + g_num_sms / 2 - 1) / (g_num_sms / 2)) * (kPN + 24) * 0.85;
+}
+
 // the tile width with the least work per SM, wider tiles first
-int pick_width(int mTiles, int N) {
+int pick_width(int mTiles, int N, double* cost = nullptr) {
     int best = 256; double bestCost = 1e30;
     for (int bn : {256, 128, 64}) {
         const long tiles = (long)mTiles * ((N + bn - 1) / bn);
-        const double cost = (double)((tiles + g_num_sms - 1) / g_num_sms) * (bn + 24);
-        if (cost < bestCost) { bestCost = cost; best = bn; }
+        const double c = (double)((tiles + g_num_sms - 1) / g_num_sms) * (bn + 24);
+        if (c < bestCost) { bestCost = c; best = bn; }
     }
+    if (cost != nullptr) *cost = bestCost;
     return best;
 }
 bool run_width(int bn, GemmTcParams& p, const void* a, int aK, int aPitch, size_t aRows, const Bf16View& w, cudaStream_t s) {
@@ -270,7 +435,10 @@ bool launch_bf16_gemm_tc(const Bf16LinearArgs& a, const GroupedRows* g, cudaStre
     p.error = g_dev_error;
     p.lenPos = nullptr; p.lenT = 0; p.outHalf = nullptr;
     if (!g) launch_stage_rows(a.a, a.b, a.w.Kp, a.M, nullptr, 1, a.ws, true, s);
-    return run_width(pick_width(p.mTiles, p.N), p, a.ws, a.w.Kp, a.w.Kp, a.M, a.w, s);
+    double cost;
+    const int width = pick_width(p.mTiles, p.N, &cost);
+    if (!g && pair_cost(a.M, p.N) <= cost && run_pair(p, a.ws, a.w.Kp, a.w.Kp, a.M, a.w, s)) return true;
+    return run_width(width, p, a.ws, a.w.Kp, a.w.Kp, a.M, a.w, s);
 }
 
 void launch_bf16_gemm_rows(const __nv_bfloat16* rows, int lda, int K, const float* pos, int T, int maxRows, const Bf16View& w, __nv_bfloat16* out, int ldo,
