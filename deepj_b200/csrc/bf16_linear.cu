@@ -287,22 +287,26 @@ void launch_bf16_store(const float* src, int rows, int cols, __nv_bfloat16* dst,
              dst_ld);
 }
 
+// False where the rows do not come in 16-byte pieces or are too long for the registers.
 template <typename OutT>
-static void stage_rows(const RowOperand& a, const RowOperand& b, int Kp, int rows, const int* map, int div, OutT* out, cudaStream_t s) {
+static bool stage_rows_in_registers(const RowOperand& a, const RowOperand& b, int Kp, int rows, const int* map, int div, OutT* out, cudaStream_t s) {
     const int K1p = pad8(a.k);
     auto aligned = [](const RowOperand& r) {
         return (((uintptr_t)r.x | (uintptr_t)r.gate | (uintptr_t)r.base | (uintptr_t)r.sum | (uintptr_t)r.gamma) & 15) == 0 &&
                ((r.k | r.ldx | (r.gate ? r.ldg : 0) | (r.base ? r.ldbase : 0) | (r.sum ? r.ldsum : 0)) & 3) == 0 && (r.groups < 2 || r.k / r.groups % 4 == 0);
     };
-    if (((uintptr_t)out & 15) == 0 && aligned(a) && (b.k == 0 || (aligned(b) && b.groups == 0)) && (a.groups == 0 || a.k <= 4096)) {
-        auto go = [&](auto kernel) { launch_k(kernel, dim3((unsigned)rows), dim3(256), 0, s, true, a, b, K1p, Kp, map, div, out); };
-        if (a.groups == 0 || a.k <= 1024) go(k_stage_rows<OutT, 1>);
-        else if (a.k <= 2048) go(k_stage_rows<OutT, 2>);
-        else go(k_stage_rows<OutT, 4>);
-        return;
-    }
+    if (((uintptr_t)out & 15) != 0 || !aligned(a) || (b.k > 0 && (!aligned(b) || b.groups > 0)) || (a.groups > 0 && a.k > 4096)) return false;
+    auto go = [&](auto kernel) { launch_k(kernel, dim3((unsigned)rows), dim3(256), 0, s, true, a, b, K1p, Kp, map, div, out); };
+    if (a.groups == 0 || a.k <= 1024) go(k_stage_rows<OutT, 1>);
+    else if (a.k <= 2048) go(k_stage_rows<OutT, 2>);
+    else go(k_stage_rows<OutT, 4>);
+    return true;
+}
+template <typename OutT>
+static void stage_rows(const RowOperand& a, const RowOperand& b, int Kp, int rows, const int* map, int div, OutT* out, cudaStream_t s) {
+    if (stage_rows_in_registers(a, b, Kp, rows, map, div, out, s)) return;
     raise_smem((const void*)k_stage_rows_any<OutT>, (size_t)Kp * 4);
-    launch_k(k_stage_rows_any<OutT>, dim3((unsigned)rows), dim3(256), (size_t)Kp * 4, s, true, a, b, K1p, Kp, map, div, out);
+    launch_k(k_stage_rows_any<OutT>, dim3((unsigned)rows), dim3(256), (size_t)Kp * 4, s, true, a, b, pad8(a.k), Kp, map, div, out);
 }
 
 void launch_stage_rows(const RowOperand& a, const RowOperand& b, int Kp, int rows, const int* map, int div, void* out, bool bf16, cudaStream_t s) {
@@ -311,6 +315,7 @@ void launch_stage_rows(const RowOperand& a, const RowOperand& b, int Kp, int row
 }
 
 void launch_norm_add(const RowOperand& x, float* out, int ldo, int rows, cudaStream_t s) {
+    if (ldo == x.k && x.k % 4 == 0 && stage_rows_in_registers(x, RowOperand(), x.k, rows, nullptr, 1, out, s)) return;
     const size_t smem = (size_t)pad8(x.k) * 4;
     raise_smem((const void*)k_norm_add, smem);
     launch_k(k_norm_add, dim3((unsigned)rows), dim3(256), smem, s, true, x, out, ldo);

@@ -268,7 +268,7 @@ DJ_PART void launch_mlstm(const MlstmArgs& a, cudaStream_t s);
 
 // ── misc ──
 void launch_embed_gather(const float* table, const float* ids, float* out, int rows, int d, int vocab, cudaStream_t s);
-// scratch: 2·16·rows ints of partial (key, index) pairs, tickets: rows zeroed self-resetting counters (rows ≤ kArgmaxRowsMax)
+// scratch: 2·32·rows ints of partial (key, index) pairs, tickets: rows zeroed self-resetting counters (rows ≤ kArgmaxRowsMax)
 constexpr int kArgmaxRowsMax = 4096;
 void launch_argmax_rows(const float* in, float* out, int rows, int cols, int* scratch, int* tickets, cudaStream_t s);
 // topK = 0 means the whole row (the reference's convention); more than 1024 candidates sort the row in `ws`

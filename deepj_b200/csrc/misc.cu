@@ -41,7 +41,7 @@ __device__ __forceinline__ int order_key(float v) {
 // keeps the lowest index among equals).  grid (parts, rows): every CTA reduces its slice of the row to one
 // (key, index) pair; the CTA that arrives last at the row (a self-resetting ticket) reduces the parts.  One CTA
 // per row costs a full load round trip per 1024 columns — 18 µs for a 32000-entry row.
-constexpr int kArgmaxParts = 16;
+constexpr int kArgmaxParts = 32;                 // 1000 columns of a 32000-entry row: one 16-byte load per thread
 __global__ void __launch_bounds__(256) k_argmax_rows(const float* __restrict__ in, float* __restrict__ out, int rows, int cols,
                                                       int* __restrict__ scratch, int* __restrict__ tickets) {
     __shared__ int s_key[8];
@@ -54,9 +54,17 @@ __global__ void __launch_bounds__(256) k_argmax_rows(const float* __restrict__ i
     const int per = ((cols + parts - 1) / parts + 3) & ~3;
     const int lo = min(cols, part * per), hi = min(cols, lo + per);
     int bestKey = INT_MIN, bestIdx = INT_MAX;
-    for (int c = lo + (int)threadIdx.x; c < hi; c += blockDim.x) {
-        int k = order_key(d[c]);
+    auto meet = [&](float v, int c) {
+        const int k = order_key(v);
         if (k > bestKey || (k == bestKey && c < bestIdx)) { bestKey = k; bestIdx = c; }
+    };
+    if ((cols & 3) == 0 && (reinterpret_cast<uintptr_t>(in) & 15) == 0) {      // lo and hi are multiples of four then
+        for (int c = lo + (int)threadIdx.x * 4; c < hi; c += blockDim.x * 4) {
+            const float4 v = *reinterpret_cast<const float4*>(d + c);
+            meet(v.x, c); meet(v.y, c + 1); meet(v.z, c + 2); meet(v.w, c + 3);
+        }
+    } else {
+        for (int c = lo + (int)threadIdx.x; c < hi; c += blockDim.x) meet(d[c], c);
     }
     auto warp_best = [&]() {
         for (int o = 16; o > 0; o >>= 1) {

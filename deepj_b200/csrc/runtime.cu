@@ -123,8 +123,8 @@ void ensure_init() {
     }
     // ticket counters of the split-attention merge and the batched linear, then the greedy pick's (kArgmaxRowsMax)
     // and its partial pairs (2 · 16 per row)
-    DJ_CUDA_CHECK(cudaMalloc((void**)&R.tickets, (kAttnTickets + kArgmaxRowsMax * 33) * sizeof(int)));
-    DJ_CUDA_CHECK(cudaMemset(R.tickets, 0, (kAttnTickets + kArgmaxRowsMax * 33) * sizeof(int)));
+    DJ_CUDA_CHECK(cudaMalloc((void**)&R.tickets, (kAttnTickets + kArgmaxRowsMax * 65) * sizeof(int)));
+    DJ_CUDA_CHECK(cudaMemset(R.tickets, 0, (kAttnTickets + kArgmaxRowsMax * 65) * sizeof(int)));
     DJ_CUDA_CHECK(cudaMalloc((void**)&g_dev_error, sizeof(int)));
     DJ_CUDA_CHECK(cudaMemset(g_dev_error, 0, sizeof(int)));
     R.inited = true;
