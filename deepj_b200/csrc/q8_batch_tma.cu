@@ -290,6 +290,18 @@ __global__ void __launch_bounds__(256) k_q8_batch_reduce(const BatchTail t, int 
     float rec[8];
     int tile = blockIdx.x;
     if (tile < nTiles) fetch(tile, rec, 0);
+    // bias and residual of a tile go out with its records
+    float bias = 0.0f, other = 0.0f;
+    auto operands = [&](int tile) {
+        const int n = tile * rowsPerTile + (SWIGLU ? r & 7 : r);
+        if (!live || n >= t.N) return;
+        if (SWIGLU) { const float* b = r < 8 ? t.bias : t.bias2; if (b) bias = b[n]; }
+        else {
+            if (t.bias) bias = t.bias[n];
+            if (t.residual) other = t.residual[(size_t)m * t.ldr + n];
+        }
+    };
+    operands(tile);
     {
         // row m's Σx²: the 16 threads of the row take the chunks r, r+16, … and meet in a fixed shuffle tree
         float ss = 0.0f;
@@ -307,27 +319,20 @@ __global__ void __launch_bounds__(256) k_q8_batch_reduce(const BatchTail t, int 
 #pragma unroll
             for (int q = 0; q < 8; q++) v += rec[q];
         }
-        v *= inv;
+        v = v * inv + bias;
+        const float res = other;
         const int next = tile + gridDim.x;
-        if (next < nTiles) fetch(next, rec, 0);
+        if (next < nTiles) { fetch(next, rec, 0); operands(next); }
         if (SWIGLU) {
             const float u = __shfl_down_sync(0xffffffffu, v, 8);      // the up projection's row sits 8 lanes on
             const int n = tile * rowsPerTile + r;
             if (m < t.M && r < 8 && n < t.N) {
-                float vv = v, uu = u;
-                if (t.bias) vv += t.bias[n];
-                if (t.bias2) uu += t.bias2[n];
-                const float sig = 1.0f / (1.0f + expf(-vv));
-                t.out[(size_t)m * t.ldo + n] = (vv * sig) * uu;
+                const float sig = 1.0f / (1.0f + expf(-v));
+                t.out[(size_t)m * t.ldo + n] = (v * sig) * u;
             }
         } else {
             const int n = tile * rowsPerTile + r;
-            if (m < t.M && n < t.N) {
-                float vv = v;
-                if (t.bias) vv += t.bias[n];
-                if (t.residual) vv += t.residual[(size_t)m * t.ldr + n];
-                t.out[(size_t)m * t.ldo + n] = vv;
-            }
+            if (m < t.M && n < t.N) t.out[(size_t)m * t.ldo + n] = v + res;
         }
     }
 }
@@ -349,7 +354,7 @@ void launch_batch_tma(const BatchTmaParams& p, cudaStream_t s) {
     const int gx = nItems < cap ? nItems : cap;
     launch_k(k_q8_gemm_i8<SWIGLU, NP, kDepth>, dim3(gx), dim3(kThreads), batch_tma_smem(kDepth), s, true, p);
     const int nChunksK = (p.K + kSlice - 1) / kSlice;
-    launch_k(k_q8_batch_reduce<SWIGLU>, dim3(p.nTiles < 4 * g_num_sms ? p.nTiles : 4 * g_num_sms), dim3(256), 0, s, true, p.tail, p.nTiles, nChunksK);
+    launch_k(k_q8_batch_reduce<SWIGLU>, dim3(p.nTiles < 8 * g_num_sms ? p.nTiles : 8 * g_num_sms), dim3(256), 0, s, true, p.tail, p.nTiles, nChunksK);
 }
 
 }  // namespace
