@@ -49,7 +49,8 @@ struct GemvTmaParams {
     const float* residual; int ldr;
     float* out; int ldo;
     int K, N, M, act;               // act 1: GELU behind the bias
-    int share, extra, depth;        // granules of 8 rows per block; the first `extra` blocks have one more; ring items per warp
+    int share, extra;               // granules of 8 rows per block; the first `extra` blocks have one more
+    int depth, chunk;               // ring items per warp; tiles between two barriers
     int* error;
     unsigned long long* trace;
 };
@@ -140,7 +141,14 @@ __global__ void __launch_bounds__(kThreads, 2) k_q8_gemv_tma(const __grid_consta
         const float4 a = *reinterpret_cast<const float4*>(q), b = *reinterpret_cast<const float4*>(q + 4);
         return ((((((a.x + a.y) + a.z) + a.w) + b.x) + b.y) + b.z) + b.w;
     };
-    // activations → digit columns in the MMA fragment's order; every warp converts the groups it consumes and goes on by itself
+    // activations → digit columns in the MMA fragment's order; every warp converts the groups it consumes and goes on by itself, the
+    // next row's first groups on their way while it converts a row's last
+    auto load_row = [&](const float* xrow) {
+#pragma unroll
+        for (int u = 0; u < kAhead; u++)
+            if (warp + kWarps * u < nGroups) xv[u] = ld4(xrow, warp + kWarps * u);
+    };
+    load_row(p.x);
     const int j8 = lane & 7, pos = j8 < 4 ? 8 * j8 : 8 * (j8 - 4) + 4;
 #pragma unroll 1
     for (int m = 0; m < p.M; m++) {
@@ -148,10 +156,6 @@ __global__ void __launch_bounds__(kThreads, 2) k_q8_gemv_tma(const __grid_consta
         int8_t* const dcol = xd + (size_t)(kGemvColsPerRow * m) * ldxs;
         float* const xscRow = xsc + (size_t)m * nBlocks;
         float ss = 0.0f, mean = 0.0f, inv = 1.0f;
-#pragma unroll
-        for (int u = 0; u < kAhead; u++)
-            if (warp + kWarps * u < nGroups) xv[u] = ld4(xrow, warp + kWarps * u);
-        if (m > 0) load_gain();
         if (GPT && p.beta) {                         // LayerNorm1D (norm/LayerNorm1D.java:34-71): the row's mean, then its biased variance, over the block
 #pragma unroll 1
             for (int pass = 0; pass < 2; pass++) {
@@ -189,9 +193,11 @@ __global__ void __launch_bounds__(kThreads, 2) k_q8_gemv_tma(const __grid_consta
                 }
                 gemv_digits4(v, gv[u], p.gamma != nullptr && !(GPT && p.beta), ss, dcol + grp * kItemK + (lane >> 3) * 32 + pos, ldxs, j8 == 0,
                              xscRow + grp * 4 + (lane >> 3));
-                if (grp + kWarps * kAhead < nGroups) {
-                    xv[u] = ld4(xrow, grp + kWarps * kAhead);
-                    if (p.gamma) gv[u] = ld4(p.gamma, grp + kWarps * kAhead);
+                const bool more = grp + kWarps * kAhead < nGroups;
+                if (more || m + 1 < p.M) {
+                    const int to = more ? grp + kWarps * kAhead : warp + kWarps * u;
+                    xv[u] = ld4(more ? xrow : xrow + p.ldx, to);
+                    if (p.gamma && nGroups > kWarps * kAhead) gv[u] = ld4(p.gamma, to);
                 }
             }
         }
@@ -222,7 +228,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_q8_gemv_tma(const __grid_consta
     const uint32_t lmChunk = (uint32_t)((lane >> 4) ^ (lrow & 7));
     int cslot = 0, limit = kSpinLimit;
     uint32_t phases = 0;
-    const int chunk = kChunk / p.M;                  // tiles between two barriers
+    const int chunk = p.chunk;
 #pragma unroll 1
     for (int tile0 = 0; tile0 < tiles; tile0 += chunk) {
         const int many = min(chunk, tiles - tile0);
@@ -323,21 +329,25 @@ __global__ void __launch_bounds__(kThreads, 2) k_q8_gemv_tma(const __grid_consta
     if (p.trace != nullptr && tid == 0) atomicMax(p.trace + 6, gtime());
 }
 
-size_t tma_smem_bytes(int K, int M, int depth) {
+size_t tma_smem_bytes(int K, int M, int depth, int chunk) {
     const size_t groups = (K + kItemK - 1) / kItemK;
     return 1024 + (size_t)kWarps * depth * kItemBytes + (size_t)kGemvColsPerRow * M * (groups * kItemK + kGemvXsPad) + M * groups * 16 +
-           (size_t)(kChunk / M) * M * 16 * kWarps * 4;
+           (size_t)chunk * M * 16 * kWarps * 4;
 }
 constexpr size_t kSmemHalf = 111 * 1024;         // two blocks per SM
 constexpr size_t kSmemWhole = 224 * 1024;        // a block with its SM to itself
-constexpr int kMinDepth = 3;
 
-// Ring items per warp, so that two blocks share an SM where that can be;
-// 0: no ring fits.
-int ring_depth(int K, int M) {
-    for (int d = kMaxDepth; d >= kMinDepth; d--)
-        if (tma_smem_bytes(K, M, d) <= kSmemHalf) return d;
-    return tma_smem_bytes(K, M, kMinDepth) <= kSmemWhole ? kMinDepth : 0;
+// Ring items per warp and tiles between two barriers beside the digits of M rows, so that two blocks share an SM; depth 0: they
+// do not fit.  Several rows that need a whole SM are taken in passes of fewer rows instead, or with shorter rings: launch to launch,
+// against one block per SM, 4 rows of 4096 → 12288 28.2 → 18.3 µs (two barriers in place of one), 2 of 11008 → 4096 25.4 → 15.9 (two ring
+// items), 4 of it 41.5 → 31.1 (two passes).  A single row may take an SM for one block.
+struct Ring { int depth, chunk; };
+Ring ring_for(int K, int M) {
+    const int full = kChunk / M;
+    for (int d = kMaxDepth; d >= 2; d--)
+        for (int c = full; c >= 1; c = d == kMaxDepth ? 0 : c / 2)
+            if (tma_smem_bytes(K, M, d, c) <= kSmemHalf) return {d, c};
+    return {M == 1 && tma_smem_bytes(K, M, 3, full) <= kSmemWhole ? 3 : 0, full};
 }
 
 template <bool SWIGLU, int NM, bool GPT>
@@ -349,8 +359,9 @@ void launch_tma(GemvTmaParams& p, cudaStream_t s) {
     }
     const int granules = (p.N + 7) / 8, gx = std::min(SWIGLU ? granules : (granules + 1) / 2, 2 * g_num_sms);
     p.share = granules / gx; p.extra = granules % gx;
-    p.depth = ring_depth(p.K, p.M);
-    launch_k(k_q8_gemv_tma<SWIGLU, NM, GPT>, dim3(gx), dim3(kThreads), tma_smem_bytes(p.K, p.M, p.depth), s, true, p);
+    const Ring r = ring_for(p.K, p.M);
+    p.depth = r.depth; p.chunk = r.chunk;
+    launch_k(k_q8_gemv_tma<SWIGLU, NM, GPT>, dim3(gx), dim3(kThreads), tma_smem_bytes(p.K, p.M, r.depth, r.chunk), s, true, p);
 }
 
 }  // namespace
@@ -390,7 +401,7 @@ bool launch_q8_gemv_tma(const Q8LinearArgs& a, cudaStream_t s) {
     const bool swiglu = a.w2.codes != nullptr, gpt = a.beta != nullptr || a.act != 0;
     if (K % 32 != 0 || g_dev_error == nullptr || (swiglu && (gpt || a.w2.K != K || a.w2.Kp != a.w.Kp || a.w2.N != a.w.N))) return false;
     if (((reinterpret_cast<uintptr_t>(a.x) | reinterpret_cast<uintptr_t>(a.gamma) | reinterpret_cast<uintptr_t>(a.beta)) & 15) != 0 || (a.M > 1 && a.ldx % 4 != 0)) return false;
-    if (ring_depth(K, 1) == 0) return false;
+    if (ring_for(K, 1).depth == 0) return false;
     GemvTmaParams p;
     if (!q8_encode_weight_maps(a.w, &p.codes, &p.scales)) return false;
     if (swiglu) {
@@ -398,7 +409,7 @@ bool launch_q8_gemv_tma(const Q8LinearArgs& a, cudaStream_t s) {
     } else { p.codes2 = p.codes; p.scales2 = p.scales; }
     for (int m0 = 0; m0 < a.M;) {
         int rows = std::min(a.M - m0, 4);            // 8 MMA columns = 2 activation rows × (3 digits + 1 unused); 3-4 rows take a second MMA
-        while (rows > 1 && ring_depth(K, rows) == 0) rows--;
+        while (rows > 1 && ring_for(K, rows).depth == 0) rows--;
         p.x = a.x + (size_t)m0 * a.ldx; p.ldx = a.ldx; p.gamma = a.gamma; p.beta = a.gamma ? a.beta : nullptr; p.eps = a.eps;
         p.bias = a.bias; p.bias2 = a.bias2; p.act = a.act;
         p.residual = a.residual ? a.residual + (size_t)m0 * a.ldr : nullptr; p.ldr = a.ldr;

@@ -52,3 +52,9 @@ def test_few_rows(K, N, M):
         check(rms * np.abs(u).max(), g / (1 + np.exp(-g)) * u, np.maximum(np.abs(w), np.abs(w2)) + np.abs(g).max() * np.abs(w2) / np.abs(u).max(), "gated pair")
     finally:
         dev.close()
+
+
+# rows whose digits leave room for: a barrier every two tiles; two ring items; two rows of three (a pass of two, a pass of one); two items and one tile
+@pytest.mark.parametrize("K,N,M", [(4096, 9600, 4), (11008, 5000, 2), (11008, 40, 3), (5632, 4744, 4)])
+def test_rings_beside_several_rows(K, N, M):
+    test_few_rows(K, N, M)
