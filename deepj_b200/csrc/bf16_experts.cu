@@ -1,7 +1,7 @@
 // Table-routed experts: a table row indexed by the token id names the `top` experts of the token, each of weight 1/top.
 //
 // Few rows, or models run in 32-bit: every (token, slot) entry is its own GEMV over its expert's weight rows
-// (bf16_linear.cu).  Many rows: the entries are sorted by expert into 128-row tiles and the feed-forward runs as two
+// (bf16_gemv.cu).  Many rows: the entries are sorted by expert into 128-row tiles and the feed-forward runs as two
 // grouped tensor-core products (bf16_gemm_tc.cu):
 //   k_expert_plan     one block: entries per expert, tile → expert, padded position → entry
 //   k_stage_rows      gathers the normed rows of the entries in that order

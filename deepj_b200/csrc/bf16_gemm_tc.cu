@@ -9,7 +9,8 @@
 //   warps 0-3  drain the other accumulator: tcgen05.ld, a shared-memory transpose, row-contiguous stores with residual,
 //            soft cap or the gated pair
 // Grouped form (table-routed experts): `tileExpert` gives each 128-row tile its expert (−1: no tile), whose weight rows
-// start at expert · N; `rowMap` scatters output rows.  Every wait is bounded (codes 211-214 in the device error word).
+// start at expert · N; `rowMap` scatters output rows.  Every wait is bounded (codes 211-214 in the device error word,
+// 215-218 in the form for pairs of SMs, whose comment stands at the kernel).
 #include "row_operand.cuh"
 #include "tc_common.cuh"
 

@@ -379,7 +379,7 @@ void dispatch_q8_linear(const Q8LinearArgs& a, cudaStream_t s) {
     const bool batchOk = batch_qualifies(a);
     if (runs_tc(a) && launch_q8_linear_tc(a, a.ws, s)) return;
     if (batchOk) {
-        // five or more rows share one pass over the weights, 16 at a time (up to four are two GEMV passes, which is as fast)
+        // five or more rows share one pass over the weights, 16 at a time (up to four take the GEMV, whose MMAs have room for them)
         bool ok = true;
         for (int m0 = 0; m0 < a.M && ok; m0 += 16) {
             const int rows = a.M - m0 < 16 ? a.M - m0 : 16;

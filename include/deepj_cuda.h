@@ -85,7 +85,7 @@ int deepj_cuda_trace_read(uint64_t* out, int32_t max_launches, int32_t* n_launch
  * captured, [3]=kernel nodes in the last replayed graph, [4]=workspace bytes,
  * [5]=device-side error flag of bounded waits (0 = none; 100 + rank: a tensor-parallel peer's data
  * never arrived; 201-207: a barrier of the tensor-core GEMM; 300-312: the whole-token kernel's grid barrier
- * or rings; 330 / 331: a bulk-copy item of the GEMV / several-row kernel never arrived),
+ * or rings; 330 - 333: a bulk-copy item of the Q8 GEMV, the several-row kernel, decode attention or the bf16 GEMV never arrived),
  * [6], [7]=bytes and number of released float buffers' blocks that are kept for later buffers (at most 256 MiB and 4096;
  * given back when an allocation of this library fails and by deepj_cuda_shutdown). */
 int deepj_cuda_stats(int64_t* counters, int32_t n);
