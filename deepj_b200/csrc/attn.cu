@@ -272,6 +272,7 @@ __global__ void __launch_bounds__(kAttnWarps * 32, 4) k_attn_decode(const AttnDe
         return;
     }
     if constexpr (CLUSTER) {
+        __syncwarp();                                                    // (the barrier's .aligned forms want whole warps)
         asm volatile("barrier.cluster.wait.aligned;" ::: "memory");      // every block of the cluster is running
         uint32_t to;
         asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(to) : "r"(smem_u32(&s_part[split][0])));
@@ -279,6 +280,7 @@ __global__ void __launch_bounds__(kAttnWarps * 32, 4) k_attn_decode(const AttnDe
 #pragma unroll 1
         for (int j = tid; j < HD; j += kAttnWarps * 32) put(j, blocks(j));
         if (tid == 0) { put(HD, M); put(HD + 1, L); }
+        __syncwarp();                                                    // heads of 16: half of the first warp has put a column
         asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
         if (split != 0) return;
         asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");

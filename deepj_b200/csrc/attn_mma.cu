@@ -258,6 +258,7 @@ __global__ void __launch_bounds__(128, 2) k_attn_prefill_mma(
             *reinterpret_cast<float2*>(po + row1 * LP + 2 * t4 + j * 8) = make_float2(o[j][2], o[j][3]);
         }
         if (t4 == 0) { pm[row0] = m0; pm[row1] = m1; pl[row0] = l0; pl[row1] = l1; }
+        __syncwarp();                                                    // the barrier's .aligned form wants whole warps
         asm volatile("barrier.cluster.arrive.release.aligned;\n barrier.cluster.wait.acquire.aligned;" ::: "memory");
         constexpr int LANES = HD / 4;                                    // threads of a row
         auto peer = [&](const float* p, int rank) {
@@ -289,6 +290,7 @@ __global__ void __launch_bounds__(128, 2) k_attn_prefill_mma(
                 *reinterpret_cast<float2*>(dst + 2) = make_float2(sum.z / L, sum.w / L);
             }
         }
+        __syncwarp();                                                    // heads of 64: the half warps' rows may end an iteration apart
         asm volatile("barrier.cluster.arrive.release.aligned;\n barrier.cluster.wait.acquire.aligned;" ::: "memory");      // nobody reads this block any more
         return;
     }
