@@ -30,7 +30,7 @@ extern int g_num_sms;
 // When true, launchers attach the programmatic-dependent-launch attribute so that
 // a kernel's weight prefetch overlaps the tail of its predecessor.
 extern bool g_use_pdl;
-// Q8 GEMV kernel choice (environment DEEPJ_CUDA_GEMV = cpasync | fma to step down: without the TMA kernels, without any tensor-pipe kernel); shapes outside a
+// Q8 GEMV kernel choice (environment DEEPJ_CUDA_GEMV = cpasync | fma to step down: without tensor copies, without any tensor-pipe kernel); shapes outside a
 // kernel's domain fall through to the next one.
 extern int g_gemv_mode;
 extern int g_tc_terms;      // deepj_cuda_tc_configure

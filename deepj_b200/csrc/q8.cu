@@ -349,7 +349,7 @@ void launch_q8_linear(const Q8LinearArgs& a0, cudaStream_t s) {
     if (a0.beta == nullptr && a0.act == 0) { dispatch_q8_linear(a0, s); return; }
     // GPT blocks: up to four rows go through the GEMV, which takes LayerNorm and GELU itself; the 16-row
     // kernels see already normalised rows and get the activation applied to their output afterwards
-    if (g_gemv_mode == 2 && a0.M < 5 && launch_q8_gemv_tma(a0, s)) return;
+    if (g_gemv_mode >= 1 && a0.M < 5 && launch_q8_gemv_tma(a0, s)) return;
     // the tensor-core kernel normalises in its pre-pass and activates in its epilogue; the 16-row kernel cannot
     if (runs_tc(a0) && launch_q8_linear_tc(a0, a0.ws, s)) return;
     Q8LinearArgs a = a0;
@@ -387,7 +387,7 @@ void dispatch_q8_linear(const Q8LinearArgs& a, cudaStream_t s) {
         }
         if (ok) return;
     }
-    if (g_gemv_mode == 2 && launch_q8_gemv_tma(a, s)) return;
+    if (g_gemv_mode >= 1 && launch_q8_gemv_tma(a, s)) return;
     if (swiglu) launch_gemv_dispatch<true>(p, a.M, s);
     else launch_gemv_dispatch<false>(p, a.M, s);
 }

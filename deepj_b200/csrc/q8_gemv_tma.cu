@@ -12,8 +12,9 @@
 // activations itself; its sums of a tile, the digits recombined, go to shared memory, and one barrier per 16 tiles (or at the
 // end) stands between them and the outputs.  (One block per SM with rings twice as deep: 5.9 against 4.7 ms for eight 7B steps, 8 warps
 // do not keep up with the stream.)  A launch of a few microseconds runs most of its code once, and fetching 1 KB of code
-// that another kernel has displaced takes 0.15 µs: the conversion is a loop over four groups in registers, rows that do not come in 16-byte
-// pieces take the FMA kernel.  Measured from the dependency wait to the last block's end, against the kernel with everything
+// that another kernel has displaced takes 0.15 µs: the conversion is a loop over four groups in registers, and rows that do not come in
+// 16-byte pieces have a form of their own (PLAIN), whose lanes also fill the rings themselves, with cp.async, so that it serves
+// without tensor maps too.  Measured from the dependency wait to the last block's end, against the kernel with everything
 // unrolled and a barrier per tile: 2048 → 2048 1.9-2.6 µs (1.9-2.9), gate and up of 5632 5.9 (7.6), 5632 → 2048 5.7 (6.0), head of
 // 32000 × 2048 13.2 (15.6), gate and up of 11008 × 4096 18.0 (19.2), 4096 → 4096 4.0 (5.2).  GPT blocks (LayerNorm, GELU, reduction lengths of 1600)
 // came from a cp.async kernel of 8.0 µs per launch: gpt2xl_request 9.5 → 8.5 ms.
@@ -43,6 +44,7 @@ constexpr int kErrTmaWait = 330;                    // device error code: an ite
 
 struct GemvTmaParams {
     CUtensorMap codes, scales, codes2, scales2;     // boxes of 8 rows; the second pair is the SwiGLU up projection
+    Q8View w, w2;                   // the same weights, for the PLAIN form
     const float* x; int ldx;
     const float* gamma; const float* beta; float eps;      // beta: LayerNorm instead of RMSNorm
     const float* bias; const float* bias2;
@@ -58,7 +60,8 @@ struct GemvTmaParams {
 __device__ __noinline__ float gelu_call(float v) { return gelu_ref(v); }
 
 // NM = 2 takes three or four activation rows in one pass over the weights (a second MMA per block).
-template <bool SWIGLU, int NM, bool GPT>
+// PLAIN: rows, gain and shift by single values; a warp copies its items itself, 16 bytes a lane and copy, laid out as the boxes are.
+template <bool SWIGLU, int NM, bool GPT, bool PLAIN>
 __global__ void __launch_bounds__(kThreads, 2) k_q8_gemv_tma(const __grid_constant__ GemvTmaParams p) {
     extern __shared__ unsigned char smem_raw[];
     __shared__ __align__(8) unsigned long long s_bar[kWarps * kMaxDepth];
@@ -85,7 +88,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_q8_gemv_tma(const __grid_consta
     const uint32_t myC = smem_u32(smem) + (uint32_t)(warp * p.depth) * kCodeBytes;
     const uint32_t myS = smem_u32(ringS) + (uint32_t)(warp * p.depth) * kScaleBytes;
     const uint32_t myBar = smem_u32(&s_bar[warp * kMaxDepth]);
-    if (lane < p.depth) mbar_init(myBar + 8 * lane, 1);
+    if (lane < p.depth) mbar_init(myBar + 8 * lane, PLAIN ? 32 : 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     __syncwarp();
 
@@ -94,7 +97,25 @@ __global__ void __launch_bounds__(kThreads, 2) k_q8_gemv_tma(const __grid_consta
     int itile = 0, igrp = warp, islot = 0;
     auto issue_next = [&]() {
         if (igrp >= nGroups || itile >= tiles) return;
-        if (lane == 0) {
+        if (PLAIN) {                                 // rows past N and columns past the row are zeros here too
+            const uint32_t bar = myBar + 8 * islot, dc = myC + (uint32_t)islot * kCodeBytes, ds = myS + (uint32_t)islot * kScaleBytes;
+            const int row = row0 + itile * (SWIGLU ? 8 : 16);
+            auto source = [&](int r, int& n) -> const Q8View& { n = row + (SWIGLU ? r & 7 : r); return SWIGLU && r >= 8 ? p.w2 : p.w; };
+#pragma unroll
+            for (int i = 0; i < 4; i++) {            // piece c of row r sits at r · 128 + ((c ^ (r & 7)) · 16)
+                const int r = i * 4 + (lane >> 3), c = lane & 7, k = igrp * kItemK + c * 16;
+                int n;
+                const Q8View& w = source(r, n);
+                const bool on = n < p.N && k < p.K;
+                cp_async16_zfill(dc + r * kItemK + ((c ^ (r & 7)) << 4), w.codes + (on ? (size_t)n * w.Kp + k : 0), on);
+            }
+            if (lane < 16) {
+                int n;
+                const Q8View& w = source(lane, n);
+                cp_async16_zfill(ds + lane * 16, w.scales + (n < p.N ? (size_t)n * w.nb + igrp * 4 : 0), n < p.N);
+            }
+            cp_async_arrive(bar);
+        } else if (lane == 0) {
             const uint32_t bar = myBar + 8 * islot, dc = myC + (uint32_t)islot * kCodeBytes, ds = myS + (uint32_t)islot * kScaleBytes;
             const int row = row0 + itile * (SWIGLU ? 8 : 16);
             if (SWIGLU) {
@@ -126,7 +147,8 @@ __global__ void __launch_bounds__(kThreads, 2) k_q8_gemv_tma(const __grid_consta
     float4 xv[kAhead], gv[kAhead];
     auto ld4 = [&](const float* q, int grp) {        // zeros behind the row's end
         const int k = grp * kItemK + lane * 4;
-        return k < p.K ? *reinterpret_cast<const float4*>(q + k) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        if (k >= p.K) return make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        return PLAIN ? make_float4(q[k], q[k + 1], q[k + 2], q[k + 3]) : *reinterpret_cast<const float4*>(q + k);
     };
     auto load_gain = [&]() {
 #pragma unroll
@@ -350,18 +372,18 @@ Ring ring_for(int K, int M) {
     return {M == 1 && tma_smem_bytes(K, M, 3, full) <= kSmemWhole ? 3 : 0, full};
 }
 
-template <bool SWIGLU, int NM, bool GPT>
+template <bool SWIGLU, int NM, bool GPT, bool PLAIN>
 void launch_tma(GemvTmaParams& p, cudaStream_t s) {
     static bool attrSet = false;
     if (!attrSet) {
-        DJ_CUDA_CHECK(cudaFuncSetAttribute(k_q8_gemv_tma<SWIGLU, NM, GPT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemWhole));
+        DJ_CUDA_CHECK(cudaFuncSetAttribute(k_q8_gemv_tma<SWIGLU, NM, GPT, PLAIN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemWhole));
         attrSet = true;
     }
     const int granules = (p.N + 7) / 8, gx = std::min(SWIGLU ? granules : (granules + 1) / 2, 2 * g_num_sms);
     p.share = granules / gx; p.extra = granules % gx;
     const Ring r = ring_for(p.K, p.M);
     p.depth = r.depth; p.chunk = r.chunk;
-    launch_k(k_q8_gemv_tma<SWIGLU, NM, GPT>, dim3(gx), dim3(kThreads), tma_smem_bytes(p.K, p.M, r.depth, r.chunk), s, true, p);
+    launch_k(k_q8_gemv_tma<SWIGLU, NM, GPT, PLAIN>, dim3(gx), dim3(kThreads), tma_smem_bytes(p.K, p.M, r.depth, r.chunk), s, true, p);
 }
 
 }  // namespace
@@ -394,19 +416,30 @@ bool q8_encode_weight_maps(const Q8View& w, CUtensorMap* codes, CUtensorMap* sca
     return true;
 }
 
-// Returns false when the shape is outside this kernel's domain: rows in 16-byte pieces, a ring beside the digits of one row, whole
-// blocks (the FMA kernel rounds less than the digits do: 1.0e-7 against 2e-7 of the result, and other lengths stay with it).
+namespace {
+
+template <bool PLAIN>
+void launch_rows(GemvTmaParams& p, bool swiglu, bool gpt, cudaStream_t s) {
+    if (swiglu) { if (p.M > 2) launch_tma<true, 2, false, PLAIN>(p, s); else launch_tma<true, 1, false, PLAIN>(p, s); }
+    else if (gpt) { if (p.M > 2) launch_tma<false, 2, true, PLAIN>(p, s); else launch_tma<false, 1, true, PLAIN>(p, s); }
+    else { if (p.M > 2) launch_tma<false, 2, false, PLAIN>(p, s); else launch_tma<false, 1, false, PLAIN>(p, s); }
+}
+
+}  // namespace
+
+// Returns false when the shape is outside this kernel's domain: a ring beside the digits of one row, whole blocks (the FMA kernel rounds
+// less than the digits do: 1.0e-7 against 2e-7 of the result, and other lengths stay with it).
 bool launch_q8_gemv_tma(const Q8LinearArgs& a, cudaStream_t s) {
     const int K = a.w.K;
     const bool swiglu = a.w2.codes != nullptr, gpt = a.beta != nullptr || a.act != 0;
     if (K % 32 != 0 || g_dev_error == nullptr || (swiglu && (gpt || a.w2.K != K || a.w2.Kp != a.w.Kp || a.w2.N != a.w.N))) return false;
-    if (((reinterpret_cast<uintptr_t>(a.x) | reinterpret_cast<uintptr_t>(a.gamma) | reinterpret_cast<uintptr_t>(a.beta)) & 15) != 0 || (a.M > 1 && a.ldx % 4 != 0)) return false;
     if (ring_for(K, 1).depth == 0) return false;
-    GemvTmaParams p;
-    if (!q8_encode_weight_maps(a.w, &p.codes, &p.scales)) return false;
-    if (swiglu) {
-        if (!q8_encode_weight_maps(a.w2, &p.codes2, &p.scales2)) return false;
-    } else { p.codes2 = p.codes; p.scales2 = p.scales; }
+    GemvTmaParams p = {};
+    // rows that do not come in 16-byte pieces, the setting that leaves tensor copies out, a driver without them
+    const bool pieces = ((reinterpret_cast<uintptr_t>(a.x) | reinterpret_cast<uintptr_t>(a.gamma) | reinterpret_cast<uintptr_t>(a.beta)) & 15) == 0 && (a.M == 1 || a.ldx % 4 == 0);
+    bool plain = !pieces || g_gemv_mode < 2 || !q8_encode_weight_maps(a.w, &p.codes, &p.scales);
+    if (!plain && swiglu) plain = !q8_encode_weight_maps(a.w2, &p.codes2, &p.scales2);
+    p.w = a.w; p.w2 = a.w2;
     for (int m0 = 0; m0 < a.M;) {
         int rows = std::min(a.M - m0, 4);            // 8 MMA columns = 2 activation rows × (3 digits + 1 unused); 3-4 rows take a second MMA
         while (rows > 1 && ring_for(K, rows).depth == 0) rows--;
@@ -417,9 +450,7 @@ bool launch_q8_gemv_tma(const Q8LinearArgs& a, cudaStream_t s) {
         p.K = K; p.N = a.w.N; p.M = rows;
         p.error = g_dev_error;
         p.trace = trace_slot();
-        if (swiglu) { if (rows > 2) launch_tma<true, 2, false>(p, s); else launch_tma<true, 1, false>(p, s); }
-        else if (gpt) { if (rows > 2) launch_tma<false, 2, true>(p, s); else launch_tma<false, 1, true>(p, s); }
-        else { if (rows > 2) launch_tma<false, 2, false>(p, s); else launch_tma<false, 1, false>(p, s); }
+        if (plain) launch_rows<true>(p, swiglu, gpt, s); else launch_rows<false>(p, swiglu, gpt, s);
         m0 += rows;
     }
     return true;

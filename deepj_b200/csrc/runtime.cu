@@ -23,7 +23,7 @@ namespace dj {
 long long g_launches = 0;
 int g_num_sms = 148;
 bool g_use_pdl = true;
-int g_gemv_mode = 2;   // 2: tensor-pipe kernels (TMA GEMV, several-row, tcgen05) with the FMA kernel as the fallback, 1: without the kernels on TMA rings, 0: FMA kernel only
+int g_gemv_mode = 2;   // 2: tensor-pipe kernels (GEMV, several-row, tcgen05) with the FMA kernel as the fallback, 1: the few-row and several-row ones without tensor copies, 0: FMA kernel only
 int* g_dev_error = nullptr;     // device int, 0 = no bounded wait has ever expired
 
 // Phase tracing (environment DEEPJ_CUDA_TRACE=1): every traced launch gets eight

@@ -1,5 +1,9 @@
 """The few-row Q8 kernel at the edges of its groups (128), its warps (8 groups), its register rounds (4 groups a warp), its tiles (16 rows,
 half tiles) and its chunks (16 tiles × rows), with RMSNorm, LayerNorm, GELU and the gated pair, against float64."""
+import os
+import subprocess
+import sys
+
 import numpy as np
 import pytest
 
@@ -18,7 +22,7 @@ def dequantized(dev, q, K, N):
 
 @pytest.mark.parametrize("K,N", SHAPES)
 @pytest.mark.parametrize("M", [1, 2, 4])
-def test_few_rows(K, N, M):
+def test_few_rows(K, N, M, off=0, pad=0):            # rows that start `off` values into their buffer and lie K + pad apart
     dev = Dev(9 << 20)
     try:
         rng = np.random.default_rng(K + N + M)
@@ -27,8 +31,11 @@ def test_few_rows(K, N, M):
         bias, res = rng.standard_normal(N).astype(np.float32), rng.standard_normal((M, N)).astype(np.float32)
         q, q2 = (dev.q8((rng.standard_normal((K, N)) * 0.05).astype(np.float32)) for _ in range(2))
         w, w2 = dequantized(dev, q, K, N), dequantized(dev, q2, K, N)
-        xb, gb, tb, bb, rb = (dev.buf(a.size, a) for a in (x, gamma, beta, bias, res))
-        ob = dev.buf(M * N)
+        spaced = np.full(off + M * (K + pad), np.nan, np.float32)
+        for m in range(M):
+            spaced[off + m * (K + pad):][:K] = x[m]
+        xb, gb, tb, bb, rb = (dev.buf(a.size, a) for a in (spaced, gamma, beta, bias, res))
+        ob, ld = dev.buf(M * N), K + pad
         x64 = x.astype(np.float64)
         rms = x64 / np.sqrt((x64 ** 2).mean(1, keepdims=True) + 1e-5) * gamma
         mean = x64.mean(1, keepdims=True)
@@ -40,14 +47,14 @@ def test_few_rows(K, N, M):
             size = (np.abs(row).max(1, keepdims=True) * np.abs(weights).sum(1)[None]) * (2.0 ** -22 + K / 256 * 2.0 ** -24) + 1e-6 * (np.abs(want) + 4)
             assert (np.abs(got - want) <= 2 * size).all(), (what, np.abs(got - want).max())
 
-        dev.flush([OP_Q8_LINEAR, xb, 0, K, -1, 0, q, -1, -1, 0, 0, ob, 0, N, M])
+        dev.flush([OP_Q8_LINEAR, xb, off, ld, -1, 0, q, -1, -1, 0, 0, ob, 0, N, M])
         check(x64, x64 @ w.T, w, "plain")
-        dev.flush([OP_Q8_LINEAR, xb, 0, K, gb, float_bits(1e-5), q, bb, rb, 0, N, ob, 0, N, M])
+        dev.flush([OP_Q8_LINEAR, xb, off, ld, gb, float_bits(1e-5), q, bb, rb, 0, N, ob, 0, N, M])
         check(rms, rms @ w.T + bias + res, w, "rms")
-        dev.flush([OP_Q8_LINEAR_LN, xb, 0, K, gb, tb, float_bits(1e-5), q, bb, -1, 0, 0, ob, 0, N, M, 1])
+        dev.flush([OP_Q8_LINEAR_LN, xb, off, ld, gb, tb, float_bits(1e-5), q, bb, -1, 0, 0, ob, 0, N, M, 1])
         z = ln @ w.T + bias
         check(ln, 0.5 * z * (1 + np.tanh(np.sqrt(2 / np.float64(np.float32(np.pi))) * (z + 0.044715 * z ** 3))), w, "layer norm and gelu")
-        dev.flush([OP_Q8_SWIGLU, xb, 0, K, gb, float_bits(1e-5), q, bb, q2, -1, ob, 0, N, M])
+        dev.flush([OP_Q8_SWIGLU, xb, off, ld, gb, float_bits(1e-5), q, bb, q2, -1, ob, 0, N, M])
         g, u = rms @ w.T + bias, rms @ w2.T
         check(rms * np.abs(u).max(), g / (1 + np.exp(-g)) * u, np.maximum(np.abs(w), np.abs(w2)) + np.abs(g).max() * np.abs(w2) / np.abs(u).max(), "gated pair")
     finally:
@@ -58,3 +65,19 @@ def test_few_rows(K, N, M):
 @pytest.mark.parametrize("K,N,M", [(4096, 9600, 4), (11008, 5000, 2), (11008, 40, 3), (5632, 4744, 4)])
 def test_rings_beside_several_rows(K, N, M):
     test_few_rows(K, N, M)
+
+
+# rows that do not come in 16-byte pieces, up to the reduction lengths beyond the FMA kernel's; a block with an SM to itself (from about 24000)
+@pytest.mark.parametrize("K,N,M,off,pad", [(128, 17, 4, 1, 1), (1056, 600, 1, 2, 0), (1600, 72, 2, 0, 1), (4096, 4800, 3, 3, 2), (11008, 40, 4, 0, 3), (16416, 24, 1, 1, 0),
+                                           (24864, 17, 2, 1, 1), (24864, 17, 1, 0, 0), (24864, 9, 4, 0, 4), (52608, 8, 1, 0, 0)])
+def test_rows_anywhere(K, N, M, off, pad):
+    test_few_rows(K, N, M, off, pad)
+
+
+def test_without_tensor_copies():
+    """The setting that leaves the kernels on tensor copies out: the same rows, lengths beyond the FMA kernel's among them."""
+    env = dict(os.environ, DEEPJ_CUDA_GEMV="cpasync")
+    here = os.path.abspath(__file__)
+    res = subprocess.run([sys.executable, "-m", "pytest", "-x", "-q", "-p", "no:cacheprovider", "-m", "gpu", here, "-k", "few_rows or rows_anywhere"], env=env,
+                         capture_output=True, text=True, timeout=600, cwd=os.path.dirname(os.path.dirname(here)))
+    assert res.returncode == 0 and f"{3 * len(SHAPES) + 10} passed" in res.stdout, res.stdout + res.stderr
