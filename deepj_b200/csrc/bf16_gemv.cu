@@ -12,6 +12,8 @@
 // held three steps of weights in registers: launch to launch): 46 MB gate and up 9.3 µs (12.6), 23 MB down 5.7 and 8.4 MB out
 // 5.1 (8.5 on average), head of 131 MB 21.2 µs = 6.2 TB/s.  Tried: asking the items behind the ring into L2 ahead of the wait (2-8 per
 // warp: 2-4 % slower steps).
+// Without tensor maps (PLAIN: a driver that gives none, or the setting that leaves tensor copies out) the lanes of a warp fill its ring with
+// cp.async, 16 bytes each; everything else is the same.
 // An item is ROWS weight rows × COLS columns.  A block owns a run of row groups; the items of that run, group by group, are cut
 // into equal parts, one per warp, so that narrow weights keep every warp busy too.  A warp sums a row group for as long as
 // its part stays in it and leaves the sum in shared memory; the end of the kernel adds the parts of a group in warp order.
@@ -41,6 +43,7 @@ constexpr int kPlain = 0, kExpertRows = 1, kExpertSum = 2;
 
 struct RgParams {
     CUtensorMap map;                             // boxes of an item, four columns to an element
+    const __nv_bfloat16* w; int wRows;           // the same weight, for the PLAIN form
     RowOperand a, b;
     int rows;                                    // activation rows of this pass, at most MR
     int N, Kp, K1p;                              // K1p: first column of segment b
@@ -126,7 +129,7 @@ __device__ __forceinline__ const float* more_of(const RowOperand& seg, int m) {
     return seg.gate ? seg.gate + (size_t)m * seg.ldg : seg.base ? seg.base + (size_t)m * seg.ldbase : nullptr;
 }
 
-template <int MR, int ROWS, int WARPS, int EXPERTS>
+template <int MR, int ROWS, int WARPS, int EXPERTS, bool PLAIN>
 __global__ void __launch_bounds__(WARPS * 32, MR == 1 ? 2 : 1) k_bf16_gemv(const __grid_constant__ RgParams p) {
     constexpr int COLS = kRgItem / 2 / ROWS, V = MR * ROWS, THREADS = WARPS * 32;
     extern __shared__ __align__(128) unsigned char smem[];
@@ -141,7 +144,7 @@ __global__ void __launch_bounds__(WARPS * 32, MR == 1 ? 2 : 1) k_bf16_gemv(const
     float* const xs = reinterpret_cast<float*>(smem + (size_t)p.warps * p.depth * kRgItem);
     float* const parts = xs + MR * row;
     const uint32_t ringAddr = smem_u32(ring), bars = smem_u32(&s_bar[warp * kRgMaxDepth]), xbar = smem_u32(&s_bar[WARPS * kRgMaxDepth]);
-    if (lane < p.depth) mbar_init(bars + 8 * lane, 1);
+    if (lane < p.depth) mbar_init(bars + 8 * lane, PLAIN ? 32 : 1);
     if (tid == 0) mbar_init(xbar, 1);
     if (tid < WARPS) s_rest[tid] = -1;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -155,7 +158,7 @@ __global__ void __launch_bounds__(WARPS * 32, MR == 1 ? 2 : 1) k_bf16_gemv(const
     int fLeft = left, fi = it, fg = g0 + p.firstGroup[more][warp], fs = 0, id = 0, slot = -1, slotRow = 0;
     auto fetch = [&] {
         fLeft--;
-        if (lane == 0) {
+        if (PLAIN || lane == 0) {
             int k = fi * COLS, n = fg * ROWS;
             if (EXPERTS != kPlain) {
                 const int s = EXPERTS == kExpertRows ? fg / p.groups : fi / p.items;
@@ -163,8 +166,18 @@ __global__ void __launch_bounds__(WARPS * 32, MR == 1 ? 2 : 1) k_bf16_gemv(const
                 if (EXPERTS == kExpertRows) n -= s * p.groups * ROWS; else k -= s * p.items * COLS;
             }
             const uint32_t bar = bars + 8 * fs;
-            mbar_arrive_expect_tx(bar, kRgItem);                     // what lies outside the weight counts, and comes as zeros
-            tma_box(ringAddr + fs * kRgItem, &p.map, k / 4, slotRow + n, bar);
+            if (PLAIN) {
+#pragma unroll 4
+                for (int i = lane; i < kRgItem / 16; i += 32) {      // piece i % (COLS / 8) of the item's row i / (COLS / 8)
+                    const int wr = slotRow + n + i / (COLS / 8), wk = k + i % (COLS / 8) * 8;
+                    const bool on = wr >= 0 && wr < p.wRows && wk < p.Kp;
+                    cp_async16_zfill(ringAddr + fs * kRgItem + i * 16, p.w + (on ? (size_t)wr * p.Kp + wk : 0), on);
+                }
+                cp_async_arrive(bar);
+            } else {
+                mbar_arrive_expect_tx(bar, kRgItem);                 // what lies outside the weight counts, and comes as zeros
+                tma_box(ringAddr + fs * kRgItem, &p.map, k / 4, slotRow + n, bar);
+            }
         }
         if (++fi == nIt) { fi = 0; fg++; }
         if (++fs == p.depth) fs = 0;
@@ -405,11 +418,12 @@ bool encode_items(CUtensorMap* map, const Bf16View& w, int cols, int rows) {
                CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-template <int MR, int ROWS, int WARPS, int EXPERTS>
+template <int MR, int ROWS, int WARPS, int EXPERTS, bool PLAIN = false>
 bool launch_rg(RgParams& p, const Bf16View& w, int tokens, cudaStream_t s) {
     constexpr int COLS = kRgItem / 2 / ROWS;
-    if (!encode_items(&p.map, w, COLS, ROWS)) throw std::runtime_error("bf16 projection: the driver refused the weight's tensor map");
-    p.Kp = w.Kp; p.error = g_dev_error;
+    if constexpr (!PLAIN)
+        if (g_gemv_mode < 2 || !encode_items(&p.map, w, COLS, ROWS)) return launch_rg<MR, ROWS, WARPS, EXPERTS, true>(p, w, tokens, s);
+    p.w = w.w; p.wRows = w.N; p.Kp = w.Kp; p.error = g_dev_error;
     p.items = (w.Kp + COLS - 1) / COLS;
     p.groups = (p.N + ROWS - 1) / ROWS;
     const int groups = p.groups * (EXPERTS == kExpertRows ? p.top : 1), items = p.items * (EXPERTS == kExpertSum ? p.top : 1);
@@ -462,10 +476,10 @@ bool launch_rg(RgParams& p, const Bf16View& w, int tokens, cudaStream_t s) {
     }
     static bool attr = false;
     if (!attr) {
-        DJ_CUDA_CHECK(cudaFuncSetAttribute(k_bf16_gemv<MR, ROWS, WARPS, EXPERTS>, cudaFuncAttributeMaxDynamicSharedMemorySize, kRgSmemMax));
+        DJ_CUDA_CHECK(cudaFuncSetAttribute(k_bf16_gemv<MR, ROWS, WARPS, EXPERTS, PLAIN>, cudaFuncAttributeMaxDynamicSharedMemorySize, kRgSmemMax));
         attr = true;
     }
-    launch_k(k_bf16_gemv<MR, ROWS, WARPS, EXPERTS>, dim3((unsigned)gx, (unsigned)tokens), dim3(WARPS * 32), smem, s, true, p);
+    launch_k(k_bf16_gemv<MR, ROWS, WARPS, EXPERTS, PLAIN>, dim3((unsigned)gx, (unsigned)tokens), dim3(WARPS * 32), smem, s, true, p);
     return true;
 }
 

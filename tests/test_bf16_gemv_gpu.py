@@ -1,5 +1,9 @@
 """The ring kernel of 1-16 rows: sizes at the edges of its items (1024 columns), row groups (two or four rows), blocks (one per
 SM), rings and staging pieces, against the product in float64."""
+import os
+import subprocess
+import sys
+
 import numpy as np
 import pytest
 
@@ -38,3 +42,13 @@ def test_ring_kernel(dev, K, N, M):  # noqa: F811
         assert (np.abs(got - want) <= 2.0 ** -24 * (K / 32 + 24) * size).all(), (normed, np.abs(got - want).max())
         if summed:
             assert np.allclose(dev.get(total, M * K).reshape(M, K), row, rtol=1e-5, atol=1e-5)
+
+
+def test_without_tensor_copies():
+    """The setting that leaves the kernels on tensor copies out, as a driver without tensor maps would: these rows, and table-routed experts."""
+    env = dict(os.environ, DEEPJ_CUDA_GEMV="cpasync")
+    here = os.path.abspath(__file__)
+    files = [here, os.path.join(os.path.dirname(here), "test_bf16_ops_gpu.py")]
+    res = subprocess.run([sys.executable, "-m", "pytest", "-x", "-q", "-p", "no:cacheprovider", "-m", "gpu", *files, "-k", "ring_kernel or experts or test_linear"],
+                         env=env, capture_output=True, text=True, timeout=600, cwd=os.path.dirname(os.path.dirname(here)))
+    assert res.returncode == 0 and " passed" in res.stdout and "skipped" not in res.stdout, res.stdout + res.stderr
