@@ -446,7 +446,7 @@ bool launch_rg(RgParams& p, const Bf16View& w, int tokens, cudaStream_t s) {
     for (p.warps = WARPS, p.depth = 0; p.depth == 0 && p.warps > 0; p.warps /= 2) {
         const int perWarp = (most * items + p.warps - 1) / p.warps;
         p.maxGroups = std::min(most, (perWarp + items - 2) / items + 1);
-        const size_t fixed = ((size_t)MR * items * COLS + std::max(scratch, WARPS * p.maxGroups * MR * ROWS)) * 4, step = (size_t)p.warps * kRgItem;
+        const size_t fixed = ((size_t)MR * items * COLS + std::max(scratch, p.warps * p.maxGroups * MR * ROWS)) * 4, step = (size_t)p.warps * kRgItem;
         auto fits = [&](size_t room) { return room > fixed ? (int)std::min<size_t>(kRgMaxDepth, (room - fixed) / step) : 0; };
         p.depth = std::min(MR == 1 && fits(kRgSmemHalf) >= 2 ? fits(kRgSmemHalf) : fits(kRgSmemMax), std::max(perWarp, 1));
         smem = fixed + p.depth * step;

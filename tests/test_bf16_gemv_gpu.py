@@ -7,7 +7,8 @@ import sys
 import numpy as np
 import pytest
 
-from deepj_b200.compute_graph import OP_BF16_LINEAR_SUM, float_bits
+from deepj_b200 import _lib
+from deepj_b200.compute_graph import OP_BF16_LINEAR_SUM, OP_TABLE_EXPERTS, float_bits
 from test_bf16_ops_gpu import bf16, dev  # noqa: F401
 
 pytestmark = pytest.mark.gpu
@@ -42,6 +43,32 @@ def test_ring_kernel(dev, K, N, M):  # noqa: F811
         assert (np.abs(got - want) <= 2.0 ** -24 * (K / 32 + 24) * size).all(), (normed, np.abs(got - want).max())
         if summed:
             assert np.allclose(dev.get(total, M * K).reshape(M, K), row, rtol=1e-5, atol=1e-5)
+
+
+# slots so many that two or four weight rows per item leave their padded rows no room (eight of 256 columns), up to the widest output whose sums still fit
+@pytest.mark.parametrize("M,k,d,ff,top", [(2, 72, 40, 8, 110), (1, 64, 24, 16, 180), (7, 16, 49152, 8, 195)])
+def test_experts_of_many_slots(dev, M, k, d, ff, top):  # noqa: F811
+    rng = np.random.default_rng(top + d)
+    vocab = 5
+    x, tok = rng.standard_normal((M, k)).astype(np.float32), rng.integers(0, vocab, M)
+    table = np.stack([rng.permutation(top) for _ in range(vocab)])
+    up, down = bf16(rng.standard_normal((top * 2 * ff, k)) * 0.3), bf16(rng.standard_normal((d, ff)) * 0.3)      # one down matrix for all experts
+    res = rng.standard_normal((M, d)).astype(np.float32)
+    U, W = dev.weight(k, top * 2 * ff, [(up, 0, 1, 0)]), dev.new()
+    _lib.check(dev.lib.deepj_cuda_bf16_alloc(W, ff, top * d))
+    src = dev.buf(down.size, down)
+    for e in range(top):
+        _lib.check(dev.lib.deepj_cuda_bf16_store(W, e * d, 1, 0, src, 0, d, ff))
+    out = dev.buf(M * d)
+    dev.flush([OP_TABLE_EXPERTS, dev.buf(x.size, x), 0, k, -1, 0, float_bits(0.0), dev.buf(M, tok), dev.buf(table.size, table), vocab, top, top, U, W, ff,
+               float_bits(7.0), dev.buf(res.size, res), 0, d, out, 0, d, d, M, 1])
+    pairs = (x.astype(np.float64) @ up.T.astype(np.float64)).reshape(M, top, ff, 2)
+    g, u = np.minimum(pairs[..., 0], 7.0), np.clip(pairs[..., 1], -7.0, 7.0)
+    y = g / (1 + np.exp(-1.702 * g)) * (u + 1)                       # [M, expert, ff]; every token names every expert
+    want = res + y.mean(1) @ down.T.astype(np.float64)
+    # fp32 chains of top · 8 / 32 ... products per lane and the warps' sums, of terms that add up to `size`; the gated values are good to 2^-21
+    size = np.abs(y).mean(1) @ np.abs(down).T.astype(np.float64) + np.abs(res)
+    assert (np.abs(dev.get(out, M * d).reshape(M, d) - want) <= (2.0 ** -21 + 2.0 ** -24 * (top / 4 + 40)) * size).all()
 
 
 def test_without_tensor_copies():
