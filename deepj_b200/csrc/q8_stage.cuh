@@ -22,8 +22,10 @@ __device__ __forceinline__ void gemv_digits4(const float4& x, const float4& gain
     amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
     amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 2));
     amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 4));
-    int sbits = 0x3f800000;                              // as digits16: s = 2^(exponent(amax)+2), q = rne(v·2^23/s)
-    if (amax > 0.0f && amax < 1e36f) sbits = (__float_as_int(amax) & 0x7f800000) + 0x01000000;
+    // as digits16: s = 2^(exponent(amax)+2), q = rne(v·2^23/s); at least the s whose 2^23/s is the largest power of two (with a gain x·γ is taken
+    // before the norm, and a block below 2^-106 would meet an infinite factor)
+    int sbits = 0x3f800000;
+    if (amax > 0.0f && amax < 1e36f) sbits = max(__float_as_int(amax) & 0x7f800000, 21 << 23) + 0x01000000;
     const float mul = __int_as_float(0x7f000000 - sbits) * 8388608.0f;
     uint32_t u[4];
 #pragma unroll

@@ -74,6 +74,23 @@ def test_rows_anywhere(K, N, M, off, pad):
     test_few_rows(K, N, M, off, pad)
 
 
+@pytest.mark.parametrize("K", [1600, 2048])
+def test_rows_of_tiny_values(K):
+    """Values below 2^-106, whose digit scale has no 32-bit inverse: the scale's last place is 2^-127, and with the weights' scales a subnormal
+    number of 12 bits or more."""
+    dev = Dev(9 << 20)
+    try:
+        rng = np.random.default_rng(K)
+        N, x = 40, (rng.standard_normal((2, K)) * 1e-33).astype(np.float32)
+        gamma, q = rng.uniform(0.5, 1.5, K).astype(np.float32), dev.q8((rng.standard_normal((K, N)) * 0.05).astype(np.float32))
+        w, ob = dequantized(dev, q, K, N), dev.buf(2 * N)
+        for g, row in ((-1, x.astype(np.float64)), (dev.buf(K, gamma), x.astype(np.float64) / np.sqrt(1e-5) * gamma)):
+            dev.flush([OP_Q8_LINEAR, dev.buf(x.size, x), 0, K, g, float_bits(1e-5), q, -1, -1, 0, 0, ob, 0, N, 2])
+            assert (np.abs(dev.get(ob, 2 * N).reshape(2, N) - row @ w.T) <= 2.0 ** -11 * (np.abs(row) @ np.abs(w).T)).all()
+    finally:
+        dev.close()
+
+
 def test_without_tensor_copies():
     """The setting that leaves the kernels on tensor copies out: the same rows, lengths beyond the FMA kernel's among them."""
     env = dict(os.environ, DEEPJ_CUDA_GEMV="cpasync")
