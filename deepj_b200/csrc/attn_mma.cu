@@ -7,7 +7,7 @@
 // product a·b is accumulated as a_hi·b_hi + a_lo·b_hi + a_hi·b_lo (the dropped lo·lo term is
 // ≈ 2^-22 of the product).
 //
-// grid (heads, ceil(T / 64), sequences × splits of the keys), the last query tiles first: they have the most keys, and started last they left the
+// grid (heads, ceil(T / 64), sequences × splits of the keys: SPLIT), the last query tiles first: they have the most keys, and started last they left the
 // chip to a few blocks at the end (32 heads of 128, 2048 tokens: 695 µs with the query tiles as the fast grid axis in rising
 // order, 545 µs this way).  128 threads.  Warp w owns query rows 16w … 16w+15 of the
 // tile; the CTA walks the keys in tiles of 32: K and V rows come from the fp32 cache, are split and
@@ -54,7 +54,7 @@ __device__ __forceinline__ void split2(float x0, float x1, uint32_t& hi, uint32_
     lo = pack_h2(__float2half_rn(x0 - __half2float(h0)), __float2half_rn(x1 - __half2float(h1)));
 }
 
-template <int HD, typename KT>
+template <int HD, typename KT, bool SPLIT>
 __global__ void __launch_bounds__(128, 2) k_attn_prefill_mma(
         const float* __restrict__ qkv, int q_off, int ld, const KT* __restrict__ kcache, const KT* __restrict__ vcache,
         int maxSeq, const float* __restrict__ posbuf, const float* __restrict__ cosT, const float* __restrict__ sinT,
@@ -72,7 +72,7 @@ __global__ void __launch_bounds__(128, 2) k_attn_prefill_mma(
     pdl_launch_dependents();
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int g = lane >> 2, t4 = lane & 3;
-    const int qt = (int)(gridDim.y - 1 - blockIdx.y), h = blockIdx.x, b = blockIdx.z / splits, split = blockIdx.z - b * splits;      // the tiles with the most keys first
+    const int qt = (int)(gridDim.y - 1 - blockIdx.y), h = blockIdx.x, b = SPLIT ? blockIdx.z / splits : blockIdx.z, split = SPLIT ? blockIdx.z - b * splits : 0;      // the tiles with the most keys first
     const int t0 = qt * kMQ;
     int pos0 = (int)posbuf[b];
     pos0 = pos0 < 0 ? 0 : pos0;
@@ -140,9 +140,16 @@ __global__ void __launch_bounds__(128, 2) k_attn_prefill_mma(
         }
     };
     // this block's tiles [from, nTiles) of the row tile's; the first into stage 0
-    const int allTiles = lastKey / kMK + 1, share = (allTiles + splits - 1) / splits;
-    const int from = split * share, nTiles = min(allTiles, from + share);
-    if (from < nTiles) {
+    const int allTiles = lastKey / kMK + 1;
+    int from = 0, nTiles = allTiles, used = 1;
+    if constexpr (SPLIT) {
+        // by the keys that there are: the cache may be far larger; two tiles of heads of 128 cost one block less than their merge
+        used = HD == 128 && allTiles == 2 ? 1 : min(splits, allTiles);
+        if (split >= used) return;                  // the whole block: a cluster barrier waits for threads that have not exited
+        const int share = (allTiles + used - 1) / used;
+        from = split * share; nTiles = min(allTiles, from + share);
+    }
+    if (!SPLIT || from < nTiles) {
         fetch(kb, from * kMK);                      // on its way while the queries are staged
         stage_q();
         put(Kh, Kl);
@@ -245,7 +252,7 @@ __global__ void __launch_bounds__(128, 2) k_attn_prefill_mma(
     }
     l0 += __shfl_xor_sync(0xffffffffu, l0, 1); l0 += __shfl_xor_sync(0xffffffffu, l0, 2);
     l1 += __shfl_xor_sync(0xffffffffu, l1, 1); l1 += __shfl_xor_sync(0xffffffffu, l1, 2);
-    if (splits > 1) {
+    if (SPLIT && used > 1) {
         // the splits of a row tile are a cluster: every block leaves its unnormalised rows in its own shared memory (the stages have been
         // read out) and adds up a share of the rows over all blocks
         constexpr int LP = HD + 4;
@@ -266,16 +273,16 @@ __global__ void __launch_bounds__(128, 2) k_attn_prefill_mma(
             asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_u32(p)), "r"(rank));
             return a;
         };
-        for (int r = split + splits * (tid / LANES); r < kMQ && t0 + r < T; r += splits * (128 / LANES)) {
+        for (int r = split + used * (tid / LANES); r < kMQ && t0 + r < T; r += used * (128 / LANES)) {
             const int c = tid % LANES * 4;
             float M = -INFINITY, L = 0.0f;
-            for (int q = 0; q < splits; q++) {
+            for (int q = 0; q < used; q++) {
                 float m;
                 asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(m) : "r"(peer(pm + r, q)) : "memory");
                 M = fmaxf(M, m);
             }
             float4 sum = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-            for (int q = 0; q < splits; q++) {
+            for (int q = 0; q < used; q++) {
                 float m, l; float4 v;
                 asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(m) : "r"(peer(pm + r, q)) : "memory");
                 asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(l) : "r"(peer(pl + r, q)) : "memory");
@@ -308,11 +315,15 @@ __global__ void __launch_bounds__(128, 2) k_attn_prefill_mma(
 
 template <int HD> constexpr size_t prefill_mma_smem() { return (size_t)(2 * kMQ + 2 * 4 * kMK) * (HD + 8) * sizeof(__half); }
 
-// Blocks that share a row tile's keys, a cluster of 2, 4 or 8: where the tiles alone leave half of the slots (two per SM) empty, and
-// the cache holds four key tiles for each.  32 heads × 64 behind 700 positions, 123 tokens: 64 blocks 79 µs, 256 blocks 32 (with the queries staged eight loads at a time behind the first keys).
-int prefill_splits(long long blocks, int maxSeq) {
+// Blocks that share a row tile's keys, a cluster of 2, 4 or 8: where the tiles alone leave half of the slots (two per SM) empty.  The
+// position is on the device, so how many of them find keys (a tile of 32 each at least) is seen by the kernel, and the others leave: with two
+// or four tiles each, or by the size of the cache, a chunk of 32 … 300 tokens in a new cache took up to 1.8 times as long.
+// With the cache append, 32 heads × 64, 123 tokens behind 700 positions: 64 blocks 63 µs, 256 blocks 26; alone 19.0 and 13.4; 32 heads × 128, 32 tokens behind
+// 700 positions 76 and 29, alone 11.4 and 11.9, 64 tokens alone 16.2 and 16.6.  Clusters of eight such blocks (104 KB each) cost 1.8 µs at launch,
+// where four cost 0.5 and gain nearly as much behind a context (24 and 29 µs): four for a single row tile of 16 heads and more.
+int prefill_splits(long long blocks, int maxSeq, int most) {
     int s = 1;
-    while (s < 8 && blocks * s * 2 <= 2 * g_num_sms && maxSeq >= s * 2 * 4 * kMK) s *= 2;
+    while (s < most && blocks * s * 2 <= 2 * g_num_sms && maxSeq >= s * 2 * kMK) s *= 2;
     return s;
 }
 
@@ -320,12 +331,13 @@ template <int HD, typename KT>
 void launch_mma(const AttnDecodeArgs& a, int T, cudaStream_t s) {
     static bool attr = false;
     if (!attr) {
-        DJ_CUDA_CHECK(cudaFuncSetAttribute(k_attn_prefill_mma<HD, KT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)prefill_mma_smem<HD>()));
+        DJ_CUDA_CHECK(cudaFuncSetAttribute(k_attn_prefill_mma<HD, KT, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)prefill_mma_smem<HD>()));
+        DJ_CUDA_CHECK(cudaFuncSetAttribute(k_attn_prefill_mma<HD, KT, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)prefill_mma_smem<HD>()));
         attr = true;
     }
-    const int qTiles = (T + kMQ - 1) / kMQ, splits = prefill_splits((long long)a.H * qTiles * a.B, a.maxSeq);
+    const int qTiles = (T + kMQ - 1) / kMQ, splits = prefill_splits((long long)a.H * qTiles * a.B, a.maxSeq, HD == 128 && qTiles == 1 && a.H * a.B >= 16 ? 4 : 8);
     const dim3 grid(a.H, qTiles, a.B * splits);
-    launch_k_cluster(k_attn_prefill_mma<HD, KT>, grid, dim3(128), prefill_mma_smem<HD>(), s, dim3(1, 1, splits), (const float*)a.qkv, a.q_off, a.ld,
+    launch_k_cluster(splits > 1 ? k_attn_prefill_mma<HD, KT, true> : k_attn_prefill_mma<HD, KT, false>, grid, dim3(128), prefill_mma_smem<HD>(), s, dim3(1, 1, splits), (const float*)a.qkv, a.q_off, a.ld,
                      (const KT*)a.kcache, (const KT*)a.vcache, a.maxSeq, a.pos, a.cosT, a.sinT, a.out, a.ldo, a.H, a.scale, T, splits);
 }
 

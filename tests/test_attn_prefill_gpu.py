@@ -41,7 +41,7 @@ def reference(q, k, v, cos, sin):
     return out
 
 
-def run_case(hd, T1, T2, B=2, H=3, seed=0):
+def run_case(hd, T1, T2, B=2, H=3, seed=0, spare=5):
     import ctypes
     from deepj_b200 import _lib
     from deepj_b200.compute_graph import OP_ATTN_PREFILL
@@ -50,7 +50,7 @@ def run_case(hd, T1, T2, B=2, H=3, seed=0):
     dev = Dev(9 << 20)
     try:
         d, L = H * hd, T1 + T2
-        max_seq = L + 5
+        max_seq = L + spare
         rng = np.random.default_rng(seed + hd + T1)
         qkv = rng.standard_normal((B, L, 3, H, hd)).astype(np.float32)
         qkv[:, :, 0] *= 2.0                                               # sharper softmax rows
