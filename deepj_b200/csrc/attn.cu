@@ -36,12 +36,16 @@ constexpr int kErrAttnWait = 332;           // device error code: a copy of cach
 // Prompt chunk: row z = (sequence b, token t) of the projection buffer holds k and v of position pos[b] + t.
 // A block per row, a thread per two interleaved pairs: rotate k (x0·c − x1·s, x0·s + x1·c — RotaryEmbedding.java:81-122), copy v.
 // 2048 rows of 32 heads × 128 took 71 µs as a block of 64 threads per head and row, 24 this way (21 µs at the copy bandwidth).
+// Chunks of 32 tokens and more let the attention kernel in at the end.  Let in at the start, its 150 … 300 blocks took as long as if some SMs had three
+// of them and others none: 32 heads × 64, 300 tokens behind 3000, both kernels 333 µs, 255 this way; 8 heads, 2048 tokens behind 700 239 and 216.
+// Shorter ones have little to wait for (2 tokens of 32 heads × 64 7.1 µs, 7.6 with the end).
+constexpr int kLateTokens = 32;
 template <typename KT>
 __global__ void __launch_bounds__(256) k_kv_append(const float* __restrict__ qkv, int k_off, int v_off, int ld, KT* __restrict__ kcache,
                             KT* __restrict__ vcache, int maxSeq, const float* __restrict__ posbuf,
                             const float* __restrict__ cosT, const float* __restrict__ sinT, int H, int hd, int T) {
     pdl_wait();
-    pdl_launch_dependents();
+    if (T < kLateTokens) pdl_launch_dependents();
     const int z = blockIdx.x, b = z / T, tok = z - b * T;
     const int p = (int)posbuf[b] + tok;
     if (p < 0 || p >= maxSeq) return;
@@ -56,6 +60,7 @@ __global__ void __launch_bounds__(256) k_kv_append(const float* __restrict__ qkv
         KvIo<KT>::st4(kcache + dst, make_float4(k.x * c.x - k.y * s.x, k.x * s.x + k.y * c.x, k.z * c.y - k.w * s.y, k.z * s.y + k.w * c.y));
         KvIo<KT>::st4(vcache + dst, v);
     }
+    if (T >= kLateTokens) pdl_launch_dependents();
 }
 
 // Ring items per warp: four blocks and a projection's beside them have to fit into an SM.
