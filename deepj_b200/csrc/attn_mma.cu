@@ -22,6 +22,8 @@
 // The arithmetic it restates: HeadOps.scaledDotProductScores / applyCausalMask / Softmax /
 // applyAttentionToValues (layers/transformer/attention/HeadOps.java:90-140, activations/Softmax.java:16-19);
 // masked terms contribute exactly 0, as exp(−1e9 − max) does in fp32.
+#include <algorithm>
+
 #include "kernels.h"
 #include "kv_cache.cuh"
 #include "q8_common.cuh"
@@ -314,6 +316,13 @@ __global__ void __launch_bounds__(128, 2) k_attn_prefill_mma(
 }
 
 template <int HD> constexpr size_t prefill_mma_smem() { return (size_t)(2 * kMQ + 2 * 4 * kMK) * (HD + 8) * sizeof(__half); }
+// Shared memory that a block of the unsplit form asks for: as much as spreads a grid of one or two blocks per SM evenly (three blocks of
+// heads of 64 fit onto an SM: 8 heads, 2048 tokens behind 3000, 256 blocks, 424 µs where they lie as they come, 377 so; behind 700 219 and 211).
+constexpr size_t kSpreadOne = 116 * 1024, kSpreadTwo = 100 * 1024;
+template <int HD> size_t prefill_smem_of(long long blocks) {
+    const size_t spread = blocks <= g_num_sms ? kSpreadOne : blocks <= 2 * g_num_sms ? kSpreadTwo : 0;
+    return std::max(prefill_mma_smem<HD>(), spread);
+}
 
 // Blocks that share a row tile's keys, a cluster of 2, 4 or 8: where the tiles alone leave half of the slots (two per SM) empty.  The
 // position is on the device, so how many of them find keys (a tile of 32 each at least) is seen by the kernel, and the others leave: with two
@@ -331,14 +340,17 @@ template <int HD, typename KT>
 void launch_mma(const AttnDecodeArgs& a, int T, cudaStream_t s) {
     static bool attr = false;
     if (!attr) {
-        DJ_CUDA_CHECK(cudaFuncSetAttribute(k_attn_prefill_mma<HD, KT, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)prefill_mma_smem<HD>()));
+        DJ_CUDA_CHECK(cudaFuncSetAttribute(k_attn_prefill_mma<HD, KT, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSpreadOne));
         DJ_CUDA_CHECK(cudaFuncSetAttribute(k_attn_prefill_mma<HD, KT, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)prefill_mma_smem<HD>()));
         attr = true;
     }
-    const int qTiles = (T + kMQ - 1) / kMQ, splits = prefill_splits((long long)a.H * qTiles * a.B, a.maxSeq, HD == 128 && qTiles == 1 && a.H * a.B >= 16 ? 4 : 8);
+    const int qTiles = (T + kMQ - 1) / kMQ;
+    const long long blocks = (long long)a.H * qTiles * a.B;
+    const int splits = prefill_splits(blocks, a.maxSeq, HD == 128 && qTiles == 1 && a.H * a.B >= 16 ? 4 : 8);
     const dim3 grid(a.H, qTiles, a.B * splits);
-    launch_k_cluster(splits > 1 ? k_attn_prefill_mma<HD, KT, true> : k_attn_prefill_mma<HD, KT, false>, grid, dim3(128), prefill_mma_smem<HD>(), s, dim3(1, 1, splits), (const float*)a.qkv, a.q_off, a.ld,
-                     (const KT*)a.kcache, (const KT*)a.vcache, a.maxSeq, a.pos, a.cosT, a.sinT, a.out, a.ldo, a.H, a.scale, T, splits);
+    launch_k_cluster(splits > 1 ? k_attn_prefill_mma<HD, KT, true> : k_attn_prefill_mma<HD, KT, false>, grid, dim3(128),
+                     splits > 1 ? prefill_mma_smem<HD>() : prefill_smem_of<HD>(blocks), s, dim3(1, 1, splits), (const float*)a.qkv, a.q_off, a.ld, (const KT*)a.kcache,
+                     (const KT*)a.vcache, a.maxSeq, a.pos, a.cosT, a.sinT, a.out, a.ldo, a.H, a.scale, T, splits);
 }
 
 }  // namespace
