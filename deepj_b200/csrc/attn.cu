@@ -63,8 +63,10 @@ __global__ void __launch_bounds__(256) k_kv_append(const float* __restrict__ qkv
     if (T >= kLateTokens) pdl_launch_dependents();
 }
 
-// Ring items per warp: four blocks and a projection's beside them have to fit into an SM.
-template <typename KT> constexpr int kRingStages = sizeof(KT) == 4 ? 2 : 3;
+// Ring items per warp, of 2 KB of K rows and their V rows: four blocks and a projection's beside them have to fit into an SM.  (fp16 rows in items of
+// half the size and lanes that read eight bytes a time: 12 heads × 64, 64 sequences at 200 17.3 µs, in place of 13.5 through cp.async rings; 13.4 this way.
+// 32 × 128, 24 tokens behind 500 52.5, 38.7 and 36.0.)
+constexpr int kRingStages = 2;
 struct AttnDecodeParams {
     const float* qkv; int q_off, k_off, v_off, ld;
     void* kcache; void* vcache; int maxSeq;
@@ -73,14 +75,16 @@ struct AttnDecodeParams {
     int* error;
 };
 
-// A lane holds elements 4·(c·LPP + gl) … +3, c = 0 … 3, of its position's rows: the lanes of a position read consecutive pieces.
+// A lane holds 16-byte pieces c·LPP + gl of its position's rows (four elements in fp32, eight in fp16): its neighbours read the pieces beside them.
 // CLUSTER: the splits of a head are one cluster, whose blocks leave their partials in the first one's shared memory.
 template <int LPP, typename KT, bool CLUSTER>   // lanes per position = hd / 16; cache element type
 __global__ void __launch_bounds__(kAttnWarps * 32, 4) k_attn_decode(const AttnDecodeParams p) {
     constexpr int HD = LPP * 16, half = HD / 2;
+    constexpr int PIECE = 16 / (int)sizeof(KT), NP = 16 / PIECE;         // elements of a piece, pieces of a lane
     constexpr int PPW = 32 / LPP;                 // positions per warp iteration
-    constexpr int G = kAttnWarps * PPW;           // positions per block iteration
-    constexpr int kStages = kRingStages<KT>, kPlane = PPW * HD * (int)sizeof(KT);      // ring items per warp: K rows of PPW consecutive positions, then their V rows
+    constexpr int GPI = 4 / (int)sizeof(KT), PPI = PPW * GPI;            // a ring item: so many groups of positions, 2 KB of K rows
+    constexpr int G = kAttnWarps * PPI;           // positions per block iteration
+    constexpr int kStages = kRingStages, kPlane = PPI * HD * (int)sizeof(KT);      // ring items per warp: K rows of PPI consecutive positions, then their V rows
     extern __shared__ __align__(128) unsigned char ring[];               // [warps][kStages][2][kPlane]
     __shared__ __align__(8) unsigned long long s_bar[kAttnWarps * kStages];
     __shared__ __align__(16) float s_acc[kAttnWarps][HD];
@@ -112,7 +116,7 @@ __global__ void __launch_bounds__(kAttnWarps * 32, 4) k_attn_decode(const AttnDe
         const int seq = pos + 1, chunk = (seq + splits - 1) / splits, start = split * chunk, end = min(seq, start + chunk);
         ownsNew = p.append && pos >= start && pos < end;
         endc = ownsNew ? pos : end;
-        at = start + warp * PPW;
+        at = start + warp * PPI;
     };
     const size_t plane = ((size_t)b * p.H + h) * p.maxSeq * HD;
     KT* const khead = static_cast<KT*>(p.kcache) + plane;
@@ -121,7 +125,7 @@ __global__ void __launch_bounds__(kAttnWarps * 32, 4) k_attn_decode(const AttnDe
     auto request = [&]() {
         if (lane == 0) {
             const int slot = asked % kStages;
-            const uint32_t bytes = min(PPW, endc - at) * HD * (int)sizeof(KT), bar = bars + 8 * slot, to = mine + slot * (2 * kPlane);
+            const uint32_t bytes = min(PPI, endc - at) * HD * (int)sizeof(KT), bar = bars + 8 * slot, to = mine + slot * (2 * kPlane);
             mbar_arrive_expect_tx(bar, 2 * bytes);
             bulk_g2s(to, khead + (size_t)at * HD, bytes, bar);
             bulk_g2s(to + kPlane, vhead + (size_t)at * HD, bytes, bar);
@@ -145,12 +149,13 @@ __global__ void __launch_bounds__(kAttnWarps * 32, 4) k_attn_decode(const AttnDe
 #pragma unroll 1
     for (int i = 0; i < kStages && at < endc && p.T == 1; i++) request();      // a chunk's own rows were written by the kernel before this one
     // the rotation tables are constants: the row of the early position is fetched before the wait too
-    float2 cs[4], sn[4];
+    float2 cs[4], sn[4];                          // of two pairs each
     auto load_tables = [&]() {
 #pragma unroll
-        for (int c = 0; c < 4; c++) {
-            cs[c] = *reinterpret_cast<const float2*>(p.cosT + (size_t)pos * half + 2 * (c * LPP + gl));
-            sn[c] = *reinterpret_cast<const float2*>(p.sinT + (size_t)pos * half + 2 * (c * LPP + gl));
+        for (int j = 0; j < 4; j++) {
+            const size_t at = (size_t)pos * half + PIECE / 2 * (j / (4 / NP) * LPP + gl) + j % (4 / NP) * 2;
+            cs[j] = *reinterpret_cast<const float2*>(p.cosT + at);
+            sn[j] = *reinterpret_cast<const float2*>(p.sinT + at);
         }
     };
     load_tables();
@@ -158,12 +163,15 @@ __global__ void __launch_bounds__(kAttnWarps * 32, 4) k_attn_decode(const AttnDe
     pdl_wait();
     pdl_launch_dependents();
     // the query row does not depend on the position: its loads go out together with the position's
-    const float* rowp = p.qkv + (size_t)z * p.ld + h * HD + 4 * gl;
-    auto load_row = [&](int off, float4 (&v)[4]) {
+    const float* rowp = p.qkv + (size_t)z * p.ld + h * HD + PIECE * gl;
+    auto load_row = [&](int off, float (&v)[16]) {
 #pragma unroll
-        for (int c = 0; c < 4; c++) v[c] = *reinterpret_cast<const float4*>(rowp + off + c * (4 * LPP));
+        for (int j = 0; j < 4; j++) {
+            const float4 a = *reinterpret_cast<const float4*>(rowp + off + j / (4 / NP) * (PIECE * LPP) + j % (4 / NP) * 4);
+            v[4 * j] = a.x; v[4 * j + 1] = a.y; v[4 * j + 2] = a.z; v[4 * j + 3] = a.w;
+        }
     };
-    float4 q[4], kx[4], vx[4];
+    float q[16], kx[16], vx[16];
     load_row(p.q_off, q);
     pos = read_pos();
     if (pos != early || p.T > 1) {
@@ -177,11 +185,13 @@ __global__ void __launch_bounds__(kAttnWarps * 32, 4) k_attn_decode(const AttnDe
         for (int i = 0; i < kStages && at < endc; i++) request();
     }
     // interleaved pairs (x0, x1) → (x0·c − x1·s, x0·s + x1·c)
-    auto rotate = [&](float4 (&v)[4]) {
+    auto rotate = [&](float (&v)[16]) {
 #pragma unroll
-        for (int c = 0; c < 4; c++)
-            v[c] = make_float4(v[c].x * cs[c].x - v[c].y * sn[c].x, v[c].x * sn[c].x + v[c].y * cs[c].x, v[c].z * cs[c].y - v[c].w * sn[c].y,
-                               v[c].z * sn[c].y + v[c].w * cs[c].y);
+        for (int i = 0; i < 8; i++) {
+            const float c = i & 1 ? cs[i / 2].y : cs[i / 2].x, s = i & 1 ? sn[i / 2].y : sn[i / 2].x, x0 = v[2 * i], x1 = v[2 * i + 1];
+            v[2 * i] = x0 * c - x1 * s;
+            v[2 * i + 1] = x0 * s + x1 * c;
+        }
     };
 
     float m = -INFINITY, l = 0.0f, acc[16];
@@ -190,32 +200,35 @@ __global__ void __launch_bounds__(kAttnWarps * 32, 4) k_attn_decode(const AttnDe
     const bool folds = ownsNew && warp == 0;      // warp-uniform
     if (folds) { load_row(p.k_off, kx); load_row(p.v_off, vx); }
     rotate(q);
-    // one group of positions a time: the new token's first (lane group 0), then what the ring holds
+    // one group of positions a time: the new token's first (lane group 0), then what the ring holds, GPI groups an item
+    const KT* item = nullptr;
+    int gi = 0;
 #pragma unroll 1
     for (bool fresh = folds; fresh || base < endc; fresh = false) {
-        bool valid = fresh ? group == 0 : base + group < endc;
+        const bool valid = fresh ? group == 0 : base + group < endc;
         if (fresh) {
             // k and v come from the projections; k is rotated, both are appended to the cache, and this step attends to what
             // later steps will read back (the rounded values of an fp16 cache)
             rotate(kx);
 #pragma unroll
-            for (int c = 0; c < 4; c++) {
+            for (int c = 0; c < NP; c++)
                 if (valid) {
-                    KvIo<KT>::st4(khead + (size_t)pos * HD + 4 * (c * LPP + gl), kx[c]);
-                    KvIo<KT>::st4(vhead + (size_t)pos * HD + 4 * (c * LPP + gl), vx[c]);
+                    KvIo<KT>::st_piece(khead + (size_t)pos * HD + PIECE * (c * LPP + gl), kx + PIECE * c);
+                    KvIo<KT>::st_piece(vhead + (size_t)pos * HD + PIECE * (c * LPP + gl), vx + PIECE * c);
                 }
-                kx[c] = make_float4(KvIo<KT>::stored(kx[c].x), KvIo<KT>::stored(kx[c].y), KvIo<KT>::stored(kx[c].z), KvIo<KT>::stored(kx[c].w));
-                vx[c] = make_float4(KvIo<KT>::stored(vx[c].x), KvIo<KT>::stored(vx[c].y), KvIo<KT>::stored(vx[c].z), KvIo<KT>::stored(vx[c].w));
-            }
-        } else {
-            const KT* item = reinterpret_cast<const KT*>(ring + (size_t)warp * (kStages * 2 * kPlane) + (taken % kStages) * (2 * kPlane)) + group * HD + 4 * gl;
-            take();
 #pragma unroll
-            for (int c = 0; c < 4; c++) { kx[c] = KvIo<KT>::ld4_shared(item + c * (4 * LPP)); vx[c] = KvIo<KT>::ld4_shared(item + PPW * HD + c * (4 * LPP)); }
+            for (int e = 0; e < 16; e++) { kx[e] = KvIo<KT>::stored(kx[e]); vx[e] = KvIo<KT>::stored(vx[e]); }
+        } else {
+            if (GPI == 1 || gi == 0) {
+                item = reinterpret_cast<const KT*>(ring + (size_t)warp * (kStages * 2 * kPlane) + (taken % kStages) * (2 * kPlane)) + group * HD + PIECE * gl;
+                take();
+            }
+#pragma unroll
+            for (int c = 0; c < NP; c++) { KvIo<KT>::ld_piece(item + c * (PIECE * LPP), kx + PIECE * c); KvIo<KT>::ld_piece(item + PPI * HD + c * (PIECE * LPP), vx + PIECE * c); }
         }
         float d[4];
 #pragma unroll
-        for (int c = 0; c < 4; c++) d[c] = fmaf(q[c].w, kx[c].w, fmaf(q[c].z, kx[c].z, fmaf(q[c].y, kx[c].y, q[c].x * kx[c].x)));
+        for (int j = 0; j < 4; j++) d[j] = fmaf(q[4 * j + 3], kx[4 * j + 3], fmaf(q[4 * j + 2], kx[4 * j + 2], fmaf(q[4 * j + 1], kx[4 * j + 1], q[4 * j] * kx[4 * j])));
         float dot = (d[0] + d[1]) + (d[2] + d[3]);
 #pragma unroll
         for (int o = LPP / 2; o > 0; o >>= 1) dot += __shfl_xor_sync(0xffffffffu, dot, o);
@@ -223,16 +236,16 @@ __global__ void __launch_bounds__(kAttnWarps * 32, 4) k_attn_decode(const AttnDe
             const float sc = dot * p.scale, mn = fmaxf(m, sc), corr = expf(m - mn), pe = expf(sc - mn);
             l = l * corr + pe;
 #pragma unroll
-            for (int c = 0; c < 4; c++) {
-                acc[4 * c] = fmaf(pe, vx[c].x, acc[4 * c] * corr);
-                acc[4 * c + 1] = fmaf(pe, vx[c].y, acc[4 * c + 1] * corr);
-                acc[4 * c + 2] = fmaf(pe, vx[c].z, acc[4 * c + 2] * corr);
-                acc[4 * c + 3] = fmaf(pe, vx[c].w, acc[4 * c + 3] * corr);
-            }
+            for (int e = 0; e < 16; e++) acc[e] = fmaf(pe, vx[e], acc[e] * corr);
             m = mn;
         }
-        if (!fresh) {
-            base += G;
+        if (!fresh && GPI > 1 && gi + 1 < GPI && base + PPW < endc) {
+            gi++;
+            base += PPW;
+            item += PPW * HD;
+        } else if (!fresh) {
+            base += G - gi * PPW;
+            gi = 0;
             __syncwarp();                         // the slot is read out before a later request may overwrite it
             if (at < endc) request();
         }
@@ -255,8 +268,8 @@ __global__ void __launch_bounds__(kAttnWarps * 32, 4) k_attn_decode(const AttnDe
         }
         if (group == 0) {
 #pragma unroll
-            for (int c = 0; c < 4; c++)
-                *reinterpret_cast<float4*>(&s_acc[warp][4 * (c * LPP + gl)]) = make_float4(acc[4 * c], acc[4 * c + 1], acc[4 * c + 2], acc[4 * c + 3]);
+            for (int j = 0; j < 4; j++)
+                *reinterpret_cast<float4*>(&s_acc[warp][j / (4 / NP) * (PIECE * LPP) + PIECE * gl + j % (4 / NP) * 4]) = make_float4(acc[4 * j], acc[4 * j + 1], acc[4 * j + 2], acc[4 * j + 3]);
         }
         if (lane == 0) { s_m[warp] = M; s_l[warp] = l; }
     }
@@ -538,7 +551,7 @@ void launch_attn_decode_t(const AttnDecodeArgs& a, cudaStream_t s) {
     }
     AttnDecodeParams p = {a.qkv, a.q_off, a.k_off, a.v_off, a.ld, kc, vc, a.maxSeq, a.pos, a.cosT, a.sinT, a.ws, a.tickets, a.out, a.ldo, a.H, a.scale, T,
                           T == 1 ? 1 : 0, g_dev_error};
-    const size_t smem = (size_t)kAttnWarps * kRingStages<KT> * 1024 * sizeof(KT);
+    const size_t smem = (size_t)kAttnWarps * kRingStages * 4096;
     // a few splits merge through the first block's shared memory instead of a ticket, a fence and a round trip to the partials
     const bool cluster = a.splits > 1 && a.splits <= kClusterSplits;
     auto go = [&](auto kernel) {
