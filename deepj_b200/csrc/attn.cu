@@ -9,7 +9,7 @@
 // x0·c − x1·s, x0·s + x1·c) and streams its slice of the cache once.  Cached rows of a head are contiguous, so a warp asks for
 // the K and the V rows of 32 / (hd / 16) positions with one bulk copy each, into a ring of its own, the first of them before the
 // dependency wait; hd/16 lanes per position, online softmax in fp32.  The block that owns the newest position takes k and v from the
-// projection buffer instead, rotates k and appends both to the cache.  Up to eight splits of a head are a cluster: each
+// projection buffer instead, rotates k and appends both to the cache.  Up to eight splits of a head are a cluster, where all clusters fit onto the chip: each
 // block leaves (acc[hd], m, l) in the first one's shared memory, one cluster barrier, done.  More splits leave them in a workspace, and the last
 // block of a head to finish (a ticket counter that it resets) merges them: a fence, the ticket and the loads are 2 µs.
 // HBM-bound with long contexts: the algorithmic traffic is the K and V rows of 0..pos.  Measured between the projections around
@@ -552,13 +552,30 @@ void launch_attn_decode_t(const AttnDecodeArgs& a, cudaStream_t s) {
     AttnDecodeParams p = {a.qkv, a.q_off, a.k_off, a.v_off, a.ld, kc, vc, a.maxSeq, a.pos, a.cosT, a.sinT, a.ws, a.tickets, a.out, a.ldo, a.H, a.scale, T,
                           T == 1 ? 1 : 0, g_dev_error};
     const size_t smem = (size_t)kAttnWarps * kRingStages * 4096;
-    // a few splits merge through the first block's shared memory instead of a ticket, a fence and a round trip to the partials
-    const bool cluster = a.splits > 1 && a.splits <= kClusterSplits;
+    // a few splits merge through the first block's shared memory instead of a ticket, a fence and a round trip to the partials,
+    bool cluster = a.splits > 1 && a.splits <= kClusterSplits;
     auto go = [&](auto kernel) {
         DJ_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024));
         launch_k_cluster(kernel, grid, block, smem, s, dim3(cluster ? a.splits : 1), p);
     };
-#define DJ_ATTN_CASE(L) case L: if (cluster) go(k_attn_decode<L, KT, true>); else go(k_attn_decode<L, KT, false>); break;
+    // where all clusters are resident at once (187 of three, 142 of four, 93 of six): a second, nearly empty wave took 8 heads × 128, 24 sequences at 1000
+    // from 20.5 µs to 33 (fp16; 35 and 41 in fp32)
+    auto fits = [&](auto kernel) {
+        if (!cluster) return false;
+        static int resident[33][kClusterSplits + 1];                     // clusters by lanes per position and splits, 0 = not asked yet
+        int& most = resident[lpp][a.splits];
+        if (most == 0) {
+            DJ_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024));
+            cudaLaunchAttribute attr;
+            attr.id = cudaLaunchAttributeClusterDimension;
+            attr.val.clusterDim.x = a.splits; attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+            cudaLaunchConfig_t cfg = {};
+            cfg.gridDim = dim3(a.splits); cfg.blockDim = block; cfg.dynamicSmemBytes = smem; cfg.attrs = &attr; cfg.numAttrs = 1;
+            DJ_CUDA_CHECK(cudaOccupancyMaxActiveClusters(&most, kernel, &cfg));
+        }
+        return rows * a.H <= most;
+    };
+#define DJ_ATTN_CASE(L) case L: cluster = fits(k_attn_decode<L, KT, true>); if (cluster) go(k_attn_decode<L, KT, true>); else go(k_attn_decode<L, KT, false>); break;
     switch (lpp) {
         DJ_ATTN_CASE(1) DJ_ATTN_CASE(2) DJ_ATTN_CASE(4) DJ_ATTN_CASE(8) DJ_ATTN_CASE(16) DJ_ATTN_CASE(32)
     }

@@ -19,10 +19,9 @@ pytestmark = pytest.mark.gpu
 # head dim, cache rows (one split per 64), cached positions of the first sequence
 @pytest.mark.parametrize("hd,max_seq,start", [(16, 40, 1), (32, 130, 63), (64, 70, 30), (64, 500, 127), (128, 60, 15), (128, 66, 33), (128, 640, 300), (256, 200, 70),
                                               (512, 140, 8), (64, 1300, 700)])
-def test_steps(hd, max_seq, start, half):
+def test_steps(hd, max_seq, start, half, B=2, H=3, steps=5):
     dev = Dev(9 << 20)
     try:
-        B, H, steps = 2, 3, 5
         d, n = H * hd, min(start + 7, max_seq - steps - 1)               # cached positions: `start` and n
         rng = np.random.default_rng(hd + max_seq)
         L = n + steps
@@ -36,7 +35,7 @@ def test_steps(hd, max_seq, start, half):
         _lib.check((dev.lib.deepj_cuda_kv_alloc_f16 if half else dev.lib.deepj_cuda_kv_alloc)(kv, 1, B, H, max_seq, hd))
         xb, pb = dev.buf(B * n * 3 * d, qkv[:, :n]), dev.buf(B, np.zeros(B))
         dev.flush([OP_ATTN_PREFILL, xb, 0, d, 2 * d, 3 * d, kv, 0, pb, cb, sb, dev.buf(B * n * d), 0, d, B, H, hd, n])
-        at = [start, n]
+        at = [start if b % 2 == 0 else n for b in range(B)]
         pb = dev.buf(B, np.array(at, dtype=np.float32))
         cmd, outs = [], []
         for s in range(steps):                                           # one stream: the position moves between the ops
@@ -59,3 +58,10 @@ def test_steps(hd, max_seq, start, half):
         assert st[5] == 0
     finally:
         dev.close()
+
+
+# three and six splits of so many heads that their clusters do not all fit onto the chip at once (187 and 93 do), and of fewer
+@pytest.mark.parametrize("half", [0, 1])
+@pytest.mark.parametrize("hd,max_seq,start,B,H", [(16, 192, 100, 24, 8), (64, 400, 300, 6, 16), (128, 192, 150, 10, 6)])
+def test_clusters_that_fit_and_do_not(hd, max_seq, start, B, H, half):
+    test_steps(hd, max_seq, start, half, B, H, 2)
