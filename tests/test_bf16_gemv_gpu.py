@@ -14,9 +14,10 @@ from test_bf16_ops_gpu import bf16, dev  # noqa: F401
 pytestmark = pytest.mark.gpu
 
 
-# K: below a piece of a warp, an item less and more one unit, rows of which half an SM holds two and one ring items, a whole SM; odd tails
+# K: below a piece of a warp, an item less and more one unit, rows of which half an SM holds two and one ring items, a whole SM; four
+# rows beside rings of half of the warps and of fewer, which go two by two; odd tails
 # N: fewer rows than warps or blocks, one row group more than the blocks, many groups per warp
-@pytest.mark.parametrize("K,N", [(8, 2), (8, 8), (24, 594), (1016, 298), (1024, 296), (1032, 2368), (2048, 66), (3000, 40), (4104, 304), (9000, 26), (20001, 18),
+@pytest.mark.parametrize("K,N", [(8, 2), (8, 8), (24, 594), (1016, 298), (1024, 296), (1032, 2368), (2048, 66), (3000, 40), (4104, 304), (9000, 26), (11840, 26), (13312, 18), (20001, 18),
                                  (50000, 10), (264, 20000)])
 @pytest.mark.parametrize("M", [1, 2, 3, 7])
 def test_ring_kernel(dev, K, N, M):  # noqa: F811
