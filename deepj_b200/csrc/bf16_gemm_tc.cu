@@ -401,10 +401,14 @@ bool run_pair(GemmTcParams& p, const void* a, int aK, int aPitch, size_t aRows, 
     launch_k_cluster(k_bf16_gemm_pair, dim3((unsigned)(2 * pairs)), dim3(kGThreads), kPSmem, s, dim3(2), p);
     return true;
 }
-// Rounds of pairs, each a little over four fifths of a round of single CTAs' 128 × 256 tiles; widths as below.
-double pair_cost(int M, int N) {
+// Rounds of pairs, in the units of the widths below.  What the pairs save is operand traffic, which bounds long reductions.  Over 32 … 3000 rows and
+// 512 … 40000 outputs, where their rounds cost as much as those of the best single width, they take 1.00 of its time up to lengths of 1024, 0.99 at
+// 2048, 0.96 at 4096 and beyond, and there the narrow widths fall behind by up to half.  Counted at 0.85 for all lengths they were taken for
+// short ones where single tiles fill the SMs better: 640 × 2048 → 40000 254 in place of 219 µs, 768 × 512 → 4096 39.4 and 35.0, 300 × 512 → 8192 38.4 and 30.9.
+constexpr int kPairLong = 3584;
+double pair_cost(int M, int N, int Kp) {
     const long tiles = (long)((M + 2 * kGM - 1) / (2 * kGM)) * ((N + kPN - 1) / kPN);
-    return (double)((tiles + g_num_sms / 2 - 1) / (g_num_sms / 2)) * (kPN + 24) * 0.85;
+    return (double)((tiles + g_num_sms / 2 - 1) / (g_num_sms / 2)) * (kPN + 24) * (Kp >= kPairLong ? 0.92 : 1.0);
 }
 
 // the tile width with the least work per SM, wider tiles first
@@ -438,7 +442,7 @@ bool launch_bf16_gemm_tc(const Bf16LinearArgs& a, const GroupedRows* g, cudaStre
     if (!g) launch_stage_rows(a.a, a.b, a.w.Kp, a.M, nullptr, 1, a.ws, true, s);
     double cost;
     const int width = pick_width(p.mTiles, p.N, &cost);
-    if (!g && pair_cost(a.M, p.N) <= cost && run_pair(p, a.ws, a.w.Kp, a.w.Kp, a.M, a.w, s)) return true;
+    if (!g && pair_cost(a.M, p.N, a.w.Kp) <= cost && run_pair(p, a.ws, a.w.Kp, a.w.Kp, a.M, a.w, s)) return true;
     return run_width(width, p, a.ws, a.w.Kp, a.w.Kp, a.M, a.w, s);
 }
 
@@ -452,3 +456,13 @@ void launch_bf16_gemm_rows(const __nv_bfloat16* rows, int lda, int K, const floa
 }
 
 }  // namespace dj
+
+// Which way `rows` rows of a many-row bf16 product go: out[0] = 1 for pairs of SMs and 0 for single ones, out[1] the tile width.
+extern "C" int deepj_cuda_bf16_route(int32_t rows, int32_t K, int32_t N, int32_t* out) {
+    if (rows < 1 || K < 1 || N < 1 || out == nullptr) { dj::set_last_error("bf16_route: bad arguments"); return 1; }
+    double cost;
+    const int width = dj::pick_width((rows + dj::kGM - 1) / dj::kGM, N, &cost);
+    out[0] = dj::pair_cost(rows, N, dj::pad8(K)) <= cost;
+    out[1] = out[0] ? dj::kPN : width;
+    return 0;
+}

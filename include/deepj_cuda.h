@@ -174,6 +174,10 @@ int deepj_cuda_tc_configure(int32_t correction_terms);
  * tuning; call deepj_cuda_init first.  No counterpart in the reference. */
 int deepj_cuda_q8_route(int32_t rows, int32_t K, int32_t N, int32_t swiglu, int32_t* out);
 
+/* How `rows` rows (more than 16) of a bf16 product K x N run: out[0] = 1 on pairs of SMs, 0 on single ones; out[1] = the tile width.  For tests
+ * and tuning; call deepj_cuda_init first.  No counterpart in the reference. */
+int deepj_cuda_bf16_route(int32_t rows, int32_t K, int32_t N, int32_t* out);
+
 /* Decode attention for callers that must not allocate.  No counterpart in the reference.
  *
  * Some hosts of this library cannot let a call reach cudaMalloc: a JVM thread inside a
