@@ -229,13 +229,15 @@ __device__ __forceinline__ float block_all(float v, float* r, F join) {      // 
 }
 
 // The row in registers, up to CH chunks of eight values per thread: one load round trip, the gain's ahead of the dependency wait.
-// 123 rows of 2048: 4.7 µs with passes over memory for each sum, 3.1 this way; 2048 rows of 4096 22 and 13.
+// 123 rows of 2048: 4.7 µs with passes over memory for each sum, 3.1 this way; 2048 rows of 4096 22 and 13.  Six chunks are one block per SM:
+// many rows of 6400 with LayerNorm took 1.4 times as long with their product as passes did, in four chunks as long.
 template <int CH>
 __global__ void __launch_bounds__(kXThreads) k_x_images(const XImages p) {
     __shared__ float red[3][kXThreads / 32];
     pdl_launch_dependents();
     const int tid = threadIdx.x, m = blockIdx.x;
-    float v[CH][8], g[CH][8];
+    constexpr bool EARLY = CH <= 4;                  // the shift too (with six chunks it would leave no registers)
+    float v[CH][8], g[CH][8], b[CH][8];
     auto load = [&](const float* from, float (&to)[CH][8], float fill) {
 #pragma unroll
         for (int i = 0; i < CH; i++)
@@ -248,6 +250,7 @@ __global__ void __launch_bounds__(kXThreads) k_x_images(const XImages p) {
             }
     };
     if (p.gamma != nullptr) load(p.gamma, g, 0.0f);
+    if (EARLY && p.beta != nullptr) load(p.beta, b, 0.0f);
     pdl_wait();
     load(p.x + (size_t)m * p.ldx, v, 0.0f);
     auto add = [](float a, float b) { return a + b; };
@@ -273,12 +276,13 @@ __global__ void __launch_bounds__(kXThreads) k_x_images(const XImages p) {
             for (int e = 0; e < 8; e++) ss = fmaf(v[i][e], v[i][e], ss);
         const float root = sqrtf(block_all(ss, red[1], add) * (1.0f / (float)p.K) + p.eps);
         if (p.beta != nullptr) {                     // LayerNorm divides by it, RMSNorm multiplies
-            float b[CH][8];
-            load(p.beta, b, 0.0f);
+            if (!EARLY) load(p.beta, b, 0.0f);
 #pragma unroll
             for (int i = 0; i < CH; i++)
+                if ((tid + i * kXThreads) * 8 < p.K) {       // (a division of zero takes the slow way)
 #pragma unroll
-                for (int e = 0; e < 8; e++) v[i][e] = __fdiv_rn(v[i][e], root) * g[i][e] + b[i][e];
+                    for (int e = 0; e < 8; e++) v[i][e] = __fdiv_rn(v[i][e], root) * g[i][e] + b[i][e];
+                }
         } else {
             const float inv = __frcp_rn(root);
 #pragma unroll
@@ -297,7 +301,7 @@ __global__ void __launch_bounds__(kXThreads) k_x_images(const XImages p) {
         if (tid + i * kXThreads < p.nS * p.per * 4) put_chunk(p, m, tid + i * kXThreads, v[i], s);
 }
 
-// Rows of any length: a pass for each sum.
+// Rows of any length: a pass for each sum, four neighbouring values a thread and step (eight, as the chunks are: 64 rows of 14336, with the product, 42 µs in place of 34).
 __global__ void __launch_bounds__(kXThreads) k_x_images_long(const XImages p) {
     __shared__ float red[3][kXThreads / 32];
     pdl_launch_dependents();
@@ -328,30 +332,25 @@ __global__ void __launch_bounds__(kXThreads) k_x_images_long(const XImages p) {
         if (p.beta != nullptr) return __fdiv_rn(v - mean, inv) * g + b;
         return p.gamma != nullptr ? (v * inv) * g : v;
     };
-    auto chunk = [&](int c, float (&v)[8]) {
-#pragma unroll
-        for (int h = 0; h < 2; h++) {
-            const int k = c * 8 + 4 * h;
-            float4 a = make_float4(0.f, 0.f, 0.f, 0.f), g = make_float4(1.f, 1.f, 1.f, 1.f), b = a;
-            const bool in = k < p.K;
-            if (in) a = *reinterpret_cast<const float4*>(xr + k);
-            if (in && p.gamma) g = *reinterpret_cast<const float4*>(p.gamma + k);
-            if (in && p.beta) b = *reinterpret_cast<const float4*>(p.beta + k);
-            v[4 * h] = in ? value(a.x, g.x, b.x) : 0.0f; v[4 * h + 1] = in ? value(a.y, g.y, b.y) : 0.0f;
-            v[4 * h + 2] = in ? value(a.z, g.z, b.z) : 0.0f; v[4 * h + 3] = in ? value(a.w, g.w, b.w) : 0.0f;
-        }
+    auto load4 = [&](int k, float* v) {
+        const float4 a = *reinterpret_cast<const float4*>(xr + k);
+        float4 g = make_float4(1.f, 1.f, 1.f, 1.f), b = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (p.gamma) g = *reinterpret_cast<const float4*>(p.gamma + k);
+        if (p.beta) b = *reinterpret_cast<const float4*>(p.beta + k);
+        v[0] = value(a.x, g.x, b.x); v[1] = value(a.y, g.y, b.y); v[2] = value(a.z, g.z, b.z); v[3] = value(a.w, g.w, b.w);
     };
     float amax = 0.0f;
-    for (int c = tid; c * 8 < p.K; c += kXThreads) {
-        float v[8];
-        chunk(c, v);
-#pragma unroll
-        for (int e = 0; e < 8; e++) amax = fmaxf(amax, fabsf(v[e]));
+    for (int k = tid * 4; k < p.K; k += 4 * kXThreads) {
+        float v[4];
+        load4(k, v);
+        amax = fmaxf(amax, fmaxf(fmaxf(fabsf(v[0]), fabsf(v[1])), fmaxf(fabsf(v[2]), fabsf(v[3]))));
     }
     const RowScale s = row_scale(block_all(amax, red[2], [](float a, float b) { return fmaxf(a, b); }), p.rowscale + m);
     for (int c = tid; c < p.nS * p.per * 4; c += kXThreads) {
-        float v[8];
-        chunk(c, v);
+        float v[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+        for (int h = 0; h < 2; h++)
+            if (c * 8 + 4 * h < p.K) load4(c * 8 + 4 * h, v + 4 * h);
         put_chunk(p, m, c, v, s);
     }
 }
@@ -858,7 +857,7 @@ bool launch_q8_linear_tc(const Q8LinearArgs& a, float* ws, cudaStream_t s) {
     float* const rowscale = ws + (size_t)p.nS * per * kBlockK * pl.nt * pl.mTiles;
     const XImages xi = {a.x, a.ldx, a.gamma, a.beta, a.eps, K, p.nS, pl.nt, per, images, rowscale};
     const int chunks = (p.nS * per * 4 + kXThreads - 1) / kXThreads;     // of eight values per thread
-    launch_k(chunks == 1 ? k_x_images<1> : chunks == 2 ? k_x_images<2> : chunks == 3 ? k_x_images<3> : chunks <= 6 ? k_x_images<6> : k_x_images_long, dim3((unsigned)M),
+    launch_k(chunks == 1 ? k_x_images<1> : chunks == 2 ? k_x_images<2> : chunks == 3 ? k_x_images<3> : chunks == 4 ? k_x_images<4> : chunks <= 6 ? k_x_images<6> : k_x_images_long, dim3((unsigned)M),
              dim3(kXThreads), 0, s, true, xi);
     p.images = images; p.rowscale = rowscale;
     p.scales = a.w.scales; p.scales2 = a.w2.scales; p.bias = a.bias; p.bias2 = a.bias2;
