@@ -51,7 +51,7 @@ struct BatchTmaParams {
     CUtensorMap codes, scales, codes2, scales2;
     const float* x; int ldx;
     const float* gamma;
-    int K, N, M, vec;                // vec: rows and gain come in 16-byte pieces
+    int K, N, M;
     int nSlices, nGroups, nTiles;
     BatchTail tail;
     int* error;
@@ -62,8 +62,6 @@ __device__ __forceinline__ void mma_s8u8_16832(int (&c)[4], uint32_t a0, uint32_
     asm("mma.sync.aligned.m16n8k32.row.col.s32.s8.u8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
         : "+r"(c[0]), "+r"(c[1]), "+r"(c[2]), "+r"(c[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
-
-__device__ __noinline__ void load16_columns(const float* from, float (&to)[16]) { load16(from, false, to); }
 
 // NP = MMA pairs per block: activation rows 0..7 (NP = 1) or 0..15 (NP = 2)
 template <bool SWIGLU, int NP, int kDepth>
@@ -121,13 +119,6 @@ __global__ void __launch_bounds__(kThreads, 2) k_q8_gemm_i8(const __grid_constan
     for (int d = 0; d < kPre; d++) issue_next();
     pdl_launch_dependents();
     if (tracing) p.trace[1] = gtime();
-    // the gain is a weight as well: that of the first slice is fetched before the wait
-    float gv[16];
-    int gained = blockIdx.x % p.nSlices;
-    auto load_row = [&](const float* from, float (&to)[16]) {
-        if (p.vec) load16(from, true, to); else load16_columns(from, to);
-    };
-    if (p.gamma && gained * kSlice + lane * 16 < p.K) load_row(p.gamma + gained * kSlice + lane * 16, gv);
     pdl_wait();
     if (tracing) p.trace[2] = gtime();
     for (int d = kPre; d < kDepth - 1; d++) issue_next();
@@ -151,49 +142,67 @@ __global__ void __launch_bounds__(kThreads, 2) k_q8_gemm_i8(const __grid_constan
         const int nGrp = groups_of(item);
         if (slice != staged) {
             __syncthreads();            // every warp is done with the previous slice's columns (and with the clearing above)
-            // a warp converts every eighth activation row, a lane 16 of its 512 values (half a block); the next row is on its way
-            const bool on = k0 + lane * 16 < p.K;
-            const float* const xk = p.x + k0 + lane * 16;
-            float xn[16];
-            if (on) load_row(xk + (size_t)min(warp, p.M - 1) * p.ldx, xn);
-            if (p.gamma && slice != gained && on) load_row(p.gamma + k0 + lane * 16, gv);
-            gained = slice;
-#pragma unroll 1
-            for (int m = warp; m < p.M; m += kWarps) {
-                float xv[16];
+            // one warp pass per activation row: 512 values; a lane converts 16 (half a block).  Two rows at once: one after the other, in half the code
+            // and with the gain loaded ahead of the wait, steps of 5 … 16 sequences took 1.02 of the time at widths of 256 … 4096, single projections of 5 rows 1.06.
+            for (int m0 = warp; m0 < p.M; m0 += 2 * kWarps) {
+                float xv[2][16], gv[2][16];
+                bool on[2];
 #pragma unroll
-                for (int j = 0; j < 16; j++) xv[j] = on ? xn[j] : 0.0f;
-                if (on && m + kWarps < p.M) load_row(xk + (size_t)(m + kWarps) * p.ldx, xn);
-                if (p.gamma) {
-                    float ss = 0.0f;
+                for (int u = 0; u < 2; u++) {
+                    const int m = m0 + u * kWarps;
+                    on[u] = m < p.M && k0 + lane * 16 < p.K;
+                    const float* xrow = p.x + (size_t)m * p.ldx + k0;
+                    const bool vec = ((reinterpret_cast<uintptr_t>(xrow) | (p.gamma ? reinterpret_cast<uintptr_t>(p.gamma + k0) : 0)) & 15) == 0;
+                    if (on[u]) {
+                        load16(xrow + lane * 16, vec, xv[u]);
+                        if (p.gamma) load16(p.gamma + k0 + lane * 16, vec, gv[u]);
+                    } else {
 #pragma unroll
-                    for (int j = 0; j < 16; j++) ss = fmaf(xv[j], xv[j], ss);
-                    for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
-                    if (lane == 0) p.tail.ssq[slice * kBatchMaxRows + m] = ss;      // every CTA that stages this slice writes the same bits
-#pragma unroll
-                    for (int j = 0; j < 16; j++) xv[j] *= gv[j];
+                        for (int j = 0; j < 16; j++) { xv[u][j] = 0.0f; gv[u][j] = 1.0f; }
+                    }
                 }
-                float amax = 0.0f;
 #pragma unroll
-                for (int j = 0; j < 16; j++) amax = fmaxf(amax, fabsf(xv[j]));
-                amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));          // the other half of the 32-k block
-                // q = rne(x · 32767 / amax) uses the whole 16-bit range; blocks whose largest value is below 2^-100 count as zero
-                const bool live = amax >= 7.8886e-31f && amax <= 3.0e38f;
-                const float mul = live ? __fdividef(32767.0f, amax) : 0.0f;
-                if (!on) continue;
-                // the block order of the MMA's B fragment (as gemv_digits4): the lane's values 4j … 4j+3 sit at 8j + 4·(half of the block)
-                unsigned char* bh = xd + (size_t)m * kLdx + (lane >> 1) * 32 + (lane & 1) * 4;
-                unsigned char* bl = bh + (size_t)kBatchMaxRows * kLdx;
+                for (int u = 0; u < 2; u++) {
+                    const int m = m0 + u * kWarps;
+                    if (m >= p.M) break;                               // warp-uniform
+                    if (p.gamma) {
+                        float ss = 0.0f;
 #pragma unroll
-                for (int j = 0; j < 4; j++) {
-                    uint32_t q[4];
+                        for (int j = 0; j < 16; j++) ss = fmaf(xv[u][j], xv[u][j], ss);
+                        for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+                        if (lane == 0) p.tail.ssq[slice * kBatchMaxRows + m] = ss;      // every CTA that stages this slice writes the same bits
 #pragma unroll
-                    for (int i = 0; i < 4; i++) q[i] = (uint32_t)min(__float2int_rn(xv[4 * j + i] * mul), 32767);
-                    const uint32_t t0 = __byte_perm(q[0], q[1], 0x5140), t1 = __byte_perm(q[2], q[3], 0x5140);
-                    *reinterpret_cast<uint32_t*>(bl + 8 * j) = __byte_perm(t0, t1, 0x5410);          // bits 0-7 of the four values
-                    *reinterpret_cast<uint32_t*>(bh + 8 * j) = __byte_perm(t0, t1, 0x7632);          // bits 8-15: the signed high byte
+                        for (int j = 0; j < 16; j++) xv[u][j] *= gv[u][j];
+                    }
+                    float amax = 0.0f;
+#pragma unroll
+                    for (int j = 0; j < 16; j++) amax = fmaxf(amax, fabsf(xv[u][j]));
+                    amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));          // the other half of the 32-k block
+                    // q = rne(x · 32767 / amax) uses the whole 16-bit range; blocks whose largest value is below 2^-100 count as zero
+                    const bool live = amax >= 7.8886e-31f && amax <= 3.0e38f;
+                    const float mul = live ? __fdividef(32767.0f, amax) : 0.0f;
+                    uint32_t whi[4], wlo[4];
+#pragma unroll
+                    for (int j = 0; j < 4; j++) {
+                        uint32_t q[4];
+#pragma unroll
+                        for (int i = 0; i < 4; i++) q[i] = (uint32_t)min(__float2int_rn(xv[u][4 * j + i] * mul), 32767);
+                        const uint32_t t0 = __byte_perm(q[0], q[1], 0x5140), t1 = __byte_perm(q[2], q[3], 0x5140);
+                        wlo[j] = __byte_perm(t0, t1, 0x5410);          // bits 0-7 of the four values
+                        whi[j] = __byte_perm(t0, t1, 0x7632);          // bits 8-15: the signed high byte
+                    }
+                    if (on[u]) {
+                        // the block order of the MMA's B fragment (as gemv_digits4): the lane's values 4j … 4j+3 sit at 8j + 4·(half of the block)
+                        unsigned char* bh = xd + (size_t)m * kLdx + (lane >> 1) * 32 + (lane & 1) * 4;
+                        unsigned char* bl = bh + (size_t)kBatchMaxRows * kLdx;
+#pragma unroll
+                        for (int j = 0; j < 4; j++) {
+                            *reinterpret_cast<uint32_t*>(bh + 8 * j) = whi[j];
+                            *reinterpret_cast<uint32_t*>(bl + 8 * j) = wlo[j];
+                        }
+                        if ((lane & 1) == 0) xs[m * kXsLd + (lane >> 1)] = live ? amax * (1.0f / 32767.0f) : 0.0f;
+                    }
                 }
-                if ((lane & 1) == 0) xs[m * kXsLd + (lane >> 1)] = live ? amax * (1.0f / 32767.0f) : 0.0f;
             }
             staged = slice;
             __syncthreads();
@@ -290,18 +299,6 @@ __global__ void __launch_bounds__(256) k_q8_batch_reduce(const BatchTail t, int 
     float rec[8];
     int tile = blockIdx.x;
     if (tile < nTiles) fetch(tile, rec, 0);
-    // bias and residual of a tile go out with its records
-    float bias = 0.0f, other = 0.0f;
-    auto operands = [&](int tile) {
-        const int n = tile * rowsPerTile + (SWIGLU ? r & 7 : r);
-        if (!live || n >= t.N) return;
-        if (SWIGLU) { const float* b = r < 8 ? t.bias : t.bias2; if (b) bias = b[n]; }
-        else {
-            if (t.bias) bias = t.bias[n];
-            if (t.residual) other = t.residual[(size_t)m * t.ldr + n];
-        }
-    };
-    operands(tile);
     {
         // row m's Σx²: the 16 threads of the row take the chunks r, r+16, … and meet in a fixed shuffle tree
         float ss = 0.0f;
@@ -319,20 +316,27 @@ __global__ void __launch_bounds__(256) k_q8_batch_reduce(const BatchTail t, int 
 #pragma unroll
             for (int q = 0; q < 8; q++) v += rec[q];
         }
-        v = v * inv + bias;
-        const float res = other;
+        v *= inv;
         const int next = tile + gridDim.x;
-        if (next < nTiles) { fetch(next, rec, 0); operands(next); }
+        if (next < nTiles) fetch(next, rec, 0);
         if (SWIGLU) {
             const float u = __shfl_down_sync(0xffffffffu, v, 8);      // the up projection's row sits 8 lanes on
             const int n = tile * rowsPerTile + r;
             if (m < t.M && r < 8 && n < t.N) {
-                const float sig = 1.0f / (1.0f + expf(-v));
-                t.out[(size_t)m * t.ldo + n] = (v * sig) * u;
+                float vv = v, uu = u;
+                if (t.bias) vv += t.bias[n];
+                if (t.bias2) uu += t.bias2[n];
+                const float sig = 1.0f / (1.0f + expf(-vv));
+                t.out[(size_t)m * t.ldo + n] = (vv * sig) * uu;
             }
         } else {
             const int n = tile * rowsPerTile + r;
-            if (m < t.M && n < t.N) t.out[(size_t)m * t.ldo + n] = v + res;
+            if (m < t.M && n < t.N) {
+                float vv = v;
+                if (t.bias) vv += t.bias[n];
+                if (t.residual) vv += t.residual[(size_t)m * t.ldr + n];
+                t.out[(size_t)m * t.ldo + n] = vv;
+            }
         }
     }
 }
@@ -354,7 +358,7 @@ void launch_batch_tma(const BatchTmaParams& p, cudaStream_t s) {
     const int gx = nItems < cap ? nItems : cap;
     launch_k(k_q8_gemm_i8<SWIGLU, NP, kDepth>, dim3(gx), dim3(kThreads), batch_tma_smem(kDepth), s, true, p);
     const int nChunksK = (p.K + kSlice - 1) / kSlice;
-    launch_k(k_q8_batch_reduce<SWIGLU>, dim3(p.nTiles < 8 * g_num_sms ? p.nTiles : 8 * g_num_sms), dim3(256), 0, s, true, p.tail, p.nTiles, nChunksK);
+    launch_k(k_q8_batch_reduce<SWIGLU>, dim3(p.nTiles < 4 * g_num_sms ? p.nTiles : 4 * g_num_sms), dim3(256), 0, s, true, p.tail, p.nTiles, nChunksK);
 }
 
 }  // namespace
@@ -377,7 +381,6 @@ bool launch_q8_linear_batch_tma(const Q8LinearArgs& a, int m0, int rows, float* 
     const int rowsPerTile = swiglu ? 8 : 16;
     p.x = a.x + (size_t)m0 * a.ldx; p.ldx = a.ldx; p.gamma = a.gamma;
     p.K = K; p.N = a.w.N; p.M = rows;
-    p.vec = ((reinterpret_cast<uintptr_t>(p.x) | reinterpret_cast<uintptr_t>(p.gamma)) & 15) == 0 && p.ldx % 4 == 0;
     p.nTiles = (a.w.N + rowsPerTile - 1) / rowsPerTile;
     p.nGroups = (p.nTiles + kWarps - 1) / kWarps;
     p.nSlices = (K + kSlice - 1) / kSlice;
