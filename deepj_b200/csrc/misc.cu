@@ -41,7 +41,9 @@ __device__ __forceinline__ int order_key(float v) {
 // keeps the lowest index among equals).  grid (parts, rows): every CTA reduces its slice of the row to one
 // (key, index) pair; the CTA that arrives last at the row (a self-resetting ticket) reduces the parts.  One CTA
 // per row costs a full load round trip per 1024 columns — 18 µs for a 32000-entry row.
-constexpr int kArgmaxParts = 32;                 // 1000 columns of a 32000-entry row: one 16-byte load per thread
+// Up to 32 parts: 1000 columns of a 32000-entry row, one 16-byte load per thread (3.1 µs, 3.3 in 16 parts).  From 17 rows on 16 parts: the blocks
+// are enough, and each costs a ticket (64 rows of 50257 entries, which do not come in 16-byte pieces, 7.2 µs, in 32 parts 8.6; of 32000 5.3 and 6.6).
+constexpr int kArgmaxParts = 32, kArgmaxFewRows = 16;
 __global__ void __launch_bounds__(256) k_argmax_rows(const float* __restrict__ in, float* __restrict__ out, int rows, int cols,
                                                       int* __restrict__ scratch, int* __restrict__ tickets) {
     __shared__ int s_key[8];
@@ -330,7 +332,7 @@ void launch_embed_gather(const float* table, const float* ids, float* out, int r
 void launch_argmax_rows(const float* in, float* out, int rows, int cols, int* scratch, int* tickets, cudaStream_t s) {
     if (rows <= 0) return;
     // short rows, or more rows than ticket counters: one CTA per row
-    const int parts = (cols >= 4096 && rows <= kArgmaxRowsMax && scratch != nullptr) ? kArgmaxParts : 1;
+    const int parts = (cols >= 4096 && rows <= kArgmaxRowsMax && scratch != nullptr) ? (rows <= kArgmaxFewRows ? kArgmaxParts : kArgmaxParts / 2) : 1;
     launch_k(k_argmax_rows, dim3(parts, rows), dim3(256), 0, s, true, in, out, rows, cols, scratch, tickets);
 }
 static int sample_pow2(int cols) { int P = 2; while (P < cols) P <<= 1; return P; }

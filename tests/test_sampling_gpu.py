@@ -58,6 +58,19 @@ def test_argmax_rows_is_the_first_index_of_a_stable_descending_sort(dev, V):
     assert list(got[1:]) == [0, 3, V // 3, V // 2 + 1]
 
 
+@pytest.mark.parametrize("V", [4096, 50257])
+@pytest.mark.parametrize("rows", [16, 17])
+def test_argmax_of_few_and_many_rows(dev, rows, V):
+    """Both sides of the line between the numbers of CTAs that share a row: the maximum in the first, the last and every other slice, twice."""
+    x = np.random.default_rng(V + rows).standard_normal((rows, V)).astype(np.float32)
+    at = np.linspace(0, V - 1, rows).astype(int)
+    x[np.arange(rows), at] = 9.0
+    x[np.arange(rows), np.minimum(at + V // 3, V - 1)] = 9.0
+    ob = dev.buf(rows)
+    dev.flush([OP_ARGMAX_ROWS, dev.buf(rows * V, x), ob, rows, V])
+    assert np.array_equal(dev.get(ob, rows).astype(np.int64), at)
+
+
 def test_sampler_rejects_what_it_does_not_cover(dev):
     lb, rb, ob = dev.buf(8), dev.buf(1), dev.buf(1)
     for top_k, t in ((-1, 1.0), (4, 0.0), (4, -1.0)):
