@@ -2,7 +2,7 @@
 //
 // HBM layout of a Q8 weight for y = x·W, W[K×N]: codes[N][Kp] int8 (one output
 // column's K-vector contiguous, Kp = K rounded up to 16 with zero padding) and
-// scales[N][nb] fp32, nb = ceil(K/32).  1.125 bytes per weight.
+// scales[N][nb] fp32, nb = ceil(K/32) rounded up to a multiple of 4 (what lies beyond is zero).  1.125 bytes per weight.
 //
 // GEMV (M small): HBM-bound.  A CTA of BLOCK threads owns the whole K extent:
 // thread t keeps the activations of its 16-wide K chunks (t, t+BLOCK, ...) in

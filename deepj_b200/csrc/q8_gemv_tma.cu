@@ -394,7 +394,7 @@ bool q8_encode_weight_maps(const Q8View& w, CUtensorMap* codes, CUtensorMap* sca
     EncodeTiledFn enc = encode_tiled_fn();
     if (!enc) return false;
     if ((reinterpret_cast<uintptr_t>(w.codes) & 15) != 0 || (reinterpret_cast<uintptr_t>(w.scales) & 15) != 0) return false;
-    if (w.Kp % 16 != 0 || (w.nb * 4) % 16 != 0) return false;
+    if (w.Kp % 16 != 0) return false;
     {
         const cuuint64_t dims[2] = {(cuuint64_t)w.Kp, (cuuint64_t)w.N};
         const cuuint64_t strides[1] = {(cuuint64_t)w.Kp};

@@ -279,7 +279,7 @@ __global__ void __launch_bounds__(kXThreads) k_x_images(const XImages p) {
             if (!EARLY) load(p.beta, b, 0.0f);
 #pragma unroll
             for (int i = 0; i < CH; i++)
-                if ((tid + i * kXThreads) * 8 < p.K) {       // (a division of zero takes the slow way)
+                if ((tid + i * kXThreads) * 8 < p.K) {       // (dividing zeros is slow: 64 rows of 512, with the product, 9.9 µs, 7.6 without)
 #pragma unroll
                     for (int e = 0; e < 8; e++) v[i][e] = __fdiv_rn(v[i][e], root) * g[i][e] + b[i][e];
                 }
@@ -371,16 +371,9 @@ struct TcParams {
 };
 
 // Four block scales from block k on; past the row's end zeros, which only meet blocks that do not exist.
-__device__ __forceinline__ float4 load_scales(const float* row, int k, int nb, bool vec, bool coarse) {
+__device__ __forceinline__ float4 load_scales(const float* row, int k, int nb, bool coarse) {
     float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (vec) {
-        if (k < nb) v = *reinterpret_cast<const float4*>(row + k);
-    } else {
-        if (k < nb) v.x = row[k];
-        if (k + 1 < nb) v.y = row[k + 1];
-        if (k + 2 < nb) v.z = row[k + 2];
-        if (k + 3 < nb) v.w = row[k + 3];
-    }
+    if (k < nb) v = *reinterpret_cast<const float4*>(row + k);       // nb is a multiple of four
     if (coarse) {
         auto cut = [](float f) { return __uint_as_float((__float_as_uint(f) + 0x1000u) & 0xffffe000u); };      // 11 bits, at any size
         v = make_float4(cut(v.x), cut(v.y), cut(v.z), cut(v.w));
@@ -435,7 +428,6 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_q8_gemm_tc(const __grid_const
         const bool second = p.swiglu && r >= kRows / 2;
         const int n = min(n0 + (second ? r - kRows / 2 : r), p.N - 1);
         const float* const srow = (second ? p.scales2 : p.scales) + (size_t)n * p.nb;
-        const bool vec = (p.nb & 3) == 0;
         const uint32_t lane_base = tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(part * S::kCols);
         unsigned long long acc[S::kCols / 2];
 #pragma unroll
@@ -459,7 +451,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_q8_gemm_tc(const __grid_const
                     *at = make_ulonglong2(move_sum(acc[2 * q], o.x), move_sum(acc[2 * q + 1], o.y));
                 }
         };
-        float4 next = load_scales(srow, kt0, p.nb, vec, p.coarse);
+        float4 next = load_scales(srow, kt0, p.nb, p.coarse);
         // accumulator and phase parity of the i-th block of group g
         auto slot_of = [](int g, int i) { return S::kSlots == 4 ? (g & 1) * 2 + i / 2 : i / S::kPer % 2; };
         auto parity_of = [](int g, int i) { return (uint32_t)(S::kSlots == 4 ? g >> 1 : S::kPer == 2 ? g : i >> 1) & 1u; };
@@ -488,7 +480,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_q8_gemm_tc(const __grid_const
                 if (b0 >= nK || !ok) break;
                 const int g = g0 + h;
                 const float4 cur = next;
-                if (b0 + kGroup < nK) next = load_scales(srow, kt0 + b0 + kGroup, p.nb, vec, p.coarse);
+                if (b0 + kGroup < nK) next = load_scales(srow, kt0 + b0 + kGroup, p.nb, p.coarse);
 #pragma unroll
                 for (int i = 0; i < kGroup; i += S::kPer) {
                     if (b0 + i >= nK) break;
@@ -845,7 +837,7 @@ bool launch_q8_linear_tc(const Q8LinearArgs& a, float* ws, cudaStream_t s) {
     const bool swiglu = a.w2.codes != nullptr;
     if (ws == nullptr || ((uintptr_t)ws & 127) != 0 || M < 1 || K % 4 != 0 || g_dev_error == nullptr) return false;
     if (((uintptr_t)a.x & 15) != 0 || a.ldx % 4 != 0 || ((uintptr_t)a.gamma & 15) != 0 || ((uintptr_t)a.beta & 15) != 0) return false;
-    if (a.w.nb % 4 == 0 && (((uintptr_t)a.w.scales & 15) != 0 || (swiglu && ((uintptr_t)a.w2.scales & 15) != 0))) return false;
+    if (((uintptr_t)a.w.scales & 15) != 0 || (swiglu && ((uintptr_t)a.w2.scales & 15) != 0)) return false;
     if (swiglu && a.act != 0) return false;
     TcParams p = {};
     if (!encode_codes(a.w, swiglu ? kRows / 2 : kRows, &p.codes) || (swiglu && !encode_codes(a.w2, kRows / 2, &p.codes2))) return false;

@@ -121,7 +121,7 @@ void ensure_init() {
         R.graphs_enabled = false;      // slots are handed out per launch, which a replayed graph would not do
     }
     // ticket counters of the split-attention merge and the batched linear, then the greedy pick's (kArgmaxRowsMax)
-    // and its partial pairs (2 · 16 per row)
+    // and its partial pairs (2 · 32 per row)
     DJ_CUDA_CHECK(cudaMalloc((void**)&R.tickets, (kAttnTickets + kArgmaxRowsMax * 65) * sizeof(int)));
     DJ_CUDA_CHECK(cudaMemset(R.tickets, 0, (kAttnTickets + kArgmaxRowsMax * 65) * sizeof(int)));
     DJ_CUDA_CHECK(cudaMalloc((void**)&g_dev_error, sizeof(int)));
